@@ -41,6 +41,32 @@ __device__ __forceinline__ float bilinear_s(const float* img, int w, int h, floa
     return (bot - top) * fy + top;
 }
 
+// upsample_at (level.cuh) from planes
+__device__ __forceinline__ float2 upsample_planes(const float* su, const float* sv, int sw, int sh, const UpsampleScale& c,
+                                                  bool zero, bool damp_now, float damp, int x, int y) {
+    int ix, iy;
+    float fx, fy;
+    cell((float)x * c.rx, sw, ix, fx);
+    cell((float)y * c.ry, sh, iy, fy);
+    const int i = iy * sw + ix;
+    const float* planes[2] = {su, sv};
+    float r[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const float* p = planes[k];
+        float q[4] = {p[i], p[i + 1], p[i + sw], p[i + sw + 1]};
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            if (zero) q[m] = 0.0f;
+            if (damp_now) q[m] = damp * q[m];
+        }
+        float top = (q[1] - q[0]) * fx + q[0];
+        float bot = (q[3] - q[2]) * fx + q[2];
+        r[k] = (bot - top) * fy + top;
+    }
+    return make_float2(r[0] * c.sx, r[1] * c.sy);
+}
+
 // One separable pass of the multi channel rule over a plane (src -> dst, both w x h in shared
 // memory): along the rows (VERT false) or the columns.
 template <int N, bool VERT>
@@ -290,14 +316,16 @@ __global__ void __launch_bounds__(COARSE_THREADS) k_solve_coarse(CoarseJob J) {
         const int dw = J.sizes[l - 1][0], dh = J.sizes[l - 1][1];
         const bool zero = zero_at_level(s_any, l, J.start);
         const bool damp_now = l == J.start && J.damp_any;
-        float* ou = l == J.last ? J.fu_out : nu;
-        float* ov = l == J.last ? J.fv_out : nv;
+        const UpsampleScale up = upsample_scale(w, h, dw, dh);
         for (int i = tid; i < dw * dh; i += NT) {
             int y = i / dw, x = i - y * dw;
-            float u, v;
-            upsample_at(fu, fv, w, h, zero, damp_now, J.damp, x, y, dw, dh, &u, &v);
-            ou[i] = u;
-            ov[i] = v;
+            const float2 f = upsample_planes(fu, fv, w, h, up, zero, damp_now, J.damp, x, y);
+            if (l == J.last) {
+                J.f_out[i] = f;
+            } else {
+                nu[i] = f.x;
+                nv[i] = f.y;
+            }
         }
         __syncthreads();
         float* t = fu;

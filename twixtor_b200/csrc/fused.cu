@@ -101,381 +101,427 @@ __global__ void __launch_bounds__(FT_THREADS) k_blur5_band(const float* __restri
     }
 }
 
-// R outputs of a pass along one line at line indices i0 .. i0 + R - 1 (global), written to
-// out[r * ostride] for r < nvalid where the index lies in [0, len). The line's element t (global
-// index) is line[(t - origin) * stride]; the region holds indices [origin, origin + rlen). The
-// register path runs only when every output is interior and every input lies in the region.
-template <int N, int R, bool MULTI, bool LEFT_FIRST>
-__device__ __forceinline__ void pass_run(const float* line, int origin, int rlen, int stride, int len, int i0,
-                                         const float* k, float* out, int ostride, int nvalid) {
-    constexpr int NV = R + 2 * N - 2;
-    bool interior = nvalid == R && len >= 2 * N && i0 >= N && i0 + R - 1 < len - N && i0 - (N - 1) >= origin &&
-                    i0 + R - 1 + (N - 1) < origin + rlen;
-    if (interior) {
-        float v[NV];
-        const float* base = line + (i0 - (N - 1) - origin) * stride;
+// ---- one solver level: the tile geometry of its kernels ----------------------------------------------
+
+// Stores of res[0 .. R-1] along a shared memory line
+template <int R, class V>
+__device__ __forceinline__ void put_run(V* out, int stride, const V* res) {
 #pragma unroll
-        for (int j = 0; j < NV; j++) v[j] = base[j * stride];
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            float s = v[r + N - 1] * k[0];
-#pragma unroll
-            for (int j = N - 1; j >= 1; j--) s = s + (v[r + N - 1 + j] + v[r + N - 1 - j]) * k[j];
-            out[r * ostride] = s;
-        }
-    } else {
-        for (int r = 0; r < nvalid; r++) {
-            int i = i0 + r;
-            if (i < 0 || i >= len) continue;
-            out[r * ostride] = pass_elem<N, MULTI, LEFT_FIRST>(line, origin, stride, len, i, k);
-        }
-    }
+    for (int r = 0; r < R; r++) out[r * stride] = res[r];
+}
+
+// The border weight sums (border_den) of n consecutive line indices from i0 on: entry t of the block's
+// table (run_pass reads them for the outputs near the line's ends). Tables are filled one after the
+// other by consecutive threads; returns the index past this one.
+template <int N>
+__device__ __forceinline__ int fill_den(float2* den, int first, int n, int i0, int len, const Taps& k) {
+    for (int t = (int)threadIdx.x - first; t < n; t += blockDim.x)
+        if (t >= 0) den[t] = border_den<N>(i0 + t, len, k.k);
+    return first + n;
+}
+// Whether a tile of w0 x h0 outputs at (X0, Y0) of a w x h level has border outputs in a filter chain that
+// reaches `reach` pixels past it
+__device__ __forceinline__ bool at_border(int X0, int Y0, int w0, int h0, int reach, int w, int h) {
+    return X0 < reach || Y0 < reach || X0 + w0 > w - reach || Y0 + h0 > h - reach;
 }
 
 // ---- one solver level: gradient, tensor and its blur (flow.rs:1275-1277) ---------------------------
 
-// mask (may be null): the level mask of X of a layered solve; the gradient is zero where the mask
-// is below 0.95 at the pixel or at one of its four neighbours that exist (flow.rs:743-761).
-// b_out (may be null): calc_b of the first iteration from the level's flow fu, fv, the image i0 and
-// the mask of Y (flow.rs:334-357), into two planes of pitch bp (plane stride bplane).
-__global__ void __launch_bounds__(FT_THREADS) k_level_init(const float* __restrict__ img, int w, int h, Taps g7,
-                                                           bool above_first, float* __restrict__ gxo,
-                                                           float* __restrict__ gyo, float* __restrict__ a0o,
-                                                           float* __restrict__ a1o, float* __restrict__ a2o,
-                                                           const float* __restrict__ mask,
-                                                           const float* __restrict__ fu, const float* __restrict__ fv,
-                                                           const float* __restrict__ i0,
-                                                           const float* __restrict__ mask_y, float* __restrict__ b_out,
-                                                           int bp, long bplane) {
-    constexpr int N = 8, HALO = N - 1;
-    constexpr int RW = FT_X + 2 * HALO, RH = FT_Y + 2 * HALO;
-    constexpr int RS = RW | 1, HS = FT_X | 1;  // row strides (odd: a warp's lanes on distinct rows hit distinct banks)
-    constexpr int R = 8;                        // outputs per thread of the register blocked passes
-    extern __shared__ float sm[];
-    float* s_t = sm;                  // 3 x RH x RS tensor
-    float* s_h = s_t + 3 * RH * RS;   // 3 x RH x HS
-    int X0 = blockIdx.x * FT_X, Y0 = blockIdx.y * FT_Y;
-    int gx0 = X0 - HALO, gy0 = Y0 - HALO;
-    for (int e = threadIdx.x; e < RW * RH; e += blockDim.x) {
-        int r = e / RW, c = e - r * RW;
-        int x = gx0 + c, y = gy0 + r;
-        float t0 = 0.0f, t1 = 0.0f, t2 = 0.0f;
+// The gradient of img at (x, y) (flow.rs:283-316): the mean of the one sided differences that exist (a
+// half is exact, so the reference's division by 2 is a product), zero in a layered solve where the
+// level mask of X is below 0.95 at the pixel or at one of its four neighbours that exist
+// (flow.rs:743-761).
+__device__ __forceinline__ float2 gradient_at(const float* __restrict__ img, const float* __restrict__ mask, int w, int h,
+                                              int x, int y) {
+    const int i = y * w + x;
+    const float cc = __ldg(img + i);
+    float nx = 0.0f, ny = 0.0f;
+    if (x >= 1) nx = (cc - __ldg(img + i - 1)) + 0.0f;
+    if (y >= 1) ny = (cc - __ldg(img + i - w)) + 0.0f;
+    if (x + 1 <= w - 1) nx = nx + (__ldg(img + i + 1) - cc);
+    if (y + 1 <= h - 1) ny = ny + (__ldg(img + i + w) - cc);
+    float2 g = make_float2(x >= 1 && x + 1 <= w - 1 ? nx * 0.5f : nx, y >= 1 && y + 1 <= h - 1 ? ny * 0.5f : ny);
+    if (mask) {
+        auto off = [&](int j) { return __ldg(mask + j) < 0.95f; };
+        if (off(i) || (y >= 1 && off(i - w)) || (y + 1 < h && off(i + w)) || (x >= 1 && off(i - 1)) ||
+            (x + 1 < w && off(i + 1)))
+            g = make_float2(0.0f, 0.0f);
+    }
+    return g;
+}
+
+template <int TX, int TY>
+struct InitGeom {
+    static constexpr int HALO = 7, R = 4;
+    static constexpr int RW = TX + 2 * HALO, RH = TY + 2 * HALO;
+    static constexpr int RS = RW | 1, HS = TX | 1;  // row strides (odd: a warp's lanes on distinct rows hit distinct banks)
+    static constexpr int NDEN = TX + TY;
+    static constexpr size_t SMEM = sizeof(float2) * (RH * RS + RH * HS + NDEN) + sizeof(float) * (RH * RS + RH * HS);
+    static_assert(TX % R == 0 && TY % R == 0, "whole runs");
+};
+
+// The tasks of the passes below, each the outputs of one run; false when they are done, true (nothing
+// written) when the run needs the general rule: the same task again with SLOW, out of line, so that the
+// main path carries no calls.
+template <int TX, int TY, bool SLOW>
+__device__ __forceinline__ bool init_row(const LevelInitArgs& P, const float2* t, const float* t2, float2* o_h, float* o_h2,
+                                         const float2* den, int i0) {
+    constexpr int R = InitGeom<TX, TY>::R;
+    float2 o[R];
+    float o2[R];
+    if (h_pass<SLOW, 8, R>(t, i0, P.w, P.g7, den, o)) return true;
+    if (h_pass<SLOW, 8, R>(t2, i0, P.w, P.g7, den, o2)) return true;
+    put_run<R>(o_h, 1, o);
+    put_run<R>(o_h2, 1, o2);
+    return false;
+}
+template <int TX, int TY, bool SLOW>
+__device__ __forceinline__ bool init_column(const LevelInitArgs& P, const float2* h, const float* h2, const float2* den,
+                                            int x, int y0) {
+    using G = InitGeom<TX, TY>;
+    constexpr int R = G::R;
+    float2 o[R];
+    float o2[R];
+    if (v_pass<SLOW, 8, R>(h, G::HS, y0, P.h, P.g7, den, P.af, o)) return true;
+    if (v_pass<SLOW, 8, R>(h2, G::HS, y0, P.h, P.g7, den, P.af, o2)) return true;
+#pragma unroll
+    for (int r = 0; r < R; r++)  // with the determinant of new_disp beside the tensor
+        if (y0 + r < P.h) P.tensor[(y0 + r) * P.w + x] = make_float4(o[r].x, o[r].y, o2[r], o[r].y * o[r].y - o2[r] * o[r].x);
+    return false;
+}
+template <int TX, int TY>
+__device__ __noinline__ void init_row_slow(const LevelInitArgs& P, const float2* t, const float* t2, float2* o_h, float* o_h2,
+                                           const float2* den, int i0) {
+    init_row<TX, TY, true>(P, t, t2, o_h, o_h2, den, i0);
+}
+template <int TX, int TY>
+__device__ __noinline__ void init_column_slow(const LevelInitArgs& P, const float2* h, const float* h2, const float2* den, int x,
+                                              int y0) {
+    init_column<TX, TY, true>(P, h, h2, den, x, y0);
+}
+
+template <int TX, int TY>
+__device__ __forceinline__ void level_init_body(const LevelInitArgs& P) {
+    using G = InitGeom<TX, TY>;
+    constexpr int N = 8, R = G::R;
+    extern __shared__ __align__(16) float sm[];
+    float2* s_t = (float2*)sm;            // RH x RS: the tensor's first two channels
+    float2* s_h = s_t + G::RH * G::RS;    // RH x HS: their horizontal pass
+    float2* den_x = s_h + G::RH * G::HS;  // the weight sums of the tile's columns and rows
+    float2* den_y = den_x + TX;
+    float* s_t2 = (float*)(den_y + TY);   // the third channel, the same two planes
+    float* s_h2 = s_t2 + G::RH * G::RS;
+    const int w = P.w, h = P.h;
+    const int X0 = blockIdx.x * TX, Y0 = blockIdx.y * TY;
+    const int gx0 = X0 - G::HALO, gy0 = Y0 - G::HALO;
+    const int nt = blockDim.x;
+    if (at_border(X0, Y0, TX, TY, N, w, h)) {
+        const int t = fill_den<N>(den_x, 0, TX, X0, w, P.g7);
+        fill_den<N>(den_y, t, TY, Y0, h, P.g7);
+    }
+    // the tile's own pixels: the flow from the coarser level, the gradient, calc_b of the first iteration
+    const bool zero = P.src && zero_at_level(P.any, P.l + 1, P.start);
+    for (int e = threadIdx.x; e < TX * TY; e += nt) {
+        const int r = e / TX, c = e - r * TX;
+        const int x = X0 + c, y = Y0 + r;
+        if (x >= w || y >= h) continue;
+        const int i = y * w + x;
+        float2 f;
+        if (P.src) {
+            f = upsample_at(P.src, P.sw, P.sh, P.up, zero, P.damp_now, P.damp, x, y);
+            P.f[i] = f;
+        } else {
+            f = P.f[i];
+        }
+        const float2 g = gradient_at(P.img, P.mask_x, w, h, x, y);
+        P.grad[i] = g;
+        const float i1 = __ldg(P.img + i);
+        float2 b;
+        calc_b_run<1>(P.i0, P.mask_y, w, h, x, y, &f, &i1, &g, &b);
+        P.b_out[(long)y * P.bp + x] = b;
+    }
+    // the tensor (flow.rs:319-328) over the tile and the blur's halo
+    for (int e = threadIdx.x; e < G::RW * G::RH; e += nt) {
+        const int r = e / G::RW, c = e - r * G::RW;
+        const int x = gx0 + c, y = gy0 + r;
+        float2 t = outside_value<float2>();
+        float t2 = outside_value<float>();
         if (x >= 0 && x < w && y >= 0 && y < h) {
-            long i = (long)y * w + x;
-            float cc = __ldg(img + i);  // flow.rs:283-316
-            float nx = 0.0f, dx = 0.0f, ny = 0.0f, dy = 0.0f;
-            if (x >= 1) { nx = (cc - __ldg(img + i - 1)) + 0.0f; dx = 1.0f; }
-            if (y >= 1) { ny = (cc - __ldg(img + i - w)) + 0.0f; dy = 1.0f; }
-            if (x + 1 <= w - 1) { nx = nx + (__ldg(img + i + 1) - cc); dx = dx + 1.0f; }
-            if (y + 1 <= h - 1) { ny = ny + (__ldg(img + i + w) - cc); dy = dy + 1.0f; }
-            float gx = nx / dx, gy = ny / dy;
-            if (mask) {
-                auto off = [&](long j) { return __ldg(mask + j) < 0.95f; };
-                if (off(i) || (y >= 1 && off(i - w)) || (y + 1 < h && off(i + w)) || (x >= 1 && off(i - 1)) ||
-                    (x + 1 < w && off(i + 1))) {
-                    gx = 0.0f;
-                    gy = 0.0f;
-                }
-            }
-            t0 = gx * gx;  // flow.rs:319-328
-            t1 = gx * gy;
-            t2 = gy * gy;
-            if (x >= X0 && x < X0 + FT_X && y >= Y0 && y < Y0 + FT_Y) {
-                gxo[i] = gx;
-                gyo[i] = gy;
-                if (b_out) {  // calc_b of the level's first iteration
-                    float b0, b1;
-                    calc_b_at(i0, mask_y, w, h, x, y, __ldg(fu + i), __ldg(fv + i), cc, gx, gy, b0, b1);
-                    b_out[(long)y * bp + x] = b0;
-                    b_out[bplane + (long)y * bp + x] = b1;
-                }
-            }
+            const float2 g = gradient_at(P.img, P.mask_x, w, h, x, y);
+            t = make_float2(g.x * g.x, g.x * g.y);
+            t2 = g.y * g.y;
         }
-        const int se = r * RS + c;
-        s_t[se] = t0;
-        s_t[RH * RS + se] = t1;
-        s_t[2 * RH * RS + se] = t2;
+        s_t[r * G::RS + c] = t;
+        s_t2[r * G::RS + c] = t2;
     }
     __syncthreads();
-    // blur7 of the tensor, register blocked (pass_run: R outputs from R + 14 inputs held in
-    // registers, each output with the interior chain, or the border rule near the image's edges):
-    // horizontal along the region's rows at the tile's columns, a lane per row
-    {
-        constexpr int NSEG = FT_X / R;
-        for (int e = threadIdx.x; e < 3 * RH * NSEG; e += blockDim.x) {
-            const int r = e % RH, rest = e / RH;
-            const int seg = rest % NSEG, ch = rest / NSEG;
-            const int Y = gy0 + r;
-            if (Y < 0 || Y >= h) continue;
-            const int c0 = seg * R;
-            pass_run<N, R, true, false>(s_t + ch * RH * RS + r * RS, gx0, RW, 1, w, X0 + c0, g7.k,
-                                        s_h + ch * RH * HS + r * HS + c0, 1, R);
-        }
+    // blur7 of the tensor: along the region's rows at the tile's columns, a lane per row
+    for (int e = threadIdx.x; e < G::RH * (TX / R); e += nt) {
+        const int r = e % G::RH, c0 = (e / G::RH) * R;
+        const float2* t = s_t + r * G::RS + c0;
+        const float* t2 = s_t2 + r * G::RS + c0;
+        float2* o = s_h + r * G::HS + c0;
+        float* o2 = s_h2 + r * G::HS + c0;
+        if (init_row<TX, TY, false>(P, t, t2, o, o2, den_x + c0, X0 + c0)) init_row_slow<TX, TY>(P, t, t2, o, o2, den_x + c0, X0 + c0);
     }
     __syncthreads();
-    //    vertical at the tile's rows, a lane per column, into the tensor planes
-    {
-        constexpr int NSEG = FT_Y / R;
-        float* outs[3] = {a0o, a1o, a2o};
-        for (int e = threadIdx.x; e < 3 * FT_X * NSEG; e += blockDim.x) {
-            const int c = e % FT_X, rest = e / FT_X;
-            const int seg = rest % NSEG, ch = rest / NSEG;
-            const int X = X0 + c;
-            if (X >= w) continue;
-            const int r0 = seg * R;
-            const float* line = s_h + ch * RH * HS + c;
-            float* dst = (ch == 0 ? outs[0] : ch == 1 ? outs[1] : outs[2]) + (long)(Y0 + r0) * w + X;  // rows past h are never written
-            if (above_first) pass_run<N, R, true, true>(line, gy0, RH, HS, h, Y0 + r0, g7.k, dst, w, R);
-            else pass_run<N, R, true, false>(line, gy0, RH, HS, h, Y0 + r0, g7.k, dst, w, R);
-        }
+    // then along the tile's columns, a lane per column
+    for (int e = threadIdx.x; e < TX * (TY / R); e += nt) {
+        const int c = e % TX, r0 = (e / TX) * R;
+        if (X0 + c >= w || Y0 + r0 >= h) continue;
+        const float2* t = s_h + r0 * G::HS + c;
+        const float* t2 = s_h2 + r0 * G::HS + c;
+        if (init_column<TX, TY, false>(P, t, t2, den_y + r0, X0 + c, Y0 + r0))
+            init_column_slow<TX, TY>(P, t, t2, den_y + r0, X0 + c, Y0 + r0);
     }
 }
 
-size_t level_init_smem() {
-    constexpr int RW = FT_X + 14, RH = FT_Y + 14;
-    return sizeof(float) * (3 * RH * (RW | 1) + 3 * RH * (FT_X | 1));
-}
+#define TW_LEVEL_INIT(TX, TY)                                                                            \
+    __global__ void __launch_bounds__(LEVEL_INIT_MAX_THREADS, 2) k_level_init_##TX##x##TY(               \
+        const __grid_constant__ LevelInitArgs P) {                                                      \
+        level_init_body<TX, TY>(P);                                                                     \
+    }
+TW_LEVEL_INIT(16, 16)
+TW_LEVEL_INIT(32, 32)
+#undef TW_LEVEL_INIT
+
+size_t level_init_smem(int tile) { return tile == LEVEL_TILE_16x16 ? InitGeom<16, 16>::SMEM : InitGeom<32, 32>::SMEM; }
 
 // ---- one solver iteration (flow.rs:1278-1282): calc_b, blur7 of B, new_disp, blur5 of the flow -----
 // mask_y (may be null): the level mask of Y of a layered solve
 //
 // calc_b depends only on the flow at its own pixel, so it is computed once per pixel where the flow
 // is made: k_level_init for the level's first iteration, each iteration's epilogue for the next one
-// (k_calc_b_pitched after the level's block matching). B lives in two planes with a pitch of a
-// multiple of 4 floats, so that an iteration loads its B region with 128-bit loads.
+// (k_calc_b_pitched after the level's block matching).
 //
 // Halos: the flow's blur5 needs new_disp on the tile + 5; new_disp needs blurred B there, which
 // needs B on the tile + 12. The tile is TX x TY outputs (a template: the host picks the shape per
-// level size from its tuning table). The separable passes are register blocked: a thread computes R
-// consecutive outputs along the pass from R + 2N - 2 inputs held in registers (each input read once
-// from shared memory instead of once per tap), each output with the reference's interior chain;
-// outputs near the image border, or at the ragged end of a region, take the element rule (interior
-// chain or border renormalisation) one by one. Horizontal passes give each lane of a warp its own
-// row (row strides are odd, so the lanes hit distinct banks), vertical passes its own column.
-
+// level size). A thread computes R consecutive outputs along a pass (run_pass) with both channels in
+// one packed operation. The vertical passes end in registers: blur7's runs go straight into new_disp,
+// blur5's into the new flow and calc_b of the next iteration. Horizontal passes give each lane of a
+// warp its own row (row strides are odd, so the lanes hit distinct banks), vertical passes its own
+// column.
+//
+// What bounds it: the FP32 pipe and, on levels of few tiles, the latency of its five stages. Per launch
+// (back to back launches on random planes, both with calc_b): 960 x 540 18.5 us with 32 x 64 tiles, 1920 x
+// 1080 59.5 us; 480 x 270 10.3 us with 32 x 32 (14.4 with 32 x 64, 14.2 with 16 x 16); 240 x 135 and 120 x
+// 67 8.3 us with 16 x 16 (10.3 with 32 x 32). Scalar planes with per tap border tests took 31, 19 and 18.6
+// us (960 x 540, 480 x 270, the smaller ones).
 template <int TX, int TY>
 struct IterGeom {
     static constexpr int HB = 12, HD = 5;
     static constexpr int BW = TX + 2 * HB, BH = TY + 2 * HB;  // B region
     static constexpr int DW = TX + 2 * HD, DH = TY + 2 * HD;  // new_disp region
-    static constexpr int BS = BW | 1;                          // row strides (odd)
-    static constexpr int HS = DW | 1;
-    static constexpr int DS = DW | 1;
-    static constexpr int FS = TX | 1;
-    // buffer 1: B (2 planes BH x BS), later the blurred B / new flow (2 planes DH x DS), last the
-    // tile's new flow (2 planes TY x TX)
-    // buffer 2: the horizontal pass of B (2 planes BH x HS), later of the flow (2 planes DH x FS)
-    static constexpr int BUF1 = 2 * BH * BS;
-    static constexpr int BUF2 = 2 * BH * HS;
-    static constexpr size_t SMEM = sizeof(float) * (BUF1 + BUF2);
-    static_assert(2 * DH * DS <= BUF1 && 2 * DH * FS <= BUF2 && 2 * TX * TY <= BUF1, "the reused buffers must fit");
+    // outputs per thread of the passes: blur7 along rows and columns, blur5 along rows and columns
+    // (short runs for the small tiles, whose time is latency)
+    static constexpr int R7H = TX == 16 ? 3 : 6, R7V = TX == 16 ? 2 : 4;
+    static constexpr int R5H = TX == 16 ? 2 : 4, R5V = TX == 16 ? 1 : TX * TY == 1024 ? 2 : 4;
+    static constexpr int S7H = (DW + R7H - 1) / R7H, S7V = (DH + R7V - 1) / R7V;  // runs of a blur7 line
+    // row strides (odd) and the columns / rows a ragged last run reads past its region
+    static constexpr int BS = (S7H * R7H + 14) | 1, HS = (S7H * R7H) | 1, DS = DW | 1, FS = TX | 1;
+    static constexpr int HH = S7V * R7V + 14;
+    // buffer 1: B (BH x BS), then the new_disp flow (DH x DS); buffer 2: blur7's horizontal pass (HH x
+    // HS), then blur5's (DH x FS); then the border weight sums
+    static constexpr int BUF1 = BH * BS > S7V * R7V * DS ? BH * BS : S7V * R7V * DS;
+    static constexpr int BUF2 = HH * HS > DH * FS ? HH * HS : DH * FS;
+    static constexpr int NDEN = S7H * R7H + S7V * R7V + TX + TY;
+    static constexpr size_t SMEM = sizeof(float2) * (BUF1 + BUF2 + NDEN);
+    static_assert(BW % 2 == 0 && HB % 2 == 0 && TX % R5H == 0 && TY % R5V == 0, "aligned pairs, whole blur5 runs");
 };
 
-template <int TX, int TY>
-__device__ __forceinline__ void level_iter_body(const float* __restrict__ b_in, int bp, long bplane,
-                                                const float* __restrict__ i1, const float* __restrict__ i0,
-                                                const float* __restrict__ gx, const float* __restrict__ gy,
-                                                const float* __restrict__ a0, const float* __restrict__ a1,
-                                                const float* __restrict__ a2, const float* __restrict__ fu,
-                                                const float* __restrict__ fv, int w, int h, const Taps& g7,
-                                                const Taps& g5, bool above_first, float* __restrict__ fu_out,
-                                                float* __restrict__ fv_out, const float* __restrict__ mask_y,
-                                                float* __restrict__ b_out) {
+// The tasks of the passes below, as those of k_level_init: the outputs of one run, or true when it needs
+// the general rule.
+// blur7 of B along a row
+template <int TX, int TY, bool SLOW>
+__device__ __forceinline__ bool iter_row7(const LevelIterArgs& P, const float2* in, float2* out, const float2* den, int i0) {
+    constexpr int R = IterGeom<TX, TY>::R7H;
+    float2 o[R];
+    if (h_pass<SLOW, 8, R>(in, i0, P.w, P.g7, den, o)) return true;
+    put_run<R>(out, 1, o);
+    return false;
+}
+// blur7 of B along column x from row y0 on, and new_disp there (flow.rs:361-371); a pixel outside the image
+// leaves what the flow's blur expects there
+template <int TX, int TY, bool SLOW>
+__device__ __forceinline__ bool iter_column7(const LevelIterArgs& P, const float2* in, float2* out, const float2* den, int x,
+                                             int y0, int y_end) {
     using G = IterGeom<TX, TY>;
-    constexpr int R7 = 6, R5 = 8;  // outputs per thread of the blur7 and blur5 passes
-    extern __shared__ float sm[];
-    float* s_b = sm;            // 2 x BH x BS
-    float* s_h = sm + G::BUF1;  // 2 x BH x HS
-    float* s_d = s_b;           // reuse: 2 x DH x DS (blurred B -> new flow)
-    float* s_f = s_h;           // reuse: 2 x DH x FS
+    constexpr int R = G::R7V;
+    float2 b[R], f[R];
+    if (v_pass<SLOW, 8, R>(in, G::HS, y0, P.h, P.g7, den, P.af, b)) return true;
+    float4 t[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int y = y0 + r;
+        f[r] = outside_value<float2>();
+        t[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (x >= 0 && x < P.w && y >= 0 && y < y_end) {
+            t[r] = __ldg(P.tensor + y * P.w + x);
+            f[r] = __ldg(P.f + y * P.w + x);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        if (fabsf(t[r].w) > 40.0f) {
+            f[r].x = (t[r].y * b[r].y - t[r].z * b[r].x) / t[r].w + f[r].x;
+            f[r].y = (t[r].y * b[r].x - t[r].x * b[r].y) / t[r].w + f[r].y;
+        }
+    }
+    put_run<R>(out, G::DS, f);
+    return false;
+}
+// blur5 of the flow along a row
+template <int TX, int TY, bool SLOW>
+__device__ __forceinline__ bool iter_row5(const LevelIterArgs& P, const float2* in, float2* out, const float2* den, int i0) {
+    constexpr int R = IterGeom<TX, TY>::R5H;
+    float2 o[R];
+    if (h_pass<SLOW, 6, R>(in, i0, P.w, P.g5, den, o)) return true;
+    put_run<R>(out, 1, o);
+    return false;
+}
+// blur5 of the flow along column x from row y0 on: the new flow, and with b_out calc_b of the next
+// iteration there (flow.rs:334-357)
+template <int TX, int TY, bool SLOW>
+__device__ __forceinline__ bool iter_column5(const LevelIterArgs& P, const float2* in, const float2* den, int x, int y0) {
+    using G = IterGeom<TX, TY>;
+    constexpr int R = G::R5V;
+    float2 f[R], g[R], b[R];
+    float i1[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int i = min(y0 + r, P.h - 1) * P.w + x;
+        g[r] = make_float2(0.0f, 0.0f);
+        i1[r] = 0.0f;
+        if (P.b_out) {
+            g[r] = __ldg(P.grad + i);
+            i1[r] = __ldg(P.i1 + i);
+        }
+    }
+    if (v_pass<SLOW, 6, R>(in, G::FS, y0, P.h, P.g5, den, P.af, f)) return true;
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (y0 + r < P.h) P.f_out[(y0 + r) * P.w + x] = f[r];
+    if (P.b_out) {
+        calc_b_run<R>(P.i0, P.mask_y, P.w, P.h, x, y0, f, i1, g, b);
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            if (y0 + r < P.h) P.b_out[(long)(y0 + r) * P.bp + x] = b[r];
+    }
+    return false;
+}
+template <int TX, int TY>
+__device__ __noinline__ void iter_row7_slow(const LevelIterArgs& P, const float2* in, float2* out, const float2* den, int i0) {
+    iter_row7<TX, TY, true>(P, in, out, den, i0);
+}
+template <int TX, int TY>
+__device__ __noinline__ void iter_column7_slow(const LevelIterArgs& P, const float2* in, float2* out, const float2* den, int x,
+                                               int y0, int y_end) {
+    iter_column7<TX, TY, true>(P, in, out, den, x, y0, y_end);
+}
+template <int TX, int TY>
+__device__ __noinline__ void iter_row5_slow(const LevelIterArgs& P, const float2* in, float2* out, const float2* den, int i0) {
+    iter_row5<TX, TY, true>(P, in, out, den, i0);
+}
+template <int TX, int TY>
+__device__ __noinline__ void iter_column5_slow(const LevelIterArgs& P, const float2* in, const float2* den, int x, int y0) {
+    iter_column5<TX, TY, true>(P, in, den, x, y0);
+}
+
+template <int TX, int TY>
+__device__ __forceinline__ void level_iter_body(const LevelIterArgs& P) {
+    using G = IterGeom<TX, TY>;
+    extern __shared__ __align__(16) float sm[];
+    float2* s1 = (float2*)sm;
+    float2* s2 = s1 + G::BUF1;
+    float2* den7x = s2 + G::BUF2;
+    float2* den7y = den7x + G::S7H * G::R7H;
+    float2* den5x = den7y + G::S7V * G::R7V;
+    float2* den5y = den5x + TX;
+    const int w = P.w, h = P.h, bp = P.bp;
     const int X0 = blockIdx.x * TX, Y0 = blockIdx.y * TY;
     const int bx0 = X0 - G::HB, by0 = Y0 - G::HB;
     const int dx0 = X0 - G::HD, dy0 = Y0 - G::HD;
     const int nt = blockDim.x;
-    // 1. B over the B region, from the planes b_in (calc_b of flow.rs:334-357, computed once per pixel
-    //    by the kernel that produced the flow): 128-bit loads of 4 columns (bx0 and the pitch are
-    //    multiples of 4, the planes 16-byte aligned), zero outside the level as calc_b gives there;
-    //    four loads per thread in flight before their stores
+    // 1. B over the B region: 128-bit loads of two columns (bx0 and the pitch are even, the plane 16-byte
+    //    aligned), four per thread in flight before their stores
     {
-        constexpr int Q = G::BW / 4;  // 128-bit groups per region row
-        constexpr int NQ = 2 * G::BH * Q;
-        static_assert(G::BW % 4 == 0 && G::HB % 4 == 0, "the B region must start and end on 4-column groups");
+        constexpr int Q = G::BW / 2, NQ = G::BH * Q;
         for (int e0 = threadIdx.x; e0 < NQ; e0 += 4 * nt) {
             float4 v[4];
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 const int e = e0 + k * nt;
-                const int q = e % Q, rest = e / Q;
-                const int r = rest % G::BH, ch = rest / G::BH;
-                const int x = bx0 + 4 * q, y = by0 + r;
-                v[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                const int r = e / Q, q = e - r * Q;
+                const int x = bx0 + 2 * q, y = by0 + r;
+                v[k] = make_float4(-0.0f, -0.0f, -0.0f, -0.0f);
                 if (e < NQ && x >= 0 && x < w && y >= 0 && y < h) {
-                    v[k] = __ldg(reinterpret_cast<const float4*>(b_in + ch * bplane + (long)y * bp + x));
-                    if (x + 1 >= w) v[k].y = 0.0f;  // the pitch's padding columns
-                    if (x + 2 >= w) v[k].z = 0.0f;
-                    if (x + 3 >= w) v[k].w = 0.0f;
+                    v[k] = __ldg(reinterpret_cast<const float4*>(P.b_in + y * bp + x));
+                    if (x + 1 >= w) v[k].z = v[k].w = -0.0f;  // the pitch's padding column
                 }
             }
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 const int e = e0 + k * nt;
                 if (e >= NQ) break;
-                const int q = e % Q, rest = e / Q;
-                const int r = rest % G::BH, ch = rest / G::BH;
-                float* d = s_b + ch * G::BH * G::BS + r * G::BS + 4 * q;
-                d[0] = v[k].x;
-                d[1] = v[k].y;
-                d[2] = v[k].z;
-                d[3] = v[k].w;
+                const int r = e / Q, q = e - r * Q;
+                float2* d = s1 + r * G::BS + 2 * q;
+                d[0] = make_float2(v[k].x, v[k].y);
+                d[1] = make_float2(v[k].z, v[k].w);
             }
         }
-    }
-    __syncthreads();
-    // 2. blur7 of B (2 channels): horizontal along the B rows, outputs at the new_disp columns
-    {
-        constexpr int NSEG = (G::DW + R7 - 1) / R7;
-        for (int e = threadIdx.x; e < 2 * G::BH * NSEG; e += nt) {
-            int r = e % G::BH, rest = e / G::BH;
-            int seg = rest % NSEG, ch = rest / NSEG;
-            int Y = by0 + r;
-            if (Y < 0 || Y >= h) continue;
-            int c0 = seg * R7;
-            const float* line = s_b + ch * G::BH * G::BS + r * G::BS;
-            pass_run<8, R7, true, false>(line, bx0, G::BW, 1, w, dx0 + c0, g7.k,
-                                         s_h + ch * G::BH * G::HS + r * G::HS + c0, 1, min(R7, G::DW - c0));
+        if (at_border(X0, Y0, TX, TY, G::HD + 8 + G::R7H, w, h)) {  // a ragged last run reaches past the region
+            int t = fill_den<8>(den7x, 0, G::S7H * G::R7H, dx0, w, P.g7);
+            t = fill_den<8>(den7y, t, G::S7V * G::R7V, dy0, h, P.g7);
+            t = fill_den<6>(den5x, t, TX, X0, w, P.g5);
+            fill_den<6>(den5y, t, TY, Y0, h, P.g5);
         }
     }
     __syncthreads();
-    //    vertical, outputs at the new_disp rows (into buffer 1, whose B is no longer needed)
-    {
-        constexpr int NSEG = (G::DH + R7 - 1) / R7;
-        for (int e = threadIdx.x; e < 2 * G::DW * NSEG; e += nt) {
-            int c = e % G::DW, rest = e / G::DW;
-            int seg = rest % NSEG, ch = rest / NSEG;
-            int X = dx0 + c;
-            if (X < 0 || X >= w) continue;
-            int r0 = seg * R7;
-            const float* line = s_h + ch * G::BH * G::HS + c;
-            float* o = s_d + ch * G::DH * G::DS + r0 * G::DS + c;
-            int nv = min(R7, G::DH - r0);
-            if (above_first) pass_run<8, R7, true, true>(line, by0, G::BH, G::HS, h, dy0 + r0, g7.k, o, G::DS, nv);
-            else pass_run<8, R7, true, false>(line, by0, G::BH, G::HS, h, dy0 + r0, g7.k, o, G::DS, nv);
-        }
+    // 2. blur7 of B along the B rows, outputs at the new_disp columns
+    for (int e = threadIdx.x; e < G::BH * G::S7H; e += nt) {
+        const int r = e % G::BH, c0 = (e / G::BH) * G::R7H;
+        const float2* in = s1 + r * G::BS + c0;
+        float2* out = s2 + r * G::HS + c0;
+        if (iter_row7<TX, TY, false>(P, in, out, den7x + c0, dx0 + c0)) iter_row7_slow<TX, TY>(P, in, out, den7x + c0, dx0 + c0);
     }
     __syncthreads();
-    // 3. new_disp over the new_disp region (flow.rs:361-371), in place on the blurred B (one element
-    //    per thread and round: batching more raises the registers past three blocks per SM, which
-    //    costs more when several solves share the GPU than the batching gains)
-    for (int e = threadIdx.x; e < G::DW * G::DH; e += nt) {
-        int r = e / G::DW, c = e - r * G::DW;
-        int x = dx0 + c, y = dy0 + r;
-        if (x < 0 || x >= w || y < 0 || y >= h) continue;
-        int i = y * w + x;
-        float aa = __ldg(a0 + i), ab = __ldg(a1 + i), ad = __ldg(a2 + i);
-        int si = r * G::DS + c;
-        float b0 = s_d[si], b1 = s_d[G::DH * G::DS + si];
-        float u = __ldg(fu + i), v = __ldg(fv + i);
-        float t = ab * ab - ad * aa;
-        if (fabsf(t) > 40.0f) {
-            u = (ab * b1 - ad * b0) / t + u;
-            v = (ab * b0 - aa * b1) / t + v;
-        }
-        s_d[si] = u;
-        s_d[G::DH * G::DS + si] = v;
+    // 3. blur7 along the columns, outputs at the new_disp rows, and new_disp
+    for (int e = threadIdx.x; e < G::DW * G::S7V; e += nt) {
+        const int c = e % G::DW, r0 = (e / G::DW) * G::R7V;
+        const float2* in = s2 + r0 * G::HS + c;
+        float2* out = s1 + r0 * G::DS + c;
+        const int y_end = min(h, dy0 + G::DH);
+        if (iter_column7<TX, TY, false>(P, in, out, den7y + r0, dx0 + c, dy0 + r0, y_end))
+            iter_column7_slow<TX, TY>(P, in, out, den7y + r0, dx0 + c, dy0 + r0, y_end);
     }
     __syncthreads();
-    // 4. blur5 of the flow: horizontal at the tile columns, then vertical at the tile rows
-    {
-        constexpr int NSEG = (TX + R5 - 1) / R5;
-        for (int e = threadIdx.x; e < 2 * G::DH * NSEG; e += nt) {
-            int r = e % G::DH, rest = e / G::DH;
-            int seg = rest % NSEG, ch = rest / NSEG;
-            int Y = dy0 + r;
-            if (Y < 0 || Y >= h) continue;
-            int c0 = seg * R5;
-            const float* line = s_d + ch * G::DH * G::DS + r * G::DS;
-            pass_run<6, R5, true, false>(line, dx0, G::DW, 1, w, X0 + c0, g5.k,
-                                         s_f + ch * G::DH * G::FS + r * G::FS + c0, 1, min(R5, TX - c0));
-        }
+    // 4. blur5 of the flow along the rows at the tile's columns
+    for (int e = threadIdx.x; e < G::DH * (TX / G::R5H); e += nt) {
+        const int r = e % G::DH, c0 = (e / G::DH) * G::R5H;
+        const float2* in = s1 + r * G::DS + c0;
+        float2* out = s2 + r * G::FS + c0;
+        if (iter_row5<TX, TY, false>(P, in, out, den5x + c0, X0 + c0)) iter_row5_slow<TX, TY>(P, in, out, den5x + c0, X0 + c0);
     }
     __syncthreads();
-    //    vertical at the tile rows, into the tile buffer (buffer 1: its new_disp region was read by the
-    //    horizontal pass)
-    float* s_o = s_b;  // 2 x TY x TX
-    {
-        constexpr int NSEG = (TY + R5 - 1) / R5;
-        for (int e = threadIdx.x; e < 2 * TX * NSEG; e += nt) {
-            int c = e % TX, rest = e / TX;
-            int seg = rest % NSEG, ch = rest / NSEG;
-            int X = X0 + c;
-            if (X >= w) continue;
-            int r0 = seg * R5;
-            const float* line = s_f + ch * G::DH * G::FS + c;
-            int nv = min(R5, TY - r0);
-            float* dst = s_o + ch * TY * TX + r0 * TX + c;  // rows past h are never written
-            if (above_first) pass_run<6, R5, true, true>(line, dy0, G::DH, G::FS, h, Y0 + r0, g5.k, dst, TX, nv);
-            else pass_run<6, R5, true, false>(line, dy0, G::DH, G::FS, h, Y0 + r0, g5.k, dst, TX, nv);
-        }
-    }
-    __syncthreads();
-    // 5. the new flow to the planes; with b_out also calc_b of the next iteration at every pixel of the
-    //    tile (flow.rs:334-357), two pixels per thread and round with their loads in flight together
-    {
-        constexpr int K = 2;
-        for (int e0 = threadIdx.x; e0 < TX * TY; e0 += K * nt) {
-            float u[K], v[K], i1v[K], gxv[K], gyv[K];
-            bool in[K];
-#pragma unroll
-            for (int k = 0; k < K; k++) {
-                const int e = e0 + k * nt;
-                const int r = e / TX, c = e - r * TX;
-                const int x = X0 + c, y = Y0 + r;
-                in[k] = e < TX * TY && x < w && y < h;
-                u[k] = v[k] = i1v[k] = gxv[k] = gyv[k] = 0.0f;
-                if (in[k]) {
-                    const int i = y * w + x;
-                    u[k] = s_o[e];
-                    v[k] = s_o[TY * TX + e];
-                    fu_out[i] = u[k];
-                    fv_out[i] = v[k];
-                    if (b_out) {
-                        i1v[k] = __ldg(i1 + i);
-                        gxv[k] = __ldg(gx + i);
-                        gyv[k] = __ldg(gy + i);
-                    }
-                }
-            }
-            if (b_out) {
-#pragma unroll
-                for (int k = 0; k < K; k++) {
-                    if (!in[k]) continue;
-                    const int e = e0 + k * nt;
-                    const int r = e / TX, c = e - r * TX;
-                    const int x = X0 + c, y = Y0 + r;
-                    float b0, b1;
-                    calc_b_at(i0, mask_y, w, h, x, y, u[k], v[k], i1v[k], gxv[k], gyv[k], b0, b1);
-                    b_out[(long)y * bp + x] = b0;
-                    b_out[bplane + (long)y * bp + x] = b1;
-                }
-            }
-        }
+    // 5. blur5 along the columns: the new flow and the next iteration's B
+    for (int e = threadIdx.x; e < TX * (TY / G::R5V); e += nt) {
+        const int c = e % TX, r0 = (e / TX) * G::R5V;
+        if (X0 + c >= w || Y0 + r0 >= h) continue;
+        const float2* in = s2 + r0 * G::FS + c;
+        if (iter_column5<TX, TY, false>(P, in, den5y + r0, X0 + c, Y0 + r0)) iter_column5_slow<TX, TY>(P, in, den5y + r0, X0 + c, Y0 + r0);
     }
 }
 
-// The iteration reads B from b_in and, with b_out (same pitch bp and plane stride bplane), writes the
-// next iteration's B; b_in and b_out are different buffers (other tiles still read b_in's halo).
-#define TW_LEVEL_ITER(TX, TY)                                                                                         \
-    __global__ void __launch_bounds__(LEVEL_ITER_MAX_THREADS) k_level_iter_##TX##x##TY(                              \
-        const float* __restrict__ b_in, int bp, long bplane, const float* __restrict__ i1,                          \
-        const float* __restrict__ i0, const float* __restrict__ gx, const float* __restrict__ gy,                    \
-        const float* __restrict__ a0, const float* __restrict__ a1, const float* __restrict__ a2,                    \
-        const float* __restrict__ fu, const float* __restrict__ fv, int w, int h, Taps g7, Taps g5,                  \
-        bool above_first, float* __restrict__ fu_out, float* __restrict__ fv_out, const float* __restrict__ mask_y,  \
-        float* __restrict__ b_out) {                                                                                 \
-        level_iter_body<TX, TY>(b_in, bp, bplane, i1, i0, gx, gy, a0, a1, a2, fu, fv, w, h, g7, g5, above_first,    \
-                                fu_out, fv_out, mask_y, b_out);                                                      \
+// The iteration reads B from b_in and, with b_out (same pitch bp), writes the next iteration's B; b_in
+// and b_out are different buffers (other tiles still read b_in's halo).
+#define TW_LEVEL_ITER(TX, TY)                                                                          \
+    __global__ void __launch_bounds__(LEVEL_ITER_MAX_THREADS, 2) k_level_iter_##TX##x##TY(             \
+        const __grid_constant__ LevelIterArgs P) {                                                    \
+        level_iter_body<TX, TY>(P);                                                                   \
     }
+TW_LEVEL_ITER(16, 16)
 TW_LEVEL_ITER(32, 32)
+TW_LEVEL_ITER(32, 64)
 TW_LEVEL_ITER(64, 32)
 TW_LEVEL_ITER(64, 64)
 #undef TW_LEVEL_ITER
@@ -484,63 +530,57 @@ size_t level_iter_smem(int tile) {
     switch (tile) {
         case LEVEL_TILE_64x32: return IterGeom<64, 32>::SMEM;
         case LEVEL_TILE_64x64: return IterGeom<64, 64>::SMEM;
+        case LEVEL_TILE_16x16: return IterGeom<16, 16>::SMEM;
+        case LEVEL_TILE_32x64: return IterGeom<32, 64>::SMEM;
         default: return IterGeom<32, 32>::SMEM;
     }
 }
 
 // calc_b (flow.rs:334-357) of the next iteration where the flow changed outside an iteration (after
-// the block matching and the user displacement of the finest level): one thread per pixel, into two
-// planes of pitch bp (plane stride bplane).
+// the block matching and the user displacement of the finest level): one thread per pixel, into a plane
+// of pitch bp.
 __global__ void k_calc_b_pitched(const float* __restrict__ i1, const float* __restrict__ i0,
-                                 const float* __restrict__ gx, const float* __restrict__ gy,
-                                 const float* __restrict__ fu, const float* __restrict__ fv, int w, int h,
-                                 const float* __restrict__ mask_y, float* __restrict__ b_out, int bp, long bplane) {
+                                 const float2* __restrict__ grad, const float2* __restrict__ f, int w, int h,
+                                 const float* __restrict__ mask_y, float2* __restrict__ b_out, int bp) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= w || y >= h) return;
     const int i = y * w + x;
-    float b0, b1;
-    calc_b_at(i0, mask_y, w, h, x, y, __ldg(fu + i), __ldg(fv + i), __ldg(i1 + i), __ldg(gx + i), __ldg(gy + i), b0, b1);
-    b_out[(long)y * bp + x] = b0;
-    b_out[bplane + (long)y * bp + x] = b1;
+    const float2 fl = __ldg(f + i), g = __ldg(grad + i);
+    const float v = __ldg(i1 + i);
+    float2 b;
+    calc_b_run<1>(i0, mask_y, w, h, x, y, &fl, &v, &g, &b);
+    b_out[(long)y * bp + x] = b;
 }
 
 // ---- the end of a level (flow.rs:1292-1303): range reset, damping, then the upsample ---------------
 
 // The coarse field (with the reset and damping of its level applied on the fly) upsampled to the
-// next finer level (flow.rs:376-391, bilinear2 of sample.rs:69-86). Applying the elementwise reset
-// and damping to the four gathered samples is the same as applying them to the whole field first.
-__global__ void k_apply_upsample(const float* __restrict__ su, const float* __restrict__ sv, int sw, int sh,
+// next finer level, for the solves whose level starts with a user displacement (the others upsample in
+// k_level_init).
+__global__ void k_apply_upsample(const float2* __restrict__ src, int sw, int sh, UpsampleScale up,
                                  const int* __restrict__ any, int l, int start, bool damp_now, float damp,
-                                 float* __restrict__ du, float* __restrict__ dv, int dw, int dh) {
+                                 float2* __restrict__ dst, int dw, int dh) {
     int x = blockIdx.x * blockDim.x + threadIdx.x;
     int y = blockIdx.y;
     if (x >= dw || y >= dh) return;
-    float u, v;
-    upsample_at(su, sv, sw, sh, zero_at_level(any, l, start), damp_now, damp, x, y, dw, dh, &u, &v);
-    long o = (long)y * dw + x;
-    du[o] = u;
-    dv[o] = v;
+    dst[(long)y * dw + x] = upsample_at(src, sw, sh, up, zero_at_level(any, l, start), damp_now, damp, x, y);
 }
 
 // The finest level: reset and damping, then the final negation (flow.rs:1305) into the
 // interleaved FlowField; flags a NaN.
-__global__ void k_apply_negate(const float* __restrict__ fu, const float* __restrict__ fv, long n,
-                              const int* __restrict__ any, int start, bool damp_now, float damp,
-                              float* __restrict__ out, int* __restrict__ nan_flag) {
+__global__ void k_apply_negate(const float2* __restrict__ f, long n, const int* __restrict__ any, int start,
+                               bool damp_now, float damp, float2* __restrict__ out, int* __restrict__ nan_flag) {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    bool zero = zero_at_level(any, 0, start);
-    float u = zero ? 0.0f : fu[i];
-    float v = zero ? 0.0f : fv[i];
+    float2 v = zero_at_level(any, 0, start) ? make_float2(0.0f, 0.0f) : f[i];
     if (damp_now) {
-        u = damp * u;
-        v = damp * v;
+        v.x = damp * v.x;
+        v.y = damp * v.y;
     }
-    u = -1.0f * u;
-    v = -1.0f * v;
-    out[2 * i] = u;
-    out[2 * i + 1] = v;
-    if (isnan(u) || isnan(v)) atomicOr(nan_flag, 1);
+    v.x = -1.0f * v.x;
+    v.y = -1.0f * v.y;
+    out[i] = v;
+    if (isnan(v.x) || isnan(v.y)) atomicOr(nan_flag, 1);
 }
 
 TW_VARIANT_END

@@ -211,44 +211,28 @@ int tw_open(int device, tw_ctx** out) {
     ctx->g5 = gaussian_taps(5.0f);
     ctx->g2 = gaussian_taps(2.0f);
     ctx->b5 = binomial5();
-    // block matching keeps one line of the field in shared memory (up to BM_MAX_LINE elements)
-    e = cudaFuncSetAttribute(k_bm_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bm_smem_bytes(BM_MAX_LINE));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_bm_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bm_smem_bytes(BM_MAX_LINE));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_level_init, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)level_init_smem());
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_level_iter_32x32, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)level_iter_smem(LEVEL_TILE_32x32));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_level_iter_64x32, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)level_iter_smem(LEVEL_TILE_64x32));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_level_iter_64x64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)level_iter_smem(LEVEL_TILE_64x64));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_solve_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)coarse_smem_bytes());
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_fill_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(FILL_COARSE_MAX_FLOATS * sizeof(float)));
-    // the fast mode's builds of the same kernels
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(fast::k_bm_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bm_smem_bytes(BM_MAX_LINE));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(fast::k_bm_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bm_smem_bytes(BM_MAX_LINE));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(fast::k_level_init, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)level_init_smem());
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(fast::k_level_iter_32x32, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)level_iter_smem(LEVEL_TILE_32x32));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(fast::k_level_iter_64x32, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)level_iter_smem(LEVEL_TILE_64x32));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(fast::k_level_iter_64x64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)level_iter_smem(LEVEL_TILE_64x64));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(fast::k_solve_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)coarse_smem_bytes());
+    // the dynamic shared memory limits, of the strict kernels and of the fast mode's builds of them; block
+    // matching keeps one line of the field in shared memory (up to BM_MAX_LINE elements)
+    auto limit = [&](const void* k, size_t smem) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    };
+#define TW_LIMIT(kernel, smem)                \
+    do {                                      \
+        limit((const void*)kernel, smem);       \
+        limit((const void*)fast::kernel, smem); \
+    } while (0)
+    TW_LIMIT(k_bm_rows, bm_smem_bytes(BM_MAX_LINE));
+    TW_LIMIT(k_bm_cols, bm_smem_bytes(BM_MAX_LINE));
+    TW_LIMIT(k_level_init_16x16, level_init_smem(LEVEL_TILE_16x16));
+    TW_LIMIT(k_level_init_32x32, level_init_smem(LEVEL_TILE_32x32));
+    TW_LIMIT(k_level_iter_16x16, level_iter_smem(LEVEL_TILE_16x16));
+    TW_LIMIT(k_level_iter_32x32, level_iter_smem(LEVEL_TILE_32x32));
+    TW_LIMIT(k_level_iter_32x64, level_iter_smem(LEVEL_TILE_32x64));
+    TW_LIMIT(k_level_iter_64x32, level_iter_smem(LEVEL_TILE_64x32));
+    TW_LIMIT(k_level_iter_64x64, level_iter_smem(LEVEL_TILE_64x64));
+    TW_LIMIT(k_solve_coarse, coarse_smem_bytes());
+#undef TW_LIMIT
+    limit((const void*)k_fill_coarse, FILL_COARSE_MAX_FLOATS * sizeof(float));
     if (e != cudaSuccess) { tw_close(ctx); return TW_ERR_CUDA; }
     if (ctx->ensure(ctx->flags, FLAGS_BYTES, "flags") != TW_OK) { tw_close(ctx); return TW_ERR_CUDA; }
     k_selfcheck<<<1, 1, 0, ctx->stream>>>(ctx->flags.as<int>());

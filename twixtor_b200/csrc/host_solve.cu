@@ -3,6 +3,8 @@
 // points.
 #include "runtime.h"
 
+#include "level.cuh"
+
 namespace tw {
 
 void flow_resolution(int q, bool hiq, int w, int h, int* r_out, int* w0, int* h0) {
@@ -69,6 +71,7 @@ void start_level(float sensitivity, int levels, int* start, float* damp) {  // f
 
 Taps gaussian_taps(float r) {  // flow/conv.rs:64-86
     Taps t{};
+    t.z = -0.0f;
     int ri = std::isnan(r) ? 0 : (int)r;
     int n = std::max(ri + 1, 0);
     n = std::min(n, MAX_TAPS);
@@ -92,6 +95,7 @@ Taps gaussian_taps(float r) {  // flow/conv.rs:64-86
 
 Taps binomial5() {  // flow/conv.rs:48
     Taps t{};
+    t.z = -0.0f;
     t.k[0] = 0.375f;
     t.k[1] = 0.25f;
     t.k[2] = 0.0625f;
@@ -110,37 +114,31 @@ void conv_planes(tw_ctx* ctx, float* const* planes, int c, int w, int h, const T
     }
 }
 
-// One solver iteration (k_level_iter_*) with the tile shape and block size of the level's choice:
-// B read from b_in; with b_out the next iteration's B written (planes of pitch bp, stride bplane).
-// Algorithmic bytes per pixel: B (2), the tensor (3) and the flow (2) read, the flow (2) written;
-// with b_out also I1, the I0 gather and the gradient (2) read and B (2) written.
-void level_iter(tw_ctx* ctx, LevelTune ic, const float* A, const float* B, const float* gx, const float* gy,
-                const float* a0, const float* a1, const float* a2, const float* fu, const float* fv, int w, int h, bool af,
-                float* nu, float* nv, const float* mask_y, bool fast, const float* b_in, float* b_out, int bp,
-                long bplane) {
-    double b = (b_out ? 60.0 : 36.0) * w * h;
-    size_t smem = level_iter_smem(ic.iter_tile);
-    if (ic.iter_tile == LEVEL_TILE_64x64) {
-        dim3 g((unsigned)((w + 63) / 64), (unsigned)((h + 63) / 64));
-        LAUNCHV(ctx, fast, b, k_level_iter_64x64, g, ic.iter_threads, smem, b_in, bp, bplane, A, B, gx, gy, a0, a1, a2, fu, fv, w,
-                h, ctx->g7, ctx->g5, af, nu, nv, mask_y, b_out);
-    } else if (ic.iter_tile == LEVEL_TILE_64x32) {
-        dim3 g((unsigned)((w + 63) / 64), (unsigned)((h + 31) / 32));
-        LAUNCHV(ctx, fast, b, k_level_iter_64x32, g, ic.iter_threads, smem, b_in, bp, bplane, A, B, gx, gy, a0, a1, a2, fu, fv, w,
-                h, ctx->g7, ctx->g5, af, nu, nv, mask_y, b_out);
-    } else {
-        LAUNCHV(ctx, fast, b, k_level_iter_32x32, tiles(w, h), ic.iter_threads, smem, b_in, bp, bplane, A, B, gx, gy, a0, a1, a2,
-                fu, fv, w, h, ctx->g7, ctx->g5, af, nu, nv, mask_y, b_out);
+// One solver iteration (k_level_iter_*) with the tile shape and block size of the level's choice.
+// Algorithmic bytes per pixel: B (8), the tensor (16) and the flow (8) read, the flow (8) written;
+// with b_out also I1 (4), the I0 gather (4) and the gradient (8) read and B (8) written.
+void level_iter(tw_ctx* ctx, LevelTune ic, const LevelIterArgs& P, bool fast) {
+    const double b = (P.b_out ? 64.0 : 40.0) * P.w * P.h;
+    const size_t smem = level_iter_smem(ic.iter_tile);
+    auto grid = [&](int tx, int ty) { return dim3((unsigned)((P.w + tx - 1) / tx), (unsigned)((P.h + ty - 1) / ty)); };
+    switch (ic.iter_tile) {
+        case LEVEL_TILE_64x64: LAUNCHV(ctx, fast, b, k_level_iter_64x64, grid(64, 64), ic.iter_threads, smem, P); break;
+        case LEVEL_TILE_64x32: LAUNCHV(ctx, fast, b, k_level_iter_64x32, grid(64, 32), ic.iter_threads, smem, P); break;
+        case LEVEL_TILE_32x64: LAUNCHV(ctx, fast, b, k_level_iter_32x64, grid(32, 64), ic.iter_threads, smem, P); break;
+        case LEVEL_TILE_16x16: LAUNCHV(ctx, fast, b, k_level_iter_16x16, grid(16, 16), ic.iter_threads, smem, P); break;
+        default: LAUNCHV(ctx, fast, b, k_level_iter_32x32, grid(32, 32), ic.iter_threads, smem, P); break;
     }
 }
 
 // The launch shapes at a level of w x h: the tuning table's entry when the autotuner measured this
-// size, else the defaults: 32 x 32 iteration tiles with 512 threads for levels of few tiles
-// (latency bound: fewer elements per thread per stage) and 256 otherwise; 256 threads per line of
-// block matching.
+// size, else the defaults: the largest tile that still gives about a block per SM (fewer, larger tiles
+// recompute less halo but leave SMs idle; the times beside k_level_iter in fused.cu).
+static long tiles_of(int w, int h, int tx, int ty) { return (long)((w + tx - 1) / tx) * ((h + ty - 1) / ty); }
+
 LevelTune default_tune(int w, int h) {
-    long tiles_n = (long)((w + 31) / 32) * ((h + 31) / 32);
-    return LevelTune{LEVEL_TILE_32x32, tiles_n <= 296 ? 512 : 256, TB, TB};
+    if (tiles_of(w, h, 16, 16) <= 148) return LevelTune{LEVEL_TILE_16x16, 512, TB, TB};
+    if (tiles_of(w, h, 32, 32) <= 148) return LevelTune{LEVEL_TILE_32x32, 512, TB, TB};
+    return LevelTune{LEVEL_TILE_32x64, 512, TB, TB};
 }
 
 LevelTune level_tune(tw_ctx* ctx, int w, int h) {
@@ -148,7 +146,7 @@ LevelTune level_tune(tw_ctx* ctx, int w, int h) {
     return it != ctx->tune_table.end() ? it->second : default_tune(w, h);
 }
 
-// Threads per CTA of the tiled pyramid and tensor kernels: a level of few tiles is latency bound
+// Threads per CTA of the tiled pyramid kernels: a level of few tiles is latency bound
 // (every CTA walks its stages one after the other), so its CTAs get more threads and each thread
 // fewer elements per stage; a level with tiles enough to fill the GPU keeps 256.
 static int level_threads(int w, int h) {
@@ -302,17 +300,16 @@ int build_user_dev(tw_ctx* ctx, const UserPairs& pr, const Geo& g, int W, int H,
 }
 
 // ---- block matching (flow.rs:551-622) -----------------------------------------------------------------
-// Rows on the row-major planes; then the field is transposed, the column sweeps run on the
-// transposed planes (AT, BT: the level's bands stored column by column), and the field goes back.
-// uT, vT: scratch for the transposed field (w * h floats each).
-void block_match(tw_ctx* ctx, const float* A, const float* B, const float* AT, const float* BT, float* fu, float* fv,
-                 float* uT, float* vT, int w, int h, bool fast) {
+// Rows on the row-major planes, the swept field going into its transpose ft (w * h elements of scratch);
+// then the column sweeps on the transposed planes (AT, BT: the level's bands stored column by column),
+// the field going back into f.
+void block_match(tw_ctx* ctx, const float* A, const float* B, const float* AT, const float* BT, float2* f, float2* ft, int w,
+                 int h, bool fast) {
     if (w < 3 || h < 3) return;  // callers refuse lines above BM_MAX_LINE before any launch
     double b = 24.0 * w * h;  // per launch (both sweeps): the field read and written (8 + 8), A and B read once (4 + 4)
     LevelTune t = level_tune(ctx, w, h);
-    // the row sweeps write the transposed field the column sweeps read, and those write it back
-    LAUNCHV(ctx, fast, b, k_bm_rows, h - 2, t.bm_rows_threads, bm_smem_bytes(w), A, B, fu, fv, w, h, uT, vT);
-    LAUNCHV(ctx, fast, b, k_bm_cols, w - 2, t.bm_cols_threads, bm_smem_bytes(h), AT, BT, uT, vT, w, h, fu, fv);
+    LAUNCHV(ctx, fast, b, k_bm_rows, h - 2, t.bm_rows_threads, bm_smem_bytes(w), A, B, f, w, h, ft);
+    LAUNCHV(ctx, fast, b, k_bm_cols, w - 2, t.bm_cols_threads, bm_smem_bytes(h), AT, BT, ft, w, h, f);
 }
 
 // ---- one solve over two resident pyramids (flow.rs:1258-1307) ------------------------------------------
@@ -329,18 +326,13 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
                        const tw_flow_settings& s, DevBuf& work, float* out, int* any, int* nan_flag,
                        const float* mx, const float* my, const float* udu,
                        const float* udv, const float* uww) {
-    size_t np0 = (size_t)g.w * g.h;
-    // planes: gx gy a0 a1 a2 u0 v0 u1 v1 uT vT, then two B buffers of two planes each, 16-byte
-    // aligned, of pitch (w + 3) & ~3 at every level (plane stride bplane: the finest level's)
-    const int NP = 11;
-    const size_t boff = (np0 * NP + 3) & ~(size_t)3;
-    const long bplane = (long)((g.w + 3) & ~3) * g.h;
-    CHECK(ctx->ensure(work, (boff + 4 * (size_t)bplane) * sizeof(float), "solve scratch"));
-    float* base = work.as<float>();
-    float *gx = base, *gy = base + np0, *a0 = base + 2 * np0, *a1 = base + 3 * np0, *a2 = base + 4 * np0;
-    float *fu = base + 5 * np0, *fv = base + 6 * np0, *nu = base + 7 * np0, *nv = base + 8 * np0;
-    float *ut = base + 9 * np0, *vt = base + 10 * np0;
-    float* bb[2] = {base + boff, base + boff + 2 * bplane};
+    // the tensor (float4), two B planes (float2, of pitch bp0 = w rounded up to even at the finest level,
+    // so 16-byte aligned), the gradient, the flow twice and its transpose (float2)
+    const size_t np0 = (size_t)g.w * g.h, bplane = (size_t)((g.w + 1) & ~1) * g.h;
+    CHECK(ctx->ensure(work, np0 * (sizeof(float4) + 4 * sizeof(float2)) + 2 * bplane * sizeof(float2), "solve scratch"));
+    float4* tensor = work.as<float4>();
+    float2* bb[2] = {(float2*)(tensor + np0), (float2*)(tensor + np0) + bplane};
+    float2 *grad = bb[1] + bplane, *f = grad + np0, *fn = f + np0, *ft = fn + np0;
     int start;
     float damp;
     start_level(s.sensitivity, g.levels, &start, &damp);
@@ -348,8 +340,7 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
     size_t off = 0;
     for (int i = 0; i < g.levels; i++) { offs[i] = off; off += (size_t)g.sizes[i][0] * g.sizes[i][1]; }
     long ns = (long)g.sizes[start][0] * g.sizes[start][1];
-    CHECK(GOP(ctx, ctx->cuda(cudaMemsetAsync(fu, 0, ns * sizeof(float), ctx->cur), "flow init")));
-    CHECK(GOP(ctx, ctx->cuda(cudaMemsetAsync(fv, 0, ns * sizeof(float), ctx->cur), "flow init")));
+    CHECK(GOP(ctx, ctx->cuda(cudaMemsetAsync(f, 0, ns * sizeof(float2), ctx->cur), "flow init")));
     CHECK(GOP(ctx, ctx->cuda(cudaMemsetAsync(any, 0, 32 * sizeof(int), ctx->cur), "range flags")));
     bool af = s.taps_above_first != 0;
     bool damp_any = std::fabs((double)damp - 1.0) >= 1e-6;
@@ -357,6 +348,7 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
     // The coarse levels whose planes fit one block's shared memory run in one launch (coarse.cu),
     // for the plain solve; the masked and the tracked solves keep the kernel by kernel path.
     int first = start;
+    bool have_flow = true;  // f holds the flow of level `first` (zero at the start level)
     if (!mx && !my && !udu) {
         int last = -1;
         for (int l = start; l >= 1; l--) {
@@ -382,8 +374,7 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
             J.g7 = ctx->g7;
             J.g5 = ctx->g5;
             J.any = any;
-            J.fu_out = fu;
-            J.fv_out = fv;
+            J.f_out = f;
             double px = 0.0;
             for (int l = start; l >= last; l--) px += (double)g.sizes[l][0] * g.sizes[l][1];
             LAUNCHV(ctx, fast, 8.0 * px, k_solve_coarse, 1, COARSE_THREADS, coarse_smem_bytes(), J);
@@ -391,55 +382,99 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
         }
     }
     for (int l = first; l >= 0; l--) {
-        int w = g.sizes[l][0], h = g.sizes[l][1];
+        const int w = g.sizes[l][0], h = g.sizes[l][1];
         const float* A = x + offs[l];
         const float* B = y + offs[l];
         const float* AT = xt + offs[l];
         const float* BT = yt + offs[l];
-        double px = (double)w * h;
-        int lt = level_threads(w, h);
-        const float* mask_x = mx ? mx + offs[l] : nullptr;
+        const double px = (double)w * h;
         const float* mask_y = my ? my + offs[l] : nullptr;
         // flow/extras.rs:198-215: the user displacement of the tracking points, flow = d / w, after the
         // start or the upsample, after the finest level's block matching and at the end of the level
         auto user = [&]() {
-            if (udu) LAUNCH(ctx, k_apply_user, grid1((long)w * h), TB, 0, fu, fv, udu + offs[l], udv + offs[l], uww + offs[l],
+            if (udu) LAUNCH(ctx, k_apply_user, grid1((long)w * h), TB, 0, f, udu + offs[l], udv + offs[l], uww + offs[l],
                             (long)w * h);
         };
+        const bool damp_up = l + 1 == start && damp_any;  // the damping of the level the flow comes up from
+        LevelInitArgs I;
+        std::memset(&I, 0, sizeof I);
+        if (!have_flow) {
+            const int cw = g.sizes[l + 1][0], ch = g.sizes[l + 1][1];
+            const UpsampleScale up = upsample_scale(cw, ch, w, h);
+            if (udu) {  // the points move the upsampled flow before the level starts
+                LAUNCHV(ctx, fast, 0, k_apply_upsample, grid2(w, h), TB, 0, f, cw, ch, up, any, l + 1, start, damp_up, damp, fn, w, h);
+            } else {
+                I.src = f;
+                I.sw = cw;
+                I.sh = ch;
+                I.up = up;
+                I.any = any;
+                I.damp = damp;
+                I.damp_now = damp_up;
+            }
+            std::swap(f, fn);
+        }
+        have_flow = false;
         user();
-        LevelTune ic = level_tune(ctx, w, h);
-        const int bp = (w + 3) & ~3;
-        // the image read, the gradient and the tensor written; the flow, I0 (gather) read and B written
-        LAUNCHV(ctx, fast, 44.0 * px, k_level_init, tiles(w, h), lt, level_init_smem(), A, w, h, ctx->g7, af, gx, gy, a0, a1, a2,
-                mask_x, fu, fv, B, mask_y, bb[0], bp, bplane);
+        I.img = A;
+        I.i0 = B;
+        I.mask_x = mx ? mx + offs[l] : nullptr;
+        I.mask_y = mask_y;
+        I.f = f;
+        I.grad = grad;
+        I.tensor = tensor;
+        I.b_out = bb[0];
+        I.w = w;
+        I.h = h;
+        I.bp = (w + 1) & ~1;
+        I.l = l;
+        I.start = start;
+        I.af = af;
+        I.g7 = ctx->g7;
+        // the image read, the gradient and the tensor written (28); the flow and the I0 gather read, B
+        // written (20)
+        if (tiles_of(w, h, 16, 16) <= 148)
+            LAUNCHV(ctx, fast, 48.0 * px, k_level_init_16x16, dim3((w + 15) / 16, (h + 15) / 16), 512,
+                    level_init_smem(LEVEL_TILE_16x16), I);
+        else
+            LAUNCHV(ctx, fast, 48.0 * px, k_level_init_32x32, tiles(w, h), tiles_of(w, h, 32, 32) <= 148 ? 512 : 256,
+                    level_init_smem(LEVEL_TILE_32x32), I);
+        LevelIterArgs P;
+        std::memset(&P, 0, sizeof P);
+        P.i1 = A;
+        P.i0 = B;
+        P.grad = grad;
+        P.tensor = tensor;
+        P.mask_y = mask_y;
+        P.w = w;
+        P.h = h;
+        P.bp = I.bp;
+        P.af = af;
+        P.g7 = ctx->g7;
+        P.g5 = ctx->g5;
+        const LevelTune ic = level_tune(ctx, w, h);
         for (int it = 0; it < 3; it++) {
             // iteration it reads B from bb[it & 1]; the next one's B comes from its epilogue, or after
             // the finest level's block matching from the pointwise pass
             const bool emit = it == 0 || (it == 1 && l != 0);
-            level_iter(ctx, ic, A, B, gx, gy, a0, a1, a2, fu, fv, w, h, af, nu, nv, mask_y, fast, bb[it & 1],
-                       emit ? bb[(it + 1) & 1] : nullptr, bp, bplane);
-            std::swap(fu, nu);
-            std::swap(fv, nv);
+            P.b_in = bb[it & 1];
+            P.b_out = emit ? bb[(it + 1) & 1] : nullptr;
+            P.f = f;
+            P.f_out = fn;
+            level_iter(ctx, ic, P, fast);
+            std::swap(f, fn);
             if (it == 1 && l == 0) {
-                if (!s.skip_refine) block_match(ctx, A, B, AT, BT, fu, fv, ut, vt, w, h, fast);
+                if (!s.skip_refine) block_match(ctx, A, B, AT, BT, f, ft, w, h, fast);
                 user();
-                LAUNCHV(ctx, fast, 32.0 * px, k_calc_b_pitched, grid2(w, h), TB, 0, A, B, gx, gy, fu, fv, w, h, mask_y, bb[0], bp,
-                        bplane);
+                LAUNCHV(ctx, fast, 40.0 * px, k_calc_b_pitched, grid2(w, h), TB, 0, A, B, grad, f, w, h, mask_y, bb[0], P.bp);
             }
         }
-        if (l != 0 && !s.skip_refine) block_match(ctx, A, B, AT, BT, fu, fv, ut, vt, w, h, fast);
+        if (l != 0 && !s.skip_refine) block_match(ctx, A, B, AT, BT, f, ft, w, h, fast);
         user();
-        LAUNCHV(ctx, fast, 0, k_range_any, grid2(w, h), TB, 0, fu, fv, w, h, any + l);
-        bool damp_now = l == start && damp_any;
-        if (l > 0) {
-            int dw = g.sizes[l - 1][0], dh = g.sizes[l - 1][1];
-            LAUNCHV(ctx, fast, 0, k_apply_upsample, grid2(dw, dh), TB, 0, fu, fv, w, h, any, l, start, damp_now, damp, nu, nv, dw, dh);
-            std::swap(fu, nu);
-            std::swap(fv, nv);
-        } else {
-            LAUNCHV(ctx, fast, 0, k_apply_negate, grid1((long)np0), TB, 0, fu, fv, (long)np0, any, start, damp_now, damp, out, nan_flag);
-        }
+        LAUNCHV(ctx, fast, 0, k_range_any, grid2(w, h), TB, 0, f, w, h, any + l);
     }
+    LAUNCHV(ctx, fast, 0, k_apply_negate, grid1((long)np0), TB, 0, f, (long)np0, any, start, start == 0 && damp_any, damp,
+            (float2*)out, nan_flag);
     return TW_OK;
 }
 
@@ -713,18 +748,15 @@ int tw_block_match(tw_ctx* ctx, const float* a, const float* b, float* flow, int
     CHECK(ctx->ensure(ctx->plane[0], n * 4, "plane A"));
     CHECK(ctx->ensure(ctx->plane[1], n * 4, "plane B"));
     CHECK(ctx->ensure(ctx->plane[2], n * 8, "flow"));
-    CHECK(ctx->ensure(ctx->work[0], n * 4 * 6, "flow planes"));
+    CHECK(ctx->ensure(ctx->work[0], n * 4 * 4, "flow planes"));
     CHECK(ctx->cuda(cudaMemcpyAsync(ctx->plane[0].p, a, n * 4, cudaMemcpyHostToDevice, ctx->stream), "upload"));
     CHECK(ctx->cuda(cudaMemcpyAsync(ctx->plane[1].p, b, n * 4, cudaMemcpyHostToDevice, ctx->stream), "upload"));
     CHECK(ctx->cuda(cudaMemcpyAsync(ctx->plane[2].p, flow, n * 8, cudaMemcpyHostToDevice, ctx->stream), "upload"));
-    float* fu = ctx->work[0].as<float>();
-    float* fv = fu + n;
-    float *at = fv + n, *bt = at + n, *ut = bt + n, *vt = ut + n;
-    LAUNCH(ctx, k_deinterleave, grid1((long)n), TB, 0, ctx->plane[2].as<float>(), (long)n, fu, fv);
+    float2* ft = ctx->work[0].as<float2>();
+    float *at = (float*)(ft + n), *bt = at + n;
     LAUNCH(ctx, k_transpose2, dim3((width + 31) / 32, (height + 31) / 32), dim3(32, 8), 0, ctx->plane[0].as<float>(),
            ctx->plane[1].as<float>(), at, bt, width, height);
-    block_match(ctx, ctx->plane[0].as<float>(), ctx->plane[1].as<float>(), at, bt, fu, fv, ut, vt, width, height);
-    LAUNCH(ctx, k_interleave, grid1((long)n), TB, 0, fu, fv, (long)n, ctx->plane[2].as<float>());
+    block_match(ctx, ctx->plane[0].as<float>(), ctx->plane[1].as<float>(), at, bt, ctx->plane[2].as<float2>(), ft, width, height);
     CHECK(ctx->cuda(cudaMemcpyAsync(flow, ctx->plane[2].p, n * 8, cudaMemcpyDeviceToHost, ctx->stream), "download"));
     int hf[1];
     return finish(ctx, hf, 1);

@@ -24,7 +24,8 @@ bool valid_threads(int t, int max) { return t >= 32 && t <= max && t % 32 == 0; 
 
 namespace {
 
-const char* tile_name(int t) { return t == LEVEL_TILE_64x64 ? "64x64" : t == LEVEL_TILE_64x32 ? "64x32" : "32x32"; }
+const char* const TILE_NAMES[] = {"32x32", "64x32", "64x64", "16x16", "32x64"};  // by LEVEL_TILE_*
+const char* tile_name(int t) { return TILE_NAMES[t]; }
 
 // The table as JSON: the device's name, then one entry per level size.
 std::string table_json(tw_ctx* ctx) {
@@ -66,8 +67,9 @@ void load_table(tw_ctx* ctx, const char* path) {
             sscanf(line, " \"%dx%d\": {\"iter_tile\": \"%15[0-9x]\", \"iter_threads\": %d, \"bm_rows_threads\": %d, "
                          "\"bm_cols_threads\": %d}",
                    &w, &h, tile, &it, &rt, &ct) == 6) {
-            int t = std::strcmp(tile, "64x64") == 0 ? LEVEL_TILE_64x64 : std::strcmp(tile, "64x32") == 0 ? LEVEL_TILE_64x32
-                                                                                                        : LEVEL_TILE_32x32;
+            int t = LEVEL_TILE_32x32;
+            for (int k = 0; k < 5; k++)
+                if (std::strcmp(tile, TILE_NAMES[k]) == 0) t = k;
             if (w > 0 && h > 0 && valid_threads(it, LEVEL_ITER_MAX_THREADS) && valid_threads(rt, 1024) &&
                 valid_threads(ct, 1024))
                 ctx->tune_table[key(w, h)] = LevelTune{t, it, rt, ct};
@@ -95,30 +97,28 @@ int tw_autotune(tw_ctx* ctx, const tw_flow_settings* s, int32_t width, int32_t h
     for (int l = 0; l < g.levels; l++)
         if (!ctx->tune_table.count(key(g.sizes[l][0], g.sizes[l][1]))) todo.push_back(l);
     if (!todo.empty()) {
-        // stand-in planes of the largest level: A, B, the gradient, the tensor, the flow in and out,
-        // the transposes, and a copy of the flow that block matching updates in place
-        size_t n0 = (size_t)g.w * g.h;
+        // stand-in planes of the largest level: the bands and their transposes, the gradient, the tensor,
+        // the flow, its output, its transpose and a copy that block matching updates in place, and two B
+        // planes of an even pitch, 16-byte aligned
+        const size_t n0 = (size_t)g.w * g.h, bplane = (size_t)((g.w + 1) & ~1) * g.h;
         DevBuf buf;
         size_t held = 0;
-        const int NP = 16;
-        // and two B buffers (two planes each) of pitch (w + 3) & ~3, 16-byte aligned
-        const size_t boff = (NP * n0 + 3) & ~(size_t)3;
-        const long bplane = (long)((g.w + 3) & ~3) * g.h;
-        cudaError_t e = buf.ensure((boff + 4 * (size_t)bplane) * sizeof(float), &held);
+        cudaError_t e = buf.ensure((n0 * (4 + 5 * 2 + 4) + 2 * 2 * bplane) * sizeof(float), &held);
         if (e != cudaSuccess) return ctx->cuda(e, "autotune buffers");
-        float* p = buf.as<float>();
-        float *A = p, *Bp = p + n0, *gx = p + 2 * n0, *gy = p + 3 * n0, *a0 = p + 4 * n0, *a1 = p + 5 * n0,
-              *a2 = p + 6 * n0, *fu = p + 7 * n0, *fv = p + 8 * n0, *nu = p + 9 * n0, *nv = p + 10 * n0,
-              *AT = p + 11 * n0, *BT = p + 12 * n0, *uT = p + 13 * n0, *vT = p + 14 * n0, *fsave = p + 15 * n0;
-        const float amps[15] = {40.f, 40.f, 8.f, 8.f, 60.f, 20.f, 60.f, 3.f, 3.f, 0.f, 0.f, 40.f, 40.f, 0.f, 0.f};
-        for (int i = 0; i < 15; i++) {
-            k_tune_fill<<<grid1((long)n0), TB, 0, ctx->stream>>>(p + i * n0, (long)n0, 0x9e3779b9u * (i + 1), amps[i]);
+        float4* tensor = buf.as<float4>();
+        float2 *bin = (float2*)(tensor + n0), *bout = bin + bplane, *grad = bout + bplane, *f = grad + n0, *fn = f + n0,
+               *ft = fn + n0, *fsave = ft + n0;
+        float *A = (float*)(fsave + n0), *Bp = A + n0, *AT = Bp + n0, *BT = AT + n0;
+        uint32_t seed = 0;
+        auto fill = [&](void* p, size_t floats, float amp) {
+            k_tune_fill<<<grid1((long)floats), TB, 0, ctx->stream>>>((float*)p, (long)floats, 0x9e3779b9u * ++seed, amp);
             ctx->launches++;
-        }
-        float* bin = p + boff;
-        float* bout = bin + 2 * bplane;
-        k_tune_fill<<<grid1(2 * bplane), TB, 0, ctx->stream>>>(bin, 2 * bplane, 0x85ebca6bu, 50.f);
-        ctx->launches++;
+        };
+        fill(tensor, 4 * n0, 60.f);
+        fill(bin, 2 * bplane, 50.f);
+        fill(grad, 2 * n0, 8.f);
+        fill(f, 2 * n0, 3.f);
+        for (float* p : {A, Bp, AT, BT}) fill(p, n0, 40.f);
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
@@ -141,13 +141,30 @@ int tw_autotune(tw_ctx* ctx, const tw_flow_settings* s, int32_t width, int32_t h
             int w = g.sizes[l][0], h = g.sizes[l][1];
             LevelTune best = default_tune(w, h);
             // the solver iteration: every tile shape with 256 and 512 threads (64 x 64 with 512)
-            const LevelTune iter_cands[5] = {{LEVEL_TILE_32x32, 256, 0, 0}, {LEVEL_TILE_32x32, 512, 0, 0},
+            const LevelTune iter_cands[9] = {{LEVEL_TILE_16x16, 256, 0, 0}, {LEVEL_TILE_16x16, 512, 0, 0},
+                                             {LEVEL_TILE_32x32, 256, 0, 0}, {LEVEL_TILE_32x32, 512, 0, 0},
+                                             {LEVEL_TILE_32x64, 256, 0, 0}, {LEVEL_TILE_32x64, 512, 0, 0},
                                              {LEVEL_TILE_64x32, 256, 0, 0}, {LEVEL_TILE_64x32, 512, 0, 0},
                                              {LEVEL_TILE_64x64, 512, 0, 0}};
+            LevelIterArgs P;
+            std::memset(&P, 0, sizeof P);
+            P.b_in = bin;
+            P.i1 = A;
+            P.i0 = Bp;
+            P.grad = grad;
+            P.tensor = tensor;
+            P.f = f;
+            P.f_out = fn;
+            P.b_out = bout;
+            P.w = w;
+            P.h = h;
+            P.bp = (w + 1) & ~1;
+            P.af = af;
+            P.g7 = ctx->g7;
+            P.g5 = ctx->g5;
             float bt = 1e30f;
             for (const LevelTune& c : iter_cands) {
-                float ms = timed([&] { level_iter(ctx, c, A, Bp, gx, gy, a0, a1, a2, fu, fv, w, h, af, nu, nv, nullptr, false, bin, bout,
-                                                  (w + 3) & ~3, bplane); });
+                float ms = timed([&] { level_iter(ctx, c, P, false); });
                 if (ms < bt) {
                     bt = ms;
                     best.iter_tile = c.iter_tile;
@@ -157,17 +174,18 @@ int tw_autotune(tw_ctx* ctx, const tw_flow_settings* s, int32_t width, int32_t h
             // block matching: the row and the column kernel, 128 to 512 threads per line (each one's
             // input field restored before every launch)
             if (w >= 3 && h >= 3) {
-                cudaMemcpyAsync(fsave, fu, (size_t)w * h * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream);
+                const size_t fbytes = (size_t)w * h * sizeof(float2);
+                cudaMemcpyAsync(fsave, f, fbytes, cudaMemcpyDeviceToDevice, ctx->stream);
                 float br = 1e30f, bc = 1e30f;
                 for (int th : {128, 256, 512}) {
                     float ms = timed([&] {
-                        cudaMemcpyAsync(fu, fsave, (size_t)w * h * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream);
-                        LAUNCH(ctx, k_bm_rows, h - 2, th, bm_smem_bytes(w), A, Bp, fu, fv, w, h, uT, vT);
+                        cudaMemcpyAsync(f, fsave, fbytes, cudaMemcpyDeviceToDevice, ctx->stream);
+                        LAUNCH(ctx, k_bm_rows, h - 2, th, bm_smem_bytes(w), A, Bp, f, w, h, ft);
                     });
                     if (ms < br) { br = ms; best.bm_rows_threads = th; }
                     ms = timed([&] {
-                        cudaMemcpyAsync(uT, fsave, (size_t)w * h * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream);
-                        LAUNCH(ctx, k_bm_cols, w - 2, th, bm_smem_bytes(h), AT, BT, uT, vT, w, h, fu, fv);
+                        cudaMemcpyAsync(ft, fsave, fbytes, cudaMemcpyDeviceToDevice, ctx->stream);
+                        LAUNCH(ctx, k_bm_cols, w - 2, th, bm_smem_bytes(h), AT, BT, ft, w, h, f);
                     });
                     if (ms < bc) { bc = ms; best.bm_cols_threads = th; }
                 }

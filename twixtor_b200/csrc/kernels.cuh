@@ -1,9 +1,10 @@
 // Declarations of the library's sm_100a kernels (strict mode) and their small device helpers.
 //
-// Layout in HBM: every multi channel buffer of the solver is PLANAR (one float plane per channel,
-// row major, pitch = width), so each pass streams coalesced lanes and the separable filter runs
-// the same code on each plane. The reference's interleaved layout only changes where samples
-// live, never the arithmetic of an element, so results are bit identical. Engine images keep the
+// Layout in HBM: the bands of a pyramid are planes; the solver's fields (flow, gradient, B) hold both
+// components of a pixel in one float2 and its tensor in one float4 (three channels and the determinant
+// of new_disp), so a pixel is one load and the separable filters run both components in packed
+// operations. The layout only changes where samples live, never the arithmetic of an element, so
+// results are bit identical. Engine images keep the
 // reference's interleaved A, R, G, B samples (one 32-bit word per 8 bpc pixel).
 #pragma once
 #include <cstdint>
@@ -28,6 +29,7 @@ constexpr int MAX_TAPS = 8;  // Gaussian r=7 has 8 half taps (flow/conv.rs:64-86
 struct Taps {
     float k[MAX_TAPS];
     int n;
+    float z;  // -0.0, the addend of the packed products (level.cuh)
 };
 // the half kernels of the matte choke's blur (matte.rs:366-385: radius a + 2.01 for a shrink of a
 // pixels, n = a + 3 taps for a whole a); shrinks up to 13 pixels
@@ -65,42 +67,19 @@ __global__ void k_conv_v_sphere(const float* __restrict__ src, float* __restrict
 __global__ void k_resample_sphere(const float* __restrict__ src, int sw, int sh, float* __restrict__ dst, int dw, int dh);
 
 // ---- solver (flow.rs:277-442) ------------------------------------------------------------------------
-// gradient (2 planes) and structure tensor (3 planes)
-__global__ void k_grad_tensor(const float* __restrict__ img, int w, int h, float* __restrict__ gx,
-                              float* __restrict__ gy, float* __restrict__ a0, float* __restrict__ a1,
-                              float* __restrict__ a2);
-__global__ void k_calc_b(const float* __restrict__ i1, const float* __restrict__ i0, const float* __restrict__ gx,
-                         const float* __restrict__ gy, const float* __restrict__ fu, const float* __restrict__ fv,
-                         int w, int h, float* __restrict__ bx, float* __restrict__ by);
-__global__ void k_new_disp(float* __restrict__ fu, float* __restrict__ fv, const float* __restrict__ a0,
-                           const float* __restrict__ a1, const float* __restrict__ a2, const float* __restrict__ bx,
-                           const float* __restrict__ by, long n);
 // sets *any_in_range when some pixel's x + u, y + v lies inside the level (flow.rs:430-442)
-__global__ void k_range_any(const float* __restrict__ fu, const float* __restrict__ fv, int w, int h,
-                            int* __restrict__ any_in_range);
-// the range reset while the check is live, then the damping of the start level (flow.rs:1292-1300)
-__global__ void k_range_apply(float* __restrict__ fu, float* __restrict__ fv, long n, int* __restrict__ state,
-                              bool damp_now, float damp);
-__global__ void k_range_init(int* __restrict__ state);
-__global__ void k_range_next(int* __restrict__ state);
-__global__ void k_upsample_flow(const float* __restrict__ su, const float* __restrict__ sv, int sw, int sh,
-                                float* __restrict__ du, float* __restrict__ dv, int dw, int dh);
-// the final negation (flow.rs:1305) into the interleaved FlowField layout
-__global__ void k_negate_interleave(const float* __restrict__ fu, const float* __restrict__ fv, long n,
-                                    float* __restrict__ out, int* __restrict__ nan_flag);
-__global__ void k_fill(float* __restrict__ p, long n, float v);
+__global__ void k_range_any(const float2* __restrict__ f, int w, int h, int* __restrict__ any_in_range);
 __global__ void k_deinterleave(const float* __restrict__ in, long n, float* __restrict__ fu, float* __restrict__ fv);
-__global__ void k_interleave(const float* __restrict__ fu, const float* __restrict__ fv, long n, float* __restrict__ out);
 
 // block matching (flow.rs:447-622): the four sweeps; one CTA per row or column, bm_smem_bytes(line)
-// shared. k_bm_rows: both sweeps of every row (left to right, then right to left) of (fu, fv), the
-// result written into the transposes (uT, vT; element (x, y) at [x * h + y]); k_bm_cols: both
-// sweeps of every column (top to bottom, then bottom to top) read from (uT, vT), with the
-// transposes of A and B, the result written back into (fu, fv). Lines 0 and last are not swept.
-__global__ void k_bm_rows(const float* __restrict__ A, const float* __restrict__ B, const float* __restrict__ fu,
-                          const float* __restrict__ fv, int w, int h, float* __restrict__ uT, float* __restrict__ vT);
-__global__ void k_bm_cols(const float* __restrict__ AT, const float* __restrict__ BT, const float* __restrict__ uT,
-                          const float* __restrict__ vT, int w, int h, float* fu, float* fv);
+// shared. k_bm_rows: both sweeps of every row (left to right, then right to left) of f, the result
+// written into the transpose ft (element (x, y) at [x * h + y]); k_bm_cols: both sweeps of every
+// column (top to bottom, then bottom to top) read from ft, with the transposes of A and B, the result
+// written back into f. Lines 0 and last are not swept.
+__global__ void k_bm_rows(const float* __restrict__ A, const float* __restrict__ B, const float2* __restrict__ f, int w,
+                          int h, float2* __restrict__ ft);
+__global__ void k_bm_cols(const float* __restrict__ AT, const float* __restrict__ BT, const float2* __restrict__ ft, int w,
+                          int h, float2* f);
 // two w x h planes into their h x w transposes; block (32, 8), grid (ceil(w/32), ceil(h/32))
 __global__ void k_transpose2(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ at,
                              float* __restrict__ bt, int w, int h);
@@ -145,40 +124,72 @@ constexpr int FUSED_TILE_X = 32, FUSED_TILE_Y = 32, FUSED_THREADS = 256;
 __global__ void k_blur5_band(const float* __restrict__ orig, const void* __restrict__ luma_src, int fmt, int luma_mode,
                              int w, int h, bool above_first, float* __restrict__ tmp_out, float* __restrict__ band_out,
                              float* __restrict__ band_t_out);
-__global__ void k_level_init(const float* __restrict__ img, int w, int h, Taps g7, bool above_first,
-                             float* __restrict__ gxo, float* __restrict__ gyo, float* __restrict__ a0o,
-                             float* __restrict__ a1o, float* __restrict__ a2o, const float* __restrict__ mask,
-                             const float* __restrict__ fu, const float* __restrict__ fv, const float* __restrict__ i0,
-                             const float* __restrict__ mask_y, float* __restrict__ b_out, int bp, long bplane);
-__global__ void k_calc_b_pitched(const float* __restrict__ i1, const float* __restrict__ i0,
-                                 const float* __restrict__ gx, const float* __restrict__ gy,
-                                 const float* __restrict__ fu, const float* __restrict__ fv, int w, int h,
-                                 const float* __restrict__ mask_y, float* __restrict__ b_out, int bp, long bplane);
-__global__ void k_binarize(float* __restrict__ p, long n);
-size_t level_init_smem();
+// The launch shapes of the level kernels. The public codes of the iteration's tiles are the first three
+// (tw_tuning_set); the last two are shapes the defaults and the autotuner choose.
+enum { LEVEL_TILE_32x32 = 0, LEVEL_TILE_64x32 = 1, LEVEL_TILE_64x64 = 2, LEVEL_TILE_COUNT = 3, LEVEL_TILE_16x16 = 3,
+       LEVEL_TILE_32x64 = 4 };
+constexpr int LEVEL_ITER_MAX_THREADS = 512, LEVEL_INIT_MAX_THREADS = 512;
+
+// The scales of an upsample (level.cuh, upsample_scale)
+struct UpsampleScale {
+    float sx, sy, rx, ry;
+};
+
+// The start of a level over TX x TY tiles: with src the flow of the level upsampled from the coarser
+// one (sw x sh, level l + 1, its reset and damping on the way) into f, else f as it is; the gradient of
+// img, masked by mask_x (may be null); calc_b of the first iteration from f, i0 and mask_y (may be null)
+// into b_out (pitch bp, even); the blurred tensor and the determinant of new_disp.
+struct LevelInitArgs {
+    const float* img;
+    const float* i0;
+    const float* mask_x;
+    const float* mask_y;
+    const float2* src;
+    const int* any;
+    float2* f;
+    float2* grad;
+    float4* tensor;
+    float2* b_out;
+    int w, h, bp, sw, sh, l, start;
+    UpsampleScale up;
+    float damp;
+    int damp_now, af;
+    Taps g7;
+};
+__global__ void k_level_init_16x16(const __grid_constant__ LevelInitArgs P);
+__global__ void k_level_init_32x32(const __grid_constant__ LevelInitArgs P);
+size_t level_init_smem(int tile);
+
 // One solver iteration (blur7 of B, new_disp, blur5 of the flow, then calc_b of the next iteration
-// at its outputs when b_out is given) over TX x TY tiles: one kernel per tile shape; the host picks
-// the shape per level size (its tuning table). B planes: pitch bp (a multiple of 4 floats), plane
-// stride bplane, 16-byte aligned.
-enum { LEVEL_TILE_32x32 = 0, LEVEL_TILE_64x32 = 1, LEVEL_TILE_64x64 = 2, LEVEL_TILE_COUNT = 3 };
-constexpr int LEVEL_ITER_MAX_THREADS = 512;
-#define TW_DECLARE_LEVEL_ITER(TX, TY)                                                                                 \
-    __global__ void k_level_iter_##TX##x##TY(                                                                       \
-        const float* __restrict__ b_in, int bp, long bplane, const float* __restrict__ i1,                          \
-        const float* __restrict__ i0, const float* __restrict__ gx, const float* __restrict__ gy,                    \
-        const float* __restrict__ a0, const float* __restrict__ a1, const float* __restrict__ a2,                    \
-        const float* __restrict__ fu, const float* __restrict__ fv, int w, int h, Taps g7, Taps g5,                  \
-        bool above_first, float* __restrict__ fu_out, float* __restrict__ fv_out, const float* __restrict__ mask_y,  \
-        float* __restrict__ b_out);
-TW_DECLARE_LEVEL_ITER(32, 32)
-TW_DECLARE_LEVEL_ITER(64, 32)
-TW_DECLARE_LEVEL_ITER(64, 64)
-#undef TW_DECLARE_LEVEL_ITER
+// at its outputs when b_out is given) over TX x TY tiles: one kernel per tile shape. The B planes hold
+// both components of a pixel, pitch bp (even), 16-byte aligned.
+struct LevelIterArgs {
+    const float2* b_in;
+    const float* i1;
+    const float* i0;
+    const float2* grad;
+    const float4* tensor;
+    const float2* f;
+    const float* mask_y;
+    float2* f_out;
+    float2* b_out;
+    int w, h, bp, af;
+    Taps g7, g5;
+};
+__global__ void k_level_iter_16x16(const __grid_constant__ LevelIterArgs P);
+__global__ void k_level_iter_32x32(const __grid_constant__ LevelIterArgs P);
+__global__ void k_level_iter_32x64(const __grid_constant__ LevelIterArgs P);
+__global__ void k_level_iter_64x32(const __grid_constant__ LevelIterArgs P);
+__global__ void k_level_iter_64x64(const __grid_constant__ LevelIterArgs P);
 size_t level_iter_smem(int tile);
+__global__ void k_calc_b_pitched(const float* __restrict__ i1, const float* __restrict__ i0,
+                                 const float2* __restrict__ grad, const float2* __restrict__ f, int w, int h,
+                                 const float* __restrict__ mask_y, float2* __restrict__ b_out, int bp);
+__global__ void k_binarize(float* __restrict__ p, long n);
 
 // The persistent coarse-level solve (coarse.cu): one block walks the levels start .. last of a solve
 // whose planes fit its shared memory (at most COARSE_MAX_PIXELS pixels and COARSE_MAX_LINE per side;
-// last >= 1), and writes the upsampled flow of level last - 1 (planar) for the tiled kernels.
+// last >= 1), and writes the upsampled flow of level last - 1 for the tiled kernels.
 constexpr int COARSE_THREADS = 1024;
 constexpr int COARSE_MAX_PIXELS = 2048;
 constexpr int COARSE_MAX_LINE = 128;
@@ -194,17 +205,15 @@ struct CoarseJob {
     bool af;      // the vertical tap above first
     Taps g7, g5;
     int* any;  // the per level range flags (32 ints, zeroed before)
-    float* fu_out;
-    float* fv_out;
+    float2* f_out;
 };
 __global__ void k_solve_coarse(CoarseJob job);
 size_t coarse_smem_bytes();
-__global__ void k_apply_upsample(const float* __restrict__ su, const float* __restrict__ sv, int sw, int sh,
+__global__ void k_apply_upsample(const float2* __restrict__ src, int sw, int sh, UpsampleScale up,
                                  const int* __restrict__ any, int l, int start, bool damp_now, float damp,
-                                 float* __restrict__ du, float* __restrict__ dv, int dw, int dh);
-__global__ void k_apply_negate(const float* __restrict__ fu, const float* __restrict__ fv, long n,
-                               const int* __restrict__ any, int start, bool damp_now, float damp,
-                               float* __restrict__ out, int* __restrict__ nan_flag);
+                                 float2* __restrict__ dst, int dw, int dh);
+__global__ void k_apply_negate(const float2* __restrict__ f, long n, const int* __restrict__ any, int start,
+                               bool damp_now, float damp, float2* __restrict__ out, int* __restrict__ nan_flag);
 
 // ---- warping code 1: Smart Blend and the hole fill (smart.cu) -----------------------------------------
 // mode 0: Nearest (the warp pa only), 1: Blend (pa = A, pb = B, w = frac); binary: the binary alpha
@@ -284,8 +293,8 @@ __global__ void k_user_splat(UserPairs pairs, int w0, int h0, int W, int H, floa
                              float* __restrict__ dv, float* __restrict__ uw);
 __global__ void k_user_finest(float* __restrict__ du, float* __restrict__ dv, float* __restrict__ uw, long n);
 __global__ void k_user_scale(float* __restrict__ du, float* __restrict__ dv, long n, float sx, float sy);
-__global__ void k_apply_user(float* __restrict__ fu, float* __restrict__ fv, const float* __restrict__ du,
-                             const float* __restrict__ dv, const float* __restrict__ uw, long n);
+__global__ void k_apply_user(float2* __restrict__ f, const float* __restrict__ du, const float* __restrict__ dv,
+                             const float* __restrict__ uw, long n);
 __global__ void k_solver_mask(const float* __restrict__ raws, int nfg, int k, const float* __restrict__ comp, long n,
                               int fmt, float* __restrict__ out);
 __global__ void k_layer_times(const void* __restrict__ src, const float* __restrict__ p, void* __restrict__ out, int fmt,

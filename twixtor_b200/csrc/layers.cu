@@ -371,15 +371,12 @@ __global__ void k_user_scale(float* __restrict__ du, float* __restrict__ dv, lon
 }
 
 // flow/extras.rs:181-194 (apply_user): flow = d / w where w != 0
-__global__ void k_apply_user(float* __restrict__ fu, float* __restrict__ fv, const float* __restrict__ du,
-                             const float* __restrict__ dv, const float* __restrict__ uw, long n) {
+__global__ void k_apply_user(float2* __restrict__ f, const float* __restrict__ du, const float* __restrict__ dv,
+                             const float* __restrict__ uw, long n) {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float k = uw[i];
-    if (k != 0.0f) {
-        fu[i] = du[i] / k;
-        fv[i] = dv[i] / k;
-    }
+    if (k != 0.0f) f[i] = make_float2(du[i] / k, dv[i] / k);
 }
 
 }  // namespace tw

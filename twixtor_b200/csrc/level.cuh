@@ -8,6 +8,73 @@
 
 namespace tw {
 
+// ---- packed pairs ------------------------------------------------------------------------------------
+// The two channels of B and of the flow (and two of the tensor's three) travel as float2 through the
+// separable passes: one packed instruction rounds both lanes as the scalar one does, so the bits are
+// the same for half the issue slots (the FP32 pipe takes a packed operation in two cycles: 127 scalar
+// results per clock and SM either way, measured).
+//
+// The assembler contracts a packed multiply and a packed add into one fused operation whatever
+// -fmad=false and the .rn say (measured: every one of a million sums differed). So a product is
+// written as a * k + z with z = -0.0, which rounds exactly as the product does, zeros and their signs
+// included, and z is a value the compiler cannot know: it comes with the kernel's parameters (Taps::z).
+__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 vmul(float2 a, float k, float z) {
+    return __ffma2_rn(a, make_float2(k, k), make_float2(z, z));
+}
+__device__ __forceinline__ float2 vmadd(float2 s, float2 a, float k, float z) {  // s + a * k
+#ifdef TW_FAST_VARIANT
+    return __ffma2_rn(a, make_float2(k, k), s);
+#else
+    return __fadd2_rn(s, vmul(a, k, z));
+#endif
+}
+__device__ __forceinline__ float vadd(float a, float b) { return a + b; }
+__device__ __forceinline__ float vmul(float a, float k, float) { return a * k; }
+__device__ __forceinline__ float vmadd(float s, float a, float k, float) { return s + a * k; }
+// a / d for a weight sum d (0.05 < d <= 1) and y = 1 / d, both correctly rounded: Markstein's division by
+// a known reciprocal (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990): q1 = a y corrected by its exact remainder is faithful, and a second correction by the
+// exact remainder of q1 rounds it correctly. Two lanes share each step. A zero keeps its sign; an
+// operand too near the range's ends for the exact remainders shows in `seen` (its magnitudes' largest and
+// smallest but zero), and the caller redoes it by the division. (A division here, even one that is
+// never taken, holds up the zero filled rows outside the image in its slow path: 7000 cycles for the
+// border rows of a tile, 3100 without.)
+struct Magnitudes {
+    float hi = 0.0f, lo = 1.0f;
+    __device__ __forceinline__ bool safe() const { return hi < 1e30f && lo > 1e-30f; }
+};
+__device__ __forceinline__ float quot1(float a, float q, Magnitudes& seen) {
+    seen.hi = fmaxf(seen.hi, fabsf(a));
+    seen.lo = fminf(seen.lo, a == 0.0f ? 1.0f : fabsf(a));
+    return a == 0.0f ? a : q;
+}
+__device__ __forceinline__ float2 vquot(float2 a, float2 dy, Magnitudes& seen) {
+    const float2 n = make_float2(-dy.x, -dy.x), y = make_float2(dy.y, dy.y);
+    float2 q = __ffma2_rn(a, y, make_float2(0.0f, 0.0f));
+    q = __ffma2_rn(__ffma2_rn(q, n, a), y, q);
+    q = __ffma2_rn(__ffma2_rn(q, n, a), y, q);
+    return make_float2(quot1(a.x, q.x, seen), quot1(a.y, q.y, seen));
+}
+__device__ __forceinline__ float vquot(float a, float2 dy, Magnitudes& seen) {
+    float q = a * dy.y;
+    q = __fmaf_rn(__fmaf_rn(q, -dy.x, a), dy.y, q);
+    q = __fmaf_rn(__fmaf_rn(q, -dy.x, a), dy.y, q);
+    return quot1(a, q, seen);
+}
+// how far the nearest sample is from the sentinel -1.0 of the border rule (0: it is the sentinel)
+__device__ __forceinline__ float from_sentinel(float2 v, float m) {
+    const float2 d = __fadd2_rn(v, make_float2(1.0f, 1.0f));
+    return fminf(fminf(m, fabsf(d.x)), fabsf(d.y));
+}
+__device__ __forceinline__ float from_sentinel(float v, float m) { return fminf(m, fabsf(v + 1.0f)); }
+template <class V>
+__device__ __forceinline__ V outside_value();  // -0.0: adding it times a tap changes no sum, not even a zero's sign
+template <>
+__device__ __forceinline__ float2 outside_value<float2>() { return make_float2(-0.0f, -0.0f); }
+template <>
+__device__ __forceinline__ float outside_value<float>() { return -0.0f; }
+
 // ---- separable pass elements ---------------------------------------------------------------------
 
 // flow/conv.rs:101-137 on a line held in shared memory: element t of the line (global index, inside
@@ -54,6 +121,115 @@ __device__ __forceinline__ float pass_elem(const float* line, int origin, int st
         return s;
     }
     return border_sm<N, MULTI, LEFT_FIRST>(line, origin, stride, len, i, k);
+}
+
+// The weight sum of the border rule at line index i (conv.rs:101-137) when no sample is the sentinel:
+// it depends on the position alone; with its reciprocal. 1 for the interior outputs, which are not
+// divided.
+template <int N>
+__device__ __forceinline__ float2 border_den(int i, int len, const float* k) {
+    if (i >= N && i < len - N) return make_float2(1.0f, 1.0f);
+    float den = k[0];
+#pragma unroll
+    for (int j = N - 1; j >= 1; j--) {
+        if (i + j >= 0 && i + j < len) den = den + k[j];
+        if (i - j >= 0 && i - j < len) den = den + k[j];
+    }
+    return make_float2(den, __frcp_rn(den));
+}
+
+// One element by the general rule, per channel, out of the main path: the multi channel rule drops
+// real samples of exactly -1.0, which run_pass sends here. line: line index `origin` at line[0].
+template <int N, bool LEFT_FIRST>
+__device__ __noinline__ float slow_elem(const float* line, int origin, int stride, int len, int i, const float* k) {
+    return pass_elem<N, true, LEFT_FIRST>(line, origin, stride, len, i, k);
+}
+template <int N, bool LEFT_FIRST>
+__device__ __forceinline__ float slow_pass(const float* line, int origin, int stride, int len, int i, const float* k) {
+    return slow_elem<N, LEFT_FIRST>(line, origin, stride, len, i, k);
+}
+template <int N, bool LEFT_FIRST>
+__device__ __forceinline__ float2 slow_pass(const float2* line, int origin, int stride, int len, int i, const float* k) {
+    const float* f = reinterpret_cast<const float*>(line);
+    return make_float2(slow_elem<N, LEFT_FIRST>(f, origin, 2 * stride, len, i, k),
+                       slow_elem<N, LEFT_FIRST>(f + 1, origin, 2 * stride, len, i, k));
+}
+
+// R consecutive outputs of a multi channel pass (conv.rs:141-190 / :268-301) at line indices i0 ..
+// i0 + R - 1, from the R + 2N - 2 samples base[0], base[stride], ... (line indices i0 - (N - 1) on),
+// each read once. Samples outside the line hold outside_value, so a border output is the plain chain
+// of its taps, one side after the other, over the position's weight sum (den[r], border_den of output
+// r): no per tap tests. Returns true, with res undefined, for the rare run near the line's ends that
+// needs the general rule: a window that holds the sentinel -1.0, or a sum that vquot does not divide; the
+// caller then runs slow_run. Outputs outside the line come out as garbage that nobody reads.
+template <int N, int R, bool LEFT_FIRST, class V>
+__device__ __forceinline__ bool run_pass(const V* base, int stride, int i0, int len, const Taps& t, const float2* den,
+                                         V* res) {
+    constexpr int NV = R + 2 * N - 2;
+    V v[NV];
+#pragma unroll
+    for (int j = 0; j < NV; j++) v[j] = base[j * stride];
+    if (i0 >= N && i0 + R - 1 < len - N) {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            V s = vmul(v[r + N - 1], t.k[0], t.z);
+#pragma unroll
+            for (int j = N - 1; j >= 1; j--) s = vmadd(s, vadd(v[r + N - 1 + j], v[r + N - 1 - j]), t.k[j], t.z);
+            res[r] = s;
+        }
+        return false;
+    }
+    // a run that touches the line's ends: both rules for every output and a select, so that the R chains
+    // stay independent (an interior output's weight sum is 1, and a value over 1 is the value)
+    Magnitudes seen;
+    float nearest = 1.0f;
+#pragma unroll
+    for (int j = 0; j < NV; j++) nearest = from_sentinel(v[j], nearest);
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int i = i0 + r;
+        V s = vmul(v[r + N - 1], t.k[0], t.z), e = s;
+#pragma unroll
+        for (int j = N - 1; j >= 1; j--) {
+            s = vmadd(s, vadd(v[r + N - 1 + j], v[r + N - 1 - j]), t.k[j], t.z);
+            e = vmadd(e, LEFT_FIRST ? v[r + N - 1 - j] : v[r + N - 1 + j], t.k[j], t.z);
+            e = vmadd(e, LEFT_FIRST ? v[r + N - 1 + j] : v[r + N - 1 - j], t.k[j], t.z);
+        }
+        const bool inner = i >= N && i < len - N;
+        const V q = vquot(e, den[r], seen);
+        res[r] = inner ? s : q;
+    }
+    return nearest == 0.0f || !seen.safe();
+}
+
+// The same outputs by the general rule, one element after the other.
+template <int N, int R, bool LEFT_FIRST, class V>
+__device__ __forceinline__ void slow_run(const V* base, int stride, int i0, int len, const Taps& t, V* res) {
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int i = i0 + r;
+        res[r] = outside_value<V>();
+        if (i >= 0 && i < len) res[r] = slow_pass<N, LEFT_FIRST>(base, i0 - (N - 1), stride, len, i, t.k);
+    }
+}
+
+// run_pass, or with SLOW slow_run, for a pass along the rows or the columns (`above_first`: the tap above
+// first).
+template <bool SLOW, int N, int R, class V>
+__device__ __forceinline__ bool h_pass(const V* base, int i0, int len, const Taps& t, const float2* den, V* res) {
+    if (!SLOW) return run_pass<N, R, false>(base, 1, i0, len, t, den, res);
+    slow_run<N, R, false>(base, 1, i0, len, t, res);
+    return false;
+}
+template <bool SLOW, int N, int R, class V>
+__device__ __forceinline__ bool v_pass(const V* base, int stride, int i0, int len, const Taps& t, const float2* den,
+                                       bool above_first, V* res) {
+    if (!SLOW)
+        return above_first ? run_pass<N, R, true>(base, stride, i0, len, t, den, res)
+                           : run_pass<N, R, false>(base, stride, i0, len, t, den, res);
+    if (above_first) slow_run<N, R, true>(base, stride, i0, len, t, res);
+    else slow_run<N, R, false>(base, stride, i0, len, t, res);
+    return false;
 }
 
 // flow.rs:474-523 (Block::cost). B(X, Y) is B[Y * w + X] for a row-major plane (COLS false) and
@@ -106,20 +282,50 @@ __device__ __forceinline__ bool bm_cost(const float* __restrict__ B, int w, int 
     return true;
 }
 
-// flow.rs:334-357 (calc_b) at pixel (x, y) whose flow is (u, v): B = (I0(x - u, y - v) - I1) * grad,
-// zero where the source point leaves the level, and in a layered solve (mask_y) where the warped
-// mask of Y is below 0.999 (flow.rs:777-845). i1v, gxv, gyv: I1 and the gradient at the pixel.
-__device__ __forceinline__ void calc_b_at(const float* __restrict__ i0, const float* __restrict__ mask_y, int w, int h,
-                                          int x, int y, float u, float v, float i1v, float gxv, float gyv, float& b0,
-                                          float& b1) {
-    const float sx = (float)x - u, sy = (float)y - v;
-    b0 = 0.0f;
-    b1 = 0.0f;
-    if (!(sx < 0.0f || (float)w - 1.0f < sx || sy < 0.0f || (float)h - 1.0f < sy) &&
-        (!mask_y || bilinear1(mask_y, w, h, sx, sy) >= 0.999f)) {
-        const float rr = bilinear1(i0, w, h, sx, sy) - i1v;
-        b0 = rr * gxv;
-        b1 = rr * gyv;
+// sample.rs:31-41 for a coordinate known to lie in [0, len - 1] (or a NaN): the conversion needs no range
+// test and the cell no lower clamp (a NaN gives cell 0 and a NaN fraction, as the general rule does)
+__device__ __forceinline__ void cell_inside(float x, int len, int& io, float& fo) {
+    int i = __float2int_rz(x);
+    float f = x - (float)i;
+    if (i >= len - 1) { i = len - 2; f = 1.0f; }
+    io = i;
+    fo = f;
+}
+
+// flow.rs:334-357 (calc_b) at R pixels (x, y + r) whose flow is f[r]: B = (I0(x - u, y - v) - I1) * grad,
+// zero where the source point leaves the level, and in a layered solve (mask_y) where the warped mask of
+// Y is below 0.999 (flow.rs:777-845). i1, g: I1 and the gradient at the pixels. Levels are at least 2 x
+// 2. The gathers of all R pixels are in flight together (a point outside reads pixel 0).
+template <int R>
+__device__ __forceinline__ void calc_b_run(const float* __restrict__ i0, const float* __restrict__ mask_y, int w, int h, int x,
+                                           int y, const float2* f, const float* i1, const float2* g, float2* b) {
+    bool in[R];
+    int at[R];
+    float fx[R], fy[R], p[R][4];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const float sx = (float)x - f[r].x, sy = (float)(y + r) - f[r].y;
+        in[r] = !(sx < 0.0f || (float)w - 1.0f < sx || sy < 0.0f || (float)h - 1.0f < sy);
+        if (in[r] && mask_y) in[r] = bilinear1(mask_y, w, h, sx, sy) >= 0.999f;
+        int ix, iy;
+        cell_inside(sx, w, ix, fx[r]);
+        cell_inside(sy, h, iy, fy[r]);
+        at[r] = in[r] ? iy * w + ix : 0;
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const float* q = i0 + at[r];
+        p[r][0] = __ldg(q);
+        p[r][1] = __ldg(q + 1);
+        p[r][2] = __ldg(q + w);
+        p[r][3] = __ldg(q + w + 1);
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const float top = (p[r][1] - p[r][0]) * fx[r] + p[r][0];
+        const float bot = (p[r][3] - p[r][2]) * fx[r] + p[r][2];
+        const float rr = ((bot - top) * fy[r] + top) - i1[r];
+        b[r] = in[r] ? make_float2(rr * g[r].x, rr * g[r].y) : make_float2(0.0f, 0.0f);
     }
 }
 
@@ -131,39 +337,45 @@ __device__ __forceinline__ bool zero_at_level(const int* any, int l, int start) 
     return check && any[l] == 0;
 }
 
-// flow.rs:376-391 (upsample_flow, bilinear2 of sample.rs:69-86) at output pixel (x, y) of dw x dh:
-// the coarse field su / sv of sw x sh with the reset (zero) and the damping of its level applied to
-// the four gathered samples, which is the same as applying them to the whole field first.
-__device__ __forceinline__ void upsample_at(const float* su, const float* sv, int sw, int sh, bool zero,
-                                            bool damp_now, float damp, int x, int y, int dw, int dh, float* u,
-                                            float* v) {
-    float sx = ((float)dw - 1.0f) / (float)(sw - 1);
-    float sy = ((float)dh - 1.0f) / (float)(sh - 1);
-    float rx = (float)(1.0 / (double)sx);
-    float ry = (float)(1.0 / (double)sy);
+// flow.rs:376-391 (upsample_flow, bilinear2 of sample.rs:69-86) from a field of sw x sh to one of dw x
+// dh: the scales sx, sy and their reciprocals, formed once on the host (the same IEEE operations).
+__host__ __device__ inline UpsampleScale upsample_scale(int sw, int sh, int dw, int dh) {
+    UpsampleScale u;
+    u.sx = ((float)dw - 1.0f) / (float)(sw - 1);
+    u.sy = ((float)dh - 1.0f) / (float)(sh - 1);
+    u.rx = (float)(1.0 / (double)u.sx);
+    u.ry = (float)(1.0 / (double)u.sy);
+    return u;
+}
+
+// The upsampled flow at output pixel (x, y), with the reset (zero) and the damping of the coarse
+// field's level applied to the four gathered samples, which is the same as applying them to the whole
+// field first.
+__device__ __forceinline__ float2 upsample_at(const float2* src, int sw, int sh, const UpsampleScale& c, bool zero,
+                                              bool damp_now, float damp, int x, int y) {
     int ix, iy;
     float fx, fy;
-    cell((float)x * rx, sw, ix, fx);
-    cell((float)y * ry, sh, iy, fy);
-    int i = iy * sw + ix;
-    const float* planes[2] = {su, sv};
-    float r[2];
+    cell((float)x * c.rx, sw, ix, fx);
+    cell((float)y * c.ry, sh, iy, fy);
+    const int i = iy * sw + ix;
+    float2 q[4] = {src[i], src[i + 1], src[i + sw], src[i + sw + 1]};
 #pragma unroll
-    for (int c = 0; c < 2; c++) {
-        const float* p = planes[c];
-        float q[4] = {p[i], p[i + 1], p[i + sw], p[i + sw + 1]};
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            float t = zero ? 0.0f : q[m];
-            if (damp_now) t = damp * t;
-            q[m] = t;
-        }
-        float top = (q[1] - q[0]) * fx + q[0];
-        float bot = (q[3] - q[2]) * fx + q[2];
-        r[c] = (bot - top) * fy + top;
+    for (int m = 0; m < 4; m++) {
+        if (zero) q[m] = make_float2(0.0f, 0.0f);
+        if (damp_now) q[m] = make_float2(damp * q[m].x, damp * q[m].y);
     }
-    *u = r[0] * sx;
-    *v = r[1] * sy;
+    float2 r;
+    {
+        float top = (q[1].x - q[0].x) * fx + q[0].x;
+        float bot = (q[3].x - q[2].x) * fx + q[2].x;
+        r.x = ((bot - top) * fy + top) * c.sx;
+    }
+    {
+        float top = (q[1].y - q[0].y) * fx + q[0].y;
+        float bot = (q[3].y - q[2].y) * fx + q[2].y;
+        r.y = ((bot - top) * fy + top) * c.sy;
+    }
+    return r;
 }
 
 }  // namespace tw

@@ -5,8 +5,7 @@
 // real-time render thread where a driver allocation can stall or is forbidden. They can still pass
 // their own device buffers for the inputs and the output. This entry point runs the four block
 // matching sweeps (flow.rs:551-622) on such buffers without allocating anything: its only scratch
-// (the field split into two float planes, the transposes of the two images and of the field for
-// the column sweeps) lives in the file-scope device array below, which every GPU that loads the
+// (a copy of the field, the transposes of the two images and of the field for the column sweeps) lives in the file-scope device array below, which every GPU that loads the
 // library holds until the process exits.
 #include <cuda_runtime.h>
 
@@ -15,8 +14,8 @@
 
 namespace {
 
-// Scratch of the allocation-free block matching: the u and v planes of the field, the transposes
-// of A and B, and the transposed field of the column sweeps (6 planes).
+// Scratch of the allocation-free block matching: the transposes of A and B, the field and its
+// transpose (6 planes).
 constexpr long NOALLOC_MAX_PIXELS = TW_NOALLOC_MAX_PIXELS;
 static __device__ __align__(256) float g_noalloc_planes[6 * NOALLOC_MAX_PIXELS];
 
@@ -35,6 +34,11 @@ int setup(float** planes) {
         return TW_ERR_CUDA;
     *planes = (float*)p;
     return TW_OK;
+}
+
+__global__ void k_copy_floats(const float* __restrict__ in, float* __restrict__ out, long n) {
+    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = in[i];
 }
 
 // One launch through cudaLaunchKernel, whose return code is this launch's own: an error that the
@@ -57,30 +61,26 @@ extern "C" int tw_block_match_noalloc(const float* a, const float* b, float* flo
     if (rc != TW_OK) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     long n = (long)width * height;
-    float* fu = planes;
-    float* fv = fu + n;
-    float *at = fv + n, *bt = at + n, *ut = bt + n, *vt = ut + n;
+    float *at = planes, *bt = at + n;
+    float2 *ft = (float2*)(bt + n), *f = ft + n;
     const int tb = 256;
-    dim3 g1((unsigned)((n + tb - 1) / tb));
     dim3 tt(32, 8), ga((width + 31) / 32, (height + 31) / 32);
-    const float* cfu = fu;
-    const float* cfv = fv;
-    const float* cut = ut;
-    const float* cvt = vt;
     // every element of the planes this call reads is written first, so the previous call's
-    // contents never reach the result
-    cudaError_t e = launch(tw::k_deinterleave, g1, dim3(tb), 0, s, (const float*)flow, n, fu, fv);
+    // contents never reach the result. The field is swept in a copy: the caller's pointer need not be
+    // aligned to a pair.
+    dim3 g2((unsigned)((2 * n + tb - 1) / tb));
+    cudaError_t e = launch(k_copy_floats, g2, dim3(tb), 0, s, (const float*)flow, (float*)f, 2 * n);
     if (e == cudaSuccess && width >= 3 && height >= 3) {
-        // the row sweeps write the transposed field (ut, vt), the column sweeps read it with the
-        // transposes of A and B and write the result back into (fu, fv)
-        e = launch(tw::k_bm_rows, dim3(height - 2), dim3(tb), tw::bm_smem_bytes(width), s, a, b, cfu, cfv, (int)width,
-                   (int)height, ut, vt);
+        // the row sweeps write the transposed field ft, the column sweeps read it with the transposes of
+        // A and B and write the result back into f
+        e = launch(tw::k_bm_rows, dim3(height - 2), dim3(tb), tw::bm_smem_bytes(width), s, a, b, (const float2*)f, (int)width,
+                   (int)height, ft);
         if (e == cudaSuccess) e = launch(tw::k_transpose2, ga, tt, 0, s, a, b, at, bt, (int)width, (int)height);
         if (e == cudaSuccess)
             e = launch(tw::k_bm_cols, dim3(width - 2), dim3(tb), tw::bm_smem_bytes(height), s, (const float*)at,
-                       (const float*)bt, cut, cvt, (int)width, (int)height, fu, fv);
+                       (const float*)bt, (const float2*)ft, (int)width, (int)height, f);
     }
-    if (e == cudaSuccess) e = launch(tw::k_interleave, g1, dim3(tb), 0, s, cfu, cfv, n, flow);
+    if (e == cudaSuccess) e = launch(k_copy_floats, g2, dim3(tb), 0, s, (const float*)f, flow, 2 * n);
     if (e != cudaSuccess) return TW_ERR_CUDA;
     if (cudaStreamSynchronize(s) != cudaSuccess) return TW_ERR_CUDA;
     return TW_OK;

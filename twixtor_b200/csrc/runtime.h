@@ -313,12 +313,9 @@ __global__ void k_set_flag(int* flags, int idx);  // flags[idx] = 1 (the injecte
 // host_solve.cu
 LevelTune level_tune(tw_ctx* ctx, int w, int h);
 LevelTune default_tune(int w, int h);
-void block_match(tw_ctx* ctx, const float* A, const float* B, const float* AT, const float* BT, float* fu, float* fv,
-                 float* uT, float* vT, int w, int h, bool fast = false);
-void level_iter(tw_ctx* ctx, LevelTune ic, const float* A, const float* B, const float* gx, const float* gy,
-                const float* a0, const float* a1, const float* a2, const float* fu, const float* fv, int w, int h, bool af,
-                float* nu, float* nv, const float* mask_y, bool fast, const float* b_in, float* b_out, int bp,
-                long bplane);
+void block_match(tw_ctx* ctx, const float* A, const float* B, const float* AT, const float* BT, float2* f, float2* ft, int w,
+                 int h, bool fast = false);
+void level_iter(tw_ctx* ctx, LevelTune ic, const LevelIterArgs& P, bool fast);
 size_t pyramid_floats(const Geo& g);
 int build_pyramid_dev(tw_ctx* ctx, const void* eng_dev, int W, int H, int fmt, const tw_flow_settings& s, const Geo& g,
                       float* out, float* out_t, DevBuf* scratch);

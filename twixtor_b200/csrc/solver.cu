@@ -203,152 +203,19 @@ __global__ void k_resample(const float* __restrict__ src, int sw, int sh, float*
     dst[(long)y * dw + x] = bilinear1(src, sw, sh, (float)x * sx, (float)y * sy);
 }
 
-// flow.rs:283-328 (calc_grad, calc_a)
-__global__ void k_grad_tensor(const float* __restrict__ img, int w, int h, float* __restrict__ gxo,
-                              float* __restrict__ gyo, float* __restrict__ a0, float* __restrict__ a1,
-                              float* __restrict__ a2) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y;
-    if (x >= w || y >= h) return;
-    long i = (long)y * w + x;
-    float c = img[i];
-    float nx = 0.0f, dx = 0.0f, ny = 0.0f, dy = 0.0f;
-    if (x >= 1) { nx = (c - img[i - 1]) + 0.0f; dx = 1.0f; }
-    if (y >= 1) { ny = (c - img[i - w]) + 0.0f; dy = 1.0f; }
-    if (x + 1 <= w - 1) { nx = nx + (img[i + 1] - c); dx = dx + 1.0f; }
-    if (y + 1 <= h - 1) { ny = ny + (img[i + w] - c); dy = dy + 1.0f; }
-    float gx = nx / dx, gy = ny / dy;
-    gxo[i] = gx;
-    gyo[i] = gy;
-    a0[i] = gx * gx;
-    a1[i] = gx * gy;
-    a2[i] = gy * gy;
-}
-
-// flow.rs:334-357 (calc_b): i1 = imgA, i0 = imgB
-__global__ void k_calc_b(const float* __restrict__ i1, const float* __restrict__ i0, const float* __restrict__ gx,
-                         const float* __restrict__ gy, const float* __restrict__ fu, const float* __restrict__ fv,
-                         int w, int h, float* __restrict__ bx, float* __restrict__ by) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y;
-    if (x >= w || y >= h) return;
-    long i = (long)y * w + x;
-    float fw = (float)w, fh = (float)h;
-    float sx = (float)x - fu[i];
-    float sy = (float)y - fv[i];
-    if (sx < 0.0f || fw - 1.0f < sx || sy < 0.0f || fh - 1.0f < sy) {
-        bx[i] = 0.0f;
-        by[i] = 0.0f;
-    } else {
-        float s = bilinear1(i0, w, h, sx, sy);
-        float r = s - i1[i];
-        bx[i] = r * gx[i];
-        by[i] = r * gy[i];
-    }
-}
-
-// flow.rs:361-371 (new_disp)
-__global__ void k_new_disp(float* __restrict__ fu, float* __restrict__ fv, const float* __restrict__ a0,
-                           const float* __restrict__ a1, const float* __restrict__ a2, const float* __restrict__ bx,
-                           const float* __restrict__ by, long n) {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float aa = a0[i], ab = a1[i], ad = a2[i];
-    float b0 = bx[i], b1 = by[i];
-    float t = ab * ab - ad * aa;
-    if (fabsf(t) > 40.0f) {
-        fu[i] = (ab * b1 - ad * b0) / t + fu[i];
-        fv[i] = (ab * b0 - aa * b1) / t + fv[i];
-    }
-}
-
 // flow.rs:430-442 (all_flow_out_of_range), as "some pixel is in range"
-__global__ void k_range_any(const float* __restrict__ fu, const float* __restrict__ fv, int w, int h,
-                            int* __restrict__ any_in_range) {
+__global__ void k_range_any(const float2* __restrict__ f, int w, int h, int* __restrict__ any_in_range) {
     int x = blockIdx.x * blockDim.x + threadIdx.x;
     int y = blockIdx.y;
     bool in = false;
     if (x < w && y < h) {
-        long i = (long)y * w + x;
-        float px = (float)x + fu[i];
-        float py = (float)y + fv[i];
+        const float2 v = f[(long)y * w + x];
+        float px = (float)x + v.x;
+        float py = (float)y + v.y;
         float fw = (float)(w - 1), fh = (float)(h - 1);
         in = 0.0f <= px && px <= fw && 0.0f <= py && py <= fh;
     }
     if (__syncthreads_or(in) && threadIdx.x == 0) atomicOr(any_in_range, 1);
-}
-
-// flow.rs:1292-1300: state[0] = check (still live), state[1] = some pixel in range at this level
-__global__ void k_range_apply(float* __restrict__ fu, float* __restrict__ fv, long n, int* __restrict__ state,
-                              bool damp_now, float damp) {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    bool zero = state[0] != 0 && state[1] == 0;
-    float u = zero ? 0.0f : fu[i];
-    float v = zero ? 0.0f : fv[i];
-    if (damp_now) {  // scale_values (flow.rs:422-427): f * p, untouched for f == 1
-        u = damp * u;
-        v = damp * v;
-    }
-    fu[i] = u;
-    fv[i] = v;
-}
-
-// the check state of a solve: check live, nothing in range yet (flow.rs:1270)
-__global__ void k_range_init(int* __restrict__ state) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        state[0] = 1;
-        state[1] = 0;
-    }
-}
-
-// the check state after a level: check = check && nothing was in range; clears the flag for the next level
-__global__ void k_range_next(int* __restrict__ state) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        state[0] = (state[0] != 0 && state[1] == 0) ? 1 : 0;
-        state[1] = 0;
-    }
-}
-
-// flow.rs:376-391 (upsample_flow) with sample.rs:69-86 (bilinear2) on the planar field
-__global__ void k_upsample_flow(const float* __restrict__ su, const float* __restrict__ sv, int sw, int sh,
-                                float* __restrict__ du, float* __restrict__ dv, int dw, int dh) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y;
-    if (x >= dw || y >= dh) return;
-    float sx = ((float)dw - 1.0f) / (float)(sw - 1);
-    float sy = ((float)dh - 1.0f) / (float)(sh - 1);
-    float rx = (float)(1.0 / (double)sx);
-    float ry = (float)(1.0 / (double)sy);
-    int ix, iy;
-    float fx, fy;
-    cell((float)x * rx, sw, ix, fx);
-    cell((float)y * ry, sh, iy, fy);
-    long i = (long)iy * sw + ix;
-    float r[2];
-    const float* planes[2] = {su, sv};
-#pragma unroll
-    for (int c = 0; c < 2; c++) {
-        const float* p = planes[c];
-        float p00 = p[i], p10 = p[i + 1], p01 = p[i + sw], p11 = p[i + sw + 1];
-        float top = (p10 - p00) * fx + p00;
-        float bot = (p11 - p01) * fx + p01;
-        r[c] = (bot - top) * fy + top;
-    }
-    long o = (long)y * dw + x;
-    du[o] = r[0] * sx;
-    dv[o] = r[1] * sy;
-}
-
-// flow.rs:1305: scale_values(flow, -1.0), written interleaved; flags a NaN
-__global__ void k_negate_interleave(const float* __restrict__ fu, const float* __restrict__ fv, long n,
-                                    float* __restrict__ out, int* __restrict__ nan_flag) {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float u = -1.0f * fu[i], v = -1.0f * fv[i];
-    out[2 * i] = u;
-    out[2 * i + 1] = v;
-    if (isnan(u) || isnan(v)) atomicOr(nan_flag, 1);
 }
 
 __global__ void k_deinterleave(const float* __restrict__ in, long n, float* __restrict__ fu, float* __restrict__ fv) {
@@ -356,18 +223,6 @@ __global__ void k_deinterleave(const float* __restrict__ in, long n, float* __re
     if (i >= n) return;
     fu[i] = in[2 * i];
     fv[i] = in[2 * i + 1];
-}
-
-__global__ void k_interleave(const float* __restrict__ fu, const float* __restrict__ fv, long n, float* __restrict__ out) {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    out[2 * i] = fu[i];
-    out[2 * i + 1] = fv[i];
-}
-
-__global__ void k_fill(float* __restrict__ p, long n, float v) {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
 }
 
 // =====================================================================================================
@@ -677,9 +532,8 @@ __device__ void bm_sweep(float* su, float* sv, float* c0, const float* s_a, int*
 // transposes its field for the column sweeps (flow.rs:583-621). A and B of a column sweep are the
 // transposed planes (element (x, y) at [x * h + y]) so that the line's patches stay contiguous.
 template <bool COLS>
-__device__ void bm_line(const float* __restrict__ A, const float* __restrict__ B, const float* src_u,
-                        const float* src_v, const float* ends_u, const float* ends_v, float* dst_u, float* dst_v, int w,
-                        int h, int fixed) {
+__device__ void bm_line(const float* __restrict__ A, const float* __restrict__ B, const float2* src, const float2* ends,
+                        float2* dst, int w, int h, int fixed) {
     extern __shared__ float sm[];
     const int len = COLS ? h : w, other = COLS ? w : h;
     if (len < 3) return;  // no interior position
@@ -695,13 +549,9 @@ __device__ void bm_line(const float* __restrict__ A, const float* __restrict__ B
     int* entry = ctl + 8;
     int* prevl = entry + nch;
     for (int i = threadIdx.x; i < len; i += blockDim.x) {
-        if (COLS && (i == 0 || i == len - 1)) {
-            su[i] = ends_u[(long)i * w + fixed];
-            sv[i] = ends_v[(long)i * w + fixed];
-        } else {
-            su[i] = src_u[(long)fixed * len + i];
-            sv[i] = src_v[(long)fixed * len + i];
-        }
+        const float2 f = COLS && (i == 0 || i == len - 1) ? ends[(long)i * w + fixed] : src[(long)fixed * len + i];
+        su[i] = f.x;
+        sv[i] = f.y;
 #pragma unroll
         for (int o = 0; o < 3; o++)  // A at offset o-1 across the line: rows y-1..y+1, or columns x-1..x+1
             s_a[o * len + i] = __ldg(A + (long)(fixed - 1 + o) * len + i);
@@ -711,8 +561,7 @@ __device__ void bm_line(const float* __restrict__ A, const float* __restrict__ B
     bm_sweep<COLS>(su, sv, c0, s_a, endp, qa, qb, ctl, entry, prevl, B, w, h, fixed, len, false);
     bm_sweep<COLS>(su, sv, c0, s_a, endp, qa, qb, ctl, entry, prevl, B, w, h, fixed, len, true);
     for (int i = threadIdx.x + 1; i <= len - 2; i += blockDim.x) {
-        dst_u[(long)i * other + fixed] = su[i];
-        dst_v[(long)i * other + fixed] = sv[i];
+        dst[(long)i * other + fixed] = make_float2(su[i], sv[i]);
     }
 }
 
@@ -738,22 +587,22 @@ __global__ void k_transpose2(const float* __restrict__ a, const float* __restric
     }
 }
 
-// The row sweeps of rows 1..h-2 of the field (fu, fv), the result into the transposed planes
-// (uT, vT; element (x, y) at [x * h + y]) at the interior of those rows
-__global__ void k_bm_rows(const float* __restrict__ A, const float* __restrict__ B, const float* __restrict__ fu,
-                          const float* __restrict__ fv, int w, int h, float* __restrict__ uT, float* __restrict__ vT) {
+// The row sweeps of rows 1..h-2 of the field f, the result into the transposed field ft (element (x,
+// y) at [x * h + y]) at the interior of those rows
+__global__ void k_bm_rows(const float* __restrict__ A, const float* __restrict__ B, const float2* __restrict__ f, int w,
+                          int h, float2* __restrict__ ft) {
     int y = blockIdx.x + 1;  // rows 1..h-2
     if (y > h - 2) return;
-    bm_line<false>(A, B, fu, fv, nullptr, nullptr, uT, vT, w, h, y);
+    bm_line<false>(A, B, f, nullptr, ft, w, h, y);
 }
 
-// The column sweeps of columns 1..w-2 from the transposed planes (uT, vT) that k_bm_rows wrote, the
-// end rows 0 and h-1 from (fu, fv); the result into (fu, fv) at rows 1..h-2 of those columns
-__global__ void k_bm_cols(const float* __restrict__ AT, const float* __restrict__ BT, const float* __restrict__ uT,
-                          const float* __restrict__ vT, int w, int h, float* fu, float* fv) {
+// The column sweeps of columns 1..w-2 from the transposed field ft that k_bm_rows wrote, the end rows 0
+// and h-1 from f; the result into f at rows 1..h-2 of those columns
+__global__ void k_bm_cols(const float* __restrict__ AT, const float* __restrict__ BT, const float2* __restrict__ ft, int w,
+                          int h, float2* f) {
     int x = blockIdx.x + 1;  // columns 1..w-2
     if (x > w - 2) return;
-    bm_line<true>(AT, BT, uT, vT, fu, fv, fu, fv, w, h, x);
+    bm_line<true>(AT, BT, ft, f, f, w, h, x);
 }
 
 TW_VARIANT_END
