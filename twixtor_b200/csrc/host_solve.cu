@@ -305,11 +305,13 @@ int build_user_dev(tw_ctx* ctx, const UserPairs& pr, const Geo& g, int W, int H,
 // the field going back into f.
 void block_match(tw_ctx* ctx, const float* A, const float* B, const float* AT, const float* BT, float2* f, float2* ft, int w,
                  int h, bool fast) {
-    if (w < 3 || h < 3) return;  // callers refuse lines above BM_MAX_LINE before any launch
+    // no block has a cost in a level of fewer than 4 x 4 pixels (flow.rs:474-500), so no vector moves there;
+    // callers refuse lines above BM_MAX_LINE before any launch
+    if (w < 4 || h < 4) return;
     double b = 24.0 * w * h;  // per launch (both sweeps): the field read and written (8 + 8), A and B read once (4 + 4)
     LevelTune t = level_tune(ctx, w, h);
-    LAUNCHV(ctx, fast, b, k_bm_rows, h - 2, t.bm_rows_threads, bm_smem_bytes(w), A, B, f, w, h, ft);
-    LAUNCHV(ctx, fast, b, k_bm_cols, w - 2, t.bm_cols_threads, bm_smem_bytes(h), AT, BT, ft, w, h, f);
+    LAUNCHV(ctx, fast, b, k_bm_rows, h - 2, std::min(t.bm_rows_threads, BM_MAX_THREADS), bm_smem_bytes(w), A, B, f, w, h, ft, ctx->g7.z);
+    LAUNCHV(ctx, fast, b, k_bm_cols, w - 2, std::min(t.bm_cols_threads, BM_MAX_THREADS), bm_smem_bytes(h), AT, BT, ft, w, h, f, ctx->g7.z);
 }
 
 // ---- one solve over two resident pyramids (flow.rs:1258-1307) ------------------------------------------

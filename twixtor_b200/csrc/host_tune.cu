@@ -173,19 +173,19 @@ int tw_autotune(tw_ctx* ctx, const tw_flow_settings* s, int32_t width, int32_t h
             }
             // block matching: the row and the column kernel, 128 to 512 threads per line (each one's
             // input field restored before every launch)
-            if (w >= 3 && h >= 3) {
+            if (w >= 4 && h >= 4) {
                 const size_t fbytes = (size_t)w * h * sizeof(float2);
                 cudaMemcpyAsync(fsave, f, fbytes, cudaMemcpyDeviceToDevice, ctx->stream);
                 float br = 1e30f, bc = 1e30f;
                 for (int th : {128, 256, 512}) {
                     float ms = timed([&] {
                         cudaMemcpyAsync(f, fsave, fbytes, cudaMemcpyDeviceToDevice, ctx->stream);
-                        LAUNCH(ctx, k_bm_rows, h - 2, th, bm_smem_bytes(w), A, Bp, f, w, h, ft);
+                        LAUNCH(ctx, k_bm_rows, h - 2, th, bm_smem_bytes(w), A, Bp, f, w, h, ft, ctx->g7.z);
                     });
                     if (ms < br) { br = ms; best.bm_rows_threads = th; }
                     ms = timed([&] {
                         cudaMemcpyAsync(ft, fsave, fbytes, cudaMemcpyDeviceToDevice, ctx->stream);
-                        LAUNCH(ctx, k_bm_cols, w - 2, th, bm_smem_bytes(h), AT, BT, ft, w, h, f);
+                        LAUNCH(ctx, k_bm_cols, w - 2, th, bm_smem_bytes(h), AT, BT, ft, w, h, f, ctx->g7.z);
                     });
                     if (ms < bc) { bc = ms; best.bm_cols_threads = th; }
                 }

@@ -75,17 +75,18 @@ __global__ void k_deinterleave(const float* __restrict__ in, long n, float* __re
 // shared. k_bm_rows: both sweeps of every row (left to right, then right to left) of f, the result
 // written into the transpose ft (element (x, y) at [x * h + y]); k_bm_cols: both sweeps of every
 // column (top to bottom, then bottom to top) read from ft, with the transposes of A and B, the result
-// written back into f. Lines 0 and last are not swept.
+// written back into f. Lines 0 and last are not swept; levels of at least 4 x 4. z: -0.0 (level.cuh).
 __global__ void k_bm_rows(const float* __restrict__ A, const float* __restrict__ B, const float2* __restrict__ f, int w,
-                          int h, float2* __restrict__ ft);
+                          int h, float2* __restrict__ ft, float z);
 __global__ void k_bm_cols(const float* __restrict__ AT, const float* __restrict__ BT, const float2* __restrict__ ft, int w,
-                          int h, float2* f);
+                          int h, float2* f, float z);
 // two w x h planes into their h x w transposes; block (32, 8), grid (ceil(w/32), ceil(h/32))
 __global__ void k_transpose2(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ at,
                              float* __restrict__ bt, int w, int h);
 size_t bm_smem_bytes(int len);
 // longest row or column block matching keeps in shared memory (9 arrays of 4-byte values per element)
 constexpr int BM_MAX_LINE = 6144;
+constexpr int BM_MAX_THREADS = 512;  // per line; larger tuning entries run with it
 
 // ---- warps and blends (warp.rs, blend.rs) ------------------------------------------------------------
 struct WarpParams {

@@ -10,9 +10,9 @@ namespace fast {
 __global__ void k_resample(const float* __restrict__ src, int sw, int sh, float* __restrict__ dst, int dw, int dh);
 __global__ void k_range_any(const float2* __restrict__ f, int w, int h, int* __restrict__ any_in_range);
 __global__ void k_bm_rows(const float* __restrict__ A, const float* __restrict__ B, const float2* __restrict__ f, int w,
-                          int h, float2* __restrict__ ft);
+                          int h, float2* __restrict__ ft, float z);
 __global__ void k_bm_cols(const float* __restrict__ AT, const float* __restrict__ BT, const float2* __restrict__ ft, int w,
-                          int h, float2* f);
+                          int h, float2* f, float z);
 __global__ void k_transpose2(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ at,
                              float* __restrict__ bt, int w, int h);
 __global__ void k_blur5_band(const float* __restrict__ orig, const void* __restrict__ luma_src, int fmt, int luma_mode,

@@ -282,6 +282,83 @@ __device__ __forceinline__ bool bm_cost(const float* __restrict__ B, int w, int 
     return true;
 }
 
+// One coordinate of a target for Block::cost (flow.rs:474-500) in a level of n >= 4 pixels along it: the
+// cost exists for targets in [1, n - 2]; the cell is the target's whole part, but at n - 2 the cell
+// before it (with the fraction 1). Any other target is moved into the range and reported as no good.
+__device__ __forceinline__ void bm_cell(float t, float top, int last, bool& ok, int& i, float& f) {
+    const float c = fminf(fmaxf(t, 1.0f), top);
+    ok = ok && c == t;
+    i = min(__float2int_rz(c), last);
+    f = c - (float)i;
+}
+
+// The level block matching reads, along one line: B row major (element (x, y) at [y * w + x]), or with COLS
+// its transpose ([x * h + y]), so that a line's patches are contiguous.
+// The costs (flow.rs:474-523) of two vectors at one position as the two lanes of packed arithmetic: lane .x
+// and lane .y their cells' first elements (at0, at1) and fractions; p: the 3 x 3 patch of A there, row by row.
+// The products carry negated weights, so that their sum adds to the patch value; the squares are the same
+// bits. z: -0.0 (see the packed pairs above).
+template <bool COLS>
+__device__ __forceinline__ float2 bm_cost2(const float* __restrict__ B, int pitch, const float p[9], float2 fx, float2 fy,
+                                           int at0, int at1, float z) {
+    float2 T[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            T[COLS ? j : i][COLS ? i : j] = make_float2(__ldg(B + at0 + i * pitch + j), __ldg(B + at1 + i * pitch + j));
+    const float2 zz = make_float2(z, z);
+    const float2 nx = make_float2(-fx.x, -fx.y), ny = make_float2(-fy.x, -fy.y);
+    const float2 w11 = __ffma2_rn(fy, fx, zz), n11 = __ffma2_rn(fy, nx, zz);
+    const float2 n10 = __fadd2_rn(w11, nx), n01 = __fadd2_rn(w11, ny);
+    const float2 n00 = __fadd2_rn(__fadd2_rn(__fadd2_rn(fx, make_float2(-1.0f, -1.0f)), fy), n11);
+    float2 s = zz;
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const int k = b * 3 + a;
+#ifdef TW_FAST_VARIANT
+            const float2 d = __ffma2_rn(n11, T[b + 1][a + 1], __ffma2_rn(n01, T[b + 1][a], __ffma2_rn(n10, T[b][a + 1],
+                             __ffma2_rn(n00, T[b][a], make_float2(p[k], p[k])))));
+            s = __ffma2_rn(d, d, s);
+#else
+            float2 q = __fadd2_rn(__ffma2_rn(n00, T[b][a], zz), __ffma2_rn(n10, T[b][a + 1], zz));
+            q = __fadd2_rn(q, __ffma2_rn(n01, T[b + 1][a], zz));
+            q = __fadd2_rn(q, __ffma2_rn(n11, T[b + 1][a + 1], zz));
+            const float2 d = __fadd2_rn(make_float2(p[k], p[k]), q);
+            const float2 sq = __ffma2_rn(d, d, zz);
+            s = k == 0 ? sq : k < 8 ? __fadd2_rn(s, sq) : __fadd2_rn(sq, s);
+#endif
+        }
+    }
+    return s;
+}
+
+// The cost of one vector there.
+template <bool COLS>
+__device__ __forceinline__ float bm_cost1(const float* __restrict__ B, int pitch, const float p[9], float fx, float fy, int at) {
+    float T[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) T[COLS ? j : i][COLS ? i : j] = __ldg(B + at + i * pitch + j);
+    const float w11 = fy * fx, w10 = fx - w11, w01 = fy - w11, w00 = ((1.0f - fx) - fy) + w11;
+    float sq[9];
+#pragma unroll
+    for (int b = 0; b < 3; b++)
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const float q = ((w00 * T[b][a] + w10 * T[b][a + 1]) + w01 * T[b + 1][a]) + w11 * T[b + 1][a + 1];
+            const float d = p[b * 3 + a] - q;
+            sq[b * 3 + a] = d * d;
+        }
+    float s = sq[0] + sq[1];
+#pragma unroll
+    for (int k = 2; k < 8; k++) s = s + sq[k];
+    return sq[8] + s;
+}
+
 // sample.rs:31-41 for a coordinate known to lie in [0, len - 1] (or a NaN): the conversion needs no range
 // test and the cell no lower clamp (a NaN gives cell 0 and a NaN fraction, as the general rule does)
 __device__ __forceinline__ void cell_inside(float x, int len, int& io, float& fo) {

@@ -70,15 +70,15 @@ extern "C" int tw_block_match_noalloc(const float* a, const float* b, float* flo
     // aligned to a pair.
     dim3 g2((unsigned)((2 * n + tb - 1) / tb));
     cudaError_t e = launch(k_copy_floats, g2, dim3(tb), 0, s, (const float*)flow, (float*)f, 2 * n);
-    if (e == cudaSuccess && width >= 3 && height >= 3) {
+    if (e == cudaSuccess && width >= 4 && height >= 4) {
         // the row sweeps write the transposed field ft, the column sweeps read it with the transposes of
         // A and B and write the result back into f
         e = launch(tw::k_bm_rows, dim3(height - 2), dim3(tb), tw::bm_smem_bytes(width), s, a, b, (const float2*)f, (int)width,
-                   (int)height, ft);
+                   (int)height, ft, -0.0f);
         if (e == cudaSuccess) e = launch(tw::k_transpose2, ga, tt, 0, s, a, b, at, bt, (int)width, (int)height);
         if (e == cudaSuccess)
             e = launch(tw::k_bm_cols, dim3(width - 2), dim3(tb), tw::bm_smem_bytes(height), s, (const float*)at,
-                       (const float*)bt, (const float2*)ft, (int)width, (int)height, f);
+                       (const float*)bt, (const float2*)ft, (int)width, (int)height, f, -0.0f);
     }
     if (e == cudaSuccess) e = launch(k_copy_floats, g2, dim3(tb), 0, s, (const float*)f, flow, 2 * n);
     if (e != cudaSuccess) return TW_ERR_CUDA;

@@ -259,40 +259,43 @@ __device__ __forceinline__ void bm_patch(const float* s_a, int len, int i, float
         for (int c = 0; c < 3; c++) p[r * 3 + c] = COLS ? s_a[c * len + (i - 1 + r)] : s_a[r * len + (i - 1 + c)];
 }
 
-// accept(i, n) of the sweep at line position i with its patch p (Block::step, flow.rs:529-546): ci is
-// the cost of the current vector (NaN when the step cannot happen at i: no target or no cost).
-template <bool COLS>
-__device__ __forceinline__ bool bm_accept_p(const float p[9], const float* __restrict__ B, int w, int h, int fixed,
-                                            int i, float nu, float nv, float ci) {
-    if (isnan(ci)) return false;  // None, or a NaN cost that nothing compares below
-    int x = COLS ? fixed : i, y = COLS ? i : fixed;
-    float c1;
-    if (!bm_cost<COLS>(B, w, h, p, (float)x - nu, (float)y - nv, c1)) return false;
-    return c1 < ci;
-}
-
+// accept(i, n) of the sweep at line position i (Block::step, flow.rs:529-546): ci is the cost of the
+// current vector (NaN when the step cannot happen at i: no target or no cost).
 template <bool COLS>
 __device__ __forceinline__ bool bm_accept(const float* s_a, int len, const float* __restrict__ B, int w, int h,
                                           int fixed, int i, float nu, float nv, float ci) {
     float p[9];
     bm_patch<COLS>(s_a, len, i, p);
-    return bm_accept_p<COLS>(p, B, w, h, fixed, i, nu, nv, ci);
+    const int x = COLS ? fixed : i, y = COLS ? i : fixed;
+    bool ok = true;
+    int ix, iy;
+    float fx, fy;
+    bm_cell((float)x - nu, (float)(w - 2), w - 3, ok, ix, fx);
+    bm_cell((float)y - nv, (float)(h - 2), h - 3, ok, iy, fy);
+    const float c1 = bm_cost1<COLS>(B, COLS ? h : w, p, fx, fy, COLS ? (ix - 1) * h + iy - 1 : (iy - 1) * w + ix - 1);
+    return ok && c1 < ci;
 }
 
-// The cost of the vector (u, v) at line position i (flow.rs:529-536): NaN when its target leaves the
-// level or the block has no cost.
+// The cost ci of the current vector (u, v) at line position i (NaN: no target, or no cost) and accept(i, n)
+// for the vector (nu, nv), evaluated together.
 template <bool COLS>
-__device__ __forceinline__ float bm_own_cost(const float p[9], const float* __restrict__ B, int w, int h, int fixed,
-                                             int i, float u, float v) {
-    float c = __int_as_float(0x7fc00000);
-    int x = COLS ? fixed : i, y = COLS ? i : fixed;
-    float tx = (float)x - u;
-    float ty = (float)y - v;
-    if (0.0f <= tx && tx <= (float)(w - 1) && 0.0f <= ty && ty <= (float)(h - 1)) {
-        float cost;
-        if (bm_cost<COLS>(B, w, h, p, tx, ty, cost)) c = cost;
-    }
-    return c;
+__device__ __forceinline__ bool bm_own_accept(const float* s_a, int len, const float* __restrict__ B, int w, int h, int fixed,
+                                              int i, float u, float v, float nu, float nv, float z, float& ci) {
+    float p[9];
+    bm_patch<COLS>(s_a, len, i, p);
+    const float x = (float)(COLS ? fixed : i), y = (float)(COLS ? i : fixed);
+    const float wtop = (float)(w - 2), htop = (float)(h - 2);
+    bool ok0 = true, ok1 = true;
+    int ix0, iy0, ix1, iy1;
+    float2 fx, fy;
+    bm_cell(x - u, wtop, w - 3, ok0, ix0, fx.x);
+    bm_cell(y - v, htop, h - 3, ok0, iy0, fy.x);
+    bm_cell(x - nu, wtop, w - 3, ok1, ix1, fx.y);
+    bm_cell(y - nv, htop, h - 3, ok1, iy1, fy.y);
+    const float2 c = bm_cost2<COLS>(B, COLS ? h : w, p, fx, fy, COLS ? (ix0 - 1) * h + iy0 - 1 : (iy0 - 1) * w + ix0 - 1,
+                                    COLS ? (ix1 - 1) * h + iy1 - 1 : (iy1 - 1) * w + ix1 - 1, z);
+    ci = ok0 ? c.x : __int_as_float(0x7fc00000);
+    return ok1 && c.y < ci;
 }
 
 // Appends val to q (counter *n) for the lanes of the warp with `want`: one atomic per warp. Every lane
@@ -326,43 +329,32 @@ __device__ __forceinline__ void bm_push(int* q, int* n, bool want, int val) {
 //      before each);
 //   4. the owner of every position (the last start at or before it, by binary lifting over the
 //      doubled tables from the chunk's entry), and v[owner] into the line.
+// What bounds it: instruction issue on the fine levels, the latency of its stages on the coarse ones. The
+// packed evaluation of step 1 (both sweeps; the reverse sweep used to queue and recompute the replaced
+// positions' costs) took the launches at 960 x 540 from 81 to 74 us (rows) and 57 to 52 us (columns). Tried
+// and slower: a warp of 32 neighbouring lines walking chunks of positions with carried vectors, chunks and
+// clusters of blocks put right afterwards (half the instructions, but 64 to 80 us at 960 x 540 and 28 to 47
+// us at 120 x 67 against 14: its steps follow one another).
 // Every cost is Block::cost bit for bit, so the result equals the sequential sweep. The in place
 // update is safe: step 4 reads only run starts, which keep their own vectors.
 template <bool COLS>
 __device__ void bm_sweep(float* su, float* sv, float* c0, const float* s_a, int* endp, int* qa, int* qb, int* ctl,
                          int* entry, int* prevl, const float* __restrict__ B, int w, int h, int fixed, int len,
-                         bool reverse) {
+                         bool reverse, float z) {
     const unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     auto line_of = [&](int q) -> int { return reverse ? len - 1 - q : q; };  // sweep position -> line index
-    // 1. the reverse sweep's costs of the replaced vectors (qa holds their line indices, ctl[3] their count)
-    if (reverse) {
-        const int n = ctl[3];
-        for (int k = tid; k < n; k += nt) {
-            const int i = qa[k];
-            float p[9];
-            bm_patch<COLS>(s_a, len, i, p);
-            c0[i] = bm_own_cost<COLS>(p, B, w, h, fixed, i, su[i], sv[i]);
-        }
-        __syncthreads();
-    }
-    //    the test of v[q-1] at q (candidate j = q - 1), the forward sweep computing c0 on the way
+    // 1. c0 and the test of v[q-1] at q (candidate j = q - 1)
     for (int qb0 = 0; qb0 < len; qb0 += nt) {
         const int q = qb0 + tid, j = q - 1;
         bool more = false;
         if (q >= 1 && q < len) {
             if (q <= len - 2) {
                 const int i = line_of(q), jl = line_of(j);
-                float p[9];
-                bm_patch<COLS>(s_a, len, i, p);
                 float ci;
-                if (!reverse) {
-                    ci = bm_own_cost<COLS>(p, B, w, h, fixed, i, su[i], sv[i]);
-                    c0[i] = ci;
-                } else {
-                    ci = c0[i];
-                }
-                if (!bm_accept_p<COLS>(p, B, w, h, fixed, i, su[jl], sv[jl], ci)) endp[j] = q;
+                const bool take = bm_own_accept<COLS>(s_a, len, B, w, h, fixed, i, su[i], sv[i], su[jl], sv[jl], z, ci);
+                c0[i] = ci;
+                if (!take) endp[j] = q;
                 else if (q + 1 <= len - 2) more = true;
                 else endp[j] = len - 1;
             } else {
@@ -483,12 +475,11 @@ __device__ void bm_sweep(float* su, float* sv, float* c0, const float* s_a, int*
             entry[k] = -1;
             prevl[k] = Lp;
         }
-        ctl[0] = ctl[1] = ctl[2] = ctl[3] = 0;  // the next sweep's counters and the list of replaced positions
+        ctl[0] = ctl[1] = ctl[2] = 0;  // the next sweep's counters
     }
     __syncthreads();
     // 4. owners by binary lifting from the chunk's entry over the doubled tables Jr[r] (2^r successors,
-    //    saturated at the chunk's end), then the scatter; the forward sweep lists the replaced
-    //    positions for the reverse sweep's costs
+    //    saturated at the chunk's end), then the scatter
     for (int c = warp; c < nch; c += nw) {
         const int base = c << 5, q = base + lane;
         int Jr[5];
@@ -517,7 +508,6 @@ __device__ void bm_sweep(float* su, float* sv, float* c0, const float* s_a, int*
             su[i] = su[o];
             sv[i] = sv[o];
         }
-        if (!reverse) bm_push(qa, ctl + 3, moved, i);
     }
     __syncthreads();
 }
@@ -533,7 +523,7 @@ __device__ void bm_sweep(float* su, float* sv, float* c0, const float* s_a, int*
 // transposed planes (element (x, y) at [x * h + y]) so that the line's patches stay contiguous.
 template <bool COLS>
 __device__ void bm_line(const float* __restrict__ A, const float* __restrict__ B, const float2* src, const float2* ends,
-                        float2* dst, int w, int h, int fixed) {
+                        float2* dst, int w, int h, int fixed, float z) {
     extern __shared__ float sm[];
     const int len = COLS ? h : w, other = COLS ? w : h;
     if (len < 3) return;  // no interior position
@@ -558,8 +548,8 @@ __device__ void bm_line(const float* __restrict__ A, const float* __restrict__ B
     }
     if (threadIdx.x < 8) ctl[threadIdx.x] = 0;
     __syncthreads();
-    bm_sweep<COLS>(su, sv, c0, s_a, endp, qa, qb, ctl, entry, prevl, B, w, h, fixed, len, false);
-    bm_sweep<COLS>(su, sv, c0, s_a, endp, qa, qb, ctl, entry, prevl, B, w, h, fixed, len, true);
+    bm_sweep<COLS>(su, sv, c0, s_a, endp, qa, qb, ctl, entry, prevl, B, w, h, fixed, len, false, z);
+    bm_sweep<COLS>(su, sv, c0, s_a, endp, qa, qb, ctl, entry, prevl, B, w, h, fixed, len, true, z);
     for (int i = threadIdx.x + 1; i <= len - 2; i += blockDim.x) {
         dst[(long)i * other + fixed] = make_float2(su[i], sv[i]);
     }
@@ -589,20 +579,20 @@ __global__ void k_transpose2(const float* __restrict__ a, const float* __restric
 
 // The row sweeps of rows 1..h-2 of the field f, the result into the transposed field ft (element (x,
 // y) at [x * h + y]) at the interior of those rows
-__global__ void k_bm_rows(const float* __restrict__ A, const float* __restrict__ B, const float2* __restrict__ f, int w,
-                          int h, float2* __restrict__ ft) {
+__global__ void __launch_bounds__(BM_MAX_THREADS) k_bm_rows(const float* __restrict__ A, const float* __restrict__ B, const float2* __restrict__ f, int w,
+                          int h, float2* __restrict__ ft, float z) {
     int y = blockIdx.x + 1;  // rows 1..h-2
     if (y > h - 2) return;
-    bm_line<false>(A, B, f, nullptr, ft, w, h, y);
+    bm_line<false>(A, B, f, nullptr, ft, w, h, y, z);
 }
 
 // The column sweeps of columns 1..w-2 from the transposed field ft that k_bm_rows wrote, the end rows 0
 // and h-1 from f; the result into f at rows 1..h-2 of those columns
-__global__ void k_bm_cols(const float* __restrict__ AT, const float* __restrict__ BT, const float2* __restrict__ ft, int w,
-                          int h, float2* f) {
+__global__ void __launch_bounds__(BM_MAX_THREADS) k_bm_cols(const float* __restrict__ AT, const float* __restrict__ BT, const float2* __restrict__ ft, int w,
+                          int h, float2* f, float z) {
     int x = blockIdx.x + 1;  // columns 1..w-2
     if (x > w - 2) return;
-    bm_line<true>(AT, BT, ft, f, f, w, h, x);
+    bm_line<true>(AT, BT, ft, f, f, w, h, x, z);
 }
 
 TW_VARIANT_END
