@@ -127,29 +127,6 @@ __device__ __forceinline__ bool at_border(int X0, int Y0, int w0, int h0, int re
 
 // ---- one solver level: gradient, tensor and its blur (flow.rs:1275-1277) ---------------------------
 
-// The gradient of img at (x, y) (flow.rs:283-316): the mean of the one sided differences that exist (a
-// half is exact, so the reference's division by 2 is a product), zero in a layered solve where the
-// level mask of X is below 0.95 at the pixel or at one of its four neighbours that exist
-// (flow.rs:743-761).
-__device__ __forceinline__ float2 gradient_at(const float* __restrict__ img, const float* __restrict__ mask, int w, int h,
-                                              int x, int y) {
-    const int i = y * w + x;
-    const float cc = __ldg(img + i);
-    float nx = 0.0f, ny = 0.0f;
-    if (x >= 1) nx = (cc - __ldg(img + i - 1)) + 0.0f;
-    if (y >= 1) ny = (cc - __ldg(img + i - w)) + 0.0f;
-    if (x + 1 <= w - 1) nx = nx + (__ldg(img + i + 1) - cc);
-    if (y + 1 <= h - 1) ny = ny + (__ldg(img + i + w) - cc);
-    float2 g = make_float2(x >= 1 && x + 1 <= w - 1 ? nx * 0.5f : nx, y >= 1 && y + 1 <= h - 1 ? ny * 0.5f : ny);
-    if (mask) {
-        auto off = [&](int j) { return __ldg(mask + j) < 0.95f; };
-        if (off(i) || (y >= 1 && off(i - w)) || (y + 1 < h && off(i + w)) || (x >= 1 && off(i - 1)) ||
-            (x + 1 < w && off(i + 1)))
-            g = make_float2(0.0f, 0.0f);
-    }
-    return g;
-}
-
 template <int TX, int TY>
 struct InitGeom {
     static constexpr int HALO = 7, R = 4;

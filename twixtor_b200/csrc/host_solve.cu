@@ -347,11 +347,10 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
     bool af = s.taps_above_first != 0;
     bool damp_any = std::fabs((double)damp - 1.0) >= 1e-6;
     const bool fast = s.fast_mode != 0;
-    // The coarse levels whose planes fit one block's shared memory run in one launch (coarse.cu),
-    // for the plain solve; the masked and the tracked solves keep the kernel by kernel path.
+    // The coarse levels whose planes fit one block's shared memory run in one launch (coarse.cu).
     int first = start;
     bool have_flow = true;  // f holds the flow of level `first` (zero at the start level)
-    if (!mx && !my && !udu) {
+    {
         int last = -1;
         for (int l = start; l >= 1; l--) {
             int w = g.sizes[l][0], h = g.sizes[l][1];
@@ -362,6 +361,11 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
             CoarseJob J{};
             J.x = x;
             J.y = y;
+            J.mx = mx;
+            J.my = my;
+            J.udu = udu;
+            J.udv = udv;
+            J.uww = udu ? uww : nullptr;
             for (int i = 0; i < g.levels; i++) {
                 J.sizes[i][0] = g.sizes[i][0];
                 J.sizes[i][1] = g.sizes[i][1];

@@ -191,12 +191,17 @@ __global__ void k_binarize(float* __restrict__ p, long n);
 // The persistent coarse-level solve (coarse.cu): one block walks the levels start .. last of a solve
 // whose planes fit its shared memory (at most COARSE_MAX_PIXELS pixels and COARSE_MAX_LINE per side;
 // last >= 1), and writes the upsampled flow of level last - 1 for the tiled kernels.
-constexpr int COARSE_THREADS = 1024;
+constexpr int COARSE_THREADS = 512;
 constexpr int COARSE_MAX_PIXELS = 2048;
 constexpr int COARSE_MAX_LINE = 128;
 struct CoarseJob {
     const float* x;  // the band pyramids of X and Y, levels concatenated finest first
     const float* y;
+    const float* mx;  // the mask pyramids of a layered solve, laid out like the bands (null: none)
+    const float* my;
+    const float* udu;  // the user displacement of tracking points, likewise (uww null: none)
+    const float* udv;
+    const float* uww;
     int sizes[32][2];
     int offs[32];  // the first element of each level
     int start, last;
@@ -208,7 +213,7 @@ struct CoarseJob {
     int* any;  // the per level range flags (32 ints, zeroed before)
     float2* f_out;
 };
-__global__ void k_solve_coarse(CoarseJob job);
+__global__ void k_solve_coarse(const __grid_constant__ CoarseJob job);
 size_t coarse_smem_bytes();
 __global__ void k_apply_upsample(const float2* __restrict__ src, int sw, int sh, UpsampleScale up,
                                  const int* __restrict__ any, int l, int start, bool damp_now, float damp,

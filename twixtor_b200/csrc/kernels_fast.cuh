@@ -33,7 +33,7 @@ __global__ void k_apply_upsample(const float2* __restrict__ src, int sw, int sh,
                                  float2* __restrict__ dst, int dw, int dh);
 __global__ void k_apply_negate(const float2* __restrict__ f, long n, const int* __restrict__ any, int start,
                                bool damp_now, float damp, float2* __restrict__ out, int* __restrict__ nan_flag);
-__global__ void k_solve_coarse(CoarseJob job);
+__global__ void k_solve_coarse(const __grid_constant__ CoarseJob job);
 
 }  // namespace fast
 }  // namespace tw
