@@ -358,7 +358,8 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
             last = l;
         }
         if (last >= 1) {
-            CoarseJob J{};
+            CoarseJob J;
+            std::memset(&J, 0, sizeof J);
             J.x = x;
             J.y = y;
             J.mx = mx;
@@ -370,6 +371,7 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
                 J.sizes[i][0] = g.sizes[i][0];
                 J.sizes[i][1] = g.sizes[i][1];
                 J.offs[i] = (int)offs[i];
+                if (i > 0) J.up[i] = upsample_scale(g.sizes[i][0], g.sizes[i][1], g.sizes[i - 1][0], g.sizes[i - 1][1]);
             }
             J.start = start;
             J.last = last;
@@ -385,6 +387,7 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
             for (int l = start; l >= last; l--) px += (double)g.sizes[l][0] * g.sizes[l][1];
             LAUNCHV(ctx, fast, 8.0 * px, k_solve_coarse, 1, COARSE_THREADS, coarse_smem_bytes(), J);
             first = last - 1;
+            have_flow = false;
         }
     }
     for (int l = first; l >= 0; l--) {

@@ -31,6 +31,11 @@ struct Taps {
     int n;
     float z;  // -0.0, the addend of the packed products (level.cuh)
 };
+// The scales of an upsample (level.cuh, upsample_scale)
+struct UpsampleScale {
+    float sx, sy, rx, ry;
+};
+
 // the half kernels of the matte choke's blur (matte.rs:366-385: radius a + 2.01 for a shrink of a
 // pixels, n = a + 3 taps for a whole a); shrinks up to 13 pixels
 constexpr int MAX_WIDE_TAPS = 16;
@@ -131,11 +136,6 @@ enum { LEVEL_TILE_32x32 = 0, LEVEL_TILE_64x32 = 1, LEVEL_TILE_64x64 = 2, LEVEL_T
        LEVEL_TILE_32x64 = 4 };
 constexpr int LEVEL_ITER_MAX_THREADS = 512, LEVEL_INIT_MAX_THREADS = 512;
 
-// The scales of an upsample (level.cuh, upsample_scale)
-struct UpsampleScale {
-    float sx, sy, rx, ry;
-};
-
 // The start of a level over TX x TY tiles: with src the flow of the level upsampled from the coarser
 // one (sw x sh, level l + 1, its reset and damping on the way) into f, else f as it is; the gradient of
 // img, masked by mask_x (may be null); calc_b of the first iteration from f, i0 and mask_y (may be null)
@@ -190,10 +190,10 @@ __global__ void k_binarize(float* __restrict__ p, long n);
 
 // The persistent coarse-level solve (coarse.cu): one block walks the levels start .. last of a solve
 // whose planes fit its shared memory (at most COARSE_MAX_PIXELS pixels and COARSE_MAX_LINE per side;
-// last >= 1), and writes the upsampled flow of level last - 1 for the tiled kernels.
+// last >= 1), and writes the flow of level `last` for the tiled kernels.
 constexpr int COARSE_THREADS = 512;
 constexpr int COARSE_MAX_PIXELS = 2048;
-constexpr int COARSE_MAX_LINE = 128;
+constexpr int COARSE_MAX_LINE = 128;  // a line is walked in segments of at most 32
 struct CoarseJob {
     const float* x;  // the band pyramids of X and Y, levels concatenated finest first
     const float* y;
@@ -203,7 +203,8 @@ struct CoarseJob {
     const float* udv;
     const float* uww;
     int sizes[32][2];
-    int offs[32];  // the first element of each level
+    int offs[32];          // the first element of each level
+    UpsampleScale up[32];  // from each level to the next finer one
     int start, last;
     bool damp_any;  // the start level's damping differs from 1
     float damp;

@@ -75,6 +75,12 @@ __device__ __forceinline__ float2 outside_value<float2>() { return make_float2(-
 template <>
 __device__ __forceinline__ float outside_value<float>() { return -0.0f; }
 
+// An element of a plane in global memory, or (LDG false) in shared memory
+template <bool LDG>
+__device__ __forceinline__ float plane_load(const float* p) {
+    return LDG ? __ldg(p) : *p;
+}
+
 // ---- separable pass elements ---------------------------------------------------------------------
 
 // flow/conv.rs:101-137 on a line held in shared memory: element t of the line (global index, inside
@@ -138,6 +144,35 @@ __device__ __forceinline__ float2 border_den(int i, int len, const float* k) {
     return make_float2(den, __frcp_rn(den));
 }
 
+// new_disp (flow.rs:361-371) at R pixels: b the blurred B, t the blurred tensor and its determinant, f the flow,
+// updated. Both components divide by the determinant: y = 1 / t once, correctly rounded, and Markstein's
+// corrections in pairs (vquot; a zero takes its sign from a y), which hold for operands within 2^60 of 1 (t
+// is above 40); others divide.
+template <int R>
+__device__ __forceinline__ void new_disp_run(const float2* b, const float4* t, float2* f) {
+    float2 a[R], q[R];
+    bool on[R], plain[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        on[r] = fabsf(t[r].w) > 40.0f;
+        a[r] = make_float2(t[r].y * b[r].y - t[r].z * b[r].x, t[r].y * b[r].x - t[r].x * b[r].y);
+        const float d = on[r] ? t[r].w : 64.0f, y = __frcp_rn(d);
+        const float lo = 8.67e-19f, hi = 1.15e18f;  // 2^-60, 2^60
+        plain[r] = on[r] && !(fabsf(d) < hi && (a[r].x == 0.0f || (fabsf(a[r].x) > lo && fabsf(a[r].x) < hi)) &&
+                              (a[r].y == 0.0f || (fabsf(a[r].y) > lo && fabsf(a[r].y) < hi)));
+        const float2 n = make_float2(-d, -d), yy = make_float2(y, y);
+        const float2 q0 = __ffma2_rn(a[r], yy, make_float2(-0.0f, -0.0f));
+        float2 v = __ffma2_rn(__ffma2_rn(q0, n, a[r]), yy, q0);
+        v = __ffma2_rn(__ffma2_rn(v, n, a[r]), yy, v);
+        q[r] = make_float2(a[r].x == 0.0f ? q0.x : v.x, a[r].y == 0.0f ? q0.y : v.y);
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        if (plain[r]) q[r] = make_float2(a[r].x / t[r].w, a[r].y / t[r].w);
+        if (on[r]) f[r] = make_float2(q[r].x + f[r].x, q[r].y + f[r].y);
+    }
+}
+
 // One element by the general rule, per channel, out of the main path: the multi channel rule drops
 // real samples of exactly -1.0, which run_pass sends here. line: line index `origin` at line[0].
 template <int N, bool LEFT_FIRST>
@@ -162,7 +197,7 @@ __device__ __forceinline__ float2 slow_pass(const float2* line, int origin, int 
 // r): no per tap tests. Returns true, with res undefined, for the rare run near the line's ends that
 // needs the general rule: a window that holds the sentinel -1.0, or a sum that vquot does not divide; the
 // caller then runs slow_run. Outputs outside the line come out as garbage that nobody reads.
-template <int N, int R, bool LEFT_FIRST, class V>
+template <int N, int R, bool LEFT_FIRST, bool SPLIT, class V>
 __device__ __forceinline__ bool run_pass(const V* base, int stride, int i0, int len, const Taps& t, const float2* den,
                                          V* res) {
     constexpr int NV = R + 2 * N - 2;
@@ -180,25 +215,38 @@ __device__ __forceinline__ bool run_pass(const V* base, int stride, int i0, int 
         return false;
     }
     // a run that touches the line's ends: both rules for every output and a select, so that the R chains
-    // stay independent (an interior output's weight sum is 1, and a value over 1 is the value)
+    // stay independent (an interior output's weight sum is 1, and a value over 1 is the value). SPLIT: the
+    // border rule first, then the interior one in a run that has both. One block whose runs are mostly at a
+    // line's ends is faster so; the tiles of a level, which have few such runs, are 13 % slower.
     Magnitudes seen;
-    float nearest = 1.0f;
+    float near4[4] = {1.0f, 1.0f, 1.0f, 1.0f};  // (SPLIT: four chains of minima)
 #pragma unroll
-    for (int j = 0; j < NV; j++) nearest = from_sentinel(v[j], nearest);
+    for (int j = 0; j < NV; j++) near4[SPLIT ? j % 4 : 0] = from_sentinel(v[j], near4[SPLIT ? j % 4 : 0]);
 #pragma unroll
     for (int r = 0; r < R; r++) {
         const int i = i0 + r;
         V s = vmul(v[r + N - 1], t.k[0], t.z), e = s;
 #pragma unroll
         for (int j = N - 1; j >= 1; j--) {
-            s = vmadd(s, vadd(v[r + N - 1 + j], v[r + N - 1 - j]), t.k[j], t.z);
+            if (!SPLIT) s = vmadd(s, vadd(v[r + N - 1 + j], v[r + N - 1 - j]), t.k[j], t.z);
             e = vmadd(e, LEFT_FIRST ? v[r + N - 1 - j] : v[r + N - 1 + j], t.k[j], t.z);
             e = vmadd(e, LEFT_FIRST ? v[r + N - 1 + j] : v[r + N - 1 - j], t.k[j], t.z);
         }
         const bool inner = i >= N && i < len - N;
         const V q = vquot(e, den[r], seen);
-        res[r] = inner ? s : q;
+        res[r] = !SPLIT && inner ? s : q;
     }
+    if (SPLIT && i0 + R - 1 >= N && i0 < len - N) {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int i = i0 + r;
+            V s = vmul(v[r + N - 1], t.k[0], t.z);
+#pragma unroll
+            for (int j = N - 1; j >= 1; j--) s = vmadd(s, vadd(v[r + N - 1 + j], v[r + N - 1 - j]), t.k[j], t.z);
+            res[r] = i >= N && i < len - N ? s : res[r];
+        }
+    }
+    const float nearest = fminf(fminf(near4[0], near4[1]), fminf(near4[2], near4[3]));
     return nearest == 0.0f || !seen.safe();
 }
 
@@ -215,71 +263,25 @@ __device__ __forceinline__ void slow_run(const V* base, int stride, int i0, int 
 
 // run_pass, or with SLOW slow_run, for a pass along the rows or the columns (`above_first`: the tap above
 // first).
-template <bool SLOW, int N, int R, class V>
+template <bool SLOW, int N, int R, bool SPLIT = false, class V>
 __device__ __forceinline__ bool h_pass(const V* base, int i0, int len, const Taps& t, const float2* den, V* res) {
-    if (!SLOW) return run_pass<N, R, false>(base, 1, i0, len, t, den, res);
+    if (!SLOW) return run_pass<N, R, false, SPLIT>(base, 1, i0, len, t, den, res);
     slow_run<N, R, false>(base, 1, i0, len, t, res);
     return false;
 }
-template <bool SLOW, int N, int R, class V>
+template <bool SLOW, int N, int R, bool SPLIT = false, class V>
 __device__ __forceinline__ bool v_pass(const V* base, int stride, int i0, int len, const Taps& t, const float2* den,
                                        bool above_first, V* res) {
     if (!SLOW)
-        return above_first ? run_pass<N, R, true>(base, stride, i0, len, t, den, res)
-                           : run_pass<N, R, false>(base, stride, i0, len, t, den, res);
+        return above_first ? run_pass<N, R, true, SPLIT>(base, stride, i0, len, t, den, res)
+                           : run_pass<N, R, false, SPLIT>(base, stride, i0, len, t, den, res);
     if (above_first) slow_run<N, R, true>(base, stride, i0, len, t, res);
     else slow_run<N, R, false>(base, stride, i0, len, t, res);
     return false;
 }
 
-// flow.rs:474-523 (Block::cost). B(X, Y) is B[Y * w + X] for a row-major plane (COLS false) and
-// B[X * h + Y] for its transpose (COLS true); the arithmetic does not depend on the layout. Indices
-// are 32-bit (a level plane holds at most 6144 x 6144 elements).
-template <bool COLS, bool LDG = true>
-__device__ __forceinline__ bool bm_cost(const float* __restrict__ B, int w, int h, const float p[9], float x2, float y2,
-                                        float& out) {
-    float wm2 = (float)(w - 2), hm2 = (float)(h - 2);
-    if (x2 > wm2 || y2 > hm2) return false;
-    int ix, iy;
-    float fx, fy;
-    if (x2 == wm2) { ix = cvtt32(wm2 - 1.0f); fx = 1.0f; }
-    else { ix = cvtt32(x2); fx = x2 - (float)ix; }
-    if (y2 == hm2) { iy = cvtt32(hm2 - 1.0f); fy = 1.0f; }
-    else { iy = cvtt32(y2); fy = y2 - (float)iy; }
-    if (ix < 1 || iy < 1) return false;
-    float w11 = fy * fx;
-    float w10 = fx - w11;
-    float w01 = fy - w11;
-    float w00 = ((1.0f - fx) - fy) + w11;
-    float t[4][4];
-    if (!COLS) {
-        const float* base = B + (iy - 1) * w + (ix - 1);
-#pragma unroll
-        for (int r = 0; r < 4; r++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) t[r][c] = LDG ? __ldg(base + r * w + c) : base[r * w + c];
-    } else {
-        const float* base = B + (ix - 1) * h + (iy - 1);
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-#pragma unroll
-            for (int r = 0; r < 4; r++) t[r][c] = LDG ? __ldg(base + c * h + r) : base[c * h + r];
-    }
-    float sq[9];
-#pragma unroll
-    for (int b = 0; b < 3; b++) {
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            float q = ((w00 * t[b][a] + w10 * t[b][a + 1]) + w01 * t[b + 1][a]) + w11 * t[b + 1][a + 1];
-            float d = p[b * 3 + a] - q;
-            sq[b * 3 + a] = d * d;
-        }
-    }
-    float s = sq[0] + sq[1];
-#pragma unroll
-    for (int k = 2; k < 8; k++) s = s + sq[k];
-    out = sq[8] + s;
-    return true;
+__device__ __forceinline__ bool same_bits(float2 a, float2 b) {
+    return __float_as_int(a.x) == __float_as_int(b.x) && __float_as_int(a.y) == __float_as_int(b.y);
 }
 
 // One coordinate of a target for Block::cost (flow.rs:474-500) in a level of n >= 4 pixels along it: the
@@ -298,7 +300,7 @@ __device__ __forceinline__ void bm_cell(float t, float top, int last, bool& ok, 
 // and lane .y their cells' first elements (at0, at1) and fractions; p: the 3 x 3 patch of A there, row by row.
 // The products carry negated weights, so that their sum adds to the patch value; the squares are the same
 // bits. z: -0.0 (see the packed pairs above).
-template <bool COLS>
+template <bool COLS, bool LDG = true>
 __device__ __forceinline__ float2 bm_cost2(const float* __restrict__ B, int pitch, const float p[9], float2 fx, float2 fy,
                                            int at0, int at1, float z) {
     float2 T[4][4];
@@ -306,7 +308,7 @@ __device__ __forceinline__ float2 bm_cost2(const float* __restrict__ B, int pitc
     for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++)
-            T[COLS ? j : i][COLS ? i : j] = make_float2(__ldg(B + at0 + i * pitch + j), __ldg(B + at1 + i * pitch + j));
+            T[COLS ? j : i][COLS ? i : j] = make_float2(plane_load<LDG>(B + at0 + i * pitch + j), plane_load<LDG>(B + at1 + i * pitch + j));
     const float2 zz = make_float2(z, z);
     const float2 nx = make_float2(-fx.x, -fx.y), ny = make_float2(-fy.x, -fy.y);
     const float2 w11 = __ffma2_rn(fy, fx, zz), n11 = __ffma2_rn(fy, nx, zz);
@@ -336,13 +338,13 @@ __device__ __forceinline__ float2 bm_cost2(const float* __restrict__ B, int pitc
 }
 
 // The cost of one vector there.
-template <bool COLS>
+template <bool COLS, bool LDG = true>
 __device__ __forceinline__ float bm_cost1(const float* __restrict__ B, int pitch, const float p[9], float fx, float fy, int at) {
     float T[4][4];
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) T[COLS ? j : i][COLS ? i : j] = __ldg(B + at + i * pitch + j);
+        for (int j = 0; j < 4; j++) T[COLS ? j : i][COLS ? i : j] = plane_load<LDG>(B + at + i * pitch + j);
     const float w11 = fy * fx, w10 = fx - w11, w01 = fy - w11, w00 = ((1.0f - fx) - fy) + w11;
     float sq[9];
 #pragma unroll
@@ -373,8 +375,8 @@ __device__ __forceinline__ void cell_inside(float x, int len, int& io, float& fo
 // zero where the source point leaves the level, and in a layered solve (mask_y) where the warped mask of
 // Y is below 0.999 (flow.rs:777-845). i1, g: I1 and the gradient at the pixels. Levels are at least 2 x
 // 2. The gathers of all R pixels are in flight together (a point outside reads pixel 0).
-template <int R>
-__device__ __forceinline__ void calc_b_run(const float* __restrict__ i0, const float* __restrict__ mask_y, int w, int h, int x,
+template <int R, bool LDG = true>
+__device__ __forceinline__ void calc_b_run(const float* i0, const float* __restrict__ mask_y, int w, int h, int x,
                                            int y, const float2* f, const float* i1, const float2* g, float2* b) {
     bool in[R];
     int at[R];
@@ -392,10 +394,10 @@ __device__ __forceinline__ void calc_b_run(const float* __restrict__ i0, const f
 #pragma unroll
     for (int r = 0; r < R; r++) {
         const float* q = i0 + at[r];
-        p[r][0] = __ldg(q);
-        p[r][1] = __ldg(q + 1);
-        p[r][2] = __ldg(q + w);
-        p[r][3] = __ldg(q + w + 1);
+        p[r][0] = plane_load<LDG>(q);
+        p[r][1] = plane_load<LDG>(q + 1);
+        p[r][2] = plane_load<LDG>(q + w);
+        p[r][3] = plane_load<LDG>(q + w + 1);
     }
 #pragma unroll
     for (int r = 0; r < R; r++) {
@@ -410,15 +412,15 @@ __device__ __forceinline__ void calc_b_run(const float* __restrict__ i0, const f
 // half is exact, so the reference's division by 2 is a product), zero in a layered solve where the
 // level mask of X is below 0.95 at the pixel or at one of its four neighbours that exist
 // (flow.rs:743-761).
-__device__ __forceinline__ float2 gradient_at(const float* __restrict__ img, const float* __restrict__ mask, int w, int h,
-                                              int x, int y) {
+template <bool LDG = true>
+__device__ __forceinline__ float2 gradient_at(const float* img, const float* __restrict__ mask, int w, int h, int x, int y) {
     const int i = y * w + x;
-    const float cc = __ldg(img + i);
+    const float cc = plane_load<LDG>(img + i);
     float nx = 0.0f, ny = 0.0f;
-    if (x >= 1) nx = (cc - __ldg(img + i - 1)) + 0.0f;
-    if (y >= 1) ny = (cc - __ldg(img + i - w)) + 0.0f;
-    if (x + 1 <= w - 1) nx = nx + (__ldg(img + i + 1) - cc);
-    if (y + 1 <= h - 1) ny = ny + (__ldg(img + i + w) - cc);
+    if (x >= 1) nx = (cc - plane_load<LDG>(img + i - 1)) + 0.0f;
+    if (y >= 1) ny = (cc - plane_load<LDG>(img + i - w)) + 0.0f;
+    if (x + 1 <= w - 1) nx = nx + (plane_load<LDG>(img + i + 1) - cc);
+    if (y + 1 <= h - 1) ny = ny + (plane_load<LDG>(img + i + w) - cc);
     float2 g = make_float2(x >= 1 && x + 1 <= w - 1 ? nx * 0.5f : nx, y >= 1 && y + 1 <= h - 1 ? ny * 0.5f : ny);
     if (mask) {
         auto off = [&](int j) { return __ldg(mask + j) < 0.95f; };
