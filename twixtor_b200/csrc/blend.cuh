@@ -9,11 +9,11 @@ namespace tw {
 template <typename P> __device__ __forceinline__ P blend_sample(P a, P b, float w);
 template <> __device__ __forceinline__ uint8_t blend_sample<uint8_t>(uint8_t a, uint8_t b, float w) {
     float af = (float)a, bf = (float)b;
-    return (uint8_t)cvtt64f((bf - af) * w + af + 0.5f);
+    return (uint8_t)cvtt_low((bf - af) * w + af + 0.5f);
 }
 template <> __device__ __forceinline__ uint16_t blend_sample<uint16_t>(uint16_t a, uint16_t b, float w) {
     float af = (float)a, bf = (float)b;
-    return (uint16_t)cvtt64f((bf - af) * w + af + 0.5f);
+    return (uint16_t)cvtt_low((bf - af) * w + af + 0.5f);
 }
 template <> __device__ __forceinline__ float blend_sample<float>(float a, float b, float w) {
     float r = (b - a) * w + a + 0.0f;
@@ -30,19 +30,19 @@ __device__ __forceinline__ void lerp_px_int(T f[4], const T s[4], float w, float
     float a = diff(0) * w + sf(0);
     float n = a / scale;
     if (!(n > 0.0f)) {
-        T z = (T)cvtt64f(0.0f);
 #pragma unroll
-        for (int i = 0; i < 4; i++) f[i] = z;
+        for (int i = 0; i < 4; i++) f[i] = T(0);
         return;
     }
     float r = diff(1) * w + sf(1), g = diff(2) * w + sf(2), b = diff(3) * w + sf(3);
     if (n > 1.0f) { r = r / n; g = g / n; b = b / n; a = scale; }
     auto clamp = [&](float c) { return c > a ? a : (0.0f > c ? 0.0f : c); };
     r = clamp(r); g = clamp(g); b = clamp(b);
-    f[1] = (T)cvtt64f(r + 0.5f);
-    f[2] = (T)cvtt64f(g + 0.5f);
-    f[3] = (T)cvtt64f(b + 0.5f);
-    f[0] = (T)cvtt64f(a + 0.5f);
+    // 0 .. scale, or a NaN that converts to 0 as the low bits of the reference's conversion are
+    f[1] = (T)__float2int_rz(r + 0.5f);
+    f[2] = (T)__float2int_rz(g + 0.5f);
+    f[3] = (T)__float2int_rz(b + 0.5f);
+    f[0] = (T)__float2int_rz(a + 0.5f);
 }
 template <> __device__ __forceinline__ void lerp_px<uint8_t>(uint8_t f[4], const uint8_t s[4], float w) {
     lerp_px_int<uint8_t>(f, s, w, 255.0f);

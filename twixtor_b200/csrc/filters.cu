@@ -101,7 +101,7 @@ __device__ __forceinline__ void blur_px(const void* src, void* dst, int w, int h
                                         bool above_first) {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long)w * h) return;
-    int y = (int)(i / w), x = (int)(i - (long)y * w);
+    int y = row_of(i, w), x = (int)(i - (long)y * w);
     const P* s = (const P*)src;
     float v[4];
     if (!cols) conv_pixel<P>(x, w, T, s + (long)y * w * 4, 4, false, v);
@@ -153,7 +153,7 @@ __global__ void k_mask_prune(const uint8_t* __restrict__ src, uint8_t* __restric
     if (gated_off(gate)) return;
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long)w * h) return;
-    int y = (int)(i / w), x = (int)(i - (long)y * w);
+    int y = row_of(i, w), x = (int)(i - (long)y * w);
     uint8_t v = src[i];
     if (v != 0 && x >= 1 && x <= w - 2 && y >= 2 && y <= h - 3 && ring_sum(src, w, x, y - 2, y, y + 2) < limit) v = 0;
     dst[i] = v;
@@ -165,7 +165,7 @@ __global__ void k_mask_dilate(const uint8_t* __restrict__ src, uint8_t* __restri
     if (gated_off(gate)) return;
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long)w * h) return;
-    int y = (int)(i / w);
+    int y = row_of(i, w);
     uint8_t v = src[i];
     if (y >= 1 && y <= h - 2 && (src[i - w] == 255 || src[i + w] == 255)) v = 255;
     dst[i] = v;
@@ -179,7 +179,7 @@ __global__ void k_mask_fill_border(const uint8_t* __restrict__ src, uint8_t* __r
     if (gated_off(gate)) return;
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long)w * h) return;
-    int y = (int)(i / w), x = (int)(i - (long)y * w);
+    int y = row_of(i, w), x = (int)(i - (long)y * w);
     int cx = min(max(x, 1), w - 2), cy = min(max(y, 1), h - 2);
     uint8_t v = src[(long)cy * w + cx];
     if (v == 0 && limit < ring_sum(src, w, cx, cy - 1, cy, cy + 1)) v = (uint8_t)value;
@@ -266,7 +266,7 @@ __device__ __forceinline__ void finish_px(P* frame, const P* blurred, uint8_t ma
             float plain = (g * sv + fl * dvv) + 0.0f;
             frame[k] = (P)(isnan(plain) ? nr::add(nr::add(nr::mul(g, sv), nr::mul(fl, dvv)), 0.0f) : plain);
         } else {
-            frame[k] = (P)cvtt64f(((float)f[k] * g + (float)s[k] * fl) + 0.5f);
+            frame[k] = (P)cvtt_low(((float)f[k] * g + (float)s[k] * fl) + 0.5f);
         }
     }
 }
@@ -382,7 +382,7 @@ __device__ __forceinline__ void motion_blur_px(const MotionBlur& B, long i, int 
                         } else if (0.0f <= qx && qx < wf && 0.0f <= qy && qy < hf) {
                             cnt++;
                             float t[4];
-                            bilerp4<P>(src, B.w, w1, h1, qx, qy, t);
+                            bilerp4<P>(src, B.w, w1, h1, qx, qy, B.flow.z, t);
 #pragma unroll
                             for (int c = 0; c < 4; c++) sum[c] = acc_add<P>(sum[c], t[c]);
                         }

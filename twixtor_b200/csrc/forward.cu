@@ -241,30 +241,32 @@ __global__ void k_fwp_blur(const void* __restrict__ in, void* __restrict__ out, 
 }
 
 template <typename P>
-__device__ __forceinline__ void fwp_resample_px(const void* src, int sw, int sh, void* dst, int dw, int dh, int x, int y) {
+__device__ __forceinline__ void fwp_resample_px(const void* src, int sw, int sh, void* dst, int dw, int dh, int x, int y,
+                                                float z) {
     float sx = ((float)sw - 1.0f) / (float)(dw - 1);
     float sy = ((float)sh - 1.0f) / (float)(dh - 1);
     float v[4];
-    bilerp4<P>((const P*)src, sw, sw - 1, sh - 1, (float)x * sx, (float)y * sy, v);
-    P* o = (P*)dst + ((long)y * dw + x) * 4;
+    bilerp4<P>((const P*)src, sw, sw - 1, sh - 1, (float)x * sx, (float)y * sy, z, v);
+    // (a sample in the depth's range: px_stored)
 #pragma unroll
-    for (int q = 0; q < 4; q++) o[q] = Pix<P>::store(v[q]);
+    for (int q = 0; q < 4; q++) v[q] = px_stored<P>(v[q]);
+    px_store((P*)dst + ((long)y * dw + x) * 4, v);
 }
 
 // pyramid.rs:258-280: the corner aligned resample of a blurred level to the next size
 __global__ void k_fwp_resample(const void* __restrict__ src, int sw, int sh, void* __restrict__ dst, int dw, int dh,
-                               int fmt) {
+                               int fmt, float z) {
     int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= dw || y >= dh) return;
-    if (fmt == 0) fwp_resample_px<uint8_t>(src, sw, sh, dst, dw, dh, x, y);
-    else if (fmt == 1) fwp_resample_px<uint16_t>(src, sw, sh, dst, dw, dh, x, y);
-    else fwp_resample_px<float>(src, sw, sh, dst, dw, dh, x, y);
+    if (fmt == 0) fwp_resample_px<uint8_t>(src, sw, sh, dst, dw, dh, x, y, z);
+    else if (fmt == 1) fwp_resample_px<uint16_t>(src, sw, sh, dst, dw, dh, x, y, z);
+    else fwp_resample_px<float>(src, sw, sh, dst, dw, dh, x, y, z);
 }
 
 // pyramid.rs:98-108: one bilinear tap at (w1 * u, h1 * v). A coordinate that leaves the image
 // (the reference indexes out of its slice there) reads nothing and raises the bad flag.
 template <typename P>
-__device__ __forceinline__ void fw_tap(const void* img, int w, int h, float u, float v, float o[4], int* bad) {
+__device__ __forceinline__ void fw_tap(const void* img, int w, int h, float u, float v, float z, float o[4], int* bad) {
     int w1 = w - 1, h1 = h - 1;
     float x = (float)w1 * u, y = (float)h1 * v;
     int ix = cvtt32(x), iy = cvtt32(y);
@@ -276,7 +278,7 @@ __device__ __forceinline__ void fw_tap(const void* img, int w, int h, float u, f
         for (int q = 0; q < 4; q++) o[q] = 0.0f;
         return;
     }
-    bilerp4<P>((const P*)img, w, w1, h1, x, y, o);
+    bilerp4<P>((const P*)img, w, w1, h1, x, y, z, o);
 }
 
 // pyramid.rs:72-95 (the hit: forward.rs:134-145)
@@ -287,16 +289,16 @@ __device__ __forceinline__ void fw_sample(const FwLevels& L, float u, float v, f
             int i = cvtt32(d);
             float frac = d - (float)i;
             float a[4], b[4];
-            fw_tap<P>(L.p[i], L.w[i], L.h[i], u, v, a, bad);
-            fw_tap<P>(L.p[i + 1], L.w[i + 1], L.h[i + 1], u, v, b, bad);
+            fw_tap<P>(L.p[i], L.w[i], L.h[i], u, v, L.z, a, bad);
+            fw_tap<P>(L.p[i + 1], L.w[i + 1], L.h[i + 1], u, v, L.z, b, bad);
 #pragma unroll
             for (int q = 0; q < 4; q++) o[q] = x86::add(x86::mul(x86::sub(b[q], a[q]), frac), a[q]);
             return;
         }
-        fw_tap<P>(L.p[L.count - 1], L.w[L.count - 1], L.h[L.count - 1], u, v, o, bad);
+        fw_tap<P>(L.p[L.count - 1], L.w[L.count - 1], L.h[L.count - 1], u, v, L.z, o, bad);
         return;
     }
-    fw_tap<P>(L.p[0], L.w[0], L.h[0], u, v, o, bad);
+    fw_tap<P>(L.p[0], L.w[0], L.h[0], u, v, L.z, o, bad);
 }
 
 // ---- the scan converter (forward/raster.rs) ------------------------------------------------------------
@@ -512,7 +514,7 @@ struct EmitSink {
         float c[4];
         if (R.pyramid) {
             if (0.0f < p[2]) fw_sample<P>(R.levels, p[0], p[1], p[2], c, R.bad);
-            else fw_tap<P>(R.levels.p[0], R.levels.w[0], R.levels.h[0], p[0], p[1], c, R.bad);
+            else fw_tap<P>(R.levels.p[0], R.levels.w[0], R.levels.h[0], p[0], p[1], R.levels.z, c, R.bad);
         } else {
 #pragma unroll
             for (int q = 0; q < 4; q++) c[q] = p[q];
@@ -730,7 +732,7 @@ __device__ __forceinline__ void store_px(void* out, uint8_t* cov, long p, const 
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         if (sizeof(P) == 4) ((float*)o)[k] = x86::add(a[k], 0.0f);
-        else o[k] = (P)cvtt64f(a[k] + 0.5f);
+        else o[k] = (P)cvtt_low(a[k] + 0.5f);
     }
     if (cov) cov[p] = n != 0 ? 0xff : 0;
 }

@@ -29,6 +29,8 @@ WarpParams warp_params(const void* src, const float* flow_interleaved, int fw, i
     p.fu = flow_interleaved;
     p.fv = flow_interleaved ? flow_interleaved + 1 : nullptr;
     p.fstride = 2;
+    p.z = -0.0f;
+    p.pairs = ((uintptr_t)flow_interleaved & 7) == 0;
     p.fw = fw;
     p.fh = fh;
     p.amount = amount;
@@ -256,6 +258,7 @@ int forward_warp_dev(tw_ctx* ctx, const void* src, const float* flow, int fw, in
     L.w[0] = W;
     L.h[0] = H;
     L.count = pyramid ? levels : 1;
+    L.z = -0.0f;
     if (pyramid && levels > 1) {
         size_t tot = 0;
         int cw = W, chh = H;
@@ -278,7 +281,7 @@ int forward_warp_dev(tw_ctx* ctx, const void* src, const float* flow, int fw, in
             LAUNCH(ctx, k_fwp_blur, gb, 128, 0, L.p[i - 1], ctx->fw_tmp[0].p, pw, ph, 0, fmt);
             LAUNCH(ctx, k_fwp_blur, gb, 128, 0, ctx->fw_tmp[0].p, ctx->fw_tmp[1].p, pw, ph, 1, fmt);
             dim3 gr((unsigned)((L.w[i] + 127) / 128), (unsigned)L.h[i]);
-            LAUNCH(ctx, k_fwp_resample, gr, 128, 0, ctx->fw_tmp[1].p, pw, ph, (void*)L.p[i], L.w[i], L.h[i], fmt);
+            LAUNCH(ctx, k_fwp_resample, gr, 128, 0, ctx->fw_tmp[1].p, pw, ph, (void*)L.p[i], L.w[i], L.h[i], fmt, L.z);
         }
     }
     // 3. count the hits of every pixel, then their offsets

@@ -9,29 +9,31 @@ namespace tw {
 
 // ---- wire -> engine (image.rs:178-206, premultiply :276-303) ----------------------------------------
 
+// The wire element of engine element i (w x h, rows bottom up with flip)
+__device__ __forceinline__ long wire_at(long i, int w, int h, bool flip) {
+    if (!flip) return i;
+    const int y = row_of(i, w);
+    return (long)(h - 1 - y) * w + (i - (long)y * w);
+}
+
 __global__ void k_from_frame_u8(const uint8_t* __restrict__ wire, uint8_t* __restrict__ eng, int w, int h, bool flip) {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     long n = (long)w * h;
     if (i >= n) return;
-    int y = (int)(i / w), x = (int)(i - (long)y * w);
-    long si = (long)(flip ? h - 1 - y : y) * w + x;
-    uchar4 p = reinterpret_cast<const uchar4*>(wire)[si];  // r, g, b, a
-    float a = (float)p.w * inv_255();
-    uchar4 o;
-    o.x = p.w;
-    o.y = (uint8_t)qround((float)p.x * a);
-    o.z = (uint8_t)qround((float)p.y * a);
-    o.w = (uint8_t)qround((float)p.z * a);
-    reinterpret_cast<uchar4*>(eng)[i] = o;
+    float p[4], o[4];  // r, g, b, a
+    px_floats<uint8_t>(wire + wire_at(i, w, h, flip) * 4, p);
+    float a = p[3] * inv_255();
+    o[0] = p[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) o[c + 1] = px_rounded(p[c] * a);
+    px_store(eng + i * 4, o);
 }
 
 __global__ void k_from_frame_u16(const uint16_t* __restrict__ wire, uint16_t* __restrict__ eng, int w, int h, bool flip) {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     long n = (long)w * h;
     if (i >= n) return;
-    int y = (int)(i / w), x = (int)(i - (long)y * w);
-    long si = (long)(flip ? h - 1 - y : y) * w + x;
-    ushort4 p = reinterpret_cast<const ushort4*>(wire)[si];
+    ushort4 p = reinterpret_cast<const ushort4*>(wire)[wire_at(i, w, h, flip)];
     uint16_t A = u16_to_q15(p.w), R = u16_to_q15(p.x), G = u16_to_q15(p.y), Bc = u16_to_q15(p.z);
     float a = (float)A * premul16_color();
     ushort4 o;
@@ -46,8 +48,7 @@ __global__ void k_from_frame_f32(const float* __restrict__ wire, float* __restri
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     long n = (long)w * h;
     if (i >= n) return;
-    int y = (int)(i / w), x = (int)(i - (long)y * w);
-    long si = (long)(flip ? h - 1 - y : y) * w + x;
+    long si = wire_at(i, w, h, flip);
     // planes G, B, R, A
     float g = wire[si], b = wire[n + si], r = wire[2 * n + si], a = wire[3 * n + si];
     float o1 = a * r, o2 = a * g, o3 = a * b;
@@ -61,28 +62,28 @@ __global__ void k_from_frame_f32(const float* __restrict__ wire, float* __restri
 
 // ---- engine -> wire (image.rs:213-245, unpremultiply :306-351) --------------------------------------
 
-__device__ __forceinline__ uchar4 unpremul_u8(uchar4 p) {  // -> r, g, b, a
-    if (p.x == 0) return make_uchar4(p.y, p.z, p.w, p.x);
-    float s = 255.0f / (float)p.x;
-    auto f = [&](uint8_t c) {
-        float v = (float)c * s;
-        if (v > 255.0f) v = 255.0f;
-        return (uint8_t)qround(v);
-    };
-    return make_uchar4(f(p.y), f(p.z), f(p.w), p.x);
+// Whole samples a, r, g, b as floats -> r, g, b, a; an opaque pixel's factor is 1
+__device__ __forceinline__ void unpremul_u8(const float p[4], float o[4]) {
+    o[0] = p[1];
+    o[1] = p[2];
+    o[2] = p[3];
+    o[3] = p[0];
+    if (p[0] == 0.0f || p[0] == 255.0f) return;
+    const float s = 255.0f / p[0];
+#pragma unroll
+    for (int c = 0; c < 3; c++) o[c] = px_rounded(fminf(o[c] * s, 255.0f));
 }
 
-__device__ __forceinline__ ushort4 unpremul_u16(ushort4 p) {  // -> wire r, g, b, a
-    ushort4 o;
-    if (p.x == 0) {
-        o = make_ushort4(p.y, p.z, p.w, p.x);
-    } else {
-        float a = (float)p.x;
-        float s = 32768.0f / a;
-        o = make_ushort4((uint16_t)qround((float)p.y * s), (uint16_t)qround((float)p.z * s),
-                         (uint16_t)qround((float)p.w * s), (uint16_t)qround(a * unpremul16_alpha()));
+__device__ __forceinline__ void unpremul_u16(const float p[4], float o[4]) {
+    uint32_t q[4] = {(uint32_t)p[1], (uint32_t)p[2], (uint32_t)p[3], (uint32_t)p[0]};
+    if (p[0] != 0.0f) {
+        const float s = p[0] == 32768.0f ? 1.0f : 32768.0f / p[0];
+#pragma unroll
+        for (int c = 0; c < 3; c++) q[c] = qround(p[c + 1] * s);
+        q[3] = qround(p[0] * unpremul16_alpha());
     }
-    return make_ushort4(q15_to_u16(o.x), q15_to_u16(o.y), q15_to_u16(o.z), q15_to_u16(o.w));
+#pragma unroll
+    for (int c = 0; c < 4; c++) o[c] = (float)q15_to_u16((uint16_t)q[c]);
 }
 
 __device__ __forceinline__ float4 unpremul_f32(float4 p) {  // -> a, r, g, b (engine order)
@@ -102,26 +103,29 @@ __global__ void k_to_frame_u8(const uint8_t* __restrict__ eng, uint8_t* __restri
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     long n = (long)w * h;
     if (i >= n) return;
-    int y = (int)(i / w), x = (int)(i - (long)y * w);
-    long si = (long)(flip ? h - 1 - y : y) * w + x;
-    reinterpret_cast<uchar4*>(wire)[i] = unpremul_u8(reinterpret_cast<const uchar4*>(eng)[si]);
+    long si = wire_at(i, w, h, flip);
+    float p[4], o[4];
+    px_floats<uint8_t>(eng + si * 4, p);
+    unpremul_u8(p, o);
+    px_store(wire + i * 4, o);
 }
 
 __global__ void k_to_frame_u16(const uint16_t* __restrict__ eng, uint16_t* __restrict__ wire, int w, int h, bool flip) {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     long n = (long)w * h;
     if (i >= n) return;
-    int y = (int)(i / w), x = (int)(i - (long)y * w);
-    long si = (long)(flip ? h - 1 - y : y) * w + x;
-    reinterpret_cast<ushort4*>(wire)[i] = unpremul_u16(reinterpret_cast<const ushort4*>(eng)[si]);
+    long si = wire_at(i, w, h, flip);
+    float p[4], o[4];
+    px_floats<uint16_t>(eng + si * 4, p);
+    unpremul_u16(p, o);
+    px_store(wire + i * 4, o);
 }
 
 __global__ void k_to_frame_f32(const float* __restrict__ eng, float* __restrict__ wire, int w, int h, bool flip) {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     long n = (long)w * h;
     if (i >= n) return;
-    int y = (int)(i / w), x = (int)(i - (long)y * w);
-    long si = (long)(flip ? h - 1 - y : y) * w + x;
+    long si = wire_at(i, w, h, flip);
     float4 o = unpremul_f32(reinterpret_cast<const float4*>(eng)[si]);
     wire[i] = o.z;          // G
     wire[n + i] = o.w;      // B
@@ -144,12 +148,10 @@ __device__ __forceinline__ void inv_warp_px(const WarpParams& p, void* out, uint
     int x = blockIdx.x * blockDim.x + threadIdx.x;
     int y = blockIdx.y;
     if (x >= w || y >= h) return;
-    P o[4];
+    float o[4];
     bool b = false;
     uint8_t c = warp_pixel<P>(p, x, y, w, h, o, b);
-    P* dst = (P*)out + ((long)y * w + x) * 4;
-#pragma unroll
-    for (int k = 0; k < 4; k++) dst[k] = o[k];
+    px_store((P*)out + ((long)y * w + x) * 4, o);
     if (cov) cov[(long)y * w + x] = c;
     if (b) atomicOr(bad, 1);
 }
@@ -194,33 +196,40 @@ __global__ void k_lerp(void* __restrict__ first, const void* __restrict__ second
 
 // ---- the fused Blend composition of warping code 0 ---------------------------------------------------
 
-template <typename P>
-__device__ __forceinline__ void store_px(const P o[4], void* out, long i, bool to_wire, long npx);
-template <>
-__device__ __forceinline__ void store_px<uint8_t>(const uint8_t o[4], void* out, long i, bool to_wire, long npx) {
-    uchar4 e = make_uchar4(o[0], o[1], o[2], o[3]);
-    reinterpret_cast<uchar4*>(out)[i] = to_wire ? unpremul_u8(e) : e;
+// Samples as floats into the engine image, or unpremultiplied into the wire frame
+__device__ __forceinline__ void store_px(const float o[4], uint8_t* out, long i, bool to_wire, long npx) {
+    float u[4] = {o[0], o[1], o[2], o[3]};
+    if (to_wire) unpremul_u8(o, u);
+    px_store(out + i * 4, u);
 }
-template <>
-__device__ __forceinline__ void store_px<uint16_t>(const uint16_t o[4], void* out, long i, bool to_wire, long npx) {
-    ushort4 e = make_ushort4(o[0], o[1], o[2], o[3]);
-    reinterpret_cast<ushort4*>(out)[i] = to_wire ? unpremul_u16(e) : e;
+__device__ __forceinline__ void store_px(const float o[4], uint16_t* out, long i, bool to_wire, long npx) {
+    float u[4] = {o[0], o[1], o[2], o[3]};
+    if (to_wire) unpremul_u16(o, u);
+    px_store(out + i * 4, u);
 }
-template <>
-__device__ __forceinline__ void store_px<float>(const float o[4], void* out, long i, bool to_wire, long npx) {
-    float4 e = make_float4(o[0], o[1], o[2], o[3]);
+__device__ __forceinline__ void store_px(const float o[4], float* out, long i, bool to_wire, long npx) {
     if (!to_wire) {
-        reinterpret_cast<float4*>(out)[i] = e;
+        px_store(out + i * 4, o);
         return;
     }
-    float4 u = unpremul_f32(e);
-    float* wire = (float*)out;
-    wire[i] = u.z;
-    wire[npx + i] = u.w;
-    wire[2 * npx + i] = u.y;
-    wire[3 * npx + i] = u.x;
+    float4 u = unpremul_f32(make_float4(o[0], o[1], o[2], o[3]));
+    out[i] = u.z;
+    out[npx + i] = u.w;
+    out[2 * npx + i] = u.y;
+    out[3 * npx + i] = u.x;
 }
 
+// blend_sample of a pair, samples and result as floats: with 0 <= w <= 1 (the common branch) an integer
+// depth's sum is in its range, and a NaN weight's is stored as 0
+template <typename P>
+__device__ __forceinline__ float2 blend_pair(float2 a, float2 b, float w, float z) {
+    float2 t = __fadd2_rn(__ffma2_rn(__ffma2_rn(a, make_float2(-1.0f, -1.0f), b), make_float2(w, w), make_float2(z, z)), a);
+    t = __fadd2_rn(t, make_float2(0.5f, 0.5f));
+    return make_float2(trunc_biased(fmaxf(t.x, 0.0f)) - PX_BIAS, trunc_biased(fmaxf(t.y, 0.0f)) - PX_BIAS);
+}
+
+// Both warps, the blend and the store of a pixel. A thread takes one pixel: a frame has some hundred times the
+// threads that the chip holds, and the gathers want many in flight.
 template <typename P>
 __device__ __forceinline__ void compose_blend_px(const WarpParams& pa, const WarpParams& pb, float wblend, int mode,
                                                  void* out, int w, int h, bool to_wire, bool flip_out, int* bad) {
@@ -228,14 +237,30 @@ __device__ __forceinline__ void compose_blend_px(const WarpParams& pa, const War
     int y = blockIdx.y;
     if (x >= w || y >= h) return;
     // the output pixel (x, y) of the engine image lands on wire row h-1-y when flip_out
-    P ta[4], tb[4], o[4];
+    float ta[4], tb[4], o[4];
     bool b = false;
     if (mode != 2) warp_pixel<P>(pa, x, y, w, h, ta, b);
     if (mode != 1) warp_pixel<P>(pb, x, y, w, h, tb, b);
-    float wl = (float)(1.0 - (double)wblend);
-    blend_px<P>(ta, tb, wblend, wl, mode, o);
+    if (mode == 0 && sizeof(P) < 4) {
+        const float2 u = blend_pair<P>(make_float2(ta[0], ta[1]), make_float2(tb[0], tb[1]), wblend, pa.z);
+        const float2 v = blend_pair<P>(make_float2(ta[2], ta[3]), make_float2(tb[2], tb[3]), wblend, pa.z);
+        o[0] = u.x; o[1] = u.y; o[2] = v.x; o[3] = v.y;
+    } else if (mode == 1 || mode == 2) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) o[k] = mode == 1 ? ta[k] : tb[k];
+    } else {
+        P qa[4], qb[4], qo[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            qa[k] = (P)ta[k];
+            qb[k] = (P)tb[k];
+        }
+        blend_px<P>(qa, qb, wblend, mode == 3 ? (float)(1.0 - (double)wblend) : 0.0f, mode, qo);
+#pragma unroll
+        for (int k = 0; k < 4; k++) o[k] = (float)qo[k];
+    }
     int oy = flip_out ? h - 1 - y : y;
-    store_px<P>(o, out, (long)oy * w + x, to_wire, (long)w * h);
+    store_px(o, (P*)out, (long)oy * w + x, to_wire, (long)w * h);
     if (b) atomicOr(bad, 1);
 }
 

@@ -105,6 +105,8 @@ struct WarpParams {
     // steps sx = amount / rx, sy = amount / ry, single precision, formed once on the host (the same
     // IEEE divisions the kernel made per pixel)
     float rx, ry, sx, sy;
+    float z;             // -0.0, the addend that keeps a packed product a product of its own
+    bool pairs;          // fu and fv interleaved and 8 byte aligned: a vector in one load
     bool copy_only;      // the |amount| early outs of inv_warp (warp.rs:751-764)
     bool hold;
     bool is360;          // wrap-around: the point wrapped into the image, the pole reflection, the 360 sampler
@@ -322,6 +324,7 @@ struct FwLevels {  // level 0 is the source
     const void* p[FW_MAX_LEVELS];
     int w[FW_MAX_LEVELS], h[FW_MAX_LEVELS];
     int count;
+    float z;  // -0.0 (WarpParams)
 };
 struct FwRaster {
     int w, h, fmt;
@@ -346,7 +349,7 @@ __global__ void k_fw_vertices(const float* __restrict__ flow, int fw, int fh, Fw
                               const uint2* __restrict__ tab, int ntab);
 __global__ void k_fwp_blur(const void* __restrict__ in, void* __restrict__ out, int w, int h, int vertical, int fmt);
 __global__ void k_fwp_resample(const void* __restrict__ src, int sw, int sh, void* __restrict__ dst, int dw, int dh,
-                               int fmt);
+                               int fmt, float z);
 __global__ void k_fw_count(FwRaster R);
 __global__ void k_fw_emit(FwRaster R);      // the Gouraud variant
 __global__ void k_fw_emit_tex(FwRaster R);  // the textured variant (R.pyramid)

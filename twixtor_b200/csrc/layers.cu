@@ -7,6 +7,7 @@
 // value itself). NaN handling follows the reference's x86 arithmetic where a NaN of a float matte
 // can reach an output (the cut, in double precision there), and its NaN rule where it uses it.
 #include "kernels.cuh"
+#include "warp.cuh"
 
 #include <climits>
 
@@ -32,7 +33,7 @@ __global__ void k_matte_extract(const void* __restrict__ wire, int fmt, int chan
     long n = (long)w * h;
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    int y = (int)(i / w), x = (int)(i - (long)y * w);
+    int y = row_of(i, w), x = (int)(i - (long)y * w);
     long si = (long)(flip ? h - 1 - y : y) * w + x;
     int c = chan == 1 ? 0 : chan == 2 ? 1 : chan == 3 ? 2 : 3;  // wire order R, G, B, A
     float v;
@@ -245,27 +246,25 @@ __global__ void k_refill_pre(void* __restrict__ img, int fmt, long n, uint8_t* _
     bool hole = false;
     if (i < n) {
         if (fmt == 0) {
-            uint8_t* p = (uint8_t*)img + i * 4;
-            if (p[0] != 0) {
-                float s = 255.0f / (float)p[0];  // image.rs:306-320
-                for (int c = 1; c < 4; c++) {
-                    float v = (float)p[c] * s;
-                    if (v > 255.0f) v = 255.0f;
-                    p[c] = (uint8_t)qround(v);
-                }
+            uint8_t* q = (uint8_t*)img + i * 4;
+            float p[4];
+            px_floats<uint8_t>(q, p);
+            if (p[0] != 0.0f && p[0] != 255.0f) {  // (an opaque pixel's factor is 1)
+                float s = 255.0f / p[0];  // image.rs:306-320
+                for (int c = 1; c < 4; c++) p[c] = px_rounded(fminf(p[c] * s, 255.0f));
+                px_store(q, p);
             }
-            hole = (uint8_t)(0xffu - p[0]) != 0;
+            hole = p[0] != 255.0f;
         } else if (fmt == 1) {
-            uint16_t* p = (uint16_t*)img + i * 4;
-            if (p[0] != 0) {
-                float inv = 65535.0f / (float)p[0];
-                for (int c = 1; c < 4; c++) {
-                    float v = (float)p[c] * inv;
-                    if (65535.0f < v) v = 65535.0f;
-                    p[c] = (uint16_t)qround(v);
-                }
+            uint16_t* q = (uint16_t*)img + i * 4;
+            float p[4];
+            px_floats<uint16_t>(q, p);
+            if (p[0] != 0.0f && p[0] != 65535.0f) {
+                float inv = 65535.0f / p[0];
+                for (int c = 1; c < 4; c++) p[c] = px_rounded(fminf(p[c] * inv, 65535.0f));
+                px_store(q, p);
             }
-            hole = (uint16_t)(0xffffu - p[0]) != 0;
+            hole = p[0] != 65535.0f;
         } else {
             float* p = (float*)img + i * 4;
             if (!(1e-7 > (double)p[0])) {
@@ -288,25 +287,31 @@ __global__ void k_refill_post(void* __restrict__ img, int fmt, long n, const flo
     if (i >= n) return;
     const float K16 = __uint_as_float(0x37800080u);
     if (fmt == 0) {
-        uint8_t* p = (uint8_t*)img + i * 4;
+        uint8_t* q = (uint8_t*)img + i * 4;
+        float p[4];
+        px_floats<uint8_t>(q, p);
         if (plane) {
             int64_t v = as_i64(plane[i]);
-            p[0] = (uint8_t)(v < 0 ? 0 : v > 255 ? 255 : v);
+            p[0] = (float)(v < 0 ? 0 : v > 255 ? 255 : (int)v);
         } else {
-            p[0] = ((const uint8_t*)frame)[i * 4];
+            p[0] = (float)((const uint8_t*)frame)[i * 4];
         }
-        float a = (float)p[0] * __uint_as_float(0x3b808081u);  // image.rs:276-280
-        for (int c = 1; c < 4; c++) p[c] = (uint8_t)qround((float)p[c] * a);
+        float a = p[0] * __uint_as_float(0x3b808081u);  // image.rs:276-280
+        for (int c = 1; c < 4; c++) p[c] = px_rounded(p[c] * a);
+        px_store(q, p);
     } else if (fmt == 1) {
-        uint16_t* p = (uint16_t*)img + i * 4;
+        uint16_t* q = (uint16_t*)img + i * 4;
+        float p[4];
+        px_floats<uint16_t>(q, p);
         if (plane) {
             int64_t v = as_i64(plane[i]);
-            p[0] = (uint16_t)(v < 0 ? 0 : v > 65535 ? 65535 : v);
+            p[0] = (float)(v < 0 ? 0 : v > 65535 ? 65535 : (int)v);
         } else {
-            p[0] = ((const uint16_t*)frame)[i * 4];
+            p[0] = (float)((const uint16_t*)frame)[i * 4];
         }
-        float f = (float)p[0] * K16;
-        for (int c = 1; c < 4; c++) p[c] = (uint16_t)qround((float)p[c] * f);
+        float f = p[0] * K16;
+        for (int c = 1; c < 4; c++) p[c] = px_rounded(p[c] * f);
+        px_store(q, p);
     } else {
         float* p = (float*)img + i * 4;
         p[0] = plane ? plane[i] : ((const float*)frame)[i * 4];

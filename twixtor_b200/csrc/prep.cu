@@ -34,7 +34,7 @@ __global__ void k_delinearize(float* __restrict__ p, long n) {
 __global__ void k_edge_map(const float* __restrict__ src, float* __restrict__ dst, int w, int h) {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long)w * h) return;
-    int y = (int)(i / w), x = (int)(i - (long)y * w);
+    int y = row_of(i, w), x = (int)(i - (long)y * w);
     float c = src[i];
     float nx = 0.0f, dx = 0.0f, ny = 0.0f, dy = 0.0f;
     if (x >= 1) { nx = (c - src[i - 1]) + 0.0f; dx = 1.0f; }

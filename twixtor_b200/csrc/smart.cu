@@ -96,9 +96,9 @@ template <> struct SPx<uint8_t> {
         float y = x + 0.5f;
         if (0.0f > y) return 0;
         if (y > 255.0f) return 255;
-        return (uint8_t)cvtt64f(y);
+        return (uint8_t)__float2int_rz(y);  // (a NaN: 0)
     }
-    __device__ static uint8_t raw(float x) { return (uint8_t)cvtt64f(x); }
+    __device__ static uint8_t raw(float x) { return (uint8_t)cvtt_low(x); }
 };
 template <> struct SPx<uint16_t> {
     static constexpr float WHITE = 65535.0f;
@@ -106,9 +106,9 @@ template <> struct SPx<uint16_t> {
         float y = x + 0.5f;
         if (0.0f > y) return 0;
         if (y > 65535.0f) return 65535;
-        return (uint16_t)cvtt64f(y);
+        return (uint16_t)__float2int_rz(y);  // (a NaN: 0)
     }
-    __device__ static uint16_t raw(float x) { return (uint16_t)cvtt64f(x); }
+    __device__ static uint16_t raw(float x) { return (uint16_t)cvtt_low(x); }
 };
 template <> struct SPx<float> {
     static constexpr float WHITE = 1.0f;
@@ -119,17 +119,17 @@ template <> struct SPx<float> {
 // One Smart Blend pixel (smartblend.rs:268-298): p1 over p2 and p2 over p1 blended at w, or the
 // binary alpha variant; the raw store where the blended alpha came out 0, else the plain store.
 template <typename P>
-__device__ __forceinline__ void smart_blend_px(const P* ta, const P* tb, float w, bool binary, P* o) {
-    float p1[4], p2[4], v[4];
-    for (int k = 0; k < 4; k++) {
-        p1[k] = (float)ta[k];
-        p2[k] = (float)tb[k];
-    }
+__device__ __forceinline__ void smart_blend_px(const float p1[4], const float p2[4], float w, bool binary, float o[4]) {
+    float v[4];
     constexpr bool R = sizeof(P) == 4;  // NaN only reaches float images
     bool raw = false;
     if (binary) binary_px<R>(p1, p2, w, SPx<P>::WHITE, v);
     else raw = smart_px<R>(p1, p2, w, SPx<P>::WHITE, v);
-    for (int k = 0; k < 4; k++) o[k] = raw ? SPx<P>::raw(v[k]) : SPx<P>::plain(v[k]);
+    if (raw) {
+        for (int k = 0; k < 4; k++) o[k] = (float)SPx<P>::raw(v[k]);
+    } else {
+        for (int k = 0; k < 4; k++) o[k] = (float)SPx<P>::plain(v[k]);
+    }
 }
 
 // One pixel of warping code 1. mode 0: Nearest (one warp: pa), 1: Blend (pa = A, pb = B, w = frac).
@@ -141,7 +141,7 @@ __device__ __forceinline__ void compose_smart_px(const WarpParams& pa, const War
     int y = blockIdx.y;
     bool hole = false;
     if (x < W && y < H) {
-        P ta[4], tb[4], o[4];
+        float ta[4], tb[4], o[4];
         bool b = false;
         uint8_t c1 = warp_pixel<P>(pa, x, y, W, H, ta, b);
         uint8_t cov = c1;
@@ -153,8 +153,7 @@ __device__ __forceinline__ void compose_smart_px(const WarpParams& pa, const War
             smart_blend_px<P>(ta, tb, w, binary, o);
         }
         long i = (long)y * W + x;
-        P* dst = (P*)out + i * 4;
-        for (int k = 0; k < 4; k++) dst[k] = o[k];
+        px_store((P*)out + i * 4, o);
         uint8_t m = (uint8_t)(0xff - cov);
         holes[i] = m;
         hole = m != 0;  // a u8 mask value is a hole iff it is not 0 (holefill.rs:124-133)
@@ -172,14 +171,21 @@ __global__ void k_compose_smart(WarpParams pa, WarpParams pb, int fmt, int mode,
 }
 
 // smartblend.rs:305-315 on whole images (the stage entry point)
+template <typename P>
+__device__ __forceinline__ void smart_blend_at(const void* p1, const void* p2, float w, bool binary, void* out, long i) {
+    float a[4], b[4], o[4];
+    px_floats<P>((const P*)p1 + 4 * i, a);
+    px_floats<P>((const P*)p2 + 4 * i, b);
+    smart_blend_px<P>(a, b, w, binary, o);
+    px_store((P*)out + 4 * i, o);
+}
 __global__ void k_smart_blend(const void* __restrict__ p1, const void* __restrict__ p2, int fmt, float w, bool binary,
                               void* __restrict__ out, long n) {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    if (fmt == 0) smart_blend_px<uint8_t>((const uint8_t*)p1 + 4 * i, (const uint8_t*)p2 + 4 * i, w, binary, (uint8_t*)out + 4 * i);
-    else if (fmt == 1)
-        smart_blend_px<uint16_t>((const uint16_t*)p1 + 4 * i, (const uint16_t*)p2 + 4 * i, w, binary, (uint16_t*)out + 4 * i);
-    else smart_blend_px<float>((const float*)p1 + 4 * i, (const float*)p2 + 4 * i, w, binary, (float*)out + 4 * i);
+    if (fmt == 0) smart_blend_at<uint8_t>(p1, p2, w, binary, out, i);
+    else if (fmt == 1) smart_blend_at<uint16_t>(p1, p2, w, binary, out, i);
+    else smart_blend_at<float>(p1, p2, w, binary, out, i);
 }
 
 // holefill.rs:124-133: a pixel is a hole when !(eps > m) in double (a NaN float value is a hole);

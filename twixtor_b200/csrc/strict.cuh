@@ -27,8 +27,20 @@ __device__ __forceinline__ int64_t cvtt64f(float x) {
     if (!(x >= -9223372036854775808.0f && x < 9223372036854775808.0f)) return INT64_MIN;
     return __float2ll_rz(x);
 }
-// image.rs:255-258: q(x) = trunc((f64)x + 0.5); callers keep the low byte / word
-__device__ __forceinline__ int64_t qround(float x) { return cvtt64d((double)x + 0.5); }
+// The low 32 bits of cvtt64f(x), by the 32 bit conversion where that holds it
+__device__ __forceinline__ uint32_t cvtt_low(float x) {
+    return fabsf(x) < 2147483648.0f ? (uint32_t)__float2int_rz(x) : (uint32_t)cvtt64f(x);
+}
+// image.rs:255-258: q(x) = trunc((f64)x + 0.5); callers keep the low byte / word. The sum rounded toward zero
+// in single precision has the same whole part as the exact one, so no doubles are needed.
+__device__ __forceinline__ uint32_t qround(float x) { return cvtt_low(__fadd_rz(x, 0.5f)); }
+// trunc(x) of 0 <= x < 2^23 as the low bits of a float, 2^23 + trunc(x): a conversion at the adders' rate
+__device__ __forceinline__ float trunc_biased(float x) { return __fadd_rz(x, 8388608.0f); }
+// i / w for an element index and a row width: in 32 bits where the index has no more (a 64 bit division takes
+// some 70 instructions, most of a per element kernel)
+__device__ __forceinline__ int row_of(long i, int w) {
+    return i >> 32 ? (int)(i / w) : (int)((uint32_t)i / (uint32_t)w);
+}
 
 // warp.rs:129-135: clamp(trunc(v + 0.5), 0, 255) through the -128 bias and two saturations
 __device__ __forceinline__ uint8_t sat_u8(float v) {
