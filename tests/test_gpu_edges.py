@@ -61,3 +61,50 @@ def test_warps_between_the_ends_of_the_range(dev, fmt, size, wa, interp):
         got = dev.compose_vectors(tw.EngineSettings(), tw.Selection(wa=np.float32(wa), interp=interp), a, b, w, h, fmt,
                                   flows[0], flows[1], (w, h))
         assert same(got, O.compose_vectors(a, b, w, h, fmt, flows[0], flows[1], w, h, np.float32(wa), interp))
+
+
+@pytest.mark.parametrize("size", [(2, 2), (3, 200), (16, 17), (33, 32), (63, 64), (64, 65), (66, 31), (130, 129)])
+@pytest.mark.parametrize("fmt,above_first", [(0, True), (1, False), (2, True), (2, False)])
+def test_pyramid_steps_at_the_ends_of_their_tiles(dev, size, fmt, above_first):
+    """Planes of one tile of each shape and a pixel more or less; float samples include zeros of both signs and
+    magnitudes that the border division by reciprocals leaves to the plain division."""
+    w, h = size
+    rng = np.random.RandomState(w * 5 + h)
+    eng = rng.random_sample(w * h * 4) * {0: 255, 1: 65535, 2: 1}[fmt]
+    eng = eng.astype(tw.DTYPES[fmt])
+    if fmt == 2:
+        eng[rng.randint(0, eng.size, eng.size // 3)] = 0.0
+        eng[rng.randint(0, eng.size, eng.size // 8)] = -0.0
+        eng[rng.randint(0, eng.size, 3)] = [1e-40, 3e35, -2e-33]
+    s = tw.FlowSettings(quality=5, taps_above_first=above_first)
+    got = dev.build_pyramid(eng, w, h, fmt, s)
+    want = O.build_pyramid(eng, w, h, fmt, quality=5, above_first=above_first)
+    assert len(got) == len(want)
+    for g, o in zip(got, want):
+        assert same(g, o)
+
+
+@pytest.mark.parametrize("size", [(3, 3), (16, 15), (17, 33), (31, 66), (65, 64), (129, 48), (200, 9)])
+@pytest.mark.parametrize("masks", [False, True])
+@pytest.mark.parametrize("points", [None, (-1.0, 0.0), (-1.0, -1.0)])
+@pytest.mark.parametrize("above_first", [False, True])
+def test_solves_at_the_ends_of_their_tiles(dev, size, masks, points, above_first):
+    """Levels of one tile of each shape and a pixel more or less, in the one block of the coarse levels and out of
+    it. The points put vectors of exactly -1.0, the sentinel of the border rule, near the corners."""
+    w, h = size
+    rng = np.random.RandomState(w * 3 + h)
+    x = np.kron(rng.randint(0, 256, ((h + 2) // 3, (w + 2) // 3, 4)), np.ones((3, 3, 1)))[:h, :w].astype(np.uint8)
+    y = np.roll(x, 1, axis=1)
+    y[:, 0] = rng.randint(0, 256, (h, 4))
+    x, y = np.ascontiguousarray(x).reshape(-1), np.ascontiguousarray(y).reshape(-1)
+    mx = my = pairs = None
+    if masks:
+        mx, my = [(rng.random_sample((h, w)) < 0.9).astype(np.float32).ravel() for _ in range(2)]
+    if points:
+        at = np.array([[1.0, 1.0], [w - 1.0, 1.0], [1.0, h - 1.0], [w / 2, h / 2]], np.float32)
+        pairs = np.concatenate([at, at + np.float32(points)], 1).astype(np.float32)
+    kw = dict(quality=5, above_first=above_first)
+    want, xl, yl, mxl, myl, ud, uw = O.solve_pyramids_with(x, y, w, h, 0, mx, my, pairs, **kw)
+    s = tw.FlowSettings(quality=5, taps_above_first=above_first)
+    got, _ = dev.solve_pyramids(s, w, h, xl, yl, mxl, myl, ud, uw)
+    assert got.tobytes() == want.tobytes()

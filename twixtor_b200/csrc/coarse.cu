@@ -38,9 +38,6 @@ constexpr int GL = 4;        // lanes per segment of a line of block matching
 constexpr int NG = NT / GL;  // segments in flight
 constexpr int PAD = 7;       // what the longest filter reads past a line
 constexpr int RUN = 2;       // outputs per thread of a pass
-// the largest padded plane of a level of at most COARSE_MAX_PIXELS (16 x 128)
-constexpr int PLANE = 4800;
-
 // e / d for 0 <= e < 4096 and 1 <= d <= COARSE_MAX_LINE, from inverse_of(d)
 __device__ __forceinline__ unsigned inverse_of(int d) { return (1u << 20) / (unsigned)d + 1u; }
 __device__ __forceinline__ int over_of(int e, unsigned inv) { return (int)((unsigned)e * inv >> 20); }
@@ -265,22 +262,23 @@ __device__ __forceinline__ void sweep(const Coarse& C, bool reverse, float z) {
 
 __global__ void __launch_bounds__(COARSE_THREADS) k_solve_coarse(const __grid_constant__ CoarseJob J) {
     extern __shared__ __align__(16) float4 coarse_sm[];
-    constexpr int M = COARSE_MAX_PIXELS;
+    // block matching's planes (the flow's copy, the costs and the tests) lie in the tensor's, which it does not need
+    const int M = J.pixels, PLANE = J.plane;
     Coarse C;
     C.tensor = coarse_sm;
+    C.fn = (float2*)C.tensor;
+    C.cost = (float*)(C.fn + M);
+    C.takes = (unsigned char*)(C.cost + M);
     C.p1 = (float2*)(C.tensor + M);
     C.p2 = C.p1 + PLANE;
     C.grad = C.p2 + PLANE;
     C.f = C.grad + M;
-    C.fn = C.f + M;
-    C.den7x = C.fn + M;
+    C.den7x = C.f + M;
     C.den7y = C.den7x + COARSE_MAX_LINE;
     C.den5x = C.den7y + COARSE_MAX_LINE;
     C.den5y = C.den5x + COARSE_MAX_LINE;
-    C.cost = (float*)(C.den5y + COARSE_MAX_LINE);
-    C.a = C.cost + M;
+    C.a = (float*)(C.den5y + COARSE_MAX_LINE);
     C.b = C.a + M;
-    C.takes = (unsigned char*)(C.b + M);
     __shared__ int s_any[32];
     const int tid = threadIdx.x;
     const bool af = J.af;
@@ -435,15 +433,16 @@ __global__ void __launch_bounds__(COARSE_THREADS) k_solve_coarse(const __grid_co
             C.fn[i] = upsample_at(C.f, w, h, J.up[l], zero, damp_now, J.damp, x, y);
         }
         __syncthreads();
-        flip();
+        for (int i = tid; i < dw * dh; i += NT) C.f[i] = C.fn[i];
     }
     const int n = J.sizes[J.last][0] * J.sizes[J.last][1];
     for (int i = tid; i < n; i += NT) J.f_out[i] = C.f[i];
 }
 
-size_t coarse_smem_bytes() {
-    return (size_t)COARSE_MAX_PIXELS * (sizeof(float4) + 3 * sizeof(float2) + 3 * sizeof(float) + 1) +
-           (2 * PLANE + 4 * COARSE_MAX_LINE) * sizeof(float2);
+int coarse_plane(int w, int h) { return (h + 2 * PAD) * ((w + 2 * PAD + RUN) | 1); }
+size_t coarse_smem_bytes(int pixels, int plane) {
+    return (size_t)pixels * (sizeof(float4) + 2 * sizeof(float2) + 2 * sizeof(float)) +
+           (2 * (size_t)plane + 4 * COARSE_MAX_LINE) * sizeof(float2);
 }
 
 TW_VARIANT_END

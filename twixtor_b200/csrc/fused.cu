@@ -12,94 +12,237 @@
 namespace tw {
 TW_VARIANT_BEGIN
 
-constexpr int FT_X = 32;  // tile width (outputs)
-constexpr int FT_Y = 32;  // tile height
-constexpr int FT_THREADS = 1024;  // the launch bound; each launch picks 256 to 1024 threads
+// ---- a step of a pyramid (flow.rs:248-275): blur5, the band and the next size, in one launch ---------------
 
-// A separable pass over a shared-memory region, both directions:
-//   src: RH x RW region whose (0,0) is global (gx0, gy0); dst: OH x OW region at global (ox0, oy0).
-// Horizontal: dst(r, c) = pass along row gy0 + r (OH == RH, oy0 == gy0) at global column ox0 + c.
-// Vertical:   dst(r, c) = pass along column ox0 + c (OW == RW, ox0 == gx0) at global row oy0 + r.
-// Elements whose output position lies outside the image are left undefined (never read).
-template <int N, bool MULTI, bool VERT, bool ABOVE_FIRST>
-__device__ __forceinline__ void region_pass(const float* src, int RW, int gx0, int gy0, float* dst, int OW, int OH,
-                                            int ox0, int oy0, int w, int h, const float* k) {
-    for (int e = threadIdx.x; e < OW * OH; e += blockDim.x) {
-        int r = e / OW, c = e - r * OW;
-        int X = ox0 + c, Y = oy0 + r;
-        if (X < 0 || X >= w || Y < 0 || Y >= h) continue;
-        float v;
-        if (!VERT) {
-            const float* line = src + (Y - gy0) * RW;
-            v = pass_elem<N, MULTI, false>(line, gx0, 1, w, X, k);
-        } else {
-            const float* line = src + (X - gx0);
-            v = pass_elem<N, MULTI, ABOVE_FIRST>(line, gy0, RW, h, Y, k);
+// The single channel border rule by the division, for a run of sums that vquot does not divide.
+template <int R>
+__device__ __noinline__ void single_slow(float2* e, const float2* den, int i0, int len, int n) {
+#pragma unroll 1
+    for (int r = 0; r < R; r++)
+        if (i0 + r < n || i0 + r >= len - n) e[r] = make_float2(e[r].x / den[r].x, e[r].y / den[r].x);
+}
+
+// R outputs of the single channel rule (conv.rs:101-137, :141-190) of a pair of lines, from their R + 2N - 2
+// samples v (line indices i0 - (N - 1) on; samples outside the line are 0, which its taps add). The outputs near
+// the line's ends are divided by the weights inside it (den: border_den of each output).
+template <int N, int R, bool LEFT_FIRST>
+__device__ __forceinline__ void single_run(const float2* v, int i0, int len, const Taps& t, const float2* den, float2* res) {
+    if (i0 >= N && i0 + R - 1 < len - N) {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            float2 s = vmul(v[r + N - 1], t.k[0], t.z);
+#pragma unroll
+            for (int j = N - 1; j >= 1; j--) s = vmadd(s, vadd(v[r + N - 1 + j], v[r + N - 1 - j]), t.k[j], t.z);
+            res[r] = s;
         }
-        dst[e] = v;
+        return;
+    }
+    Magnitudes seen;
+    float2 sums[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int i = i0 + r;
+        const bool inner = i >= N && i < len - N;
+        const float2 c = vmul(v[r + N - 1], t.k[0], t.z);
+        float2 s = c, e = c;
+#pragma unroll
+        for (int j = N - 1; j >= 1; j--) {
+            s = vmadd(s, vadd(v[r + N - 1 + j], v[r + N - 1 - j]), t.k[j], t.z);
+            e = vmadd(e, LEFT_FIRST ? v[r + N - 1 - j] : v[r + N - 1 + j], t.k[j], t.z);
+            e = vmadd(e, LEFT_FIRST ? v[r + N - 1 + j] : v[r + N - 1 - j], t.k[j], t.z);
+        }
+        sums[r] = inner ? s : e;
+        const float2 q = vquot(e, den[r], seen);
+        res[r] = inner ? s : q;
+    }
+    if (!seen.safe()) {
+        single_slow<R>(sums, den, i0, len, N);
+#pragma unroll
+        for (int r = 0; r < R; r++) res[r] = sums[r];
     }
 }
 
-template <int N, bool MULTI>
-__device__ __forceinline__ void vpass(const float* src, int RW, int gx0, int gy0, float* dst, int OW, int OH, int ox0,
-                                      int oy0, int w, int h, const float* k, bool above_first) {
-    if (above_first) region_pass<N, MULTI, true, true>(src, RW, gx0, gy0, dst, OW, OH, ox0, oy0, w, h, k);
-    else region_pass<N, MULTI, true, false>(src, RW, gx0, gy0, dst, OW, OH, ox0, oy0, w, h, k);
+// flow/extras.rs:64-72: v >= 0.95 gives 1, else 0 (a NaN gives 0)
+__device__ __forceinline__ float binarized(float v) { return v >= 0.95f ? 1.0f : 0.0f; }
+
+// The tile of a step: T x T source pixels, their blur with one column and row more (the resample's second
+// taps) and the halo of the blur. The row pass takes the rows y and y + HP as a pair (rows a lane apart, so
+// that the lanes' loads fall into different banks), the column pass two columns next to each other; 4 outputs
+// per thread. Strides keep the scalar accesses free of conflicts and the pairs aligned.
+template <int T>
+struct PyramidGeom {
+    static constexpr int N = 3, HALO = N - 1, R = 4;
+    static constexpr int OUT = T + 1, SEG = (OUT + R - 1) / R, RC = T + 8, RS = RC + 1;
+    static constexpr int HP = (OUT + 2 * HALO + 1) / 2, HS = R * SEG + 2, HROWS = R * SEG + 2 * HALO;
+    static constexpr int CP = (OUT + 1) / 2, VS = 2 * CP + 1, VROWS = R * SEG;
+    static constexpr int DEN = R * SEG, CELLS = T + 2;
+    static_assert(2 * HP <= HROWS && R * SEG + 2 * HALO <= RC && HS % 2 == 0, "the planes hold every run");
+    static constexpr int O_H = 2 * HP * RS, O_V = O_H + HROWS * HS, O_TAB = (O_V + VROWS * VS + 1) / 2 * 2;
+    static constexpr int FLOATS = O_TAB + 2 * (2 * DEN + 2 * CELLS);
+};
+
+// The region's rows r, r + 1, ... (a warp each) and then its last 8 columns, through at(X, Y)
+template <int T, int NT, class At>
+__device__ __forceinline__ void pyramid_load(float* s_in, int X0, int Y0, int w, int h, At at) {
+    using G = PyramidGeom<T>;
+    const int tid = threadIdx.x;
+    constexpr int ROWS = 2 * G::HP, PER = NT / T, A = (ROWS + PER - 1) / PER, B = (ROWS * 8 + NT - 1) / NT;
+    float v[A + B];
+    const int c = tid % T, r0 = tid / T, X = X0 - G::HALO + c;
+#pragma unroll
+    for (int j = 0; j < A; j++) {
+        const int Y = Y0 - G::HALO + r0 + j * PER;
+        v[j] = X >= 0 && X < w && Y >= 0 && Y < h ? at(X, Y) : 0.0f;
+    }
+#pragma unroll
+    for (int j = 0; j < B; j++) {
+        const int e = tid + j * NT, X1 = X0 - G::HALO + T + e % 8, Y = Y0 - G::HALO + e / 8;
+        v[A + j] = e % 8 < G::OUT + 2 * G::HALO - T && X1 < w && Y >= 0 && Y < h ? at(X1, Y) : 0.0f;
+    }
+#pragma unroll
+    for (int j = 0; j < A; j++)
+        if (r0 + j * PER < ROWS) s_in[(r0 + j * PER) * G::RS + c] = v[j];
+#pragma unroll
+    for (int j = 0; j < B; j++) {
+        const int e = tid + j * NT;
+        if (e < ROWS * 8) s_in[e / 8 * G::RS + T + e % 8] = v[A + j];
+    }
 }
 
-// ---- pyramid: blur5 + band (flow.rs:261-268) and the first reduction step --------------------------
+// One step: blur = blur5(src) (src a plane, or the luma of an engine image computed on the way,
+// prep.rs:168-235), band = src - blur and its transpose, and dst = blur resampled to dw x dh
+// (sample.rs:91-112): each output belongs to the tile of its first tap; the sizes are such that a step is at
+// least 1 (dw = w / 2, and no less than 2). bin_in, bin_out: a mask's pyramid (flow/extras.rs:76-123), src and
+// dst binarized. sm: PyramidGeom<T>::FLOATS floats.
+template <int T, int NT>
+__device__ __forceinline__ void pyramid_step(const PyramidStep& P, float* sm, int X0, int Y0) {
+    using G = PyramidGeom<T>;
+    constexpr int R = G::R;
+    float *s_in = sm, *s_h = sm + G::O_H, *s_v = sm + G::O_V;
+    float2 *s_dx = (float2*)(sm + G::O_TAB), *s_dy = s_dx + G::DEN, *s_cx = s_dy + G::DEN, *s_cy = s_cx + G::CELLS;
+    const int w = P.w, h = P.h, tid = threadIdx.x;
+    if (P.luma_src) {
+        const int fmt = P.fmt, mode = P.luma_mode;
+        const void* img = P.luma_src;
+        auto load = [&](auto at) { pyramid_load<T, NT>(s_in, X0, Y0, w, h, at); };
+        // (the plain luma of each depth without the tests of a depth and a mode per sample)
+        if (mode == 0 && fmt == 0) load([&](int X, int Y) { return luma_px(img, 0, (long)Y * w + X, 0); });
+        else if (mode == 0 && fmt == 1) load([&](int X, int Y) { return luma_px(img, 1, (long)Y * w + X, 0); });
+        else if (mode == 0) load([&](int X, int Y) { return luma_px(img, 2, (long)Y * w + X, 0); });
+        else load([&](int X, int Y) { return luma_px(img, fmt, (long)Y * w + X, mode); });
+    } else if (P.bin_in) {
+        pyramid_load<T, NT>(s_in, X0, Y0, w, h, [&](int X, int Y) { return binarized(P.src[(long)Y * w + X]); });
+    } else {
+        pyramid_load<T, NT>(s_in, X0, Y0, w, h, [&](int X, int Y) { return P.src[(long)Y * w + X]; });
+    }
+    // the outputs xa .. (nx of them), ya .. (ny) whose first tap can lie in the tile: its ends over the step
+    int xa = 0, nx = 0, ya = 0, ny = 0;
+    if (P.dst) {
+        auto range = [](int at, int len, float step, int n, int& lo, int& count) {
+            lo = (int)((float)at / step);
+            count = min((at + T < len - 1 ? min((int)((float)(at + T) / step), n - 1) : n - 1) - lo + 1, G::CELLS);
+        };
+        range(X0, w, P.sx, P.dw, xa, nx);
+        range(Y0, h, P.sy, P.dh, ya, ny);
+    }
+    // the tables: border weights, and the cells of the outputs (first tap in the tile, or -1; fraction)
+    auto cell_at = [](int i, float step, int len, int at) {
+        int k;
+        float f;
+        cell((float)i * step, len, k, f);
+        k -= at;
+        return make_float2(__int_as_float(k >= 0 && k < T ? k : -1), f);
+    };
+    for (int i = tid; i < G::DEN; i += NT) {
+        s_dx[i] = border_den<G::N>(X0 + i, w, P.t.k);
+        s_dy[i] = border_den<G::N>(Y0 + i, h, P.t.k);
+    }
+    for (int i = NT - 1 - tid; i < G::CELLS; i += NT) {
+        if (i < nx) s_cx[i] = cell_at(xa + i, P.sx, w, X0);
+        if (i < ny) s_cy[i] = cell_at(ya + i, P.sy, h, Y0);
+    }
+    __syncthreads();
+    for (int e = tid; e < G::HP * G::SEG; e += NT) {
+        const int seg = e / G::HP, y = e - seg * G::HP;
+        const float *a = s_in + y * G::RS + seg * R, *b = a + G::HP * G::RS;
+        float2 in[R + 2 * G::N - 2], o[R];
+#pragma unroll
+        for (int j = 0; j < R + 2 * G::N - 2; j++) in[j] = make_float2(a[j], b[j]);
+        single_run<G::N, R, false>(in, X0 + seg * R, w, P.t, s_dx + seg * R, o);
+        float* out = s_h + y * G::HS + seg * R;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            out[r] = o[r].x;
+            out[G::HP * G::HS + r] = o[r].y;
+        }
+    }
+    __syncthreads();
+    for (int e = tid; e < G::CP * G::SEG; e += NT) {
+        const int seg = e / G::CP, c = e - seg * G::CP;
+        float2 in[R + 2 * G::N - 2], o[R];
+#pragma unroll
+        for (int j = 0; j < R + 2 * G::N - 2; j++) in[j] = *(const float2*)(s_h + (seg * R + j) * G::HS + 2 * c);
+        if (P.above_first) single_run<G::N, R, true>(in, Y0 + seg * R, h, P.t, s_dy + seg * R, o);
+        else single_run<G::N, R, false>(in, Y0 + seg * R, h, P.t, s_dy + seg * R, o);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            s_v[(seg * R + r) * G::VS + 2 * c] = o[r].x;
+            s_v[(seg * R + r) * G::VS + 2 * c + 1] = o[r].y;
+        }
+    }
+    __syncthreads();
+    const float* centre = s_in + G::HALO * G::RS + G::HALO;
+    const int u = tid % T, v0 = tid / T;
+    if (P.band && X0 + u < w) {
+        float* out = P.band + (long)(Y0 + v0) * w + X0 + u;
+#pragma unroll
+        for (int j = 0; j < T; j += NT / T)
+            if (Y0 + v0 + j < h) out[(long)j * w] = centre[(v0 + j) * G::RS + u] - s_v[(v0 + j) * G::VS + u];
+    }
+    if (P.band_t && Y0 + u < h) {  // element (x, y) at [x * h + y], for the column sweeps
+        float* out = P.band_t + (long)(X0 + v0) * h + Y0 + u;
+#pragma unroll
+        for (int j = 0; j < T; j += NT / T)
+            if (X0 + v0 + j < w) out[(long)j * h] = centre[u * G::RS + v0 + j] - s_v[u * G::VS + v0 + j];
+    }
+    constexpr int COLS = T / 2 + 2;  // the outputs across a tile at a step of 2
+    for (int x0 = 0; x0 < nx; x0 += COLS) {
+        for (int e = tid; e < COLS * ny; e += NT) {
+            const int y = e / COLS, x = x0 + e - y * COLS;
+            if (x >= nx) continue;
+            const float2 cx = s_cx[x], cy = s_cy[y];
+            const int ix = __float_as_int(cx.x), iy = __float_as_int(cy.x);
+            if (ix < 0 || iy < 0) continue;
+            const float* q = s_v + iy * G::VS + ix;
+            const float top = (q[1] - q[0]) * cx.y + q[0], bot = (q[G::VS + 1] - q[G::VS]) * cx.y + q[G::VS];
+            const float r = (bot - top) * cy.y + top;
+            P.dst[(long)(ya + y) * P.dw + xa + x] = P.bin_out ? binarized(r) : r;
+        }
+    }
+}
 
-// tmp = blur5(orig) and band = orig - tmp over one tile; orig is a plane, or (luma_src != nullptr)
-// the luma of an engine image computed on the fly (prep.rs:168-235; luma_mode: the LUMA_* bits).
-__global__ void __launch_bounds__(FT_THREADS) k_blur5_band(const float* __restrict__ orig, const void* __restrict__ luma_src,
-                                                           int fmt, int luma_mode, int w, int h, bool above_first,
-                                                           float* __restrict__ tmp_out, float* __restrict__ band_out,
-                                                           float* __restrict__ band_t_out) {
-    constexpr int N = 3, HALO = N - 1;
-    constexpr int RW = FT_X + 2 * HALO, RH = FT_Y + 2 * HALO;
-    __shared__ float s_in[RH * RW];
-    __shared__ float s_h[RH * FT_X];
-    __shared__ float s_t[FT_Y][FT_X + 1];  // the band tile, for the transposed copy
-    const float k[3] = {0.375f, 0.25f, 0.0625f};  // flow/conv.rs:48
-    int X0 = blockIdx.x * FT_X, Y0 = blockIdx.y * FT_Y;
-    int gx0 = X0 - HALO, gy0 = Y0 - HALO;
-    for (int e = threadIdx.x; e < RW * RH; e += blockDim.x) {
-        int r = e / RW, c = e - r * RW;
-        int X = gx0 + c, Y = gy0 + r;
-        float v = 0.0f;
-        if (X >= 0 && X < w && Y >= 0 && Y < h) {
-            long i = (long)Y * w + X;
-            v = luma_src ? luma_px(luma_src, fmt, i, luma_mode) : orig[i];
-        }
-        s_in[e] = v;
-    }
-    __syncthreads();
-    region_pass<N, false, false, false>(s_in, RW, gx0, gy0, s_h, FT_X, RH, X0, gy0, w, h, k);
-    __syncthreads();
-    for (int e = threadIdx.x; e < FT_X * FT_Y; e += blockDim.x) {
-        int r = e / FT_X, c = e - r * FT_X;
-        int X = X0 + c, Y = Y0 + r;
-        if (X >= w || Y >= h) continue;
-        const float* line = s_h + c;
-        float v = above_first ? pass_elem<N, false, true>(line, gy0, FT_X, h, Y, k)
-                              : pass_elem<N, false, false>(line, gy0, FT_X, h, Y, k);
-        long i = (long)Y * w + X;
-        tmp_out[i] = v;
-        if (band_out) {
-            float bv = s_in[(Y - gy0) * RW + (X - gx0)] - v;
-            band_out[i] = bv;
-            s_t[r][c] = bv;
-        }
-    }
-    if (band_t_out) {  // the band transposed (element (x, y) at [x * h + y]) for the column sweeps
+// Bound by issue at the large sizes (130 instructions per 8 bit pixel, 200 before) and by latency at the small
+// ones. A step was two launches with the blur's plane stored in between, scalar passes and a test per tap:
+// 1920 x 1080 to 960 x 540 22 us, now 17; 480 x 270 11, now 7.
+__global__ void __launch_bounds__(PYRAMID_THREADS_32) k_pyramid_step_32(const __grid_constant__ PyramidStep P) {
+    __shared__ __align__(16) float sm[PyramidGeom<32>::FLOATS];
+    pyramid_step<32, PYRAMID_THREADS_32>(P, sm, blockIdx.x * 32, blockIdx.y * 32);
+}
+__global__ void __launch_bounds__(PYRAMID_THREADS_16) k_pyramid_step_16(const __grid_constant__ PyramidStep P) {
+    __shared__ __align__(16) float sm[PyramidGeom<16>::FLOATS];
+    pyramid_step<16, PYRAMID_THREADS_16>(P, sm, blockIdx.x * 16, blockIdx.y * 16);
+}
+
+// The last steps of a pyramid, whose planes are one tile of 64 x 64 each: one block, a step after the other
+// (each plane but the first is this block's own of the step before).
+__global__ void __launch_bounds__(PYRAMID_TAIL_THREADS) k_pyramid_tail(const __grid_constant__ PyramidTail P) {
+    extern __shared__ __align__(16) float tail_sm[];
+    for (int i = 0; i < P.n; i++) {
+        pyramid_step<PYRAMID_TAIL, PYRAMID_TAIL_THREADS>(P.step[i], tail_sm, 0, 0);
         __syncthreads();
-        for (int e = threadIdx.x; e < FT_X * FT_Y; e += blockDim.x) {
-            int c = e / FT_Y, r = e - c * FT_Y;
-            int X = X0 + c, Y = Y0 + r;
-            if (X < w && Y < h) band_t_out[(long)X * h + Y] = s_t[r][c];
-        }
     }
 }
+size_t pyramid_tail_smem() { return PyramidGeom<PYRAMID_TAIL>::FLOATS * sizeof(float); }
 
 // ---- one solver level: the tile geometry of its kernels ----------------------------------------------
 
@@ -565,10 +708,10 @@ TW_VARIANT_END
 
 namespace tw {
 TW_VARIANT_BEGIN
-// flow/extras.rs:64-72: v >= 0.95 gives 1, else 0 (a NaN gives 0), in place
+// flow/extras.rs:64-72 of a plane in place
 __global__ void k_binarize(float* __restrict__ p, long n) {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = p[i] >= 0.95f ? 1.0f : 0.0f;
+    if (i < n) p[i] = binarized(p[i]);
 }
 TW_VARIANT_END
 }  // namespace tw

@@ -230,7 +230,8 @@ int tw_open(int device, tw_ctx** out) {
     TW_LIMIT(k_level_iter_32x64, level_iter_smem(LEVEL_TILE_32x64));
     TW_LIMIT(k_level_iter_64x32, level_iter_smem(LEVEL_TILE_64x32));
     TW_LIMIT(k_level_iter_64x64, level_iter_smem(LEVEL_TILE_64x64));
-    TW_LIMIT(k_solve_coarse, coarse_smem_bytes());
+    TW_LIMIT(k_pyramid_tail, pyramid_tail_smem());
+    TW_LIMIT(k_solve_coarse, coarse_smem_bytes(COARSE_MAX_PIXELS, COARSE_MAX_PLANE));
 #undef TW_LIMIT
     limit((const void*)k_fill_coarse, FILL_COARSE_MAX_FLOATS * sizeof(float));
     if (e != cudaSuccess) { tw_close(ctx); return TW_ERR_CUDA; }

@@ -250,7 +250,6 @@ static int layers_dev(tw_ctx* ctx, const tw_retime_settings& s, const tw_selecti
     float* scr = M + o_scr;
     int* flags = ctx->flags.as<int>();
     CHECK(ctx->cuda(cudaMemsetAsync(flags, 0, FLAGS_BYTES, ctx->stream), "flags"));
-    CHECK(ctx->cuda(cudaMemsetAsync(flags + FL_ONE, 0x01, sizeof(int), ctx->stream), "flags"));
     const void* frame[2] = {ctx->eng[0].p, ctx->eng[1].p};
     // the raw planes, the cut planes of a shrink (in the motion path's rows, as the plates run), the
     // per-level range flags are not in use yet
@@ -304,7 +303,7 @@ static int layers_dev(tw_ctx* ctx, const tw_retime_settings& s, const tw_selecti
             CHECK(build_pyramid_dev(ctx, img(side, k), W, H, fmt, fp, gk, pyr(g, side), pyr(g, side) + pf, LL.scratch[side]));
             LAUNCH(ctx, k_solver_mask, grid1(n), TB, 0, raw + (size_t)side * nfg * n, nfg, k,
                    comp + ((size_t)side * L + k) * n, n, fmt, sm);
-            CHECK(build_mask_pyramid_dev(ctx, sm, W, H, fs, gk, mpyr(g, side), sc, sc + n, flags + FL_ONE));
+            CHECK(build_mask_pyramid_dev(ctx, sm, W, H, fs, gk, mpyr(g, side), sc, sc + n));
             if (np_k > 0 && (side == 0 ? need_ab : need_ba)) {
                 UserPairs pr;
                 float* u = user + ((size_t)g * 2 + side) * 3 * pf;

@@ -149,15 +149,59 @@ LevelTune level_tune(tw_ctx* ctx, int w, int h) {
 // Threads per CTA of the tiled pyramid kernels: a level of few tiles is latency bound
 // (every CTA walks its stages one after the other), so its CTAs get more threads and each thread
 // fewer elements per stage; a level with tiles enough to fill the GPU keeps 256.
-static int level_threads(int w, int h) {
-    long tiles_n = (long)((w + 31) / 32) * ((h + 31) / 32);
-    return tiles_n <= 148 ? 1024 : tiles_n <= 296 ? 512 : 256;
+// ---- a step of a pyramid: the blur5 of src (or of the luma of luma_src), its band and transposed band, and the
+// next size's plane, each where asked for. Tiles of 32 x 32, or of 16 x 16 while the larger ones would not fill
+// the chip's 148 SMs (a 240 x 135 level: see pyramid_step's figures).
+PyramidStep pyramid_step_of(tw_ctx* ctx, const float* src, int w, int h, bool above_first, float* dst, int dw, int dh) {
+    PyramidStep P{};
+    P.src = src;
+    P.w = w;
+    P.h = h;
+    P.above_first = above_first;
+    P.dst = dst;
+    P.dw = dw;
+    P.dh = dh;
+    if (dst) {
+        P.sx = ((float)w - 1.0f) / (float)(dw - 1);
+        P.sy = ((float)h - 1.0f) / (float)(dh - 1);
+    }
+    P.t = ctx->b5;
+    return P;
 }
+
+// Queues steps: those of planes of at most 64 x 64 wait for each other in the tail and go in one launch of
+// one block (finish). A launch of a small step takes 5 us, nearly all of it latency.
+struct PyramidSteps {
+    tw_ctx* ctx;
+    bool fast;
+    PyramidTail tail;
+    double tail_bytes = 0;
+    PyramidSteps(tw_ctx* c, bool f) : ctx(c), fast(f) { std::memset(&tail, 0, sizeof tail); }
+    void add(const PyramidStep& P) {
+        double px = (double)P.w * P.h, in = P.luma_src ? 4.0 * sample_bytes(P.fmt) : 4.0;
+        double bytes = px * (in + (P.band ? 4.0 : 0.0) + (P.band_t ? 4.0 : 0.0)) + (P.dst ? 4.0 * P.dw * P.dh : 0.0);
+        if (P.w <= PYRAMID_TAIL && P.h <= PYRAMID_TAIL) {
+            if (tail.n == PYRAMID_TAIL_STEPS) finish();
+            tail.step[tail.n++] = P;
+            tail_bytes += bytes;
+            return;
+        }
+        auto grid = [&](int t) { return dim3((unsigned)((P.w + t - 1) / t), (unsigned)((P.h + t - 1) / t)); };
+        const dim3 g = grid(32);
+        if ((long)g.x * g.y <= 148) LAUNCHV(ctx, fast, bytes, k_pyramid_step_16, grid(16), PYRAMID_THREADS_16, 0, P);
+        else LAUNCHV(ctx, fast, bytes, k_pyramid_step_32, g, PYRAMID_THREADS_32, 0, P);
+    }
+    void finish() {
+        if (tail.n) LAUNCHV(ctx, fast, tail_bytes, k_pyramid_tail, 1, PYRAMID_TAIL_THREADS, pyramid_tail_smem(), tail);
+        tail.n = 0;
+        tail_bytes = 0;
+    }
+};
 
 // ---- the pyramid of one engine image (flow.rs:242-275) ----------------------------------------------
 // Builds the band pass levels into `out` (levels concatenated, finest first) and their transposes
 // into out_t. Luma, the reduction steps (prep.rs:252-259) and each level's blur5 + band run as
-// tiled kernels (k_blur5_band), each followed by the corner aligned resample to the next size.
+// tiled kernels (k_pyramid_step), each with the corner aligned resample to the next size.
 int build_pyramid_dev(tw_ctx* ctx, const void* eng_dev, int W, int H, int fmt, const tw_flow_settings& s, const Geo& g,
                       float* out, float* out_t, DevBuf* scratch) {
     if (s.video_range_luma && s.track_alpha)
@@ -202,20 +246,25 @@ int build_pyramid_dev(tw_ctx* ctx, const void* eng_dev, int W, int H, int fmt, c
         }
         return TW_OK;
     }
+    PyramidSteps steps(ctx, fast);
     if (g.reduction == 0) {
         long n = (long)W * H;
         LAUNCH(ctx, k_luma, grid1(n), TB, 0, eng_dev, fmt, cur, W, H, s.track_alpha != 0, s.video_range_luma != 0);
     }
     for (int r = 0; r < g.reduction; r++) {  // prep.rs:252-259; the first step reads the luma on the fly
-        LAUNCHV(ctx, fast, (r == 0 ? 4.0 * sample_bytes(fmt) : 4.0) * cw * ch + 4.0 * cw * ch, k_blur5_band, tiles(cw, ch),
-                FUSED_THREADS, 0, r == 0 ? (const float*)nullptr : cur, r == 0 ? eng_dev : nullptr, fmt, lmode, cw, ch, af, tmp,
-                (float*)nullptr, (float*)nullptr);
         int nw = cw / 2, nh = ch / 2;
-        LAUNCHV(ctx, fast, 0, k_resample, grid2(nw, nh), TB, 0, tmp, cw, ch, nxt, nw, nh);
+        PyramidStep P = pyramid_step_of(ctx, cur, cw, ch, af, nxt, nw, nh);
+        if (r == 0) {
+            P.luma_src = eng_dev;
+            P.fmt = fmt;
+            P.luma_mode = lmode;
+        }
+        steps.add(P);
         std::swap(cur, nxt);
         cw = nw;
         ch = nh;
     }
+    if (s.prep_delinearize || s.prep_contrast_edge) steps.finish();
     // flow.rs:248-253: the image prep of level 0, Delinearize then Contrast / Edge Enhance
     if (s.prep_delinearize) LAUNCH(ctx, k_delinearize, grid1((long)cw * ch), TB, 0, cur, (long)cw * ch);
     if (s.prep_contrast_edge) {
@@ -224,18 +273,18 @@ int build_pyramid_dev(tw_ctx* ctx, const void* eng_dev, int W, int H, int fmt, c
         std::swap(cur, nxt);
     }
     size_t off = 0;
-    size_t pf = pyramid_floats(g);
     for (int i = 0; i < g.levels; i++) {
         int lw = g.sizes[i][0], lh = g.sizes[i][1];
-        LAUNCHV(ctx, fast, 16.0 * lw * lh, k_blur5_band, tiles(lw, lh), level_threads(lw, lh), 0, cur, (const void*)nullptr, fmt, 0, lw,
-                lh, af, tmp, out + off, out_t ? out_t + off : (float*)nullptr);
-        if (i + 1 < g.levels) {
-            int nw = g.sizes[i + 1][0], nh = g.sizes[i + 1][1];
-            LAUNCHV(ctx, fast, 0, k_resample, grid2(nw, nh), TB, 0, tmp, lw, lh, cur, nw, nh);
-        }
+        const bool more = i + 1 < g.levels;
+        PyramidStep P = pyramid_step_of(ctx, cur, lw, lh, af, more ? nxt : nullptr, more ? g.sizes[i + 1][0] : 0,
+                                        more ? g.sizes[i + 1][1] : 0);
+        P.band = out + off;
+        P.band_t = out_t ? out_t + off : nullptr;
+        steps.add(P);
+        std::swap(cur, nxt);
         off += (size_t)lw * lh;
     }
-    (void)pf;
+    steps.finish();
     return TW_OK;
 }
 
@@ -373,6 +422,10 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
                 J.offs[i] = (int)offs[i];
                 if (i > 0) J.up[i] = upsample_scale(g.sizes[i][0], g.sizes[i][1], g.sizes[i - 1][0], g.sizes[i - 1][1]);
             }
+            for (int l = start; l >= last; l--) {
+                J.pixels = std::max(J.pixels, g.sizes[l][0] * g.sizes[l][1]);
+                J.plane = std::max(J.plane, coarse_plane(g.sizes[l][0], g.sizes[l][1]));
+            }
             J.start = start;
             J.last = last;
             J.damp_any = damp_any;
@@ -385,7 +438,8 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
             J.f_out = f;
             double px = 0.0;
             for (int l = start; l >= last; l--) px += (double)g.sizes[l][0] * g.sizes[l][1];
-            LAUNCHV(ctx, fast, 8.0 * px, k_solve_coarse, 1, COARSE_THREADS, coarse_smem_bytes(), J);
+            LAUNCHV(ctx, fast, 8.0 * px, k_solve_coarse, 1, COARSE_THREADS,
+                    coarse_smem_bytes(J.pixels, J.plane), J);
             first = last - 1;
             have_flow = false;
         }
@@ -490,46 +544,38 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
 // The binary mask pyramid of a matte (flow/extras.rs:76-123): binarize at 0.95, then per reduction
 // step and per level the blur5 (the pyramid's tap order), the corner aligned resample, binarize.
 // matte: w*h values 0..1 on the device (consumed); out: pyramid_floats(g) values, laid out like
-// the band pyramid; scratch: two planes of w*h. `one` points at a nonzero device int (the stack
-// passes run unconditionally).
+// the band pyramid; scratch: two planes of w*h.
 int build_mask_pyramid_dev(tw_ctx* ctx, float* matte, int W, int H, const tw_flow_settings& s, const Geo& g, float* out,
-                           float* scratch0, float* scratch1, const int* one) {
-    float* cur = matte;
-    float* tmp = scratch0;
-    float* nxt = scratch1;
+                           float* scratch0, float* scratch1) {
+    PyramidSteps steps(ctx, false);
+    const float* cur = matte;
+    float* planes[2] = {scratch0, scratch1};
     bool af = s.taps_above_first != 0;
-    // prep::blur5 of one plane into tmp: the band pyramid's tiled kernel (both passes in one launch)
-    auto blur5 = [&](const float* p, int w, int h) {
-        LAUNCHB(ctx, 8.0 * w * h, k_blur5_band, tiles(w, h), level_threads(w, h), 0, p, (const void*)nullptr, 0, 0, w, h,
-                af, tmp, (float*)nullptr, (float*)nullptr);
-    };
-    auto resample = [&](const float* src, int sw, int sh, float* dst, int dw, int dh) {
-        dim3 gp((unsigned)((dw + TB - 1) / TB), (unsigned)dh, 1);
-        LAUNCH(ctx, k_stack_resample, gp, TB, 0, src, sw, sh, (long)sw * sh, dst, dw, dh, (long)dw * dh, 0, one);
-        LAUNCH(ctx, k_binarize, grid1((long)dw * dh), TB, 0, dst, (long)dw * dh);
-    };
     int cw = W, ch = H;
-    LAUNCH(ctx, k_binarize, grid1((long)W * H), TB, 0, cur, (long)W * H);
-    for (int r = 0; r < g.reduction; r++) {
+    for (int r = 0; r < g.reduction; r++) {  // the last one leaves level 0
         int nw = cw / 2, nh = ch / 2;
-        blur5(cur, cw, ch);
-        resample(tmp, cw, ch, nxt, nw, nh);
-        std::swap(cur, nxt);
+        float* dst = r + 1 < g.reduction ? planes[r & 1] : out;
+        PyramidStep P = pyramid_step_of(ctx, cur, cw, ch, af, dst, nw, nh);
+        P.bin_in = r == 0;
+        P.bin_out = true;
+        steps.add(P);
+        cur = dst;
         cw = nw;
         ch = nh;
     }
-    size_t off = 0;
-    for (int i = 0; i < g.levels; i++) {
-        int lw = g.sizes[i][0], lh = g.sizes[i][1];
-        CHECK(ctx->cuda(cudaMemcpyAsync(out + off, cur, (size_t)lw * lh * sizeof(float), cudaMemcpyDeviceToDevice, ctx->cur),
-                        "mask level"));
-        off += (size_t)lw * lh;
-        if (i + 1 < g.levels) {
-            blur5(cur, lw, lh);
-            resample(tmp, lw, lh, nxt, g.sizes[i + 1][0], g.sizes[i + 1][1]);
-            std::swap(cur, nxt);
-        }
+    if (g.reduction == 0) {
+        long n = (long)W * H;
+        LAUNCH(ctx, k_binarize, grid1(n), TB, 0, matte, n);
+        CHECK(ctx->cuda(cudaMemcpyAsync(out, matte, (size_t)n * sizeof(float), cudaMemcpyDeviceToDevice, ctx->cur), "mask level"));
     }
+    for (int i = 0; i + 1 < g.levels; i++) {
+        float* next = out + (size_t)g.sizes[i][0] * g.sizes[i][1];
+        PyramidStep P = pyramid_step_of(ctx, out, g.sizes[i][0], g.sizes[i][1], af, next, g.sizes[i + 1][0], g.sizes[i + 1][1]);
+        P.bin_out = true;
+        steps.add(P);
+        out = next;
+    }
+    steps.finish();
     return TW_OK;
 }
 
@@ -633,12 +679,10 @@ int tw_solve_masked(tw_ctx* ctx, const tw_image* x, const tw_image* y, const tw_
         float* mt = ctx->holes.as<float>();
         CHECK(ctx->cuda(cudaMemcpyAsync(mt, matte_x, n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream), "matte upload"));
         CHECK(ctx->cuda(cudaMemcpyAsync(mt + n, matte_y, n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream), "matte upload"));
-        // a nonzero int for the stack passes' "run" flag
-        CHECK(ctx->cuda(cudaMemsetAsync(flags + FL_ONE, 0x01, sizeof(int), ctx->stream), "flags"));
         mx = ctx->masks.as<float>();
         my = mx + pf;
-        CHECK(build_mask_pyramid_dev(ctx, mt, W, H, *s, g, mx, mt + 2 * n, mt + 3 * n, flags + FL_ONE));
-        CHECK(build_mask_pyramid_dev(ctx, mt + n, W, H, *s, g, my, mt + 2 * n, mt + 3 * n, flags + FL_ONE));
+        CHECK(build_mask_pyramid_dev(ctx, mt, W, H, *s, g, mx, mt + 2 * n, mt + 3 * n));
+        CHECK(build_mask_pyramid_dev(ctx, mt + n, W, H, *s, g, my, mt + 2 * n, mt + 3 * n));
     }
     size_t fb = (size_t)g.w * g.h * 2 * sizeof(float);
     CHECK(ctx->ensure(ctx->flow[0], fb, "flow"));

@@ -128,10 +128,31 @@ __global__ void k_compose_blend(WarpParams pa, WarpParams pb, int fmt, float wbl
                                 int w, int h, bool to_wire, bool flip_out, int* __restrict__ bad);
 
 // ---- fused, shared-memory tiled kernels (fused.cu) -----------------------------------------------------
-constexpr int FUSED_TILE_X = 32, FUSED_TILE_Y = 32, FUSED_THREADS = 256;
-__global__ void k_blur5_band(const float* __restrict__ orig, const void* __restrict__ luma_src, int fmt, int luma_mode,
-                             int w, int h, bool above_first, float* __restrict__ tmp_out, float* __restrict__ band_out,
-                             float* __restrict__ band_t_out);
+// A step of a pyramid (fused.cu)
+struct PyramidStep {
+    const float* src;
+    const void* luma_src;  // not null: an engine image (fmt, luma_mode: the LUMA_* bits) whose luma is the source
+    int fmt, luma_mode;
+    int w, h;
+    bool above_first;
+    bool bin_in, bin_out;
+    float *band, *band_t;  // may be null
+    float* dst;            // the next size's plane, dw x dh (may be null)
+    int dw, dh;
+    float sx, sy;          // the resample's steps, (w - 1) / (dw - 1) and (h - 1) / (dh - 1)
+    Taps t;
+};
+constexpr int PYRAMID_THREADS_16 = 128, PYRAMID_THREADS_32 = 256;
+__global__ void k_pyramid_step_16(const __grid_constant__ PyramidStep P);
+__global__ void k_pyramid_step_32(const __grid_constant__ PyramidStep P);
+// The steps of the planes of at most PYRAMID_TAIL pixels a side
+constexpr int PYRAMID_TAIL = 64, PYRAMID_TAIL_THREADS = 512, PYRAMID_TAIL_STEPS = 8;
+struct PyramidTail {
+    PyramidStep step[PYRAMID_TAIL_STEPS];
+    int n;
+};
+__global__ void k_pyramid_tail(const __grid_constant__ PyramidTail P);
+size_t pyramid_tail_smem();
 // The launch shapes of the level kernels. The public codes of the iteration's tiles are the first three
 // (tw_tuning_set); the last two are shapes the defaults and the autotuner choose.
 enum { LEVEL_TILE_32x32 = 0, LEVEL_TILE_64x32 = 1, LEVEL_TILE_64x64 = 2, LEVEL_TILE_COUNT = 3, LEVEL_TILE_16x16 = 3,
@@ -208,6 +229,7 @@ struct CoarseJob {
     int offs[32];          // the first element of each level
     UpsampleScale up[32];  // from each level to the next finer one
     int start, last;
+    int pixels, plane;  // the most of a level and of its padded plane (coarse_plane)
     bool damp_any;  // the start level's damping differs from 1
     float damp;
     bool refine;  // block matching (not skip_refine)
@@ -217,7 +239,9 @@ struct CoarseJob {
     float2* f_out;
 };
 __global__ void k_solve_coarse(const __grid_constant__ CoarseJob job);
-size_t coarse_smem_bytes();
+int coarse_plane(int w, int h);
+constexpr int COARSE_MAX_PLANE = 4686;  // of 16 x 128, the largest padded plane of COARSE_MAX_PIXELS
+size_t coarse_smem_bytes(int pixels, int plane);
 __global__ void k_apply_upsample(const float2* __restrict__ src, int sw, int sh, UpsampleScale up,
                                  const int* __restrict__ any, int l, int start, bool damp_now, float damp,
                                  float2* __restrict__ dst, int dw, int dh);

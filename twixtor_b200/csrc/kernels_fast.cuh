@@ -7,7 +7,6 @@
 namespace tw {
 namespace fast {
 
-__global__ void k_resample(const float* __restrict__ src, int sw, int sh, float* __restrict__ dst, int dw, int dh);
 __global__ void k_range_any(const float2* __restrict__ f, int w, int h, int* __restrict__ any_in_range);
 __global__ void k_bm_rows(const float* __restrict__ A, const float* __restrict__ B, const float2* __restrict__ f, int w,
                           int h, float2* __restrict__ ft, float z);
@@ -15,9 +14,9 @@ __global__ void k_bm_cols(const float* __restrict__ AT, const float* __restrict_
                           int h, float2* f, float z);
 __global__ void k_transpose2(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ at,
                              float* __restrict__ bt, int w, int h);
-__global__ void k_blur5_band(const float* __restrict__ orig, const void* __restrict__ luma_src, int fmt, int luma_mode,
-                             int w, int h, bool above_first, float* __restrict__ tmp_out, float* __restrict__ band_out,
-                             float* __restrict__ band_t_out);
+__global__ void k_pyramid_step_16(const __grid_constant__ PyramidStep P);
+__global__ void k_pyramid_step_32(const __grid_constant__ PyramidStep P);
+__global__ void k_pyramid_tail(const __grid_constant__ PyramidTail P);
 __global__ void k_level_init_16x16(const __grid_constant__ LevelInitArgs P);
 __global__ void k_level_init_32x32(const __grid_constant__ LevelInitArgs P);
 __global__ void k_level_iter_16x16(const __grid_constant__ LevelIterArgs P);

@@ -85,7 +85,7 @@ __device__ __forceinline__ float plane_load(const float* p) {
 
 // flow/conv.rs:101-137 on a line held in shared memory: element t of the line (global index, inside
 // [0, len)) lives at line[(t - origin) * stride].
-template <int N, bool MULTI, bool LEFT_FIRST>
+template <int N, bool LEFT_FIRST>
 __device__ __forceinline__ float border_sm(const float* line, int origin, int stride, int len, int i, const float* k) {
     float centre = line[(i - origin) * stride];
     float num = k[0] * centre;
@@ -98,18 +98,11 @@ __device__ __forceinline__ float border_sm(const float* line, int origin, int st
             bool right = (side == 0) != LEFT_FIRST;
             int t = right ? i + j : i - j;
             bool inside = t >= 0 && t < len;
-            float xv, wv;
-            if (!MULTI) {
-                xv = inside ? line[(t - origin) * stride] : 0.0f;
-                wv = inside ? kj : 0.0f;
-            } else {
-                float v = inside ? line[(t - origin) * stride] : -1.0f;
-                float mask = (v != -1.0f) ? 1.0f : 0.0f;
-                xv = v;
-                wv = mask * kj;
-            }
+            float v = inside ? line[(t - origin) * stride] : -1.0f;
+            float mask = (v != -1.0f) ? 1.0f : 0.0f;
+            float wv = mask * kj;
             den = den + wv;
-            num = num + xv * wv;
+            num = num + v * wv;
         }
     }
     return num / den;
@@ -117,7 +110,7 @@ __device__ __forceinline__ float border_sm(const float* line, int origin, int st
 
 // One output of a pass along a line (conv.rs:141-190 horizontally, :268-301 vertically): the
 // interior chain for elements whose taps all lie inside [n, len - n), the border rule otherwise.
-template <int N, bool MULTI, bool LEFT_FIRST>
+template <int N, bool LEFT_FIRST>
 __device__ __forceinline__ float pass_elem(const float* line, int origin, int stride, int len, int i, const float* k) {
     if (len >= 2 * N && i >= N && i < len - N) {
         const float* c = line + (i - origin) * stride;
@@ -126,7 +119,7 @@ __device__ __forceinline__ float pass_elem(const float* line, int origin, int st
         for (int j = N - 1; j >= 1; j--) s = s + (c[j * stride] + c[-j * stride]) * k[j];
         return s;
     }
-    return border_sm<N, MULTI, LEFT_FIRST>(line, origin, stride, len, i, k);
+    return border_sm<N, LEFT_FIRST>(line, origin, stride, len, i, k);
 }
 
 // The weight sum of the border rule at line index i (conv.rs:101-137) when no sample is the sentinel:
@@ -177,7 +170,7 @@ __device__ __forceinline__ void new_disp_run(const float2* b, const float4* t, f
 // real samples of exactly -1.0, which run_pass sends here. line: line index `origin` at line[0].
 template <int N, bool LEFT_FIRST>
 __device__ __noinline__ float slow_elem(const float* line, int origin, int stride, int len, int i, const float* k) {
-    return pass_elem<N, true, LEFT_FIRST>(line, origin, stride, len, i, k);
+    return pass_elem<N, LEFT_FIRST>(line, origin, stride, len, i, k);
 }
 template <int N, bool LEFT_FIRST>
 __device__ __forceinline__ float slow_pass(const float* line, int origin, int stride, int len, int i, const float* k) {

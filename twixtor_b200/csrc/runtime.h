@@ -268,13 +268,13 @@ void launch_kernel(tw_ctx* ctx, void (*k)(P...), dim3 grid, dim3 block, size_t s
 constexpr int TB = 256;
 // device flags (ints): [0..31] per-level range flags of solve 0, [32..63] of solve 1, [64] NaN in a
 // flow, [65] a warp refused a sample coordinate
-constexpr int FL_ANY0 = 0, FL_ANY1 = 32, FL_NAN = 64, FL_BAD = 65, FL_HOLE = 66, FL_SIDE1 = 67, FL_ONE = 68, FL_WB = 69,
+constexpr int FL_ANY0 = 0, FL_ANY1 = 32, FL_NAN = 64, FL_BAD = 65, FL_HOLE = 66, FL_SIDE1 = 67, FL_WB = 69,
               FL_BOUND = 70;  // [70] a device loop reached its bound
 constexpr size_t FLAGS_BYTES = 128 * sizeof(int);
 
 inline dim3 grid2(int w, int h) { return dim3((unsigned)((w + TB - 1) / TB), (unsigned)h); }
 inline unsigned grid1(long n) { return (unsigned)((n + TB - 1) / TB); }
-inline dim3 tiles(int w, int h) { return dim3((unsigned)((w + FUSED_TILE_X - 1) / FUSED_TILE_X), (unsigned)((h + FUSED_TILE_Y - 1) / FUSED_TILE_Y)); }
+inline dim3 tiles(int w, int h) { return dim3((unsigned)((w + 31) / 32), (unsigned)((h + 31) / 32)); }
 
 // Scratch of the warping code 1 composition: the composite (engine image), its holes mask, the
 // fill's planes, and the device flag "some pixel is a hole".
@@ -327,7 +327,7 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
                        const float* mx = nullptr, const float* my = nullptr, const float* udu = nullptr,
                        const float* udv = nullptr, const float* uww = nullptr);
 int build_mask_pyramid_dev(tw_ctx* ctx, float* matte, int W, int H, const tw_flow_settings& s, const Geo& g, float* out,
-                           float* scratch0, float* scratch1, const int* one);
+                           float* scratch0, float* scratch1);
 
 // host_compose.cu
 bool warp_copy_only(float amount, int fw, int width);
