@@ -108,3 +108,35 @@ def test_solves_at_the_ends_of_their_tiles(dev, size, masks, points, above_first
     s = tw.FlowSettings(quality=5, taps_above_first=above_first)
     got, _ = dev.solve_pyramids(s, w, h, xl, yl, mxl, myl, ud, uw)
     assert got.tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("size", [(2, 2), (2, 33), (32, 32), (33, 65), (66, 31), (129, 97)])
+@pytest.mark.parametrize("fmt", [0, 1, 2, "flow"])
+@pytest.mark.parametrize("above_first", [False, True])
+def test_hole_fill_at_the_ends_of_its_tiles(dev, size, fmt, above_first):
+    """Images of one tile and a pixel more or less: sparse holes, all holes and tiles without one, and for floats
+    zeros of both signs, infinities and NaNs (signalling ones too) in and beside the holes."""
+    w, h = size
+    n = w * h
+    rng = np.random.RandomState(w + 7 * h)
+    channels = 2 if fmt == "flow" else 4
+    if fmt in (0, 1):
+        img = rng.randint(0, 256 if fmt == 0 else 65536, n * channels).astype(tw.DTYPES[fmt])
+    else:
+        img = (rng.random_sample(n * channels) * 2 - 1).astype(np.float32)
+        img[rng.randint(0, img.size, max(img.size // 9, 1))] = 0.0
+        img[rng.randint(0, img.size, max(img.size // 9, 1))] = -0.0
+    masks = [(rng.random_sample(n) < p).astype(np.uint8) for p in (0.02, 0.5)] + [np.ones(n, np.uint8)]
+    masks.append((np.arange(n) % w < 3).astype(np.uint8))
+    for k, mask in enumerate(masks):
+        src = img.copy()
+        if fmt in (2, "flow") and k % 2:
+            src.view(np.uint32)[rng.randint(0, src.size, 3)] = [0x7fc00123, 0xffc04567, 0x7f800001]
+            src[rng.randint(0, src.size, 2)] = [np.inf, -np.inf]
+        if fmt == "flow":
+            got = dev.fill_flow_holes(src.copy(), w, h, mask, taps_above_first=above_first)
+            want = O.fill_flow_holes(src.copy(), w, h, mask, 1, above_first)
+        else:
+            got = dev.fill_holes(src.copy(), w, h, fmt, mask, taps_above_first=above_first)
+            want = O.fill_holes(src.copy(), w, h, fmt, mask, 1, above_first)
+        assert same(got, want)

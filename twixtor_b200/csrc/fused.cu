@@ -14,54 +14,6 @@ TW_VARIANT_BEGIN
 
 // ---- a step of a pyramid (flow.rs:248-275): blur5, the band and the next size, in one launch ---------------
 
-// The single channel border rule by the division, for a run of sums that vquot does not divide.
-template <int R>
-__device__ __noinline__ void single_slow(float2* e, const float2* den, int i0, int len, int n) {
-#pragma unroll 1
-    for (int r = 0; r < R; r++)
-        if (i0 + r < n || i0 + r >= len - n) e[r] = make_float2(e[r].x / den[r].x, e[r].y / den[r].x);
-}
-
-// R outputs of the single channel rule (conv.rs:101-137, :141-190) of a pair of lines, from their R + 2N - 2
-// samples v (line indices i0 - (N - 1) on; samples outside the line are 0, which its taps add). The outputs near
-// the line's ends are divided by the weights inside it (den: border_den of each output).
-template <int N, int R, bool LEFT_FIRST>
-__device__ __forceinline__ void single_run(const float2* v, int i0, int len, const Taps& t, const float2* den, float2* res) {
-    if (i0 >= N && i0 + R - 1 < len - N) {
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            float2 s = vmul(v[r + N - 1], t.k[0], t.z);
-#pragma unroll
-            for (int j = N - 1; j >= 1; j--) s = vmadd(s, vadd(v[r + N - 1 + j], v[r + N - 1 - j]), t.k[j], t.z);
-            res[r] = s;
-        }
-        return;
-    }
-    Magnitudes seen;
-    float2 sums[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-        const int i = i0 + r;
-        const bool inner = i >= N && i < len - N;
-        const float2 c = vmul(v[r + N - 1], t.k[0], t.z);
-        float2 s = c, e = c;
-#pragma unroll
-        for (int j = N - 1; j >= 1; j--) {
-            s = vmadd(s, vadd(v[r + N - 1 + j], v[r + N - 1 - j]), t.k[j], t.z);
-            e = vmadd(e, LEFT_FIRST ? v[r + N - 1 - j] : v[r + N - 1 + j], t.k[j], t.z);
-            e = vmadd(e, LEFT_FIRST ? v[r + N - 1 + j] : v[r + N - 1 - j], t.k[j], t.z);
-        }
-        sums[r] = inner ? s : e;
-        const float2 q = vquot(e, den[r], seen);
-        res[r] = inner ? s : q;
-    }
-    if (!seen.safe()) {
-        single_slow<R>(sums, den, i0, len, N);
-#pragma unroll
-        for (int r = 0; r < R; r++) res[r] = sums[r];
-    }
-}
-
 // flow/extras.rs:64-72: v >= 0.95 gives 1, else 0 (a NaN gives 0)
 __device__ __forceinline__ float binarized(float v) { return v >= 0.95f ? 1.0f : 0.0f; }
 

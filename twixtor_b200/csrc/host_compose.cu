@@ -74,64 +74,61 @@ FillGeo fill_geometry(int w, int h) {  // holefill.rs:140-171
     return g;
 }
 
-// one blur of a stack of planes, out of place (src stays as it is): both passes in one tiled launch
-void fill_blur(tw_ctx* ctx, const float* src, float* dst, int w, int h, long stride, int planes, const Taps& t, int n,
-               bool above_first, int rule, const int* any) {
-    dim3 g((unsigned)((w + 31) / 32), (unsigned)((h + 31) / 32), (unsigned)planes);
-    double pb = 8.0 * w * h * planes;  // every plane read once and written once
-    LAUNCHB(ctx, pb, k_stack_blur, g, 256, 0, src, dst, w, h, stride, t, n, above_first ? 1 : 0, rule, any);
-}
-
-void fill_resample(tw_ctx* ctx, const float* src, int sw, int sh, float* dst, int dw, int dh, int planes, int rule,
-                   const int* any) {
-    dim3 g((unsigned)((dw + TB - 1) / TB), (unsigned)dh, (unsigned)planes);
-    LAUNCHB(ctx, 4.0 * planes * ((double)sw * sh + (double)dw * dh), k_stack_resample, g, TB, 0, src, sw, sh, (long)sw * sh, dst,
-            dw, dh, (long)dw * dh, rule, any);
-}
-
 // The pull-push fill of an engine image in place (holefill.rs:260-350, :452-491) with the u8
 // holes mask; every kernel returns at once when *any (no hole) is 0. Per level a stack of the
 // channels' value planes and the weights: five planes for an engine image, three for an
-// interleaved flow (fmt FILL_FLOW, holefill.rs:497-518). Float images and flows run the NaN rule
-// arithmetic (for numbers the plain arithmetic bit for bit, and where a NaN reaches the result the
-// bits of the reference's repeat with the rule).
+// interleaved flow (fmt FILL_FLOW, holefill.rs:497-518); level 0 is the image itself. Float images and
+// flows run the NaN rule arithmetic (for numbers the plain arithmetic bit for bit, and where a NaN
+// reaches the result the bits of the reference's repeat with the rule).
 int fill_dev(tw_ctx* ctx, void* img, int W, int H, int fmt, const uint8_t* holes, const int* any, bool above_first,
              DevBuf& fb) {
     int rule = fmt == TW_F32 || fmt == FILL_FLOW;
     int nc = fmt == FILL_FLOW ? 2 : 4;  // value planes; the weights are plane nc
     int np = nc + 1;
     FillGeo g = fill_geometry(W, H);
-    long n0 = (long)W * H;
-    size_t offs[40];
-    size_t tot = 0;
-    for (int k = 0; k <= g.top; k++) { offs[k] = tot; tot += np * (size_t)g.dims[k][0] * g.dims[k][1]; }
-    size_t o_ta = tot, o_sa = tot + np * n0, o_sb = o_sa + nc * n0;
-    tot = o_sb + nc * n0;
-    CHECK(ctx->ensure(fb, tot * sizeof(float), "hole fill planes"));
-    float* base = fb.as<float>();
-    float* ta = base + o_ta;
-    LAUNCH(ctx, k_fill_load, grid1(n0), TB, 0, img, fmt, holes, base + offs[0], n0, any);
     // the coarse levels k0 .. top (every stack of them fits one block's shared memory) run in one
     // launch, k_fill_coarse: the finest such level k0 >= 1 is built by the pull below, the launch
-    // pulls on from it, pushes down to it and leaves the push's level k0 - 1 in the solution planes
-    int k0 = g.top + 1;
-    for (int k = 1; k <= g.top; k++)
-        if (fill_coarse_floats(g.dims, k, g.top, np, nc) <= FILL_COARSE_MAX_FLOATS) { k0 = k; break; }
-    const int pull_to = k0 <= g.top ? k0 : g.top;
-    for (int k = 1; k <= pull_to; k++) {  // pull: blur5 and the resample of the values and the weights
-        int pw = g.dims[k - 1][0], ph = g.dims[k - 1][1], cw = g.dims[k][0], chh = g.dims[k][1];
-        long pn = (long)pw * ph;
-        // the level k - 1 planes stay for the push: the blur writes ta
-        fill_blur(ctx, base + offs[k - 1], ta, pw, ph, pn, np, ctx->b5, 3, above_first, rule, any);
-        fill_resample(ctx, ta, pw, ph, base + offs[k], cw, chh, np, rule, any);
+    // pulls on from it, pushes down to it and leaves the push's level k0 - 1 in the solution planes. There is
+    // one: the top level is 2 x 2.
+    int k0 = 1;
+    while (k0 < g.top && fill_coarse_floats(g.dims, k0, g.top, np, nc) > FILL_COARSE_MAX_FLOATS) k0++;
+    auto pixels = [&](int k) { return (size_t)g.dims[k][0] * g.dims[k][1]; };
+    size_t offs[40];
+    size_t tot = 0;
+    for (int k = 1; k <= k0; k++) { offs[k] = tot; tot += (np * pixels(k) + 3) / 4 * 4; }
+    const size_t o_sol = tot, o_a = o_sol + (nc * pixels(k0 - 1) + 3) / 4 * 4, o_b = o_a + (nc * pixels(1) + 3) / 4 * 4;
+    tot = o_b + nc * pixels(1);
+    CHECK(ctx->ensure(fb, tot * sizeof(float), "hole fill planes"));
+    float* base = fb.as<float>();
+    auto grid = [&](int k, int z) { return dim3((unsigned)((g.dims[k][0] + 31) / 32), (unsigned)((g.dims[k][1] + 31) / 32), (unsigned)z); };
+    auto step = [](int from, int to) { return ((float)from - 1.0f) / (float)(to - 1); };
+    for (int k = 1; k <= k0; k++) {  // pull: blur5 and the resample of the values and the weights
+        FillPull P{};
+        if (k == 1) {
+            P.img = img;
+            P.holes = holes;
+        } else {
+            P.vals = base + offs[k - 1];
+        }
+        P.dst = base + offs[k];
+        P.fmt = fmt;
+        P.nc = nc;
+        P.w = g.dims[k - 1][0];
+        P.h = g.dims[k - 1][1];
+        P.dw = g.dims[k][0];
+        P.dh = g.dims[k][1];
+        P.sx = step(P.w, P.dw);
+        P.sy = step(P.h, P.dh);
+        P.t = ctx->b5;
+        P.above_first = above_first;
+        P.rule = rule;
+        P.any = any;
+        LAUNCHB(ctx, 4.0 * np * ((double)pixels(k - 1) + (double)pixels(k)), k_fill_pull, grid(k - 1, nc / 2 + 1), FILL_THREADS, 0, P);
     }
-    float* sol = base + o_sa;
-    float* nxt = base + o_sb;
-    int push_from = g.top;
-    if (k0 <= g.top) {
+    {
         FillCoarseJob J{};
         J.s_k0 = base + offs[k0];
-        J.out = sol;
+        J.out = base + o_sol;
         for (int k = 0; k <= g.top; k++) {
             J.dims[k][0] = g.dims[k][0];
             J.dims[k][1] = g.dims[k][1];
@@ -146,27 +143,38 @@ int fill_dev(tw_ctx* ctx, void* img, int W, int H, int fmt, const uint8_t* holes
         J.g5 = ctx->g5;
         J.any = any;
         // the stack of level k0 read, the push's level k0 - 1 written
-        double b = 4.0 * ((double)np * g.dims[k0][0] * g.dims[k0][1] + (double)nc * g.dims[k0 - 1][0] * g.dims[k0 - 1][1]);
+        double b = 4.0 * ((double)np * pixels(k0) + (double)nc * pixels(k0 - 1));
         LAUNCHB(ctx, b, k_fill_coarse, 1, FILL_COARSE_THREADS, fill_coarse_floats(g.dims, k0, g.top, np, nc) * sizeof(float), J);
-        push_from = k0 - 1;
-    } else {
-        long tn = (long)g.dims[g.top][0] * g.dims[g.top][1];
-        LAUNCH(ctx, k_stack_zero, grid1(nc * tn), TB, 0, sol, nc * tn, any);
     }
-    for (int lv = push_from; lv >= 0; lv--) {  // push
-        int lw = g.dims[lv][0], lh = g.dims[lv][1];
-        long ln = (long)lw * lh;
-        LAUNCH(ctx, k_fill_combine, grid1(ln), TB, 0, sol, base + offs[lv], ln, nc, rule, any);
-        fill_blur(ctx, sol, ta, lw, lh, ln, nc, ctx->g5, 6, above_first, rule, any);  // the blurred solution in ta
+    float* blurred[2] = {base + o_a, base + o_b};
+    for (int lv = k0 - 1; lv >= 0; lv--) {  // push
+        FillPush P{};
         if (lv == 0) {
-            LAUNCH(ctx, k_fill_combine, grid1(ln), TB, 0, ta, base + offs[0], ln, nc, rule, any);
-            sol = ta;
+            P.img = img;
+            P.holes = holes;
         } else {
-            fill_resample(ctx, ta, lw, lh, nxt, g.dims[lv - 1][0], g.dims[lv - 1][1], nc, rule, any);
-            std::swap(sol, nxt);
+            P.vals = base + offs[lv];
+            P.out = (float2*)blurred[lv & 1];
         }
+        if (lv == k0 - 1) {
+            P.direct = base + o_sol;
+        } else {
+            P.coarse = (const float2*)blurred[(lv + 1) & 1];
+            P.cw = g.dims[lv + 1][0];
+            P.ch = g.dims[lv + 1][1];
+            P.sx = step(P.cw, g.dims[lv][0]);
+            P.sy = step(P.ch, g.dims[lv][1]);
+        }
+        P.fmt = fmt;
+        P.nc = nc;
+        P.w = g.dims[lv][0];
+        P.h = g.dims[lv][1];
+        P.t = ctx->g5;
+        P.above_first = above_first;
+        P.rule = rule;
+        P.any = any;
+        LAUNCHB(ctx, 4.0 * (np + nc) * (double)pixels(lv), k_fill_push, grid(lv, nc / 2), FILL_THREADS, 0, P);
     }
-    LAUNCH(ctx, k_fill_store, grid1(n0), TB, 0, img, fmt, sol, n0, any);
     return TW_OK;
 }
 

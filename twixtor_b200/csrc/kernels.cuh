@@ -260,22 +260,37 @@ __global__ void k_cov_holes(const uint8_t* __restrict__ c1, const uint8_t* __res
                             long n, int* __restrict__ any_hole);
 __global__ void k_mask_holes(const void* __restrict__ mask, int kind, uint8_t* __restrict__ holes, long n,
                              int* __restrict__ any_hole);
-// The format code of an interleaved 2 channel flow in the hole fill (k_fill_load, k_fill_store, fill_dev)
+// The format code of an interleaved 2 channel flow in the hole fill (fill_dev)
 constexpr int FILL_FLOW = 3;
-__global__ void k_fill_load(const void* __restrict__ img, int fmt, const uint8_t* __restrict__ holes,
-                            float* __restrict__ stack, long n, const int* __restrict__ any_hole);
-// both passes of the fill's blur (horizontal, then vertical, the vertical border taps above first
-// with above_first) out of place, 32 x 32 output tiles per block and plane; 256 threads; n: 3
-// (blur5) or 6 (Gaussian r5) taps; rule: the NaN rule arithmetic (float images and flows)
-__global__ void k_stack_blur(const float* __restrict__ src, float* __restrict__ dst, int w, int h, long pstride, Taps t,
-                             int n, int above_first, int rule, const int* __restrict__ any_hole);
-__global__ void k_stack_resample(const float* __restrict__ src, int sw, int sh, long sstride, float* __restrict__ dst,
-                                 int dw, int dh, long dstride, int rule, const int* __restrict__ any_hole);
-__global__ void k_fill_combine(float* __restrict__ sol, const float* __restrict__ vals, long n, int nc, int rule,
-                               const int* __restrict__ any_hole);
-__global__ void k_fill_store(void* __restrict__ img, int fmt, const float* __restrict__ sol, long n,
-                             const int* __restrict__ any_hole);
-__global__ void k_stack_zero(float* __restrict__ p, long n, const int* __restrict__ any_hole);
+constexpr int FILL_THREADS = 256;
+// A level of the hole fill up and down (smart.cu). The stack of a level is planes of single channels: nc
+// values, then the weights.
+struct FillPull {
+    const void* img;       // level 0 (vals null): the image or flow, its holes mask
+    const uint8_t* holes;
+    const float* vals;     // the stack of level k - 1, w x h
+    float* dst;            // the stack of level k, dw x dh
+    int fmt, nc, w, h, dw, dh;
+    float sx, sy;          // the resample's steps
+    Taps t;
+    bool above_first, rule;
+    const int* any;
+};
+struct FillPush {
+    void* img;             // level 0: the image or flow, filled in place, and its holes mask; else null
+    const uint8_t* holes;
+    const float* vals;     // the stack of the level, w x h
+    const float* direct;   // the coarser solution at this level's size, planes of single channels, or (null)
+    const float2* coarse;  // of cw x ch, planes of pairs of channels
+    float2* out;           // the blurred solution, likewise
+    int fmt, nc, w, h, cw, ch;
+    float sx, sy;
+    Taps t;
+    bool above_first, rule;
+    const int* any;
+};
+__global__ void k_fill_pull(const __grid_constant__ FillPull P);
+__global__ void k_fill_push(const __grid_constant__ FillPush P);
 __global__ void k_hole_side1(const int* __restrict__ any_hole, int* __restrict__ flag);
 // The coarse levels of the pull-push fill in one block: the pull from level k0 (its stack given,
 // np planes) up to the top level and the push from the top down to level k0, every stack of those

@@ -2,13 +2,13 @@
 //
 // k_compose_smart: the two inverse warps with their coverage (warp.rs:504-561, hold off), the
 // Smart Blend composite (smartblend.rs:168-262) and the holes mask (255 - max of the coverages,
-// smartblend.rs:335-345), one pixel per thread. The fill (holefill.rs) then runs on "plane stacks":
-// the four channels and the weight plane of a level side by side (blockIdx.z picks the plane),
-// every kernel a no-op when the mask has no hole (the fill is the identity then). Float images
-// run the fill's operations with the NaN rule throughout: for numbers it is the plain arithmetic
-// bit for bit, and where a NaN reaches the result it gives the bits the reference's repeat with the
-// rule gives.
+// smartblend.rs:335-345), one pixel per thread. The fill (holefill.rs) then goes up a pyramid of the
+// values and their weights and down again, a launch per level and direction, every kernel a no-op
+// when the mask has no hole (the fill is the identity then). Float images run the fill's operations
+// with the NaN rule: for numbers it is the plain arithmetic bit for bit, and an element that comes
+// out as a NaN is taken again with the rule, which gives the bits the reference's repeat gives.
 #include "kernels.cuh"
+#include "level.cuh"
 #include "warp.cuh"
 
 namespace tw {
@@ -225,36 +225,6 @@ __global__ void k_cov_holes(const uint8_t* __restrict__ c1, const uint8_t* __res
 
 // ---- the hole fill on plane stacks (holefill.rs) ------------------------------------------------------
 
-// holefill.rs:300-313 + :452-491: level 0 of the value planes (the four channels, holes zeroed)
-// and of the weight plane (0 at a hole, else 1).
-template <typename P>
-__device__ __forceinline__ void fill_load_px(const void* img, const uint8_t* holes, float* stack, long n, long i) {
-    const P* px = (const P*)img + i * 4;
-    bool hole = holes[i] != 0;
-    for (int c = 0; c < 4; c++) stack[c * n + i] = hole ? 0.0f : (float)px[c];
-    stack[4 * n + i] = hole ? 0.0f : 1.0f;
-}
-
-// holefill.rs:510-517: the two components of an interleaved flow (FILL_FLOW) as value planes
-__device__ __forceinline__ void fill_load_flow(const void* img, const uint8_t* holes, float* stack, long n, long i) {
-    float2 v = ((const float2*)img)[i];
-    bool hole = holes[i] != 0;
-    stack[i] = hole ? 0.0f : v.x;
-    stack[n + i] = hole ? 0.0f : v.y;
-    stack[2 * n + i] = hole ? 0.0f : 1.0f;
-}
-
-__global__ void k_fill_load(const void* __restrict__ img, int fmt, const uint8_t* __restrict__ holes,
-                            float* __restrict__ stack, long n, const int* __restrict__ any_hole) {
-    if (!*any_hole) return;
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (fmt == 0) fill_load_px<uint8_t>(img, holes, stack, n, i);
-    else if (fmt == 1) fill_load_px<uint16_t>(img, holes, stack, n, i);
-    else if (fmt == FILL_FLOW) fill_load_flow(img, holes, stack, n, i);
-    else fill_load_px<float>(img, holes, stack, n, i);
-}
-
 // flow/conv.rs border element (1 channel rule) over an arithmetic set
 template <bool R, bool LEFT_FIRST, int N>
 __device__ __forceinline__ float border1(const float* line, long stride, int len, int i, const float* k) {
@@ -306,7 +276,7 @@ __device__ __forceinline__ float stack_pass_px(const float* __restrict__ s, int 
     return r;
 }
 
-// ---- both passes of the fill's blur in one launch ---------------------------------------------------
+// ---- the fill's levels in tiles ----------------------------------------------------------------------
 
 // One element of a pass along a line held in shared memory: element t (global index in [0, len)) of
 // the line at line[(t - origin) * stride]; the interior chain or the 1 channel border rule, the
@@ -339,51 +309,330 @@ __device__ __forceinline__ float stack_elem(const float* line, int origin, int s
     return Ar<R>::div(num, den);
 }
 
-// dst = the separable blur (horizontal, then vertical) of the stack src, out of place: a 32 x 32
-// output tile per block and plane (blockIdx.z), its region with the halo of N - 1 in shared memory
-// (the halo's horizontal pass computed again by the neighbouring tiles).
-constexpr int SB_TX = 32, SB_TY = 32, SB_MAXN = 6;  // the tile and the widest kernel (the push's r5 Gaussian)
-constexpr int SB_IN = (SB_TY + 2 * SB_MAXN - 2) * (SB_TX + 2 * SB_MAXN - 1), SB_H = (SB_TY + 2 * SB_MAXN - 2) * (SB_TX + 1);
+// The NaN rule's results, out of the main path
+template <int N, bool LEFT_FIRST>
+__device__ __noinline__ float2 fill_rule_elem(const float2* line, int origin, int stride, int len, int i, const Taps& t) {
+    const float* f = reinterpret_cast<const float*>(line);
+    return make_float2(stack_elem<true, N, LEFT_FIRST>(f, origin, 2 * stride, len, i, t),
+                       stack_elem<true, N, LEFT_FIRST>(f + 1, origin, 2 * stride, len, i, t));
+}
+__device__ __noinline__ float2 fill_rule_mix(float2 a, float2 b, float2 c, float2 d, float fx, float fy) {
+    auto mix = [&](float a, float b, float c, float d) {
+        return lerp_r<true>(lerp_r<true>(a, b, fx), lerp_r<true>(c, d, fx), fy);
+    };
+    return make_float2(mix(a.x, b.x, c.x, d.x), mix(a.y, b.y, c.y, d.y));
+}
+__device__ __noinline__ float2 fill_rule_quot(float2 v, float d) { return make_float2(nr::div(v.x, d), nr::div(v.y, d)); }
+__device__ __forceinline__ bool any_nan(float2 v) { return isnan(v.x) || isnan(v.y); }
 
-template <bool R, int N, bool ABOVE_FIRST>
-__device__ __forceinline__ void stack_blur_tile(const float* __restrict__ src, float* __restrict__ dst, int w, int h,
-                                                long pstride, const Taps& t, float* s_in, float* s_h) {
-    constexpr int TX = SB_TX, TY = SB_TY, HL = N - 1, RW = TX + 2 * HL, RH = TY + 2 * HL, RS = RW + 1, HS = TX + 1;
-    static_assert(N <= SB_MAXN && RH * RS <= SB_IN && RH * HS <= SB_H, "the shared buffers hold the widest region");
-    const float* s = src + blockIdx.z * pstride;
-    const int X0 = blockIdx.x * TX, Y0 = blockIdx.y * TY, gx0 = X0 - HL, gy0 = Y0 - HL;
-    for (int e = threadIdx.x; e < RH * RW; e += blockDim.x) {
-        const int r = e / RW, c = e - r * RW, X = gx0 + c, Y = gy0 + r;
-        s_in[r * RS + c] = (X >= 0 && X < w && Y >= 0 && Y < h) ? s[(long)Y * w + X] : 0.0f;
+// v / d: the reciprocal correctly rounded and Markstein's corrections in a pair (level.cuh) for operands within
+// 2^60 of 1; others divide. Most weights are 1.
+__device__ __forceinline__ float2 fill_quot(float2 v, float d, bool rule) {
+    float2 q = v;
+    if (d != 1.0f) {
+        const float lo = 8.67e-19f, hi = 1.15e18f;  // 2^-60, 2^60
+        auto in = [&](float x) { return fabsf(x) > lo && fabsf(x) < hi; };
+        if (in(d) && (v.x == 0.0f || in(v.x)) && (v.y == 0.0f || in(v.y))) {
+            const float y = __frcp_rn(d);
+            const float2 n = make_float2(-d, -d), yy = make_float2(y, y);
+            const float2 q0 = __ffma2_rn(v, yy, make_float2(-0.0f, -0.0f));
+            q = __ffma2_rn(__ffma2_rn(q0, n, v), yy, q0);
+            q = __ffma2_rn(__ffma2_rn(q, n, v), yy, q);
+            q = make_float2(v.x == 0.0f ? q0.x : q.x, v.y == 0.0f ? q0.y : q.y);
+        } else {
+            q = make_float2(v.x / d, v.y / d);
+        }
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < RH * TX; e += blockDim.x) {
-        const int r = e / TX, c = e - r * TX, X = X0 + c, Y = gy0 + r;
-        if (X < w && Y >= 0 && Y < h) s_h[r * HS + c] = stack_elem<R, N, false>(s_in + r * RS, gx0, 1, w, X, t);
+    return rule && any_nan(q) ? fill_rule_quot(v, d) : q;
+}
+
+// Four taps a b / c d of a pair mixed (flow/sample.rs:91-112)
+__device__ __forceinline__ float2 fill_mix(float2 a, float2 b, float2 c, float2 d, float fx, float fy, float z, bool rule) {
+    const float2 fx2 = make_float2(fx, fx), z2 = make_float2(z, z);
+    const float2 top = px_lerp(a, a, b, fx2, z2), bot = px_lerp(c, c, d, fx2, z2);
+    const float2 r = px_lerp(top, top, bot, make_float2(fy, fy), z2);
+    return rule && any_nan(r) ? fill_rule_mix(a, b, c, d, fx, fy) : r;
+}
+
+// The tile of a level: 32 x 32 outputs of the blur with N taps (the pull: blur5, one output more each way for the
+// resample's second taps; the push: the Gaussian), two channels of a pixel as a pair. 4 outputs per thread,
+// rows a lane apart in the row pass and columns a lane apart in the column pass.
+template <int N>
+struct FillGeom {
+    static constexpr int T = 32, R = 4, HALO = N - 1, OUT = N == 3 ? T + 1 : T, SEG = (OUT + R - 1) / R;
+    static constexpr int ROWS = OUT + 2 * HALO, RUNS = R * SEG + 2 * HALO, RS = RUNS | 1, HS = R * SEG | 1, VS = OUT | 1;
+    static constexpr int EX = N == 3 ? 8 : 16;  // the region's columns right of the first 32 (RUNS - T of them)
+    static constexpr int IN = ROWS * RS, MID = RUNS * HS;
+    static_assert(RUNS - T <= EX && SEG * R * VS <= IN, "the planes hold every run");
+};
+
+// The region of a tile at (X0, Y0), at(X, Y) inside the image and 0 outside
+template <int N, class At>
+__device__ __forceinline__ void fill_region(float2* s_in, int X0, int Y0, int w, int h, At at) {
+    using G = FillGeom<N>;
+    const int tid = threadIdx.x, c = tid % G::T, r0 = tid / G::T;
+    constexpr int PER = FILL_THREADS / G::T, A = (G::ROWS + PER - 1) / PER, B = (G::ROWS * G::EX + FILL_THREADS - 1) / FILL_THREADS;
+    float2 v[A + B];
+    // column and row of the region (no others are looked at: `at` may hold tables of the region's size)
+    auto value = [&](int x, int y) {
+        const int X = X0 - G::HALO + x, Y = Y0 - G::HALO + y;
+        return x < G::RUNS && y < G::ROWS && X >= 0 && X < w && Y >= 0 && Y < h ? at(X, Y) : make_float2(0.0f, 0.0f);
+    };
+#pragma unroll
+    for (int j = 0; j < A; j++) v[j] = value(c, r0 + j * PER);
+#pragma unroll
+    for (int j = 0; j < B; j++) {
+        const int e = tid + j * FILL_THREADS;
+        v[A + j] = value(G::T + e % G::EX, e / G::EX);
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < TY * TX; e += blockDim.x) {
-        const int r = e / TX, c = e - r * TX, X = X0 + c, Y = Y0 + r;
-        if (X < w && Y < h)
-            dst[blockIdx.z * pstride + (long)Y * w + X] = stack_elem<R, N, ABOVE_FIRST>(s_h + c, gy0, HS, h, Y, t);
+#pragma unroll
+    for (int j = 0; j < A; j++)
+        if (r0 + j * PER < G::ROWS) s_in[(r0 + j * PER) * G::RS + c] = v[j];
+#pragma unroll
+    for (int j = 0; j < B; j++) {
+        const int e = tid + j * FILL_THREADS;
+        if (e / G::EX < G::ROWS && e % G::EX < G::RUNS - G::T) s_in[e / G::EX * G::RS + G::T + e % G::EX] = v[A + j];
     }
 }
 
-__global__ void __launch_bounds__(256) k_stack_blur(const float* __restrict__ src, float* __restrict__ dst, int w, int h,
-                                                    long pstride, Taps t, int n, int above_first, int rule,
-                                                    const int* __restrict__ any_hole) {
-    if (!*any_hole) return;
-    __shared__ float s_in[SB_IN];
-    __shared__ float s_h[SB_H];
-#define TW_SB(Rr, Nn, Aa) stack_blur_tile<Rr, Nn, Aa>(src, dst, w, h, pstride, t, s_in, s_h)
+// A run of R outputs of a pass: line is the sample at index i0 - (N - 1), `first` the first one held
+template <int N, bool LEFT_FIRST>
+__device__ __forceinline__ void fill_run(const float2* line, int stride, int i0, int len, int held, const Taps& t,
+                                         const float2* den, bool rule, float2* o) {
+    constexpr int R = FillGeom<N>::R;
+    float2 v[R + 2 * N - 2];
+#pragma unroll
+    for (int j = 0; j < R + 2 * N - 2; j++) v[j] = line[j * stride];
+    single_run<N, R, LEFT_FIRST>(v, i0, len, t, den, o);
     if (rule) {
-        if (n == 3) { if (above_first) TW_SB(true, 3, true); else TW_SB(true, 3, false); }
-        else { if (above_first) TW_SB(true, 6, true); else TW_SB(true, 6, false); }
-    } else {
-        if (n == 3) { if (above_first) TW_SB(false, 3, true); else TW_SB(false, 3, false); }
-        else { if (above_first) TW_SB(false, 6, true); else TW_SB(false, 6, false); }
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            if (any_nan(o[r]) && i0 + r < min(len, held)) o[r] = fill_rule_elem<N, LEFT_FIRST>(line, i0 - (N - 1), stride, len, i0 + r, t);
     }
-#undef TW_SB
+}
+
+// Both passes of the region in s_in through s_h; out(seg, x, values): the 4 outputs of column x from row 4 * seg on
+template <int N, class Out>
+__device__ __forceinline__ void fill_blur(const float2* s_in, float2* s_h, const float2* s_dx, const float2* s_dy, int X0, int Y0,
+                                          int w, int h, const Taps& t, bool above_first, bool rule, Out out) {
+    using G = FillGeom<N>;
+    for (int e = threadIdx.x; e < G::ROWS * G::SEG; e += FILL_THREADS) {
+        const int seg = e / G::ROWS, y = e - seg * G::ROWS;
+        float2 o[G::R];
+        fill_run<N, false>(s_in + y * G::RS + seg * G::R, 1, X0 + seg * G::R, w, X0 + G::OUT, t, s_dx + seg * G::R, rule, o);
+#pragma unroll
+        for (int r = 0; r < G::R; r++) s_h[y * G::HS + seg * G::R + r] = o[r];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < G::OUT * G::SEG; e += FILL_THREADS) {
+        const int seg = e / G::OUT, x = e - seg * G::OUT;
+        float2 o[G::R];
+        const float2* line = s_h + seg * G::R * G::HS + x;
+        if (above_first) fill_run<N, true>(line, G::HS, Y0 + seg * G::R, h, Y0 + G::OUT, t, s_dy + seg * G::R, rule, o);
+        else fill_run<N, false>(line, G::HS, Y0 + seg * G::R, h, Y0 + G::OUT, t, s_dy + seg * G::R, rule, o);
+        out(seg, x, o);
+    }
+}
+
+// Channels 2 * pair and 2 * pair + 1 of an image's pixel i (a flow's vector)
+template <int FMT>
+__device__ __forceinline__ float2 fill_sample(const void* img, long i, int pair) {
+    if (FMT == FILL_FLOW) return ((const float2*)img)[i];
+    if (FMT == 2) return ((const float2*)img)[2 * i + pair];
+    if (FMT == 0) {
+        const Px4 q = px_load((const uint8_t*)img + 4 * i);
+        return px_value<uint8_t>(pair ? q.b : q.a);
+    }
+    const Px4 q = px_load((const uint16_t*)img + 4 * i);
+    return px_value<uint16_t>(pair ? q.b : q.a);
+}
+
+template <int FMT>
+__device__ __forceinline__ void fill_pull_image(const FillPull& P, float2* s_in, int X0, int Y0, int pair) {
+    const bool weights = 2 * pair == P.nc;
+    fill_region<3>(s_in, X0, Y0, P.w, P.h, [&](int X, int Y) {
+        const long i = (long)Y * P.w + X;
+        if (P.holes[i]) return make_float2(0.0f, 0.0f);
+        return weights ? make_float2(1.0f, 0.0f) : fill_sample<FMT>(P.img, i, pair);
+    });
+}
+
+// One level up (holefill.rs:300-350): blur5 of level k - 1 and the resample to level k, a pair of channels
+// or the weights (blockIdx.z); level 0 is the image itself with its holes at zero weight. Each output belongs
+// to the tile of its first tap.
+//
+// Bound by issue. With planes of single channels, a launch for the load, the blur and the resample each and a
+// test per tap, a 1080p level 0 took 14 + 50 + 12 us. Flows filled at 1080p: 38 us for a level's
+// blur and resample on average, now 19.
+__global__ void __launch_bounds__(FILL_THREADS) k_fill_pull(const __grid_constant__ FillPull P) {
+    using G = FillGeom<3>;
+    if (!*P.any) return;
+    __shared__ float2 s_in[G::IN], s_h[G::MID];
+    __shared__ float2 s_dx[G::R * G::SEG], s_dy[G::R * G::SEG], s_cx[G::T + 2], s_cy[G::T + 2];
+    const int w = P.w, h = P.h, X0 = blockIdx.x * G::T, Y0 = blockIdx.y * G::T, pair = blockIdx.z, tid = threadIdx.x;
+    const long n = (long)w * h;
+    const bool rule = P.rule, weights = 2 * pair == P.nc;
+    if (P.vals) {
+        const float *a = P.vals + 2 * pair * n, *b = weights ? nullptr : a + n;
+        fill_region<3>(s_in, X0, Y0, w, h, [&](int X, int Y) {
+            const long i = (long)Y * w + X;
+            return make_float2(a[i], b ? b[i] : 0.0f);
+        });
+    } else if (P.fmt == 0) fill_pull_image<0>(P, s_in, X0, Y0, pair);
+    else if (P.fmt == 1) fill_pull_image<1>(P, s_in, X0, Y0, pair);
+    else if (P.fmt == 2) fill_pull_image<2>(P, s_in, X0, Y0, pair);
+    else fill_pull_image<FILL_FLOW>(P, s_in, X0, Y0, pair);
+    // the outputs whose first tap can lie in the tile, from its ends over the step (at least 1)
+    auto range = [](int at, int len, float step, int n, int& lo, int& count) {
+        lo = (int)((float)at / step);
+        count = min((at + G::T < len - 1 ? min((int)((float)(at + G::T) / step), n - 1) : n - 1) - lo + 1, G::T + 2);
+    };
+    int xa, nx, ya, ny;
+    range(X0, w, P.sx, P.dw, xa, nx);
+    range(Y0, h, P.sy, P.dh, ya, ny);
+    auto cell_at = [](int i, float step, int len, int at) {
+        int k;
+        float f;
+        cell((float)i * step, len, k, f);
+        k -= at;
+        return make_float2(__int_as_float(k >= 0 && k < G::T ? k : -1), f);
+    };
+    if (tid < G::R * G::SEG) {
+        s_dx[tid] = border_den<3>(X0 + tid, w, P.t.k);
+        s_dy[tid] = border_den<3>(Y0 + tid, h, P.t.k);
+    }
+    const int k = FILL_THREADS - 1 - tid;
+    if (k < nx) s_cx[k] = cell_at(xa + k, P.sx, w, X0);
+    if (k < ny) s_cy[k] = cell_at(ya + k, P.sy, h, Y0);
+    __syncthreads();
+    float2* s_v = s_in;  // (the column pass reads s_h alone)
+    fill_blur<3>(s_in, s_h, s_dx, s_dy, X0, Y0, w, h, P.t, P.above_first, rule, [&](int seg, int x, const float2* o) {
+#pragma unroll
+        for (int r = 0; r < G::R; r++) s_v[(seg * G::R + r) * G::VS + x] = o[r];
+    });
+    __syncthreads();
+    constexpr int COLS = G::T / 2 + 2;  // the outputs across a tile at a step of 2
+    const long dn = (long)P.dw * P.dh;
+    float *da = P.dst + 2 * pair * dn, *db = weights ? nullptr : da + dn;
+    for (int x0 = 0; x0 < nx; x0 += COLS) {
+        for (int e = tid; e < COLS * ny; e += FILL_THREADS) {
+            const int y = e / COLS, x = x0 + e - y * COLS;
+            if (x >= nx) continue;
+            const float2 cx = s_cx[x], cy = s_cy[y];
+            const int ix = __float_as_int(cx.x), iy = __float_as_int(cy.x);
+            if (ix < 0 || iy < 0) continue;
+            const float2* q = s_v + iy * G::VS + ix;
+            const float2 r = fill_mix(q[0], q[1], q[G::VS], q[G::VS + 1], cx.y, cy.y, P.t.z, rule);
+            const long i = (long)(ya + y) * P.dw + xa + x;
+            da[i] = r.x;
+            if (db) db[i] = r.y;
+        }
+    }
+}
+
+// A sample as stored (holefill.rs:379-404)
+template <int FMT>
+__device__ __forceinline__ void fill_put(void* img, long i, int pair, float2 v) {
+    if (FMT == 0) ((uchar2*)img)[2 * i + pair] = make_uchar2(SPx<uint8_t>::plain(v.x), SPx<uint8_t>::plain(v.y));
+    else if (FMT == 1) ((ushort2*)img)[2 * i + pair] = make_ushort2(SPx<uint16_t>::plain(v.x), SPx<uint16_t>::plain(v.y));
+    else if (FMT == 2) ((float2*)img)[2 * i + pair] = v;
+    else ((float2*)img)[i] = v;
+}
+
+// The solution of the coarser level at (X, Y): resampled, or given at this size
+__device__ __forceinline__ float2 fill_coarser(const FillPush& P, const float2* s_cx, const float2* s_cy, int X0, int Y0, int X,
+                                               int Y, int pair) {
+    if (P.direct) {
+        const long n = (long)P.w * P.h, i = (long)Y * P.w + X;
+        return make_float2(P.direct[2 * pair * n + i], P.direct[(2 * pair + 1) * n + i]);
+    }
+    const float2 cx = s_cx[X - X0], cy = s_cy[Y - Y0];
+    const float2* q = P.coarse + (long)pair * P.cw * P.ch + (long)__float_as_int(cy.x) * P.cw + __float_as_int(cx.x);
+    return fill_mix(q[0], q[1], q[P.cw], q[P.cw + 1], cx.y, cy.y, P.t.z, P.rule);
+}
+
+template <int FMT>  // -1: a level of planes
+__device__ __forceinline__ void fill_push(const FillPush& P, float2* s_in, float2* s_h, const float2* s_dx, const float2* s_dy,
+                                          const float2* s_cx, const float2* s_cy) {
+    using G = FillGeom<6>;
+    const int w = P.w, h = P.h, X0 = blockIdx.x * G::T, Y0 = blockIdx.y * G::T, pair = blockIdx.z;
+    const int HX = X0 - G::HALO, HY = Y0 - G::HALO;
+    const long n = (long)w * h;
+    const float *va = P.vals + 2 * pair * n, *wt = P.vals + P.nc * n;
+    fill_region<6>(s_in, X0, Y0, w, h, [&](int X, int Y) {
+        const long i = (long)Y * w + X;
+        if (FMT >= 0) {
+            if (P.holes[i]) return fill_coarser(P, s_cx, s_cy, HX, HY, X, Y, pair);
+            return fill_quot(fill_sample<FMT>(P.img, i, pair), 1.0f, P.rule);
+        }
+        const float d = wt[i];
+        if (d == 0.0f) return fill_coarser(P, s_cx, s_cy, HX, HY, X, Y, pair);
+        return fill_quot(make_float2(va[i], va[n + i]), d, P.rule);
+    });
+    __syncthreads();
+    fill_blur<6>(s_in, s_h, s_dx, s_dy, X0, Y0, w, h, P.t, P.above_first, P.rule, [&](int seg, int x, const float2* o) {
+#pragma unroll
+        for (int r = 0; r < G::R; r++) {
+            const int X = X0 + x, Y = Y0 + seg * G::R + r;
+            if (X >= w || Y >= h) continue;
+            const long i = (long)Y * w + X;
+            if (FMT < 0) P.out[pair * n + i] = o[r];
+            else if (P.holes[i]) fill_put<(FMT < 0 ? 0 : FMT)>(P.img, i, pair, o[r]);
+        }
+    });
+}
+
+// One level down (holefill.rs:352-404): the values over their weights, the coarser solution where there is no
+// weight, and the Gaussian of it; a pair of channels (blockIdx.z). At level 0 (an image) the holes take it and
+// the other pixels stay as they are, but for a NaN that the rule's division by 1 quiets; a tile without a
+// hole has nothing to do. No tile reads what another writes: a hole's own sample is not looked at.
+//
+// Bound by issue. The launches of a 1080p level 0 (combine, blur, combine, store) took 10 + 48 + 10 + 15 us.
+__global__ void __launch_bounds__(FILL_THREADS) k_fill_push(const __grid_constant__ FillPush P) {
+    using G = FillGeom<6>;
+    if (!*P.any) return;
+    __shared__ float2 s_in[G::IN], s_h[G::MID];
+    __shared__ float2 s_dx[G::R * G::SEG], s_dy[G::R * G::SEG], s_cx[G::RUNS], s_cy[G::RUNS];
+    const int w = P.w, h = P.h, X0 = blockIdx.x * G::T, Y0 = blockIdx.y * G::T, pair = blockIdx.z, tid = threadIdx.x;
+    if (P.img) {
+        bool hole = false;
+        const int X = X0 + tid % G::T;
+        for (int Y = Y0 + tid / G::T; Y < min(Y0 + G::T, h); Y += FILL_THREADS / G::T) {
+            if (X >= w) continue;
+            const long i = (long)Y * w + X;
+            if (P.holes[i]) {
+                hole = true;
+            } else if (P.rule) {
+                const float2 v = P.fmt == 2 ? fill_sample<2>(P.img, i, pair) : fill_sample<FILL_FLOW>(P.img, i, pair);
+                if (any_nan(v)) {
+                    if (P.fmt == 2) fill_put<2>(P.img, i, pair, fill_rule_quot(v, 1.0f));
+                    else fill_put<FILL_FLOW>(P.img, i, pair, fill_rule_quot(v, 1.0f));
+                }
+            }
+        }
+        if (!__syncthreads_or(hole)) return;
+    }
+    if (tid < G::R * G::SEG) {
+        s_dx[tid] = border_den<6>(X0 + tid, w, P.t.k);
+        s_dy[tid] = border_den<6>(Y0 + tid, h, P.t.k);
+    }
+    const int k = FILL_THREADS - 1 - tid;
+    if (!P.direct && k < G::RUNS) {
+        auto cell_at = [](int i, float step, int len) {
+            int c;
+            float f;
+            cell((float)i * step, len, c, f);
+            return make_float2(__int_as_float(c), f);
+        };
+        s_cx[k] = cell_at(X0 - G::HALO + k, P.sx, P.cw);
+        s_cy[k] = cell_at(Y0 - G::HALO + k, P.sy, P.ch);
+    }
+    __syncthreads();
+    if (!P.img) fill_push<-1>(P, s_in, s_h, s_dx, s_dy, s_cx, s_cy);
+    else if (P.fmt == 0) fill_push<0>(P, s_in, s_h, s_dx, s_dy, s_cx, s_cy);
+    else if (P.fmt == 1) fill_push<1>(P, s_in, s_h, s_dx, s_dy, s_cx, s_cy);
+    else if (P.fmt == 2) fill_push<2>(P, s_in, s_h, s_dx, s_dy, s_cx, s_cy);
+    else fill_push<FILL_FLOW>(P, s_in, s_h, s_dx, s_dy, s_cx, s_cy);
 }
 
 // flow/sample.rs:91-112 at element (x, y) of a dw x dh plane from the sw x sh plane s (the lerps
@@ -401,36 +650,6 @@ __device__ __forceinline__ float stack_resample_px(const float* __restrict__ s, 
     float top = lerp_r<R>(s[i], s[i + 1], fx);
     float bot = lerp_r<R>(s[i + sw], s[i + sw + 1], fx);
     return lerp_r<R>(top, bot, fy);
-}
-
-template <bool R>
-__device__ __forceinline__ void stack_resample(const float* __restrict__ src, int sw, int sh, long sstride,
-                                               float* __restrict__ dst, int dw, int dh, long dstride) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y;
-    if (x >= dw || y >= dh) return;
-    dst[blockIdx.z * dstride + (long)y * dw + x] = stack_resample_px<R>(src + blockIdx.z * sstride, sw, sh, dw, dh, x, y);
-}
-
-__global__ void k_stack_resample(const float* __restrict__ src, int sw, int sh, long sstride, float* __restrict__ dst,
-                                 int dw, int dh, long dstride, int rule, const int* __restrict__ any_hole) {
-    if (!*any_hole) return;
-    if (rule) stack_resample<true>(src, sw, sh, sstride, dst, dw, dh, dstride);
-    else stack_resample<false>(src, sw, sh, sstride, dst, dw, dh, dstride);
-}
-
-// holefill.rs:371-377: sol = weight != 0 ? value / weight : sol, for the nc channels (4 of an
-// engine image, 2 of a flow); the weights are plane nc of the level's stack
-__global__ void k_fill_combine(float* __restrict__ sol, const float* __restrict__ vals, long n, int nc, int rule,
-                               const int* __restrict__ any_hole) {
-    if (!*any_hole) return;
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float wt = vals[nc * n + i];
-    if (wt != 0.0f) {
-        for (int c = 0; c < nc; c++)
-            sol[c * n + i] = rule ? Ar<true>::div(vals[c * n + i], wt) : Ar<false>::div(vals[c * n + i], wt);
-    }
 }
 
 // ---- the coarse levels of the fill in one block ------------------------------------------------------
@@ -527,34 +746,6 @@ __global__ void __launch_bounds__(FILL_COARSE_THREADS) k_fill_coarse(FillCoarseJ
     extern __shared__ float fsm[];
     if (J.rule) fill_coarse_body<true>(J, fsm);
     else fill_coarse_body<false>(J, fsm);
-}
-
-// holefill.rs:379-404 (+ the f32 bit copy): the filled channels back into the engine image
-template <typename P>
-__device__ __forceinline__ void fill_store_px(void* img, const float* sol, long n, long i) {
-    P* px = (P*)img + i * 4;
-    for (int c = 0; c < 4; c++) {
-        float v = sol[c * n + i];
-        if (sizeof(P) == 4) ((float*)px)[c] = v;
-        else px[c] = SPx<P>::plain(v);
-    }
-}
-
-__global__ void k_fill_store(void* __restrict__ img, int fmt, const float* __restrict__ sol, long n,
-                             const int* __restrict__ any_hole) {
-    if (!*any_hole) return;
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (fmt == 0) fill_store_px<uint8_t>(img, sol, n, i);
-    else if (fmt == 1) fill_store_px<uint16_t>(img, sol, n, i);
-    else if (fmt == FILL_FLOW) ((float2*)img)[i] = make_float2(sol[i], sol[n + i]);
-    else fill_store_px<float>(img, sol, n, i);
-}
-
-__global__ void k_stack_zero(float* __restrict__ p, long n, const int* __restrict__ any_hole) {
-    if (!*any_hole) return;
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = 0.0f;
 }
 
 // a hole in an image with a side of 1 pixel: the fill refuses it (holefill.rs:273-277)
