@@ -140,3 +140,32 @@ def test_hole_fill_at_the_ends_of_its_tiles(dev, size, fmt, above_first):
             got = dev.fill_holes(src.copy(), w, h, fmt, mask, taps_above_first=above_first)
             want = O.fill_holes(src.copy(), w, h, fmt, mask, 1, above_first)
         assert same(got, want)
+
+
+@pytest.mark.parametrize("pyramid", [True, False])
+@pytest.mark.parametrize("case", ["payload", "rows", "far", "whole"])
+def test_forward_warp_where_its_plain_arithmetic_ends(dev, pyramid, case):
+    """Samples around and above 10^6, rows closer than 10^-6, corners far outside, vertices on pixels."""
+    w, h = 37, 29
+    rng = np.random.RandomState(2)
+    src = rng.random_sample(w * h * 4).astype(np.float32)
+    flow = rng.uniform(-2, 2, (h, w, 2)).astype(np.float32)
+    if case == "payload":
+        src[rng.randint(0, src.size, 200)] = rng.choice(np.float32([9.99e5, 1e6, -1e6, 3e8, -2e30, 3e38]), 200)
+    elif case == "rows":
+        flow[..., 1] = np.where(rng.random_sample((h, w)) < 0.5, 0.0, rng.uniform(-3e-6, 3e-6, (h, w)))
+        flow[::5, :, 1] -= 1.0
+    elif case == "far":
+        at = rng.randint(0, h, 12), rng.randint(0, w, 12)
+        flow[at] = rng.choice(np.float32([-3e5, 9.9e5, 2e6, -4e7]), (12, 2))
+    else:
+        flow = np.round(flow)
+    flow = flow.astype(np.float32).reshape(-1)
+    try:
+        want = O.forward_warp(src, w, h, 2, flow, w, h, 1.0, pyramid, True)
+    except ValueError:
+        with pytest.raises(tw.Unsupported):
+            dev.forward_warp(src, w, h, 2, flow, (w, h), 1.0, pyramid, True)
+        return
+    got = dev.forward_warp(src, w, h, 2, flow, (w, h), 1.0, pyramid, True)
+    assert same(got[0], want[0]) and same(got[1], want[1])

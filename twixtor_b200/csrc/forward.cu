@@ -490,101 +490,220 @@ __device__ __forceinline__ void triangle(const Vt* t, int w1, int h1, Ar aa, Ar 
 }
 
 // ---- the two raster passes ------------------------------------------------------------------------------
-struct CountSink {
-    uint32_t* cnt;
-    int w;
-    int* out_flag;
-    __device__ void hit(int x, int y, const float*) { atomicAdd(&cnt[(long)y * w + x], 1u); }
-    __device__ void outside() { atomicOr(out_flag, 1); }
+// The spans of a triangle without its payload: the same scan as `triangle` (a bound of its work is the set-up,
+// for most triangles of a grid cover one pixel or none). Sorted vertices number 0 .. 2; an edge remembers its
+// ends and how many rows it has gone, so that its payload can be formed where a span has pixels.
+struct Corner {
+    float x, y;
+    int at;  // the vertex's pixel
+};
+struct ScanEdge {
+    float ay, by, x, dx, t, inv;
+    int a, b, rows;
+    float2 p[2], dp[2];  // the payload after `done` rows (-1: not formed)
+    int done;
 };
 
-template <typename P>
-struct EmitSink {
-    const FwRaster& R;
-    uint32_t tri;
-    __device__ void hit(int x, int y, const float* p) {
-        long px = (long)y * R.w + x;
-        uint32_t k = atomicAdd(&R.fill[px], 1u);
-        if (k >= R.cnt[px]) {  // the count pass saw fewer hits: never expected, never written
-            atomicOr(R.bad, 2);
-            return;
-        }
-        uint32_t slot = R.off[px] + k;
-        R.keys[slot] = tri;
-        float c[4];
-        if (R.pyramid) {
-            if (0.0f < p[2]) fw_sample<P>(R.levels, p[0], p[1], p[2], c, R.bad);
-            else fw_tap<P>(R.levels.p[0], R.levels.w[0], R.levels.h[0], p[0], p[1], R.levels.z, c, R.bad);
-        } else {
-#pragma unroll
-            for (int q = 0; q < 4; q++) c[q] = p[q];
-        }
-        R.cols[slot] = make_float4(c[0], c[1], c[2], c[3]);
-    }
-    __device__ void outside() { atomicOr(R.outside, 1); }
-};
-
-// The Gouraud variant's sink: the hit's interpolated colours; its pointers copied out of the kernel
-// parameters (a reference to them, which the textured sink's mip level table needs, makes every
-// thread copy the whole parameter block to local memory)
-struct EmitSinkG {
-    uint32_t* fill;
-    const uint32_t* cnt;
-    const uint32_t* off;
-    uint32_t* keys;
-    float4* cols;
-    int* bad;
-    int* out_flag;
-    int w;
-    uint32_t tri;
-    __device__ void hit(int x, int y, const float* p) {
-        long px = (long)y * w + x;
-        uint32_t k = atomicAdd(&fill[px], 1u);
-        if (k >= cnt[px]) {  // the count pass saw fewer hits: never expected, never written
-            atomicOr(bad, 2);
-            return;
-        }
-        uint32_t slot = off[px] + k;
-        keys[slot] = tri;
-        cols[slot] = make_float4(p[0], p[1], p[2], p[3]);
-    }
-    __device__ void outside() { atomicOr(out_flag, 1); }
-};
-
-template <typename P>
-__device__ __forceinline__ void load_vertex(const FwRaster& R, int r, int c, Vt& v) {
-    long i = (long)r * R.w + c;
-    v.x = R.vx[i];
-    v.y = R.vy[i];
-    if (R.pyramid) {
-        v.p[0] = (float)c / (float)(R.w - 1);
-        v.p[1] = (float)r / (float)(R.h - 1);
-        v.p[2] = R.vd ? R.vd[i] : 0.0f;
-        v.p[3] = 0.0f;
-    } else {
-        const P* s = (const P*)R.levels.p[0] + i * 4;
-#pragma unroll
-        for (int q = 0; q < 4; q++) v.p[q] = (float)s[q];
+__device__ __forceinline__ void scan_edge(const Corner& a, const Corner& b, int ia, int ib, float y, ScanEdge e[2], int& count) {
+    if (a.y <= y && y < b.y) {
+        ScanEdge s;
+        const float dx = b.x - a.x;
+        s.inv = 1.0f / (b.y - a.y);
+        s.t = ((y - 1.0f) - a.y) * s.inv;
+        s.ay = a.y;
+        s.by = b.y;
+        s.x = dx * s.t + a.x;
+        s.dx = dx * s.inv;
+        s.a = ia;
+        s.b = ib;
+        s.rows = 0;
+        s.done = -1;
+        if (count != 0) e[1] = s;
+        else e[0] = s;
+        count += 1;
     }
 }
 
-// MODE 0: the count pass; 1: the emit of the Gouraud variant; 2: the emit of the textured variant
-template <typename P, int MODE>
-__device__ __forceinline__ void raster_one(const FwRaster& R) {
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    long cells = (long)(R.w - 1) * (R.h - 1);
-    if (t >= 2 * cells) return;
-    long cell = t >> 1;
-    int r = (int)(cell / (R.w - 1)), c = (int)(cell - (long)r * (R.w - 1));
+// raster.rs:171-300: span(x0, x1, lx, width, row, left edge, right edge) for each row with pixels,
+// last(x0, x1, lx, width, row, left vertex, right vertex) for the degenerate last row
+template <typename Span, typename Last>
+__device__ __forceinline__ void scan_triangle(const Corner* t, Corner* vs, int w1, int h1, Span span, Last last) {
+    const float w1f = (float)w1, h1f = (float)h1;
+    const bool ok = (0.0f <= t[0].x || 0.0f <= t[1].x || 0.0f <= t[2].x) && (0.0f <= t[0].y || 0.0f <= t[1].y || 0.0f <= t[2].y) &&
+                    (t[0].x <= w1f || t[1].x <= w1f || t[2].x <= w1f) && (t[0].y <= h1f || t[1].y <= h1f || t[2].y <= h1f);
+    if (!ok) return;
+    {  // raster.rs:90-113
+        const float y0 = t[0].y, y1 = t[1].y, y2 = t[2].y;
+        int a, b, c;
+        if (y1 < y0) {
+            if (y2 < y0) {
+                if (y2 < y1) { a = 2; b = 1; c = 0; }
+                else { a = 1; b = 2; c = 0; }
+            } else { a = 1; b = 0; c = 2; }
+        } else if (y2 < y1) {
+            if (y0 < y2) { a = 0; b = 2; c = 1; }
+            else { a = 2; b = 0; c = 1; }
+        } else { a = 0; b = 1; c = 2; }
+        auto pick = [&](int k) { return k == 0 ? t[0] : k == 1 ? t[1] : t[2]; };
+        vs[0] = pick(a);
+        vs[1] = pick(b);
+        vs[2] = pick(c);
+    }
+    float y = ceilf(vs[0].y), y_end = floorf(vs[2].y);
+    if (y < 0.0f) y = 0.0f;
+    if (h1f < y_end) y_end = h1f;
+    if (y <= y_end) {
+        int vi = 0, count = 0;
+        ScanEdge e[2] = {};
+        for (;;) {  // at most h rows: y advances by 1 from >= 0 to <= h1
+            while (vi < 3) {
+                if (y < (vi == 0 ? vs[0].y : vi == 1 ? vs[1].y : vs[2].y)) break;
+                if (count == 1) {
+                    if (e[0].ay <= y && e[0].by <= y) count = 0;
+                } else if (count == 2) {
+                    if (y < e[1].ay || y < e[1].by) {
+                        if (!(y < e[0].ay || y < e[0].by)) {
+                            e[0] = e[1];
+                            count = 1;
+                        }
+                    } else if (e[0].ay <= y && e[0].by <= y) {
+                        count = 0;
+                    } else {
+                        count = 1;
+                    }
+                }
+                if (vi == 0) {
+                    scan_edge(vs[0], vs[1], 0, 1, y, e, count);
+                    scan_edge(vs[0], vs[2], 0, 2, y, e, count);
+                } else if (vi == 1) {
+                    scan_edge(vs[1], vs[2], 1, 2, y, e, count);
+                    scan_edge(vs[1], vs[0], 1, 0, y, e, count);
+                } else {
+                    scan_edge(vs[2], vs[0], 2, 0, y, e, count);
+                    scan_edge(vs[2], vs[1], 2, 1, y, e, count);
+                }
+                vi += 1;
+            }
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                e[k].x += e[k].dx;
+                e[k].rows++;
+            }
+            if (count == 2) {
+                const bool sw = e[1].x < e[0].x;  // the left edge is e[1]
+                const float lx = sw ? e[1].x : e[0].x, rx = sw ? e[0].x : e[1].x;
+                const int x0 = max(cvtt32(ceilf(lx)), 0), x1 = min(cvtt32(floorf(rx)), w1);
+                const float wid = rx - lx;
+                if (x0 <= x1 && (double)wid > 1e-08) span(x0, x1, lx, wid, cvtt32(y), sw, e);
+            }
+            y += 1.0f;
+            if (!(y <= y_end)) break;
+        }
+    }
+    const Corner &mid = vs[1], &bot = vs[2];
+    if (mid.y == h1f && mid.y == bot.y) {
+        const bool bl = bot.x <= mid.x;  // the left vertex is bot
+        const float lx = bl ? bot.x : mid.x, rx = bl ? mid.x : bot.x;
+        const float yy = bl ? bot.y : mid.y, yt = (float)cvtt32(yy);
+        if (0.0f <= yt && yt <= h1f && !((double)(yy - yt) > 0.01)) {
+            const int x0 = max(cvtt32(ceilf(lx)), 0), x1 = min(cvtt32(floorf(rx)), w1);
+            const float wid = rx - lx;
+            if ((double)wid > 1e-05) last(x0, x1, lx, wid, cvtt32(yt), bl ? 2 : 1, bl ? 1 : 2);
+        }
+    }
+}
+
+// The vertices of triangle t of the grid, T1 = (v[r][c], v[r][c+1], v[r+1][c]) and T2 = (v[r+1][c+1], v[r][c+1],
+// v[r+1][c]) of every cell; false past the last one
+__device__ __forceinline__ bool grid_triangle(const FwRaster& R, long t, Corner* v) {
+    const int cw = R.w - 1;
+    if (t >= 2l * cw * (R.h - 1)) return false;
+    const long cell = t >> 1;
+    const int r = row_of(cell, cw), c = (int)(cell - (long)r * cw);
+    const int i = r * R.w + c;  // (the hits of an image, and so its pixels, are below 2^31)
+    v[0].at = (t & 1) == 0 ? i : i + R.w + 1;
+    v[1].at = i + 1;
+    v[2].at = i + R.w;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        v[k].x = R.vx[v[k].at];
+        v[k].y = R.vy[v[k].at];
+    }
+    return true;
+}
+
+__global__ void __launch_bounds__(128) k_fw_count(const __grid_constant__ FwRaster R) {
+    Corner v[3], vs[3];
+    if (!grid_triangle(R, (long)blockIdx.x * blockDim.x + threadIdx.x, v)) return;
+    const int w1 = R.w - 1, h1 = R.h - 1;
+    auto hit = [&](int x, int y) { atomicAdd(&R.cnt[(long)y * R.w + x], 1u); };
+    scan_triangle(
+        v, vs, w1, h1,
+        [&](int x0, int x1, float, float, int y, bool, ScanEdge*) {
+            for (int x = x0; x <= x1; x++) hit(x, y);
+        },
+        [&](int x0, int x1, float, float, int y, int, int) {  // a run of at least one pixel, checked (raster.rs:116-153)
+            int x = x0;
+            do {
+                if (x < 0 || x > w1 || y < 0 || y > h1) atomicOr(R.outside, 1);
+                else hit(x, y);
+            } while (x0 != x1 && x++ < x1);
+        });
+}
+
+// A hit of triangle tri at (x, y): its slot, its key and its colour
+template <typename P, bool TEXTURED>
+__device__ __forceinline__ void emit_hit(const FwRaster& R, uint32_t tri, int x, int y, const float* p) {
+    const long px = (long)y * R.w + x;
+    const uint32_t k = atomicAdd(&R.fill[px], 1u);
+    if (k >= R.cnt[px]) {  // the count pass saw fewer hits: never expected, never written
+        atomicOr(R.bad, 2);
+        return;
+    }
+    const uint32_t slot = R.off[px] + k;
+    R.keys[slot] = tri;
+    float c[4];
+    if (TEXTURED) {
+        if (0.0f < p[2]) fw_sample<P>(R.levels, p[0], p[1], p[2], c, R.bad);
+        else fw_tap<P>(R.levels.p[0], R.levels.w[0], R.levels.h[0], p[0], p[1], R.levels.z, c, R.bad);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; q++) c[q] = p[q];
+    }
+    R.cols[slot] = make_float4(c[0], c[1], c[2], c[3]);
+}
+
+template <typename P, bool TEXTURED>
+struct EmitSink {
+    const FwRaster& R;
+    uint32_t tri;
+    __device__ void hit(int x, int y, const float* p) { emit_hit<P, TEXTURED>(R, tri, x, y, p); }
+    __device__ void outside() { atomicOr(R.outside, 1); }
+};
+
+// The payload of the vertex at pixel i: the texture coordinates and the mip level, or the colours
+template <typename P, bool TEXTURED>
+__device__ __forceinline__ void vertex_payload(const FwRaster& R, int i, float p[4]) {
+    if (TEXTURED) {
+        const int r = row_of(i, R.w), c = i - r * R.w;
+        p[0] = (float)c / (float)(R.w - 1);
+        p[1] = (float)r / (float)(R.h - 1);
+        p[2] = R.vd ? R.vd[i] : 0.0f;
+        p[3] = 0.0f;
+    } else {
+        px_floats<P>((const P*)R.levels.p[0] + (long)i * 4, p);
+    }
+}
+
+// A triangle in the reference's arithmetic of NaNs, out of the main path
+template <typename P, bool TEXTURED>
+__device__ __noinline__ void emit_general(const FwRaster& R, uint32_t t, const Corner* c) {
     Vt v[3];
-    if ((t & 1) == 0) {  // T1 = (v[r][c], v[r][c+1], v[r+1][c])
-        load_vertex<P>(R, r, c, v[0]);
-        load_vertex<P>(R, r, c + 1, v[1]);
-        load_vertex<P>(R, r + 1, c, v[2]);
-    } else {  // T2 = (v[r+1][c+1], v[r][c+1], v[r+1][c])
-        load_vertex<P>(R, r + 1, c + 1, v[0]);
-        load_vertex<P>(R, r, c + 1, v[1]);
-        load_vertex<P>(R, r + 1, c, v[2]);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        v[k].x = c[k].x;
+        v[k].y = c[k].y;
+        vertex_payload<P, TEXTURED>(R, c[k].at, v[k].p);
     }
     // raster.rs:158-166: the rule when a payload of the triangle is NaN (per scan: the Gouraud
     // variant's two scans, colours 0..2 and colour 3, choose on their own)
@@ -594,37 +713,118 @@ __device__ __forceinline__ void raster_one(const FwRaster& R) {
         na = na || isnan(v[k].p[0]) || isnan(v[k].p[1]) || isnan(v[k].p[2]);
         nb = nb || isnan(v[k].p[3]);
     }
-    Ar aa{na}, ab{nb};
-    if (MODE == 2) {
-        EmitSink<P> s{R, (uint32_t)t};
-        triangle(v, R.w - 1, R.h - 1, aa, ab, s);
-    } else if (MODE == 1) {
-        EmitSinkG s{R.fill, R.cnt, R.off, R.keys, R.cols, R.bad, R.outside, R.w, (uint32_t)t};
-        triangle(v, R.w - 1, R.h - 1, aa, ab, s);
-    } else {
-        CountSink s{R.cnt, R.w, R.outside};
-        triangle(v, R.w - 1, R.h - 1, aa, ab, s);
-    }
+    EmitSink<P, TEXTURED> s{R, t};
+    triangle(v, R.w - 1, R.h - 1, Ar{na}, Ar{nb}, s);
 }
 
-__global__ void __launch_bounds__(128) k_fw_count(FwRaster R) {
-    if (R.fmt == 0) raster_one<uint8_t, 0>(R);
-    else if (R.fmt == 1) raster_one<uint16_t, 0>(R);
-    else raster_one<float, 0>(R);
+// The emit of a triangle. Bound by issue and by the divergence of triangles with and without pixels, so the
+// payload (two pairs of channels) is formed where a span has pixels and steps on from there. No product of
+// the scan overflows where the corners and the payload are below 10^6 and no two rows are closer than 10^-6
+// (an edge's t is below 10^13 and its payload below 10^20; a span starts at most a rounding past its width): no
+// NaN can come up then, and the plain arithmetic gives the reference's bits. Other triangles go by emit_general.
+template <typename P, bool TEXTURED>
+__device__ __forceinline__ void emit_triangle(const FwRaster& R) {
+    const long tri = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    Corner v[3], vs[3];
+    if (!grid_triangle(R, tri, v)) return;
+    const float z = R.levels.z;
+    const float2 zz = make_float2(z, z);
+    bool plain = true;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const float dy = fabsf(v[k].y - v[(k + 1) % 3].y);
+        plain = plain && fabsf(v[k].x) < 1e6f && fabsf(v[k].y) < 1e6f && (dy == 0.0f || dy > 1e-6f);
+        if (TEXTURED) plain = plain && (!R.vd || fabsf(R.vd[v[k].at]) < 1e6f);
+        if (!TEXTURED && sizeof(P) == 4) {
+            float p[4];
+            vertex_payload<P, TEXTURED>(R, v[k].at, p);
+            plain = plain && fabsf(p[0]) < 1e6f && fabsf(p[1]) < 1e6f && fabsf(p[2]) < 1e6f && fabsf(p[3]) < 1e6f;
+        }
+    }
+    if (!plain) {
+        const Corner general[3] = {v[0], v[1], v[2]};  // (a copy: the corners stay in registers)
+        emit_general<P, TEXTURED>(R, (uint32_t)tri, general);
+        return;
+    }
+    const int w1 = R.w - 1, h1 = R.h - 1;
+    auto sub = [](float2 b, float2 a) { return __ffma2_rn(a, make_float2(-1.0f, -1.0f), b); };
+    auto mul = [&](float2 a, float k) { return __ffma2_rn(a, make_float2(k, k), zz); };
+    auto vertex = [&](int k, float2* p) {
+        float f[4];
+        vertex_payload<P, TEXTURED>(R, k == 0 ? vs[0].at : k == 1 ? vs[1].at : vs[2].at, f);
+        p[0] = make_float2(f[0], f[1]);
+        p[1] = make_float2(f[2], f[3]);
+    };
+    auto edge = [&](ScanEdge& e) {
+        if (e.done < 0) {
+            float2 pa[2], pb[2];
+            vertex(e.a, pa);
+            vertex(e.b, pb);
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const float2 d = sub(pb[q], pa[q]);
+                e.p[q] = __fadd2_rn(mul(d, e.t), pa[q]);
+                e.dp[q] = mul(d, e.inv);
+            }
+            e.done = 0;
+        }
+        for (; e.done < e.rows; e.done++) {
+#pragma unroll
+            for (int q = 0; q < 2; q++) e.p[q] = __fadd2_rn(e.p[q], e.dp[q]);
+        }
+    };
+    // one closed span with the payload lerped from l to r (raster.rs:116-153, :252-299)
+    auto run = [&](int x0, int x1, float lx, float wid, int y, const float2* l, const float2* r, bool check) {
+        const float inv = 1.0f / wid, t = ((float)x0 - lx) * inv;
+        float2 p[2], s[2];
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const float2 d = sub(r[q], l[q]);
+            p[q] = __fadd2_rn(mul(d, t), l[q]);
+            s[q] = mul(d, inv);
+        }
+        for (int x = x0;; x++) {
+            const float f[4] = {p[0].x, p[0].y, p[1].x, p[1].y};
+            if (check && (x < 0 || x > w1 || y < 0 || y > h1)) atomicOr(R.outside, 1);
+            else emit_hit<P, TEXTURED>(R, (uint32_t)tri, x, y, f);
+            if (x >= x1) break;
+#pragma unroll
+            for (int q = 0; q < 2; q++) p[q] = __fadd2_rn(p[q], s[q]);
+        }
+    };
+    scan_triangle(
+        v, vs, w1, h1,
+        [&](int x0, int x1, float lx, float wid, int y, bool sw, ScanEdge* e) {
+            edge(e[0]);
+            edge(e[1]);
+            float2 l[2], r[2];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                l[q] = sw ? e[1].p[q] : e[0].p[q];
+                r[q] = sw ? e[0].p[q] : e[1].p[q];
+            }
+            run(x0, x1, lx, wid, y, l, r, false);
+        },
+        [&](int x0, int x1, float lx, float wid, int y, int left, int right) {
+            float2 l[2], r[2];
+            vertex(left, l);
+            vertex(right, r);
+            run(x0, x1, lx, wid, y, l, r, true);
+        });
 }
 
 // the emit of the Gouraud variant (R.pyramid false)
-__global__ void __launch_bounds__(128, 6) k_fw_emit(FwRaster R) {
-    if (R.fmt == 0) raster_one<uint8_t, 1>(R);
-    else if (R.fmt == 1) raster_one<uint16_t, 1>(R);
-    else raster_one<float, 1>(R);
+__global__ void __launch_bounds__(128, 6) k_fw_emit(const __grid_constant__ FwRaster R) {
+    if (R.fmt == 0) emit_triangle<uint8_t, false>(R);
+    else if (R.fmt == 1) emit_triangle<uint16_t, false>(R);
+    else emit_triangle<float, false>(R);
 }
 
 // the emit of the textured variant (R.pyramid true)
-__global__ void __launch_bounds__(128, 4) k_fw_emit_tex(FwRaster R) {
-    if (R.fmt == 0) raster_one<uint8_t, 2>(R);
-    else if (R.fmt == 1) raster_one<uint16_t, 2>(R);
-    else raster_one<float, 2>(R);
+__global__ void __launch_bounds__(128, 4) k_fw_emit_tex(const __grid_constant__ FwRaster R) {
+    if (R.fmt == 0) emit_triangle<uint8_t, true>(R);
+    else if (R.fmt == 1) emit_triangle<uint16_t, true>(R);
+    else emit_triangle<float, true>(R);
 }
 
 // ---- the exclusive scan of the per pixel counts ---------------------------------------------------------

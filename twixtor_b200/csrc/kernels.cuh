@@ -389,9 +389,9 @@ __global__ void k_fw_vertices(const float* __restrict__ flow, int fw, int fh, Fw
 __global__ void k_fwp_blur(const void* __restrict__ in, void* __restrict__ out, int w, int h, int vertical, int fmt);
 __global__ void k_fwp_resample(const void* __restrict__ src, int sw, int sh, void* __restrict__ dst, int dw, int dh,
                                int fmt, float z);
-__global__ void k_fw_count(FwRaster R);
-__global__ void k_fw_emit(FwRaster R);      // the Gouraud variant
-__global__ void k_fw_emit_tex(FwRaster R);  // the textured variant (R.pyramid)
+__global__ void k_fw_count(const __grid_constant__ FwRaster R);
+__global__ void k_fw_emit(const __grid_constant__ FwRaster R);      // the Gouraud variant
+__global__ void k_fw_emit_tex(const __grid_constant__ FwRaster R);  // the textured variant (R.pyramid)
 constexpr int FW_SCAN_BLOCK = 2048;
 __global__ void k_scan_block(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, long n,
                              uint32_t* __restrict__ sums, uint32_t* __restrict__ maxc);
