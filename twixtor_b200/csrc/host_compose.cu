@@ -86,20 +86,20 @@ int fill_dev(tw_ctx* ctx, void* img, int W, int H, int fmt, const uint8_t* holes
     int nc = fmt == FILL_FLOW ? 2 : 4;  // value planes; the weights are plane nc
     int np = nc + 1;
     FillGeo g = fill_geometry(W, H);
-    // the coarse levels k0 .. top (every stack of them fits one block's shared memory) run in one
-    // launch, k_fill_coarse: the finest such level k0 >= 1 is built by the pull below, the launch
-    // pulls on from it, pushes down to it and leaves the push's level k0 - 1 in the solution planes. There is
-    // one: the top level is 2 x 2.
+    // the levels k0 .. top of one tile go in one launch, k_fill_tail: the finest of them is built by the
+    // pull below, the launch pulls on from it and pushes down to it. There is one: the top level is 2 x 2.
     int k0 = 1;
-    while (k0 < g.top && fill_coarse_floats(g.dims, k0, g.top, np, nc) > FILL_COARSE_MAX_FLOATS) k0++;
+    while (g.dims[k0][0] > FILL_TAIL || g.dims[k0][1] > FILL_TAIL) k0++;
     auto pixels = [&](int k) { return (size_t)g.dims[k][0] * g.dims[k][1]; };
-    size_t offs[40];
+    FillTail J;
+    std::memset(&J, 0, sizeof J);
     size_t tot = 0;
-    for (int k = 1; k <= k0; k++) { offs[k] = tot; tot += (np * pixels(k) + 3) / 4 * 4; }
-    const size_t o_sol = tot, o_a = o_sol + (nc * pixels(k0 - 1) + 3) / 4 * 4, o_b = o_a + (nc * pixels(1) + 3) / 4 * 4;
+    for (int k = 1; k <= g.top; k++) { J.offs[k] = (long)tot; tot += (np * pixels(k) + 3) / 4 * 4; }
+    const size_t o_a = tot, o_b = o_a + (nc * pixels(1) + 3) / 4 * 4;
     tot = o_b + nc * pixels(1);
     CHECK(ctx->ensure(fb, tot * sizeof(float), "hole fill planes"));
     float* base = fb.as<float>();
+    float2* blurred[2] = {(float2*)(base + o_a), (float2*)(base + o_b)};
     auto grid = [&](int k, int z) { return dim3((unsigned)((g.dims[k][0] + 31) / 32), (unsigned)((g.dims[k][1] + 31) / 32), (unsigned)z); };
     auto step = [](int from, int to) { return ((float)from - 1.0f) / (float)(to - 1); };
     for (int k = 1; k <= k0; k++) {  // pull: blur5 and the resample of the values and the weights
@@ -108,9 +108,9 @@ int fill_dev(tw_ctx* ctx, void* img, int W, int H, int fmt, const uint8_t* holes
             P.img = img;
             P.holes = holes;
         } else {
-            P.vals = base + offs[k - 1];
+            P.vals = base + J.offs[k - 1];
         }
-        P.dst = base + offs[k];
+        P.dst = base + J.offs[k];
         P.fmt = fmt;
         P.nc = nc;
         P.w = g.dims[k - 1][0];
@@ -125,46 +125,36 @@ int fill_dev(tw_ctx* ctx, void* img, int W, int H, int fmt, const uint8_t* holes
         P.any = any;
         LAUNCHB(ctx, 4.0 * np * ((double)pixels(k - 1) + (double)pixels(k)), k_fill_pull, grid(k - 1, nc / 2 + 1), FILL_THREADS, 0, P);
     }
-    {
-        FillCoarseJob J{};
-        J.s_k0 = base + offs[k0];
-        J.out = base + o_sol;
-        for (int k = 0; k <= g.top; k++) {
-            J.dims[k][0] = g.dims[k][0];
-            J.dims[k][1] = g.dims[k][1];
-        }
-        J.k0 = k0;
-        J.top = g.top;
-        J.np = np;
-        J.nc = nc;
-        J.rule = rule;
-        J.above_first = above_first;
-        J.b5 = ctx->b5;
-        J.g5 = ctx->g5;
-        J.any = any;
-        // the stack of level k0 read, the push's level k0 - 1 written
-        double b = 4.0 * ((double)np * pixels(k0) + (double)nc * pixels(k0 - 1));
-        LAUNCHB(ctx, b, k_fill_coarse, 1, FILL_COARSE_THREADS, fill_coarse_floats(g.dims, k0, g.top, np, nc) * sizeof(float), J);
+    J.base = base;
+    for (int i = 0; i < 2; i++) J.blurred[i] = blurred[i];
+    for (int k = 0; k <= g.top; k++) {
+        J.dims[k][0] = g.dims[k][0];
+        J.dims[k][1] = g.dims[k][1];
     }
-    float* blurred[2] = {base + o_a, base + o_b};
+    J.k0 = k0;
+    J.top = g.top;
+    J.nc = nc;
+    J.above_first = above_first;
+    J.rule = rule;
+    J.b5 = ctx->b5;
+    J.g5 = ctx->g5;
+    J.any = any;
+    // the stack of level k0 read, its solution written
+    LAUNCHB(ctx, 4.0 * (np + nc) * (double)pixels(k0), k_fill_tail, 1, FILL_TAIL_GROUPS * FILL_THREADS, fill_tail_smem(), J);
     for (int lv = k0 - 1; lv >= 0; lv--) {  // push
         FillPush P{};
         if (lv == 0) {
             P.img = img;
             P.holes = holes;
         } else {
-            P.vals = base + offs[lv];
-            P.out = (float2*)blurred[lv & 1];
+            P.vals = base + J.offs[lv];
+            P.out = blurred[lv & 1];
         }
-        if (lv == k0 - 1) {
-            P.direct = base + o_sol;
-        } else {
-            P.coarse = (const float2*)blurred[(lv + 1) & 1];
-            P.cw = g.dims[lv + 1][0];
-            P.ch = g.dims[lv + 1][1];
-            P.sx = step(P.cw, g.dims[lv][0]);
-            P.sy = step(P.ch, g.dims[lv][1]);
-        }
+        P.coarse = blurred[(lv + 1) & 1];
+        P.cw = g.dims[lv + 1][0];
+        P.ch = g.dims[lv + 1][1];
+        P.sx = step(P.cw, g.dims[lv][0]);
+        P.sy = step(P.ch, g.dims[lv][1]);
         P.fmt = fmt;
         P.nc = nc;
         P.w = g.dims[lv][0];

@@ -233,7 +233,7 @@ int tw_open(int device, tw_ctx** out) {
     TW_LIMIT(k_pyramid_tail, pyramid_tail_smem());
     TW_LIMIT(k_solve_coarse, coarse_smem_bytes(COARSE_MAX_PIXELS, COARSE_MAX_PLANE));
 #undef TW_LIMIT
-    limit((const void*)k_fill_coarse, FILL_COARSE_MAX_FLOATS * sizeof(float));
+    limit((const void*)k_fill_tail, fill_tail_smem());
     if (e != cudaSuccess) { tw_close(ctx); return TW_ERR_CUDA; }
     if (ctx->ensure(ctx->flags, FLAGS_BYTES, "flags") != TW_OK) { tw_close(ctx); return TW_ERR_CUDA; }
     k_selfcheck<<<1, 1, 0, ctx->stream>>>(ctx->flags.as<int>());

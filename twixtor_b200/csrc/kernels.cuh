@@ -280,8 +280,7 @@ struct FillPush {
     void* img;             // level 0: the image or flow, filled in place, and its holes mask; else null
     const uint8_t* holes;
     const float* vals;     // the stack of the level, w x h
-    const float* direct;   // the coarser solution at this level's size, planes of single channels, or (null)
-    const float2* coarse;  // of cw x ch, planes of pairs of channels
+    const float2* coarse;  // the coarser solution, cw x ch, planes of pairs of channels
     float2* out;           // the blurred solution, likewise
     int fmt, nc, w, h, cw, ch;
     float sx, sy;
@@ -292,23 +291,21 @@ struct FillPush {
 __global__ void k_fill_pull(const __grid_constant__ FillPull P);
 __global__ void k_fill_push(const __grid_constant__ FillPush P);
 __global__ void k_hole_side1(const int* __restrict__ any_hole, int* __restrict__ flag);
-// The coarse levels of the pull-push fill in one block: the pull from level k0 (its stack given,
-// np planes) up to the top level and the push from the top down to level k0, every stack of those
-// levels in shared memory; the push's result resampled to level k0 - 1 goes to out (nc planes of
-// that level). Level sizes as the fill's geometry (holefill.rs:140-171). fill_coarse_floats: the
-// shared memory it needs, in floats.
-constexpr int FILL_COARSE_THREADS = 1024;
-constexpr int FILL_COARSE_MAX_FLOATS = 50 * 1024;  // 200 KB
-struct FillCoarseJob {
-    const float* s_k0;
-    float* out;
+// The levels k0 .. top of the fill, of at most 32 x 32, in one block: the stack of level k0 given, its blurred
+// solution left in blurred[k0 & 1].
+constexpr int FILL_TAIL = 32, FILL_TAIL_GROUPS = 3;
+struct FillTail {
+    float* base;
+    float2* blurred[2];
+    long offs[40];  // the stacks of the levels from base on
     int dims[40][2];
-    int k0, top, np, nc, rule, above_first;
+    int k0, top, nc;
+    bool above_first, rule;
     Taps b5, g5;
     const int* any;
 };
-__global__ void k_fill_coarse(FillCoarseJob J);
-long fill_coarse_floats(const int dims[][2], int k0, int top, int np, int nc);
+__global__ void k_fill_tail(const __grid_constant__ FillTail J);
+size_t fill_tail_smem();
 
 __global__ void k_encode_vectors(const float* __restrict__ flow, int fw, int fh, void* __restrict__ out, int W, int H,
                                  int fmt, float sx, float sy, float kx, float ky, int zero);

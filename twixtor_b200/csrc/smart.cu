@@ -225,62 +225,11 @@ __global__ void k_cov_holes(const uint8_t* __restrict__ c1, const uint8_t* __res
 
 // ---- the hole fill on plane stacks (holefill.rs) ------------------------------------------------------
 
-// flow/conv.rs border element (1 channel rule) over an arithmetic set
-template <bool R, bool LEFT_FIRST, int N>
-__device__ __forceinline__ float border1(const float* line, long stride, int len, int i, const float* k) {
-    float centre = line[(long)i * stride];
-    float num = Ar<R>::mul(k[0], centre);
-    float den = k[0];
-#pragma unroll
-    for (int j = N - 1; j >= 1; j--) {
-        float kj = k[j];
-#pragma unroll
-        for (int side = 0; side < 2; side++) {
-            bool right = (side == 0) != LEFT_FIRST;
-            int t = right ? i + j : i - j;
-            bool inside = t >= 0 && t < len;
-            float xv = inside ? line[(long)t * stride] : 0.0f;
-            float wv = inside ? kj : 0.0f;
-            den = den + wv;
-            num = Ar<R>::add(num, Ar<R>::mul(xv, wv));
-        }
-    }
-    return Ar<R>::div(num, den);
-}
-
-// One element (x, y) of one pass of the 1 channel convolution of a plane s into d (conv.rs:141-190,
-// :268-301).
-template <bool R, int N, bool VERT, bool ABOVE_FIRST>
-__device__ __forceinline__ float stack_pass_px(const float* __restrict__ s, int w, int h, int x, int y, const Taps& t) {
-    float r;
-    if (!VERT) {
-        const float* row = s + (long)y * w;
-        if (w >= 2 * N && x >= N && x < w - N) {
-            r = Ar<R>::mul(row[x], t.k[0]);
-#pragma unroll
-            for (int j = N - 1; j >= 1; j--) r = Ar<R>::add(r, Ar<R>::mul(Ar<R>::add(row[x + j], row[x - j]), t.k[j]));
-        } else {
-            r = border1<R, false, N>(row, 1, w, x, t.k);
-        }
-    } else {
-        const float* col = s + x;
-        if (h >= 2 * N && y >= N && y < h - N) {
-            r = Ar<R>::mul(col[(long)y * w], t.k[0]);
-#pragma unroll
-            for (int j = N - 1; j >= 1; j--)
-                r = Ar<R>::add(r, Ar<R>::mul(Ar<R>::add(col[(long)(y + j) * w], col[(long)(y - j) * w]), t.k[j]));
-        } else {
-            r = border1<R, ABOVE_FIRST, N>(col, w, h, y, t.k);
-        }
-    }
-    return r;
-}
-
 // ---- the fill's levels in tiles ----------------------------------------------------------------------
 
 // One element of a pass along a line held in shared memory: element t (global index in [0, len)) of
-// the line at line[(t - origin) * stride]; the interior chain or the 1 channel border rule, the
-// operations of stack_pass_px / border1 in their order.
+// the line at line[(t - origin) * stride]; the interior chain or the 1 channel border rule (conv.rs:101-137,
+// :141-190, :268-301).
 template <bool R, int N, bool LEFT_FIRST>
 __device__ __forceinline__ float stack_elem(const float* line, int origin, int stride, int len, int i, const Taps& t) {
     if (len >= 2 * N && i >= N && i < len - N) {
@@ -366,11 +315,29 @@ struct FillGeom {
     static_assert(RUNS - T <= EX && SEG * R * VS <= IN, "the planes hold every run");
 };
 
+// A tile's shared memory
+template <int N>
+struct FillShared {
+    using G = FillGeom<N>;
+    float2 in[G::IN], mid[G::MID], dx[G::R * G::SEG], dy[G::R * G::SEG], cx[G::RUNS], cy[G::RUNS];
+};
+// The threads of a tile: a whole block, or one of a block's groups of FILL_THREADS, with a barrier of its own
+struct FillBlock {
+    static __device__ __forceinline__ int tid() { return threadIdx.x; }
+    static __device__ __forceinline__ void sync() { __syncthreads(); }
+};
+struct FillGroup {
+    static __device__ __forceinline__ int tid() { return threadIdx.x % FILL_THREADS; }
+    static __device__ __forceinline__ void sync() {
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / FILL_THREADS), "n"(FILL_THREADS) : "memory");
+    }
+};
+
 // The region of a tile at (X0, Y0), at(X, Y) inside the image and 0 outside
 template <int N, class At>
-__device__ __forceinline__ void fill_region(float2* s_in, int X0, int Y0, int w, int h, At at) {
+__device__ __forceinline__ void fill_region(float2* s_in, int tid, int X0, int Y0, int w, int h, At at) {
     using G = FillGeom<N>;
-    const int tid = threadIdx.x, c = tid % G::T, r0 = tid / G::T;
+    const int c = tid % G::T, r0 = tid / G::T;
     constexpr int PER = FILL_THREADS / G::T, A = (G::ROWS + PER - 1) / PER, B = (G::ROWS * G::EX + FILL_THREADS - 1) / FILL_THREADS;
     float2 v[A + B];
     // column and row of the region (no others are looked at: `at` may hold tables of the region's size)
@@ -411,25 +378,25 @@ __device__ __forceinline__ void fill_run(const float2* line, int stride, int i0,
     }
 }
 
-// Both passes of the region in s_in through s_h; out(seg, x, values): the 4 outputs of column x from row 4 * seg on
-template <int N, class Out>
-__device__ __forceinline__ void fill_blur(const float2* s_in, float2* s_h, const float2* s_dx, const float2* s_dy, int X0, int Y0,
-                                          int w, int h, const Taps& t, bool above_first, bool rule, Out out) {
+// Both passes of the region in S.in; out(seg, x, values): the 4 outputs of column x from row 4 * seg on
+template <int N, class Threads, class Out>
+__device__ __forceinline__ void fill_blur(FillShared<N>& S, int X0, int Y0, int w, int h, const Taps& t, bool above_first, bool rule,
+                                          Out out) {
     using G = FillGeom<N>;
-    for (int e = threadIdx.x; e < G::ROWS * G::SEG; e += FILL_THREADS) {
+    for (int e = Threads::tid(); e < G::ROWS * G::SEG; e += FILL_THREADS) {
         const int seg = e / G::ROWS, y = e - seg * G::ROWS;
         float2 o[G::R];
-        fill_run<N, false>(s_in + y * G::RS + seg * G::R, 1, X0 + seg * G::R, w, X0 + G::OUT, t, s_dx + seg * G::R, rule, o);
+        fill_run<N, false>(S.in + y * G::RS + seg * G::R, 1, X0 + seg * G::R, w, X0 + G::OUT, t, S.dx + seg * G::R, rule, o);
 #pragma unroll
-        for (int r = 0; r < G::R; r++) s_h[y * G::HS + seg * G::R + r] = o[r];
+        for (int r = 0; r < G::R; r++) S.mid[y * G::HS + seg * G::R + r] = o[r];
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < G::OUT * G::SEG; e += FILL_THREADS) {
+    Threads::sync();
+    for (int e = Threads::tid(); e < G::OUT * G::SEG; e += FILL_THREADS) {
         const int seg = e / G::OUT, x = e - seg * G::OUT;
         float2 o[G::R];
-        const float2* line = s_h + seg * G::R * G::HS + x;
-        if (above_first) fill_run<N, true>(line, G::HS, Y0 + seg * G::R, h, Y0 + G::OUT, t, s_dy + seg * G::R, rule, o);
-        else fill_run<N, false>(line, G::HS, Y0 + seg * G::R, h, Y0 + G::OUT, t, s_dy + seg * G::R, rule, o);
+        const float2* line = S.mid + seg * G::R * G::HS + x;
+        if (above_first) fill_run<N, true>(line, G::HS, Y0 + seg * G::R, h, Y0 + G::OUT, t, S.dy + seg * G::R, rule, o);
+        else fill_run<N, false>(line, G::HS, Y0 + seg * G::R, h, Y0 + G::OUT, t, S.dy + seg * G::R, rule, o);
         out(seg, x, o);
     }
 }
@@ -450,11 +417,75 @@ __device__ __forceinline__ float2 fill_sample(const void* img, long i, int pair)
 template <int FMT>
 __device__ __forceinline__ void fill_pull_image(const FillPull& P, float2* s_in, int X0, int Y0, int pair) {
     const bool weights = 2 * pair == P.nc;
-    fill_region<3>(s_in, X0, Y0, P.w, P.h, [&](int X, int Y) {
+    fill_region<3>(s_in, threadIdx.x, X0, Y0, P.w, P.h, [&](int X, int Y) {
         const long i = (long)Y * P.w + X;
         if (P.holes[i]) return make_float2(0.0f, 0.0f);
         return weights ? make_float2(1.0f, 0.0f) : fill_sample<FMT>(P.img, i, pair);
     });
+}
+
+// A level's stack: the pair's planes, or the weights and nothing
+__device__ __forceinline__ void fill_pull_planes(const float* vals, float2* s_in, int tid, int X0, int Y0, int w, int h, int nc, int pair) {
+    const long n = (long)w * h;
+    const float *a = vals + 2 * pair * n, *b = 2 * pair == nc ? nullptr : a + n;
+    fill_region<3>(s_in, tid, X0, Y0, w, h, [&](int X, int Y) {
+        const long i = (long)Y * w + X;
+        return make_float2(a[i], b ? b[i] : 0.0f);
+    });
+}
+
+// The rest of a pull: the blur of the region and the outputs whose first tap lies in the tile
+template <class Threads>
+__device__ __forceinline__ void fill_pull_tile(FillShared<3>& S, int X0, int Y0, int w, int h, int dw, int dh, float sx, float sy,
+                                               float* dst, int nc, int pair, const Taps& t, bool above_first, bool rule) {
+    using G = FillGeom<3>;
+    const int tid = Threads::tid();
+    // the outputs whose first tap can lie in the tile, from its ends over the step (at least 1)
+    auto range = [](int at, int len, float step, int n, int& lo, int& count) {
+        lo = (int)((float)at / step);
+        count = min((at + G::T < len - 1 ? min((int)((float)(at + G::T) / step), n - 1) : n - 1) - lo + 1, G::T + 2);
+    };
+    int xa, nx, ya, ny;
+    range(X0, w, sx, dw, xa, nx);
+    range(Y0, h, sy, dh, ya, ny);
+    auto cell_at = [](int i, float step, int len, int at) {
+        int k;
+        float f;
+        cell((float)i * step, len, k, f);
+        k -= at;
+        return make_float2(__int_as_float(k >= 0 && k < G::T ? k : -1), f);
+    };
+    if (tid < G::R * G::SEG) {
+        S.dx[tid] = border_den<3>(X0 + tid, w, t.k);
+        S.dy[tid] = border_den<3>(Y0 + tid, h, t.k);
+    }
+    const int k = FILL_THREADS - 1 - tid;
+    if (k < nx) S.cx[k] = cell_at(xa + k, sx, w, X0);
+    if (k < ny) S.cy[k] = cell_at(ya + k, sy, h, Y0);
+    Threads::sync();
+    float2* s_v = S.in;  // (the column pass reads S.mid alone)
+    fill_blur<3, Threads>(S, X0, Y0, w, h, t, above_first, rule, [&](int seg, int x, const float2* o) {
+#pragma unroll
+        for (int r = 0; r < G::R; r++) s_v[(seg * G::R + r) * G::VS + x] = o[r];
+    });
+    Threads::sync();
+    constexpr int COLS = G::T / 2 + 2;  // the outputs across a tile at a step of 2
+    const long dn = (long)dw * dh;
+    float *da = dst + 2 * pair * dn, *db = 2 * pair == nc ? nullptr : da + dn;
+    for (int x0 = 0; x0 < nx; x0 += COLS) {
+        for (int e = tid; e < COLS * ny; e += FILL_THREADS) {
+            const int y = e / COLS, x = x0 + e - y * COLS;
+            if (x >= nx) continue;
+            const float2 cx = S.cx[x], cy = S.cy[y];
+            const int ix = __float_as_int(cx.x), iy = __float_as_int(cy.x);
+            if (ix < 0 || iy < 0) continue;
+            const float2* q = s_v + iy * G::VS + ix;
+            const float2 r = fill_mix(q[0], q[1], q[G::VS], q[G::VS + 1], cx.y, cy.y, t.z, rule);
+            const long i = (long)(ya + y) * dw + xa + x;
+            da[i] = r.x;
+            if (db) db[i] = r.y;
+        }
+    }
 }
 
 // One level up (holefill.rs:300-350): blur5 of level k - 1 and the resample to level k, a pair of channels
@@ -465,69 +496,15 @@ __device__ __forceinline__ void fill_pull_image(const FillPull& P, float2* s_in,
 // test per tap, a 1080p level 0 took 14 + 50 + 12 us. Flows filled at 1080p: 38 us for a level's
 // blur and resample on average, now 19.
 __global__ void __launch_bounds__(FILL_THREADS) k_fill_pull(const __grid_constant__ FillPull P) {
-    using G = FillGeom<3>;
     if (!*P.any) return;
-    __shared__ float2 s_in[G::IN], s_h[G::MID];
-    __shared__ float2 s_dx[G::R * G::SEG], s_dy[G::R * G::SEG], s_cx[G::T + 2], s_cy[G::T + 2];
-    const int w = P.w, h = P.h, X0 = blockIdx.x * G::T, Y0 = blockIdx.y * G::T, pair = blockIdx.z, tid = threadIdx.x;
-    const long n = (long)w * h;
-    const bool rule = P.rule, weights = 2 * pair == P.nc;
-    if (P.vals) {
-        const float *a = P.vals + 2 * pair * n, *b = weights ? nullptr : a + n;
-        fill_region<3>(s_in, X0, Y0, w, h, [&](int X, int Y) {
-            const long i = (long)Y * w + X;
-            return make_float2(a[i], b ? b[i] : 0.0f);
-        });
-    } else if (P.fmt == 0) fill_pull_image<0>(P, s_in, X0, Y0, pair);
-    else if (P.fmt == 1) fill_pull_image<1>(P, s_in, X0, Y0, pair);
-    else if (P.fmt == 2) fill_pull_image<2>(P, s_in, X0, Y0, pair);
-    else fill_pull_image<FILL_FLOW>(P, s_in, X0, Y0, pair);
-    // the outputs whose first tap can lie in the tile, from its ends over the step (at least 1)
-    auto range = [](int at, int len, float step, int n, int& lo, int& count) {
-        lo = (int)((float)at / step);
-        count = min((at + G::T < len - 1 ? min((int)((float)(at + G::T) / step), n - 1) : n - 1) - lo + 1, G::T + 2);
-    };
-    int xa, nx, ya, ny;
-    range(X0, w, P.sx, P.dw, xa, nx);
-    range(Y0, h, P.sy, P.dh, ya, ny);
-    auto cell_at = [](int i, float step, int len, int at) {
-        int k;
-        float f;
-        cell((float)i * step, len, k, f);
-        k -= at;
-        return make_float2(__int_as_float(k >= 0 && k < G::T ? k : -1), f);
-    };
-    if (tid < G::R * G::SEG) {
-        s_dx[tid] = border_den<3>(X0 + tid, w, P.t.k);
-        s_dy[tid] = border_den<3>(Y0 + tid, h, P.t.k);
-    }
-    const int k = FILL_THREADS - 1 - tid;
-    if (k < nx) s_cx[k] = cell_at(xa + k, P.sx, w, X0);
-    if (k < ny) s_cy[k] = cell_at(ya + k, P.sy, h, Y0);
-    __syncthreads();
-    float2* s_v = s_in;  // (the column pass reads s_h alone)
-    fill_blur<3>(s_in, s_h, s_dx, s_dy, X0, Y0, w, h, P.t, P.above_first, rule, [&](int seg, int x, const float2* o) {
-#pragma unroll
-        for (int r = 0; r < G::R; r++) s_v[(seg * G::R + r) * G::VS + x] = o[r];
-    });
-    __syncthreads();
-    constexpr int COLS = G::T / 2 + 2;  // the outputs across a tile at a step of 2
-    const long dn = (long)P.dw * P.dh;
-    float *da = P.dst + 2 * pair * dn, *db = weights ? nullptr : da + dn;
-    for (int x0 = 0; x0 < nx; x0 += COLS) {
-        for (int e = tid; e < COLS * ny; e += FILL_THREADS) {
-            const int y = e / COLS, x = x0 + e - y * COLS;
-            if (x >= nx) continue;
-            const float2 cx = s_cx[x], cy = s_cy[y];
-            const int ix = __float_as_int(cx.x), iy = __float_as_int(cy.x);
-            if (ix < 0 || iy < 0) continue;
-            const float2* q = s_v + iy * G::VS + ix;
-            const float2 r = fill_mix(q[0], q[1], q[G::VS], q[G::VS + 1], cx.y, cy.y, P.t.z, rule);
-            const long i = (long)(ya + y) * P.dw + xa + x;
-            da[i] = r.x;
-            if (db) db[i] = r.y;
-        }
-    }
+    __shared__ FillShared<3> S;
+    const int X0 = blockIdx.x * FillGeom<3>::T, Y0 = blockIdx.y * FillGeom<3>::T, pair = blockIdx.z;
+    if (P.vals) fill_pull_planes(P.vals, S.in, threadIdx.x, X0, Y0, P.w, P.h, P.nc, pair);
+    else if (P.fmt == 0) fill_pull_image<0>(P, S.in, X0, Y0, pair);
+    else if (P.fmt == 1) fill_pull_image<1>(P, S.in, X0, Y0, pair);
+    else if (P.fmt == 2) fill_pull_image<2>(P, S.in, X0, Y0, pair);
+    else fill_pull_image<FILL_FLOW>(P, S.in, X0, Y0, pair);
+    fill_pull_tile<FillBlock>(S, X0, Y0, P.w, P.h, P.dw, P.dh, P.sx, P.sy, P.dst, P.nc, pair, P.t, P.above_first, P.rule);
 }
 
 // A sample as stored (holefill.rs:379-404)
@@ -539,45 +516,80 @@ __device__ __forceinline__ void fill_put(void* img, long i, int pair, float2 v) 
     else ((float2*)img)[i] = v;
 }
 
-// The solution of the coarser level at (X, Y): resampled, or given at this size
-__device__ __forceinline__ float2 fill_coarser(const FillPush& P, const float2* s_cx, const float2* s_cy, int X0, int Y0, int X,
-                                               int Y, int pair) {
-    if (P.direct) {
-        const long n = (long)P.w * P.h, i = (long)Y * P.w + X;
-        return make_float2(P.direct[2 * pair * n + i], P.direct[(2 * pair + 1) * n + i]);
-    }
-    const float2 cx = s_cx[X - X0], cy = s_cy[Y - Y0];
-    const float2* q = P.coarse + (long)pair * P.cw * P.ch + (long)__float_as_int(cy.x) * P.cw + __float_as_int(cx.x);
-    return fill_mix(q[0], q[1], q[P.cw], q[P.cw + 1], cx.y, cy.y, P.t.z, P.rule);
+// The coarser solution (planes of pairs of channels, null: zero) at the region's (X, Y), by the tables of S
+__device__ __forceinline__ float2 fill_coarser(const float2* coarse, int cw, int ch, const FillShared<6>& S, int x, int y, int pair,
+                                               float z, bool rule) {
+    if (!coarse) return make_float2(0.0f, 0.0f);
+    const float2 cx = S.cx[x], cy = S.cy[y];
+    const float2* q = coarse + (long)pair * cw * ch + (long)__float_as_int(cy.x) * cw + __float_as_int(cx.x);
+    return fill_mix(q[0], q[1], q[cw], q[cw + 1], cx.y, cy.y, z, rule);
 }
 
-template <int FMT>  // -1: a level of planes
-__device__ __forceinline__ void fill_push(const FillPush& P, float2* s_in, float2* s_h, const float2* s_dx, const float2* s_dy,
-                                          const float2* s_cx, const float2* s_cy) {
+// The tables of a push: the border weights, and the cells of the region in the coarser level
+template <class Threads>
+__device__ __forceinline__ void fill_push_tables(FillShared<6>& S, int X0, int Y0, int w, int h, int cw, int ch, float sx, float sy,
+                                                 const Taps& t) {
     using G = FillGeom<6>;
-    const int w = P.w, h = P.h, X0 = blockIdx.x * G::T, Y0 = blockIdx.y * G::T, pair = blockIdx.z;
-    const int HX = X0 - G::HALO, HY = Y0 - G::HALO;
+    const int tid = Threads::tid(), k = FILL_THREADS - 1 - tid;
+    if (tid < G::R * G::SEG) {
+        S.dx[tid] = border_den<6>(X0 + tid, w, t.k);
+        S.dy[tid] = border_den<6>(Y0 + tid, h, t.k);
+    }
+    if (k < G::RUNS) {
+        auto cell_at = [](int i, float step, int len) {
+            int c;
+            float f;
+            cell((float)i * step, len, c, f);
+            return make_float2(__int_as_float(c), f);
+        };
+        S.cx[k] = cell_at(X0 - G::HALO + k, sx, cw);
+        S.cy[k] = cell_at(Y0 - G::HALO + k, sy, ch);
+    }
+    Threads::sync();
+}
+
+// A level of planes: the values over their weights or the coarser solution, blurred into out
+template <class Threads>
+__device__ __forceinline__ void fill_push_planes(FillShared<6>& S, int X0, int Y0, int w, int h, const float* vals, const float2* coarse,
+                                                 int cw, int ch, float2* out, int nc, int pair, const Taps& t, bool above_first,
+                                                 bool rule) {
+    using G = FillGeom<6>;
     const long n = (long)w * h;
-    const float *va = P.vals + 2 * pair * n, *wt = P.vals + P.nc * n;
-    fill_region<6>(s_in, X0, Y0, w, h, [&](int X, int Y) {
+    const float *va = vals + 2 * pair * n, *wt = vals + nc * n;
+    fill_region<6>(S.in, Threads::tid(), X0, Y0, w, h, [&](int X, int Y) {
         const long i = (long)Y * w + X;
-        if (FMT >= 0) {
-            if (P.holes[i]) return fill_coarser(P, s_cx, s_cy, HX, HY, X, Y, pair);
-            return fill_quot(fill_sample<FMT>(P.img, i, pair), 1.0f, P.rule);
-        }
         const float d = wt[i];
-        if (d == 0.0f) return fill_coarser(P, s_cx, s_cy, HX, HY, X, Y, pair);
-        return fill_quot(make_float2(va[i], va[n + i]), d, P.rule);
+        if (d == 0.0f) return fill_coarser(coarse, cw, ch, S, X - X0 + G::HALO, Y - Y0 + G::HALO, pair, t.z, rule);
+        return fill_quot(make_float2(va[i], va[n + i]), d, rule);
+    });
+    Threads::sync();
+    fill_blur<6, Threads>(S, X0, Y0, w, h, t, above_first, rule, [&](int seg, int x, const float2* o) {
+#pragma unroll
+        for (int r = 0; r < G::R; r++) {
+            const int X = X0 + x, Y = Y0 + seg * G::R + r;
+            if (X < w && Y < h) out[pair * n + (long)Y * w + X] = o[r];
+        }
+    });
+}
+
+// Level 0, the image: the holes take the blurred solution
+template <int FMT>
+__device__ __forceinline__ void fill_push_image(FillShared<6>& S, const FillPush& P, int X0, int Y0, int pair) {
+    using G = FillGeom<6>;
+    const int w = P.w, h = P.h;
+    fill_region<6>(S.in, threadIdx.x, X0, Y0, w, h, [&](int X, int Y) {
+        const long i = (long)Y * w + X;
+        if (P.holes[i]) return fill_coarser(P.coarse, P.cw, P.ch, S, X - X0 + G::HALO, Y - Y0 + G::HALO, pair, P.t.z, P.rule);
+        return fill_quot(fill_sample<FMT>(P.img, i, pair), 1.0f, P.rule);
     });
     __syncthreads();
-    fill_blur<6>(s_in, s_h, s_dx, s_dy, X0, Y0, w, h, P.t, P.above_first, P.rule, [&](int seg, int x, const float2* o) {
+    fill_blur<6, FillBlock>(S, X0, Y0, w, h, P.t, P.above_first, P.rule, [&](int seg, int x, const float2* o) {
 #pragma unroll
         for (int r = 0; r < G::R; r++) {
             const int X = X0 + x, Y = Y0 + seg * G::R + r;
             if (X >= w || Y >= h) continue;
             const long i = (long)Y * w + X;
-            if (FMT < 0) P.out[pair * n + i] = o[r];
-            else if (P.holes[i]) fill_put<(FMT < 0 ? 0 : FMT)>(P.img, i, pair, o[r]);
+            if (P.holes[i]) fill_put<FMT>(P.img, i, pair, o[r]);
         }
     });
 }
@@ -591,8 +603,7 @@ __device__ __forceinline__ void fill_push(const FillPush& P, float2* s_in, float
 __global__ void __launch_bounds__(FILL_THREADS) k_fill_push(const __grid_constant__ FillPush P) {
     using G = FillGeom<6>;
     if (!*P.any) return;
-    __shared__ float2 s_in[G::IN], s_h[G::MID];
-    __shared__ float2 s_dx[G::R * G::SEG], s_dy[G::R * G::SEG], s_cx[G::RUNS], s_cy[G::RUNS];
+    __shared__ FillShared<6> S;
     const int w = P.w, h = P.h, X0 = blockIdx.x * G::T, Y0 = blockIdx.y * G::T, pair = blockIdx.z, tid = threadIdx.x;
     if (P.img) {
         bool hole = false;
@@ -612,141 +623,49 @@ __global__ void __launch_bounds__(FILL_THREADS) k_fill_push(const __grid_constan
         }
         if (!__syncthreads_or(hole)) return;
     }
-    if (tid < G::R * G::SEG) {
-        s_dx[tid] = border_den<6>(X0 + tid, w, P.t.k);
-        s_dy[tid] = border_den<6>(Y0 + tid, h, P.t.k);
-    }
-    const int k = FILL_THREADS - 1 - tid;
-    if (!P.direct && k < G::RUNS) {
-        auto cell_at = [](int i, float step, int len) {
-            int c;
-            float f;
-            cell((float)i * step, len, c, f);
-            return make_float2(__int_as_float(c), f);
-        };
-        s_cx[k] = cell_at(X0 - G::HALO + k, P.sx, P.cw);
-        s_cy[k] = cell_at(Y0 - G::HALO + k, P.sy, P.ch);
-    }
-    __syncthreads();
-    if (!P.img) fill_push<-1>(P, s_in, s_h, s_dx, s_dy, s_cx, s_cy);
-    else if (P.fmt == 0) fill_push<0>(P, s_in, s_h, s_dx, s_dy, s_cx, s_cy);
-    else if (P.fmt == 1) fill_push<1>(P, s_in, s_h, s_dx, s_dy, s_cx, s_cy);
-    else if (P.fmt == 2) fill_push<2>(P, s_in, s_h, s_dx, s_dy, s_cx, s_cy);
-    else fill_push<FILL_FLOW>(P, s_in, s_h, s_dx, s_dy, s_cx, s_cy);
+    fill_push_tables<FillBlock>(S, X0, Y0, w, h, P.cw, P.ch, P.sx, P.sy, P.t);
+    if (!P.img)
+        fill_push_planes<FillBlock>(S, X0, Y0, w, h, P.vals, P.coarse, P.cw, P.ch, P.out, P.nc, pair, P.t, P.above_first, P.rule);
+    else if (P.fmt == 0) fill_push_image<0>(S, P, X0, Y0, pair);
+    else if (P.fmt == 1) fill_push_image<1>(S, P, X0, Y0, pair);
+    else if (P.fmt == 2) fill_push_image<2>(S, P, X0, Y0, pair);
+    else fill_push_image<FILL_FLOW>(S, P, X0, Y0, pair);
 }
 
-// flow/sample.rs:91-112 at element (x, y) of a dw x dh plane from the sw x sh plane s (the lerps
-// over the arithmetic set)
-template <bool R>
-__device__ __forceinline__ float stack_resample_px(const float* __restrict__ s, int sw, int sh, int dw, int dh, int x,
-                                                   int y) {
-    float sx = ((float)sw - 1.0f) / (float)(dw - 1);
-    float sy = ((float)sh - 1.0f) / (float)(dh - 1);
-    int ix, iy;
-    float fx, fy;
-    cell((float)x * sx, sw, ix, fx);
-    cell((float)y * sy, sh, iy, fy);
-    long i = (long)iy * sw + ix;
-    float top = lerp_r<R>(s[i], s[i + 1], fx);
-    float bot = lerp_r<R>(s[i + sw], s[i + sw + 1], fx);
-    return lerp_r<R>(top, bot, fy);
-}
-
-// ---- the coarse levels of the fill in one block ------------------------------------------------------
-
-long fill_coarse_floats(const int dims[][2], int k0, int top, int np, int nc) {
-    long f = 0;
-    for (int k = k0; k <= top; k++) f += (long)np * dims[k][0] * dims[k][1];  // the stacks
-    long n0 = (long)dims[k0][0] * dims[k0][1];
-    return f + 2 * np * n0 + 2 * nc * n0;  // two pass scratches, the solution and the next one
-}
-
-// holefill.rs:260-377 over the levels k0 .. top, the same elements as the stack kernels (the pull's
-// blur5 and resample, the push's combine, Gaussian r5 and resample), block barriers between them.
-// The pull reads level k - 1 directly (the stack kernels blur a copy, which keeps it for the push;
-// here the blur writes scratch planes and the level stays as it is).
-template <bool R>
-__device__ void fill_coarse_body(const FillCoarseJob& J, float* fsm) {
-    const int np = J.np, nc = J.nc, k0 = J.k0, top = J.top;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    auto n_of = [&](int k) { return J.dims[k][0] * J.dims[k][1]; };
-    auto stack_at = [&](int k) {
-        float* p = fsm;
-        for (int j = k0; j < k; j++) p += np * n_of(j);
-        return p;
-    };
-    const int n0 = n_of(k0);
-    float* T = stack_at(top + 1);
-    float* U = T + np * n0;
-    float* sol = U + np * n0;
-    float* nxt = sol + nc * n0;
-    for (int i = tid; i < np * n0; i += nt) fsm[i] = J.s_k0[i];
-    __syncthreads();
-    // pull: blur5 of level k - 1 (horizontal into U, vertical into T), resampled into level k
-    for (int k = k0 + 1; k <= top; k++) {
-        const int pw = J.dims[k - 1][0], ph = J.dims[k - 1][1], cw = J.dims[k][0], chh = J.dims[k][1];
-        const int pn = pw * ph, cn = cw * chh;
-        const float* P = stack_at(k - 1);
-        float* C = stack_at(k);
-        for (int i = tid; i < np * pn; i += nt) {
-            const int pl = i / pn, e = i - pl * pn, y = e / pw, x = e - y * pw;
-            U[i] = stack_pass_px<R, 3, false, false>(P + pl * pn, pw, ph, x, y, J.b5);
-        }
-        __syncthreads();
-        for (int i = tid; i < np * pn; i += nt) {
-            const int pl = i / pn, e = i - pl * pn, y = e / pw, x = e - y * pw;
-            T[i] = J.above_first ? stack_pass_px<R, 3, true, true>(U + pl * pn, pw, ph, x, y, J.b5)
-                                 : stack_pass_px<R, 3, true, false>(U + pl * pn, pw, ph, x, y, J.b5);
-        }
-        __syncthreads();
-        for (int i = tid; i < np * cn; i += nt) {
-            const int pl = i / cn, e = i - pl * cn, y = e / cw, x = e - y * cw;
-            C[i] = stack_resample_px<R>(T + pl * pn, pw, ph, cw, chh, x, y);
-        }
-        __syncthreads();
-    }
-    // push: the solution starts at zero on the top level
-    for (int i = tid; i < nc * n_of(top); i += nt) sol[i] = 0.0f;
-    __syncthreads();
-    for (int lv = top; lv >= k0; lv--) {
-        const int lw = J.dims[lv][0], lh = J.dims[lv][1], ln = lw * lh;
-        const float* V = stack_at(lv);
-        for (int i = tid; i < ln; i += nt) {  // holefill.rs:371-377
-            const float wt = V[nc * ln + i];
-            if (wt != 0.0f)
-                for (int c = 0; c < nc; c++) sol[c * ln + i] = Ar<R>::div(V[c * ln + i], wt);
-        }
-        __syncthreads();
-        for (int i = tid; i < nc * ln; i += nt) {
-            const int pl = i / ln, e = i - pl * ln, y = e / lw, x = e - y * lw;
-            U[i] = stack_pass_px<R, 6, false, false>(sol + pl * ln, lw, lh, x, y, J.g5);
-        }
-        __syncthreads();
-        for (int i = tid; i < nc * ln; i += nt) {
-            const int pl = i / ln, e = i - pl * ln, y = e / lw, x = e - y * lw;
-            sol[i] = J.above_first ? stack_pass_px<R, 6, true, true>(U + pl * ln, lw, lh, x, y, J.g5)
-                                   : stack_pass_px<R, 6, true, false>(U + pl * ln, lw, lh, x, y, J.g5);
-        }
-        __syncthreads();
-        const int dw = J.dims[lv - 1][0], dh = J.dims[lv - 1][1], dn = dw * dh;
-        float* dst = lv > k0 ? nxt : J.out;  // level k0 - 1 is the host's to push further
-        for (int i = tid; i < nc * dn; i += nt) {
-            const int pl = i / dn, e = i - pl * dn, y = e / dw, x = e - y * dw;
-            dst[i] = stack_resample_px<R>(sol + pl * ln, lw, lh, dw, dh, x, y);
-        }
-        __syncthreads();
-        float* t = sol;
-        sol = nxt;
-        nxt = t;
-    }
-}
-
-__global__ void __launch_bounds__(FILL_COARSE_THREADS) k_fill_coarse(FillCoarseJob J) {
+// The levels k0 .. top, of one tile each, up from level k0 and down to it in one block: a group of threads per
+// pair of channels and for the weights, the level's planes in global memory (the block's own, and in its L1). A
+// level and direction takes some 4 us. (One block over planes in shared memory, a thread per element of a
+// plane with a division for its place, took 100 us for these levels and 60 x 33, this and two launches 50.)
+union FillTailShared {
+    FillShared<3> up;
+    FillShared<6> down;
+};
+__global__ void __launch_bounds__(FILL_TAIL_GROUPS * FILL_THREADS) k_fill_tail(const __grid_constant__ FillTail J) {
     if (!*J.any) return;
-    extern __shared__ float fsm[];
-    if (J.rule) fill_coarse_body<true>(J, fsm);
-    else fill_coarse_body<false>(J, fsm);
+    extern __shared__ __align__(16) unsigned char tail_sm[];
+    const int pair = threadIdx.x / FILL_THREADS;
+    FillTailShared& S = reinterpret_cast<FillTailShared*>(tail_sm)[pair];
+    auto step = [](int from, int to) { return ((float)from - 1.0f) / (float)(to - 1); };
+    for (int k = J.k0 + 1; k <= J.top; k++) {
+        const int w = J.dims[k - 1][0], h = J.dims[k - 1][1], dw = J.dims[k][0], dh = J.dims[k][1];
+        if (2 * pair <= J.nc) {
+            fill_pull_planes(J.base + J.offs[k - 1], S.up.in, FillGroup::tid(), 0, 0, w, h, J.nc, pair);
+            fill_pull_tile<FillGroup>(S.up, 0, 0, w, h, dw, dh, step(w, dw), step(h, dh), J.base + J.offs[k], J.nc, pair, J.b5,
+                                      J.above_first, J.rule);
+        }
+        __syncthreads();
+    }
+    for (int k = J.top; k >= J.k0; k--) {
+        const int w = J.dims[k][0], h = J.dims[k][1], cw = k < J.top ? J.dims[k + 1][0] : 2, ch = k < J.top ? J.dims[k + 1][1] : 2;
+        if (2 * pair < J.nc) {
+            fill_push_tables<FillGroup>(S.down, 0, 0, w, h, cw, ch, step(cw, w), step(ch, h), J.g5);
+            fill_push_planes<FillGroup>(S.down, 0, 0, w, h, J.base + J.offs[k], k < J.top ? J.blurred[(k + 1) & 1] : nullptr, cw, ch,
+                                        J.blurred[k & 1], J.nc, pair, J.g5, J.above_first, J.rule);
+        }
+        __syncthreads();
+    }
 }
+size_t fill_tail_smem() { return FILL_TAIL_GROUPS * sizeof(FillTailShared); }
 
 // a hole in an image with a side of 1 pixel: the fill refuses it (holefill.rs:273-277)
 __global__ void k_hole_side1(const int* __restrict__ any_hole, int* __restrict__ flag) {
