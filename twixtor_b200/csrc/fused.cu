@@ -473,6 +473,11 @@ __device__ __forceinline__ bool iter_column5(const LevelIterArgs& P, const float
 #pragma unroll
     for (int r = 0; r < R; r++)
         if (y0 + r < P.h) P.f_out[(y0 + r) * P.w + x] = f[r];
+    if (P.any) {
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            if (y0 + r < P.h) check_range(P.any, x, y0 + r, f[r], P.w, P.h);
+    }
     if (P.b_out) {
         calc_b_run<R>(P.i0, P.mask_y, P.w, P.h, x, y0, f, i1, g, b);
 #pragma unroll

@@ -351,16 +351,17 @@ int build_user_dev(tw_ctx* ctx, const UserPairs& pr, const Geo& g, int W, int H,
 // ---- block matching (flow.rs:551-622) -----------------------------------------------------------------
 // Rows on the row-major planes, the swept field going into its transpose ft (w * h elements of scratch);
 // then the column sweeps on the transposed planes (AT, BT: the level's bands stored column by column),
-// the field going back into f.
+// the field going back into f. any (may be null): the level's range flag, checked on the way.
 void block_match(tw_ctx* ctx, const float* A, const float* B, const float* AT, const float* BT, float2* f, float2* ft, int w,
-                 int h, bool fast) {
+                 int h, bool fast, int* any) {
     // no block has a cost in a level of fewer than 4 x 4 pixels (flow.rs:474-500), so no vector moves there;
     // callers refuse lines above BM_MAX_LINE before any launch
     if (w < 4 || h < 4) return;
     double b = 24.0 * w * h;  // per launch (both sweeps): the field read and written (8 + 8), A and B read once (4 + 4)
     LevelTune t = level_tune(ctx, w, h);
     LAUNCHV(ctx, fast, b, k_bm_rows, h - 2, std::min(t.bm_rows_threads, BM_MAX_THREADS), bm_smem_bytes(w), A, B, f, w, h, ft, ctx->g7.z);
-    LAUNCHV(ctx, fast, b, k_bm_cols, w - 2, std::min(t.bm_cols_threads, BM_MAX_THREADS), bm_smem_bytes(h), AT, BT, ft, w, h, f, ctx->g7.z);
+    LAUNCHV(ctx, fast, b, k_bm_cols, w - 2, std::min(t.bm_cols_threads, BM_MAX_THREADS), bm_smem_bytes(h), AT, BT, ft, w, h, f, ctx->g7.z,
+            any);
 }
 
 // ---- one solve over two resident pyramids (flow.rs:1258-1307) ------------------------------------------
@@ -516,6 +517,8 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
         P.g7 = ctx->g7;
         P.g5 = ctx->g5;
         const LevelTune ic = level_tune(ctx, w, h);
+        // the range check goes with the level's last kernel, unless the points move its flow after that
+        const bool match_last = l != 0 && !s.skip_refine && w >= 4 && h >= 4;
         for (int it = 0; it < 3; it++) {
             // iteration it reads B from bb[it & 1]; the next one's B comes from its epilogue, or after
             // the finest level's block matching from the pointwise pass
@@ -524,17 +527,18 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
             P.b_out = emit ? bb[(it + 1) & 1] : nullptr;
             P.f = f;
             P.f_out = fn;
+            P.any = it == 2 && !match_last && !udu ? any + l : nullptr;
             level_iter(ctx, ic, P, fast);
             std::swap(f, fn);
             if (it == 1 && l == 0) {
-                if (!s.skip_refine) block_match(ctx, A, B, AT, BT, f, ft, w, h, fast);
+                if (!s.skip_refine) block_match(ctx, A, B, AT, BT, f, ft, w, h, fast, nullptr);
                 user();
                 LAUNCHV(ctx, fast, 40.0 * px, k_calc_b_pitched, grid2(w, h), TB, 0, A, B, grad, f, w, h, mask_y, bb[0], P.bp);
             }
         }
-        if (l != 0 && !s.skip_refine) block_match(ctx, A, B, AT, BT, f, ft, w, h, fast);
+        if (match_last) block_match(ctx, A, B, AT, BT, f, ft, w, h, fast, udu ? nullptr : any + l);
         user();
-        LAUNCHV(ctx, fast, 0, k_range_any, grid2(w, h), TB, 0, f, w, h, any + l);
+        if (udu) LAUNCHV(ctx, fast, 0, k_range_any, grid2(w, h), TB, 0, f, w, h, any + l);
     }
     LAUNCHV(ctx, fast, 0, k_apply_negate, grid1((long)np0), TB, 0, f, (long)np0, any, start, start == 0 && damp_any, damp,
             (float2*)out, nan_flag);

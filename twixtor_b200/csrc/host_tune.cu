@@ -185,7 +185,7 @@ int tw_autotune(tw_ctx* ctx, const tw_flow_settings* s, int32_t width, int32_t h
                     if (ms < br) { br = ms; best.bm_rows_threads = th; }
                     ms = timed([&] {
                         cudaMemcpyAsync(ft, fsave, fbytes, cudaMemcpyDeviceToDevice, ctx->stream);
-                        LAUNCH(ctx, k_bm_cols, w - 2, th, bm_smem_bytes(h), AT, BT, ft, w, h, f, ctx->g7.z);
+                        LAUNCH(ctx, k_bm_cols, w - 2, th, bm_smem_bytes(h), AT, BT, ft, w, h, f, ctx->g7.z, (int*)nullptr);
                     });
                     if (ms < bc) { bc = ms; best.bm_cols_threads = th; }
                 }

@@ -80,11 +80,12 @@ __global__ void k_deinterleave(const float* __restrict__ in, long n, float* __re
 // shared. k_bm_rows: both sweeps of every row (left to right, then right to left) of f, the result
 // written into the transpose ft (element (x, y) at [x * h + y]); k_bm_cols: both sweeps of every
 // column (top to bottom, then bottom to top) read from ft, with the transposes of A and B, the result
-// written back into f. Lines 0 and last are not swept; levels of at least 4 x 4. z: -0.0 (level.cuh).
+// written back into f. Lines 0 and last are not swept; levels of at least 4 x 4. z: -0.0 (level.cuh); any (may
+// be null): set when some pixel's flow is in range, as k_range_any does.
 __global__ void k_bm_rows(const float* __restrict__ A, const float* __restrict__ B, const float2* __restrict__ f, int w,
                           int h, float2* __restrict__ ft, float z);
 __global__ void k_bm_cols(const float* __restrict__ AT, const float* __restrict__ BT, const float2* __restrict__ ft, int w,
-                          int h, float2* f, float z);
+                          int h, float2* f, float z, int* any);
 // two w x h planes into their h x w transposes; block (32, 8), grid (ceil(w/32), ceil(h/32))
 __global__ void k_transpose2(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ at,
                              float* __restrict__ bt, int w, int h);
@@ -197,6 +198,7 @@ struct LevelIterArgs {
     const float* mask_y;
     float2* f_out;
     float2* b_out;
+    int* any;  // the level's range flag (may be null)
     int w, h, bp, af;
     Taps g7, g5;
 };

@@ -11,7 +11,7 @@ __global__ void k_range_any(const float2* __restrict__ f, int w, int h, int* __r
 __global__ void k_bm_rows(const float* __restrict__ A, const float* __restrict__ B, const float2* __restrict__ f, int w,
                           int h, float2* __restrict__ ft, float z);
 __global__ void k_bm_cols(const float* __restrict__ AT, const float* __restrict__ BT, const float2* __restrict__ ft, int w,
-                          int h, float2* f, float z);
+                          int h, float2* f, float z, int* any);
 __global__ void k_transpose2(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ at,
                              float* __restrict__ bt, int w, int h);
 __global__ void k_pyramid_step_16(const __grid_constant__ PyramidStep P);

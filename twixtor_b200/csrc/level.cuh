@@ -480,6 +480,15 @@ __device__ __forceinline__ bool zero_at_level(const int* any, int l, int start) 
     return check && any[l] == 0;
 }
 
+// The range check at pixel (x, y) with flow f (flow.rs:430-442, all_flow_out_of_range, as "some pixel is in
+// range"), where a level's last kernel writes the flow: nearly every pixel is in range, so the flag is set within
+// the first ones and read by the others.
+__device__ __forceinline__ void check_range(int* any, int x, int y, float2 f, int w, int h) {
+    const float px = (float)x + f.x, py = (float)y + f.y;
+    const bool in = 0.0f <= px && px <= (float)(w - 1) && 0.0f <= py && py <= (float)(h - 1);
+    if (in && *(volatile int*)any == 0) atomicOr(any, 1);
+}
+
 // flow.rs:376-391 (upsample_flow, bilinear2 of sample.rs:69-86) from a field of sw x sh to one of dw x
 // dh: the scales sx, sy and their reciprocals, formed once on the host (the same IEEE operations).
 __host__ __device__ inline UpsampleScale upsample_scale(int sw, int sh, int dw, int dh) {

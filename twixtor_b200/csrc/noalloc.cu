@@ -78,7 +78,7 @@ extern "C" int tw_block_match_noalloc(const float* a, const float* b, float* flo
         if (e == cudaSuccess) e = launch(tw::k_transpose2, ga, tt, 0, s, a, b, at, bt, (int)width, (int)height);
         if (e == cudaSuccess)
             e = launch(tw::k_bm_cols, dim3(width - 2), dim3(tb), tw::bm_smem_bytes(height), s, (const float*)at,
-                       (const float*)bt, (const float2*)ft, (int)width, (int)height, f, -0.0f);
+                       (const float*)bt, (const float2*)ft, (int)width, (int)height, f, -0.0f, (int*)nullptr);
     }
     if (e == cudaSuccess) e = launch(k_copy_floats, g2, dim3(tb), 0, s, (const float*)f, flow, 2 * n);
     if (e != cudaSuccess) return TW_ERR_CUDA;

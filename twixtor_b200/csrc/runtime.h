@@ -314,7 +314,7 @@ __global__ void k_set_flag(int* flags, int idx);  // flags[idx] = 1 (the injecte
 LevelTune level_tune(tw_ctx* ctx, int w, int h);
 LevelTune default_tune(int w, int h);
 void block_match(tw_ctx* ctx, const float* A, const float* B, const float* AT, const float* BT, float2* f, float2* ft, int w,
-                 int h, bool fast = false);
+                 int h, bool fast = false, int* any = nullptr);
 void level_iter(tw_ctx* ctx, LevelTune ic, const LevelIterArgs& P, bool fast);
 size_t pyramid_floats(const Geo& g);
 int build_pyramid_dev(tw_ctx* ctx, const void* eng_dev, int W, int H, int fmt, const tw_flow_settings& s, const Geo& g,

@@ -203,19 +203,11 @@ __global__ void k_resample(const float* __restrict__ src, int sw, int sh, float*
     dst[(long)y * dw + x] = bilinear1(src, sw, sh, (float)x * sx, (float)y * sy);
 }
 
-// flow.rs:430-442 (all_flow_out_of_range), as "some pixel is in range"
+// The range check of a level whose flow the tracking points move at its end
 __global__ void k_range_any(const float2* __restrict__ f, int w, int h, int* __restrict__ any_in_range) {
     int x = blockIdx.x * blockDim.x + threadIdx.x;
     int y = blockIdx.y;
-    bool in = false;
-    if (x < w && y < h) {
-        const float2 v = f[(long)y * w + x];
-        float px = (float)x + v.x;
-        float py = (float)y + v.y;
-        float fw = (float)(w - 1), fh = (float)(h - 1);
-        in = 0.0f <= px && px <= fw && 0.0f <= py && py <= fh;
-    }
-    if (__syncthreads_or(in) && threadIdx.x == 0) atomicOr(any_in_range, 1);
+    if (x < w && y < h) check_range(any_in_range, x, y, f[(long)y * w + x], w, h);
 }
 
 __global__ void k_deinterleave(const float* __restrict__ in, long n, float* __restrict__ fu, float* __restrict__ fv) {
@@ -523,7 +515,7 @@ __device__ void bm_sweep(float* su, float* sv, float* c0, const float* s_a, int*
 // transposed planes (element (x, y) at [x * h + y]) so that the line's patches stay contiguous.
 template <bool COLS>
 __device__ void bm_line(const float* __restrict__ A, const float* __restrict__ B, const float2* src, const float2* ends,
-                        float2* dst, int w, int h, int fixed, float z) {
+                        float2* dst, int w, int h, int fixed, float z, int* any) {
     extern __shared__ float sm[];
     const int len = COLS ? h : w, other = COLS ? w : h;
     if (len < 3) return;  // no interior position
@@ -552,6 +544,13 @@ __device__ void bm_line(const float* __restrict__ A, const float* __restrict__ B
     bm_sweep<COLS>(su, sv, c0, s_a, endp, qa, qb, ctl, entry, prevl, B, w, h, fixed, len, true, z);
     for (int i = threadIdx.x + 1; i <= len - 2; i += blockDim.x) {
         dst[(long)i * other + fixed] = make_float2(su[i], sv[i]);
+    }
+    if (COLS && any) {  // the range check of the level: this column, and the end ones, which are not swept
+        for (int i = threadIdx.x; i < len; i += blockDim.x) {
+            check_range(any, fixed, i, make_float2(su[i], sv[i]), w, h);
+            if (fixed == 1) check_range(any, 0, i, dst[(long)i * w], w, h);
+            if (fixed == w - 2) check_range(any, w - 1, i, dst[(long)i * w + w - 1], w, h);
+        }
     }
 }
 
@@ -583,16 +582,16 @@ __global__ void __launch_bounds__(BM_MAX_THREADS) k_bm_rows(const float* __restr
                           int h, float2* __restrict__ ft, float z) {
     int y = blockIdx.x + 1;  // rows 1..h-2
     if (y > h - 2) return;
-    bm_line<false>(A, B, f, nullptr, ft, w, h, y, z);
+    bm_line<false>(A, B, f, nullptr, ft, w, h, y, z, nullptr);
 }
 
 // The column sweeps of columns 1..w-2 from the transposed field ft that k_bm_rows wrote, the end rows 0
-// and h-1 from f; the result into f at rows 1..h-2 of those columns
+// and h-1 from f; the result into f at rows 1..h-2 of those columns; any (may be null): the level's range flag
 __global__ void __launch_bounds__(BM_MAX_THREADS) k_bm_cols(const float* __restrict__ AT, const float* __restrict__ BT, const float2* __restrict__ ft, int w,
-                          int h, float2* f, float z) {
+                          int h, float2* f, float z, int* any) {
     int x = blockIdx.x + 1;  // columns 1..w-2
     if (x > w - 2) return;
-    bm_line<true>(AT, BT, ft, f, f, w, h, x, z);
+    bm_line<true>(AT, BT, ft, f, f, w, h, x, z, any);
 }
 
 TW_VARIANT_END
