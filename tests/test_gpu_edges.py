@@ -169,3 +169,33 @@ def test_forward_warp_where_its_plain_arithmetic_ends(dev, pyramid, case):
         return
     got = dev.forward_warp(src, w, h, 2, flow, (w, h), 1.0, pyramid, True)
     assert same(got[0], want[0]) and same(got[1], want[1])
+
+
+@pytest.mark.parametrize("w,h,fw,fh", [(2, 2, 2, 2), (33, 9, 17, 5), (31, 33, 31, 33), (65, 8, 22, 3), (20, 41, 61, 83)])
+@pytest.mark.parametrize("smooth", [False, True])
+def test_adjoint_at_the_ends_of_its_columns(dev, w, h, fw, fh, smooth):
+    """Rows and columns that end inside a warp's strip, vectors that share corners (smooth) and that do not, on
+    and beyond the border: within 1e-3 of the double precision gradients (float32 sums of at most a few dozen
+    terms in any order), as in test_gpu_adjoint."""
+    import torch
+
+    from twixtor_b200 import adjoint
+    import os
+    import sys
+    sys.path.insert(0, os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "oracle"))
+    import adjoint_fp64 as A
+    n, wa = 2, 0.35
+    rng = np.random.RandomState(w * 3 + fh)
+    a, b, g = (rng.rand(n, h, w, 4).astype(np.float32) for _ in range(3))
+    fab, fba = ((np.full((n, fh, fw, 2), 1.25) + rng.uniform(-0.01, 0.01, (n, fh, fw, 2)) if smooth
+                 else rng.uniform(-9, 9, (n, fh, fw, 2))).astype(np.float32) for _ in range(2))
+    host = (a, b, fab, fba)
+    xs = [torch.from_numpy(x).cuda().requires_grad_(True) for x in host]
+    out = adjoint.warp_blend(*xs, wa, dev)
+    out.backward(torch.from_numpy(g).cuda())
+    for i in range(n):
+        _, _, *refs = A.warp_blend_grads(*[x[i].reshape(-1) for x in host], w, h, fw, fh, wa, pos32=True,
+                                         grad_out=g[i].reshape(-1))
+        for x, ref in zip(xs, refs):
+            got = x.grad[i].cpu().numpy().astype(np.float64)
+            assert np.linalg.norm(got.reshape(-1) - np.asarray(ref).reshape(-1)) <= 1e-3 * max(np.linalg.norm(ref), 1e-6)

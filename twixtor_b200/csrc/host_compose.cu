@@ -1033,19 +1033,14 @@ int tw_warp_blend_adjoint(tw_ctx* ctx, const float* a, const float* b, const flo
     P.rx = (float)(flow_w - 1) / (float)(width - 1);
     P.ry = (float)(flow_h - 1) / (float)(height - 1);
     P.wa = wa;
-    P.tiled = P.rx <= 1.0f && P.ry <= 1.0f;
-    if (!ctx->adj_smem_set) {
-        CHECK(ctx->cuda(cudaFuncSetAttribute(k_warp_blend_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, ADJ_SMEM),
-                        "adjoint shared memory"));
-        ctx->adj_smem_set = true;
-    }
+    P.z = -0.0f;
     dim3 grid((unsigned)((width + ADJ_TX - 1) / ADJ_TX), (unsigned)((height + ADJ_TY - 1) / ADJ_TY), (unsigned)batch);
     // algorithmic bytes: A, B and the target or output gradient read, the output and the four
     // gradients written once, the flows read once
     double img = 16.0 * width * height * batch, fl = 8.0 * flow_w * flow_h * batch;
     double bytes = img * (2 + (target || grad_out ? 1 : 0) + (out ? 1 : 0) + (da ? 1 : 0) + (db ? 1 : 0)) +
                    fl * (2 + (df_ab ? 1 : 0) + (df_ba ? 1 : 0));
-    LAUNCHB(ctx, bytes, k_warp_blend_adjoint, grid, ADJ_THREADS, ADJ_SMEM, P);
+    LAUNCHB(ctx, bytes, k_warp_blend_adjoint, grid, ADJ_THREADS, 0, P);
     return ctx->cuda(cudaGetLastError(), "launch");
 }
 

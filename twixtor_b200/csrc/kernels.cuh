@@ -463,13 +463,11 @@ struct AdjParams {
     float* df_ba;
     int w, h, fw, fh;
     float rx, ry, wa;
-    bool tiled;             // rx <= 1 and ry <= 1: the flow gradients gather in shared memory first
+    float z;                // -0.0 (WarpParams)
 };
-constexpr int ADJ_TX = 32, ADJ_TY = 32, ADJ_THREADS = 256;  // the output tile of a CTA
-constexpr int ADJ_BOX_PX = 1536;                            // the shared image gradient tile, per side
-// dynamic shared memory: two image tiles (float4) and two flow tiles ((TX + 2) x (TY + 2) x 2 floats)
-constexpr int ADJ_SMEM = 2 * ADJ_BOX_PX * 16 + 2 * (ADJ_TX + 2) * (ADJ_TY + 2) * 2 * 4;
-__global__ void k_warp_blend_adjoint(AdjParams P);
+constexpr int ADJ_TX = 32, ADJ_TY = 32, ADJ_THREADS = 128;  // the output tile of a CTA
+constexpr int ADJ_ROWS = ADJ_TY / (ADJ_THREADS / 32);       // the rows of a warp
+__global__ void k_warp_blend_adjoint(const __grid_constant__ AdjParams P);
 
 // ---- Vectors In (vecin.cu) ----
 // vectors.rs:474-528 + :555-561 with the hole rule of holefill.rs:124-133: the flow of an encoded

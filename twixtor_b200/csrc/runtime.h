@@ -162,7 +162,6 @@ struct tw_ctx {
     DevBuf wb_wt[2], wb_tmp[2], wb_mask[2], wb_cov[2];  // Weighted Blend (the calls on the context's stream)
     DevBuf pre_blur, comp_e;  // Blur Compensation: the composite before the blur, the engine result
     DevBuf vi_clip[3], vi_out, vi_wire[5];  // Vectors In: the clips on the device, the output clip, one frame's wires
-    bool adj_smem_set = false;  // the adjoint kernel's dynamic shared memory limit is raised
     DevBuf host_stage;  // unused placeholder for pinned staging
     std::vector<cudaEvent_t> ev_pool;  // the profiler's events (KernelProfile)
     // the forward warp: vertices, mip pyramid, per pixel counts / offsets, hit lists, flags
