@@ -199,3 +199,28 @@ def test_adjoint_at_the_ends_of_its_columns(dev, w, h, fw, fh, smooth):
         for x, ref in zip(xs, refs):
             got = x.grad[i].cpu().numpy().astype(np.float64)
             assert np.linalg.norm(got.reshape(-1) - np.asarray(ref).reshape(-1)) <= 1e-3 * max(np.linalg.norm(ref), 1e-6)
+
+
+@pytest.mark.parametrize("size", [(3, 3), (3, 40), (33, 4), (5, 5), (32, 32), (33, 33), (65, 34), (97, 66)])
+@pytest.mark.parametrize("fmt", [0, 2])
+@pytest.mark.parametrize("density", [0.02, 0.3, 0.7])
+def test_sharpening_mask_at_the_ends_of_its_tiles(dev, size, fmt, density):
+    """Weighted Blend compositions of frames that differ in scattered blocks, single pixels and along the border:
+    the difference mask's clean-up across tiles of 32 x 32, with borders on, before and after a tile's edge."""
+    w, h = size
+    rng = np.random.RandomState(w + 5 * h)
+    top = 255 if fmt == 0 else 1.0
+    a = rng.random_sample((h, w, 4)) * top * 0.3
+    a[..., 0] = top
+    b = a.copy()
+    on = rng.random_sample((h, w)) < density
+    on |= np.kron(rng.random_sample((h // 4 + 1, w // 4 + 1)) < density / 2, np.ones((4, 4)))[:h, :w] > 0
+    on[:, 0] |= rng.random_sample(h) < 0.5
+    on[-1] |= rng.random_sample(w) < 0.5
+    b[on, 1:] = top
+    a, b = (x.reshape(-1).astype(tw.DTYPES[fmt]) for x in (a, b))
+    flows = [rng.uniform(-1.5, 1.5, w * h * 2).astype(np.float32) for _ in range(2)]
+    sel = tw.Selection(wa=np.float32(0.4), interp=2)
+    cs = tw.EngineSettings(taps_above_first=True)
+    got = dev.compose_vectors(cs, sel, a, b, w, h, fmt, flows[0], flows[1], (w, h))
+    assert same(got, O.compose_vectors3(a, b, w, h, fmt, flows[0], flows[1], w, h, sel, cs))

@@ -111,12 +111,6 @@ __device__ __forceinline__ void blur_px(const void* src, void* dst, int w, int h
     for (int l = 0; l < 4; l++) d[l] = wb_store<P>(v[l]);
 }
 
-__device__ __forceinline__ int ring_sum(const uint8_t* t, int w, int cx, int r0, int r1, int r2) {  // filters.rs:339-345
-    auto at = [&](int y, int xx) { return (int)t[(long)y * w + xx]; };
-    return at(r0, cx) + at(r0, cx - 1) + at(r0, cx + 1) + at(r1, cx - 1) + at(r1, cx + 1) + at(r2, cx - 1) +
-           at(r2, cx) + at(r2, cx + 1);
-}
-
 }  // namespace
 
 // filters.rs:254-280, one pass: along the rows (cols == false) or along the columns of src
@@ -128,62 +122,104 @@ __global__ void k_wb_blur(const void* __restrict__ src, void* __restrict__ dst, 
     else blur_px<float>(src, dst, w, h, T, cols, above_first);
 }
 
-// filters.rs:301-334: 255 where (|dR| + |dG|) + |dB| >= limit (differences in float), else 0
+// filters.rs:301-334: (|dR| + |dG|) + |dB| >= limit at pixel i (differences in float)
+__device__ __forceinline__ bool differs(const void* a, const void* b, int fmt, long i, float limit) {
+    float pa[4], pb[4];
+    if (fmt == 0) { px_floats((const uint8_t*)a + i * 4, pa); px_floats((const uint8_t*)b + i * 4, pb); }
+    else if (fmt == 1) { px_floats((const uint16_t*)a + i * 4, pa); px_floats((const uint16_t*)b + i * 4, pb); }
+    else { px_floats((const float*)a + i * 4, pa); px_floats((const float*)b + i * 4, pb); }
+    const float sum = (fabsf(pa[1] - pb[1]) + fabsf(pa[2] - pb[2])) + fabsf(pa[3] - pb[3]);
+    return sum >= limit;
+}
+
+// The mask without its clean-up: 255 or 0
 __global__ void k_wb_diff_mask(const void* __restrict__ a, const void* __restrict__ b, int fmt, long n, float limit,
                                uint8_t* __restrict__ mask, const int* __restrict__ gate) {
     if (gated_off(gate)) return;
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float d[4];
-#pragma unroll
-    for (int c = 1; c < 4; c++) {
-        float va, vb;
-        if (fmt == 0) { va = (float)((const uint8_t*)a)[i * 4 + c]; vb = (float)((const uint8_t*)b)[i * 4 + c]; }
-        else if (fmt == 1) { va = (float)((const uint16_t*)a)[i * 4 + c]; vb = (float)((const uint16_t*)b)[i * 4 + c]; }
-        else { va = ((const float*)a)[i * 4 + c]; vb = ((const float*)b)[i * 4 + c]; }
-        d[c] = fabsf(va - vb);
+    if (i < n) mask[i] = differs(a, b, fmt, i, limit) ? 0xff : 0;
+}
+
+// The difference mask and its clean-up (filters.rs:301-334, :507-520) of a frame of at least 3 x 3: the prunes
+// 254 and 509 (:360-375; with h >= 5), the dilate of the rows (:406-418), the fills 254 -> 255 twice, 254 -> 128
+// and 127 -> 64 (:387-400), each with the border replicated (:425-496: the fill's result at the coordinate
+// clamped to the inner rectangle 1..w-2 x 1..h-2). A 32 x 32 tile with what the steps reach around it (a
+// clamped coordinate one further): steps at the region's edge are wrong there and never reach the tile.
+//
+// Bound by latency: launches of their own, a byte a thread and a 64 bit division for its row, took 8 of
+// 3 to 5 us for 720 x 486. A region without a difference stays empty.
+constexpr int WBM_T = 32, WBM_HX = 8, WBM_HY = 10, WBM_W = WBM_T + 2 * WBM_HX, WBM_H = WBM_T + 2 * WBM_HY;
+
+__global__ void __launch_bounds__(WBM_THREADS) k_wb_mask(const void* __restrict__ a, const void* __restrict__ b, int fmt, int w, int h,
+                                                         float limit, uint8_t* __restrict__ mask, const int* __restrict__ gate) {
+    if (gated_off(gate)) return;
+    __shared__ uint8_t s_m[2][WBM_W * WBM_H];
+    const int X0 = blockIdx.x * WBM_T, Y0 = blockIdx.y * WBM_T, gx = X0 - WBM_HX, gy = Y0 - WBM_HY;
+    bool any = false;
+    for (int e = threadIdx.x; e < WBM_W * WBM_H; e += WBM_THREADS) {
+        const int r = e / WBM_W, X = gx + e - r * WBM_W, Y = gy + r;
+        bool on = false;
+        if (X >= 0 && X < w && Y >= 0 && Y < h) on = differs(a, b, fmt, (long)Y * w + X, limit);
+        s_m[0][e] = on ? 0xff : 0;
+        any = any || on;
     }
-    float sum = (d[1] + d[2]) + d[3];
-    mask[i] = sum >= limit ? 0xff : 0;
-}
-
-// filters.rs:360-375 (mask_prune) from the snapshot src into dst; needs w >= 3 and h >= 5
-__global__ void k_mask_prune(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int w, int h, int limit,
-                             const int* __restrict__ gate) {
-    if (gated_off(gate)) return;
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long)w * h) return;
-    int y = row_of(i, w), x = (int)(i - (long)y * w);
-    uint8_t v = src[i];
-    if (v != 0 && x >= 1 && x <= w - 2 && y >= 2 && y <= h - 3 && ring_sum(src, w, x, y - 2, y, y + 2) < limit) v = 0;
-    dst[i] = v;
-}
-
-// filters.rs:406-418 (mask_dilate_rows); needs h >= 3
-__global__ void k_mask_dilate(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int w, int h,
-                              const int* __restrict__ gate) {
-    if (gated_off(gate)) return;
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long)w * h) return;
-    int y = row_of(i, w);
-    uint8_t v = src[i];
-    if (y >= 1 && y <= h - 2 && (src[i - w] == 255 || src[i + w] == 255)) v = 255;
-    dst[i] = v;
-}
-
-// filters.rs:387-400 (mask_fill) followed by :425-496 (mask_replicate_border), for w >= 3 and
-// h >= 3: there the border copy is the fill's result at the coordinate clamped to the inner
-// rectangle 1..w-2 x 1..h-2
-__global__ void k_mask_fill_border(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int w, int h, int limit,
-                                   int value, const int* __restrict__ gate) {
-    if (gated_off(gate)) return;
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long)w * h) return;
-    int y = row_of(i, w), x = (int)(i - (long)y * w);
-    int cx = min(max(x, 1), w - 2), cy = min(max(y, 1), h - 2);
-    uint8_t v = src[(long)cy * w + cx];
-    if (v == 0 && limit < ring_sum(src, w, cx, cy - 1, cy, cy + 1)) v = (uint8_t)value;
-    dst[i] = v;
+    if (__syncthreads_or(any)) {
+        uint8_t *src = s_m[0], *dst = s_m[1];
+        // one step: at(p, x, y) the new value at the region's pixel p, image pixel (x, y), from src
+        auto step = [&](auto at) {
+            for (int e = threadIdx.x; e < WBM_W * WBM_H; e += WBM_THREADS) {
+                const int r = e / WBM_W, c = e - r * WBM_W;
+                const bool inside = c >= 2 && c < WBM_W - 2 && r >= 2 && r < WBM_H - 2;
+                dst[e] = inside ? at(e, gx + c, gy + r) : src[e];
+            }
+            __syncthreads();
+            uint8_t* t = src;
+            src = dst;
+            dst = t;
+        };
+        auto ring = [&](int p, int dy) {  // filters.rs:339-345
+            const uint8_t *m = src + p, *u = m - dy * WBM_W, *d = m + dy * WBM_W;
+            return (int)u[0] + u[-1] + u[1] + m[-1] + m[1] + d[-1] + d[0] + d[1];
+        };
+        auto prune = [&](int lim) {
+            step([&](int p, int x, int y) {
+                uint8_t v = src[p];
+                if (v != 0 && x >= 1 && x <= w - 2 && y >= 2 && y <= h - 3 && ring(p, 2) < lim) v = 0;
+                return v;
+            });
+        };
+        auto fill = [&](int lim, int value) {
+            step([&](int p, int x, int y) {
+                const int q = p + min(max(x, 1), w - 2) - x + (min(max(y, 1), h - 2) - y) * WBM_W;
+                // (a pixel outside the image, or at the region's edge, may have its inner pixel out of reach)
+                if (x < 0 || x >= w || y < 0 || y >= h || q < WBM_W + 1 || q >= WBM_W * (WBM_H - 1) - 1) return src[p];
+                uint8_t v = src[q];
+                if (v == 0 && lim < ring(q, 1)) v = (uint8_t)value;
+                return v;
+            });
+        };
+        if (h >= 5) {
+            prune(254);
+            prune(509);
+        }
+        step([&](int p, int, int y) {
+            uint8_t v = src[p];
+            if (y >= 1 && y <= h - 2 && (src[p - WBM_W] == 255 || src[p + WBM_W] == 255)) v = 255;
+            return v;
+        });
+        fill(254, 255);
+        fill(254, 255);
+        fill(254, 128);
+        fill(127, 64);
+        if (src != s_m[0]) {
+            for (int e = threadIdx.x; e < WBM_W * WBM_H; e += WBM_THREADS) s_m[0][e] = src[e];
+            __syncthreads();
+        }
+    }
+    for (int e = threadIdx.x; e < WBM_T * WBM_T; e += WBM_THREADS) {
+        const int r = e / WBM_T, c = e % WBM_T;
+        if (X0 + c < w && Y0 + r < h) mask[(long)(Y0 + r) * w + X0 + c] = s_m[0][(r + WBM_HY) * WBM_W + c + WBM_HX];
+    }
 }
 
 // filters.rs:507-520 for frames with a side below 3, by one thread: the dilate (h >= 3) and four

@@ -410,28 +410,13 @@ int sharpen_dev(tw_ctx* ctx, void* frame, const void* orig, int W, int H, int fm
         CHECK(ctx->ensure(*ws.mask[i], (size_t)n, "sharpening mask"));
     }
     uint8_t* cur = ws.mask[0]->as<uint8_t>();
-    uint8_t* nxt = ws.mask[1]->as<uint8_t>();
     float white = fmt == TW_U8 ? 255.0f : fmt == TW_U16 ? 65535.0f : 1.0f;
     float limit = 0.4f * white * 0.4f * 0.4f * 3.0f;  // filters.rs:293-295, MASK_THRESHOLD 0.4
-    LAUNCH(ctx, k_wb_diff_mask, grid1(n), TB, 0, frame, orig, fmt, n, limit, cur, gate);
-    // filters.rs:507-520: prune 254 and 509, dilate, fill 254 -> 255 twice, 254 -> 128, 127 -> 64
     if (W >= 3 && H >= 3) {
-        auto step = [&]() { std::swap(cur, nxt); };
-        if (H >= 5) {
-            LAUNCH(ctx, k_mask_prune, grid1(n), TB, 0, cur, nxt, W, H, 254, gate);
-            step();
-            LAUNCH(ctx, k_mask_prune, grid1(n), TB, 0, cur, nxt, W, H, 509, gate);
-            step();
-        }
-        LAUNCH(ctx, k_mask_dilate, grid1(n), TB, 0, cur, nxt, W, H, gate);
-        step();
-        const int fills[4][2] = {{254, 255}, {254, 255}, {254, 128}, {127, 64}};
-        for (auto& f : fills) {
-            LAUNCH(ctx, k_mask_fill_border, grid1(n), TB, 0, cur, nxt, W, H, f[0], f[1], gate);
-            step();
-        }
+        LAUNCH(ctx, k_wb_mask, tiles(W, H), WBM_THREADS, 0, frame, orig, fmt, W, H, limit, cur, gate);
     } else {
-        LAUNCH(ctx, k_mask_clean_small, 1, 1, 0, cur, nxt, W, H, gate);
+        LAUNCH(ctx, k_wb_diff_mask, grid1(n), TB, 0, frame, orig, fmt, n, limit, cur, gate);
+        LAUNCH(ctx, k_mask_clean_small, 1, 1, 0, cur, ws.mask[1]->as<uint8_t>(), W, H, gate);
     }
     // the blur (radius 3.0, filters.rs:75-93: taps 1, 1/2, 1/16, 1/512 over their sum, from powf)
     WbTaps T{};

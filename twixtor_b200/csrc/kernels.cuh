@@ -409,12 +409,9 @@ __global__ void k_wb_blur(const void* __restrict__ src, void* __restrict__ dst, 
                           bool above_first, const int* __restrict__ gate);
 __global__ void k_wb_diff_mask(const void* __restrict__ a, const void* __restrict__ b, int fmt, long n, float limit,
                                uint8_t* __restrict__ mask, const int* __restrict__ gate);
-__global__ void k_mask_prune(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int w, int h, int limit,
-                             const int* __restrict__ gate);
-__global__ void k_mask_dilate(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int w, int h,
-                              const int* __restrict__ gate);
-__global__ void k_mask_fill_border(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int w, int h, int limit,
-                                   int value, const int* __restrict__ gate);
+constexpr int WBM_THREADS = 256;
+__global__ void k_wb_mask(const void* __restrict__ a, const void* __restrict__ b, int fmt, int w, int h, float limit,
+                          uint8_t* __restrict__ mask, const int* __restrict__ gate);
 __global__ void k_mask_clean_small(uint8_t* __restrict__ m, uint8_t* __restrict__ scratch, int w, int h,
                                    const int* __restrict__ gate);
 __global__ void k_wb_finish(void* __restrict__ frame, const void* __restrict__ blurred, const uint8_t* __restrict__ mask,
