@@ -110,6 +110,33 @@ def test_solves_at_the_ends_of_their_tiles(dev, size, masks, points, above_first
     assert got.tobytes() == want.tobytes()
 
 
+@pytest.mark.parametrize("size", [(256, 32), (32, 256), (128, 64), (254, 33), (258, 32), (32, 258), (130, 64)])
+@pytest.mark.parametrize("masks", [False, True])
+@pytest.mark.parametrize("content", ["blocks", "smooth"])
+def test_solves_at_the_limits_of_the_coarse_block(dev, size, masks, content):
+    """Levels of exactly 2048 pixels and 128 a side, which one block solves, and the next larger ones, which the
+    tiled kernels take: block matching walks lines in several segments there, and walks a segment again where a
+    run reaches into it (short runs with blocks of noise, runs across segments with smooth textures)."""
+    w, h = size
+    rng = np.random.RandomState(w * 3 + h)
+    cell = 3 if content == "blocks" else 12
+    x = np.kron(rng.randint(0, 256, (h // cell + 1, w // cell + 1, 4)), np.ones((cell, cell, 1)))[:h, :w]
+    if content == "smooth":
+        for axis in (0, 1):
+            x = sum(np.roll(x, k, axis=axis) for k in range(-4, 5)) / 9.0
+    y = x.copy()
+    for i in range(0, h, 16):  # bands that move on their own
+        y[i:i + 16] = np.roll(x[i:i + 16], rng.randint(-5, 6), axis=1)
+    y[:, w // 3:w // 2] = np.roll(y[:, w // 3:w // 2], 3, axis=0)
+    x, y = (np.ascontiguousarray(np.clip(v, 0, 255)).astype(np.uint8).reshape(-1) for v in (x, y))
+    mx = my = None
+    if masks:
+        mx, my = [(rng.random_sample((h, w)) < 0.98).astype(np.float32).ravel() for _ in range(2)]
+    want, xl, yl, mxl, myl, ud, uw = O.solve_pyramids_with(x, y, w, h, 0, mx, my, None, quality=5, above_first=True)
+    got, _ = dev.solve_pyramids(tw.FlowSettings(quality=5, taps_above_first=True), w, h, xl, yl, mxl, myl, ud, uw)
+    assert got.tobytes() == want.tobytes()
+
+
 @pytest.mark.parametrize("size", [(2, 2), (2, 33), (32, 32), (33, 65), (66, 31), (129, 97)])
 @pytest.mark.parametrize("fmt", [0, 1, 2, "flow"])
 @pytest.mark.parametrize("above_first", [False, True])

@@ -234,18 +234,20 @@ __device__ __forceinline__ void sweep(const Coarse& C, bool reverse, float z) {
                 const int e = elem(line, min(max(q + gl, 1), len - 2));
                 // an accepted position whose vector was this one already: the rest stands
                 const unsigned met = group_ballot(live && gl < n && same_bits(C.fn[e], cur));
+                // the refusing position keeps its own vector; if it did before, the rest stands. Only the lane that
+                // stores it reads it (a ballot orders no memory accesses: another lane could read what was stored).
+                const int r = elem(line, min(max(q + n, 1), len - 2));
+                const bool changes = group_ballot(gl == 0 && live && refused && !met && !same_bits(C.fn[r], f[r])) != 0;
                 if (live) {
                     if (gl < (met ? __ffs(met) - 1 : n)) C.fn[e] = cur;
                     if (met) {
                         carry = false;
                     } else {
                         q += n;
-                        if (refused) {  // the position keeps its own vector; if it did before, the rest stands
-                            const int r = elem(line, q);
-                            const float2 own = f[r];
-                            carry = !same_bits(C.fn[r], own);
-                            if (carry && gl == 0) C.fn[r] = own;
-                            cur = own;
+                        if (refused) {
+                            cur = f[r];
+                            if (changes && gl == 0) C.fn[r] = cur;
+                            carry = changes;
                             q++;
                         }
                         if (q >= end) carry = false;
