@@ -228,6 +228,31 @@ def test_adjoint_at_the_ends_of_its_columns(dev, w, h, fw, fh, smooth):
             assert np.linalg.norm(got.reshape(-1) - np.asarray(ref).reshape(-1)) <= 1e-3 * max(np.linalg.norm(ref), 1e-6)
 
 
+@pytest.mark.parametrize("value", [0x7f800000, 0xff800000, 0x7fc00000, 0x7fc00001], ids=hex)
+@pytest.mark.parametrize("push", [(500.0, 0.25), (0.25, -500.0), (-500.0, 500.0)])
+@pytest.mark.parametrize("where", ["gradient", "frame"])
+def test_adjoint_of_clamped_positions_with_values_that_are_not_finite(dev, value, push, where):
+    """An axis on which every position is clamped has no gradient: exactly 0, also where the output's gradient or
+    the frames hold infinities and NaNs (of any payload); the other axis has NaNs then."""
+    import torch
+
+    from twixtor_b200 import adjoint
+    w, h, fw, fh = 40, 37, 20, 19
+    rng = np.random.RandomState(4)
+    a, b, g = (rng.rand(1, h, w, 4).astype(np.float32) for _ in range(3))
+    for x in (g,) if where == "gradient" else (a, b):
+        x.reshape(-1).view(np.uint32)[rng.randint(0, x.size, x.size // 4)] = value
+    fab, fba = (np.tile(np.array(push, np.float32), (1, fh, fw, 1)) for _ in range(2))
+    xs = [torch.from_numpy(x).cuda().requires_grad_(True) for x in (a, b, fab, fba)]
+    adjoint.warp_blend(*xs, 0.35, dev).backward(torch.from_numpy(g).cuda())
+    for f in xs[2:]:
+        for axis in range(2):
+            if abs(push[axis]) > 1.0:
+                assert (f.grad[..., axis] == 0.0).all()
+            else:
+                assert torch.isnan(f.grad[..., axis]).any()
+
+
 @pytest.mark.parametrize("size", [(3, 3), (3, 40), (33, 4), (5, 5), (32, 32), (33, 33), (65, 34), (97, 66)])
 @pytest.mark.parametrize("fmt", [0, 2])
 @pytest.mark.parametrize("density", [0.02, 0.3, 0.7])

@@ -59,13 +59,18 @@ struct FlowCell {
     float fx, fy;
 };
 
-// One side: the sample of S at p + F(p r) (s / r), sx, sy = s / r, and its derivatives along x and y (zero
-// along an axis on which the position was clamped)
+// One side: the sample of S at p + F(p r) (s / r), sx, sy = s / r, and its derivatives along x and y. Along an axis
+// on which the position was clamped there is none: the derivative's first channel holds CLAMPED then, a NaN that no
+// operation gives (their NaNs are 0x7fffffff, whatever payload came in).
 struct Side {
     int ix, iy;      // top left corner
     float fx, fy;    // fractions
     Px val, dx, dy;
 };
+constexpr int CLAMPED = 0x7fc00001;
+__device__ __forceinline__ float along(Px g, Px d, float s) {
+    return __float_as_int(d.a.x) == CLAMPED ? 0.0f : dot4(g, d) * s;
+}
 
 __device__ __forceinline__ Side side_at(const float* S, const float* F, const AdjParams& P, const FlowCell& q, int x, int y,
                                         float sx, float sy) {
@@ -86,9 +91,10 @@ __device__ __forceinline__ Side side_at(const float* S, const float* F, const Ad
     const Px c00 = ld4(S, i00), c10 = ld4(S, i00 + 1), c01 = ld4(S, i01), c11 = ld4(S, i01 + 1);
     const Px d0 = sub4(c10, c00), d1 = sub4(c11, c01), e0 = sub4(c01, c00), e1 = sub4(c11, c10);
     d.val = mix4(step4(c00, d0, d.fx, P.z), step4(c01, d1, d.fx, P.z), d.fy, P.z);
-    const Px zero = {both(0.0f), both(0.0f)};
-    d.dx = cx ? zero : fused4(d0, sub4(d1, d0), d.fy);
-    d.dy = cy ? zero : fused4(e0, sub4(e1, e0), d.fx);
+    d.dx = fused4(d0, sub4(d1, d0), d.fy);
+    d.dy = fused4(e0, sub4(e1, e0), d.fx);
+    if (cx) d.dx.a.x = __int_as_float(CLAMPED);
+    if (cy) d.dy.a.x = __int_as_float(CLAMPED);
     return d;
 }
 
@@ -170,7 +176,8 @@ __device__ __forceinline__ void next_texels(FlowSums& s, int from, int to, const
 
 __device__ __forceinline__ void sum_texels(FlowSums& s, const Side& d, Px g, const FlowCell& q, float sx, float sy, bool live) {
     if (!live) return;
-    const float2 v = make_float2(dot4(g, d.dx) * sx, dot4(g, d.dy) * sy);
+    // (0 along a clamped axis whatever g is: an infinity times a derivative of 0 would be a NaN)
+    const float2 v = make_float2(along(g, d.dx, sx), along(g, d.dy, sy));
     s.up = __ffma2_rn(v, both(1.0f - q.fy), s.up);
     s.low = __ffma2_rn(v, both(q.fy), s.low);
 }
@@ -181,8 +188,9 @@ __device__ __forceinline__ void sum_texels(FlowSums& s, const Side& d, Px g, con
 // warps.
 //
 // Bound by the gathers' latency at 16 warps an SM (128 registers; 20 warps with 96 spill: 721 us, and 4 rows a
-// thread, more corners left over, 774). 16 x 1280 x 720 with the L1 loss: 568 us; floats added to tiles of
-// the gradients in shared memory, a loop of compare and swap each and 40 a pixel, took 1.40 ms.
+// thread, more corners left over, 774). 16 x 1280 x 720 with the L1 loss: 574 us (612 with the clamped axes in
+// flags of their own); floats added to tiles of the gradients in shared memory, a loop of compare and swap each
+// and 40 a pixel, took 1.40 ms.
 __global__ void __launch_bounds__(ADJ_THREADS, 4) k_warp_blend_adjoint(const __grid_constant__ AdjParams P) {
     constexpr unsigned FULL = 0xffffffffu;
     const int b = blockIdx.z, lane = threadIdx.x & 31;
