@@ -20,6 +20,7 @@
 // single precision steps with its NaN handling: the x86 results (NaN operands propagated quieted,
 // the default NaN for invalid operations) where the reference runs plain arithmetic, the NaN rule
 // (nanrule.rs) where it switches to the rule.
+#include "forward_grid.h"
 #include "kernels.cuh"
 #include "twlog.h"
 #include "warp.cuh"
@@ -495,7 +496,7 @@ __device__ __forceinline__ void triangle(const Vt* t, int w1, int h1, Ar aa, Ar 
 // ends and how many rows it has gone, so that its payload can be formed where a span has pixels.
 struct Corner {
     float x, y;
-    int at;  // the vertex's pixel
+    int at;  // the vertex's pixel, from the first one of its cell on
 };
 struct ScanEdge {
     float ay, by, x, dx, t, inv;
@@ -613,28 +614,24 @@ __device__ __forceinline__ void scan_triangle(const Corner* t, Corner* vs, int w
     }
 }
 
-// The vertices of triangle t of the grid, T1 = (v[r][c], v[r][c+1], v[r+1][c]) and T2 = (v[r+1][c+1], v[r][c+1],
-// v[r+1][c]) of every cell; false past the last one
-__device__ __forceinline__ bool grid_triangle(const FwRaster& R, long t, Corner* v) {
-    const int cw = R.w - 1;
-    if (t >= 2l * cw * (R.h - 1)) return false;
-    const long cell = t >> 1;
-    const int r = row_of(cell, cw), c = (int)(cell - (long)r * cw);
-    const int i = r * R.w + c;  // (the hits of an image, and so its pixels, are below 2^31)
-    v[0].at = (t & 1) == 0 ? i : i + R.w + 1;
-    v[1].at = i + 1;
-    v[2].at = i + R.w;
+// The vertices of triangle t of the grid and the pixel of its cell's first one; false past the last triangle
+__device__ __forceinline__ bool grid_triangle(const FwRaster& R, long t, Corner* v, long& first) {
+    GridTriangle g;
+    if (!grid_triangle_at(t, R.w, R.h, g)) return false;
+    first = g.first;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        v[k].x = R.vx[v[k].at];
-        v[k].y = R.vy[v[k].at];
+        v[k].at = g.at[k];
+        v[k].x = R.vx[first + g.at[k]];
+        v[k].y = R.vy[first + g.at[k]];
     }
     return true;
 }
 
 __global__ void __launch_bounds__(128) k_fw_count(const __grid_constant__ FwRaster R) {
     Corner v[3], vs[3];
-    if (!grid_triangle(R, (long)blockIdx.x * blockDim.x + threadIdx.x, v)) return;
+    long first;
+    if (!grid_triangle(R, (long)blockIdx.x * blockDim.x + threadIdx.x, v, first)) return;
     const int w1 = R.w - 1, h1 = R.h - 1;
     auto hit = [&](int x, int y) { atomicAdd(&R.cnt[(long)y * R.w + x], 1u); };
     scan_triangle(
@@ -683,27 +680,27 @@ struct EmitSink {
 
 // The payload of the vertex at pixel i: the texture coordinates and the mip level, or the colours
 template <typename P, bool TEXTURED>
-__device__ __forceinline__ void vertex_payload(const FwRaster& R, int i, float p[4]) {
+__device__ __forceinline__ void vertex_payload(const FwRaster& R, long i, float p[4]) {
     if (TEXTURED) {
-        const int r = row_of(i, R.w), c = i - r * R.w;
+        const int r = row_of(i, R.w), c = (int)(i - (long)r * R.w);
         p[0] = (float)c / (float)(R.w - 1);
         p[1] = (float)r / (float)(R.h - 1);
         p[2] = R.vd ? R.vd[i] : 0.0f;
         p[3] = 0.0f;
     } else {
-        px_floats<P>((const P*)R.levels.p[0] + (long)i * 4, p);
+        px_floats<P>((const P*)R.levels.p[0] + i * 4, p);
     }
 }
 
 // A triangle in the reference's arithmetic of NaNs, out of the main path
 template <typename P, bool TEXTURED>
-__device__ __noinline__ void emit_general(const FwRaster& R, uint32_t t, const Corner* c) {
+__device__ __noinline__ void emit_general(const FwRaster& R, uint32_t t, const Corner* c, long first) {
     Vt v[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         v[k].x = c[k].x;
         v[k].y = c[k].y;
-        vertex_payload<P, TEXTURED>(R, c[k].at, v[k].p);
+        vertex_payload<P, TEXTURED>(R, first + c[k].at, v[k].p);
     }
     // raster.rs:158-166: the rule when a payload of the triangle is NaN (per scan: the Gouraud
     // variant's two scans, colours 0..2 and colour 3, choose on their own)
@@ -726,7 +723,8 @@ template <typename P, bool TEXTURED>
 __device__ __forceinline__ void emit_triangle(const FwRaster& R) {
     const long tri = (long)blockIdx.x * blockDim.x + threadIdx.x;
     Corner v[3], vs[3];
-    if (!grid_triangle(R, tri, v)) return;
+    long first;
+    if (!grid_triangle(R, tri, v, first)) return;
     const float z = R.levels.z;
     const float2 zz = make_float2(z, z);
     bool plain = true;
@@ -734,16 +732,16 @@ __device__ __forceinline__ void emit_triangle(const FwRaster& R) {
     for (int k = 0; k < 3; k++) {
         const float dy = fabsf(v[k].y - v[(k + 1) % 3].y);
         plain = plain && fabsf(v[k].x) < 1e6f && fabsf(v[k].y) < 1e6f && (dy == 0.0f || dy > 1e-6f);
-        if (TEXTURED) plain = plain && (!R.vd || fabsf(R.vd[v[k].at]) < 1e6f);
+        if (TEXTURED) plain = plain && (!R.vd || fabsf(R.vd[first + v[k].at]) < 1e6f);
         if (!TEXTURED && sizeof(P) == 4) {
             float p[4];
-            vertex_payload<P, TEXTURED>(R, v[k].at, p);
+            vertex_payload<P, TEXTURED>(R, first + v[k].at, p);
             plain = plain && fabsf(p[0]) < 1e6f && fabsf(p[1]) < 1e6f && fabsf(p[2]) < 1e6f && fabsf(p[3]) < 1e6f;
         }
     }
     if (!plain) {
         const Corner general[3] = {v[0], v[1], v[2]};  // (a copy: the corners stay in registers)
-        emit_general<P, TEXTURED>(R, (uint32_t)tri, general);
+        emit_general<P, TEXTURED>(R, (uint32_t)tri, general, first);
         return;
     }
     const int w1 = R.w - 1, h1 = R.h - 1;
@@ -751,7 +749,7 @@ __device__ __forceinline__ void emit_triangle(const FwRaster& R) {
     auto mul = [&](float2 a, float k) { return __ffma2_rn(a, make_float2(k, k), zz); };
     auto vertex = [&](int k, float2* p) {
         float f[4];
-        vertex_payload<P, TEXTURED>(R, k == 0 ? vs[0].at : k == 1 ? vs[1].at : vs[2].at, f);
+        vertex_payload<P, TEXTURED>(R, first + (k == 0 ? vs[0].at : k == 1 ? vs[1].at : vs[2].at), f);
         p[0] = make_float2(f[0], f[1]);
         p[1] = make_float2(f[2], f[3]);
     };
