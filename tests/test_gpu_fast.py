@@ -97,3 +97,16 @@ def test_fast_mode_clip_through_the_lanes(dev):
     p = _psnr(fast, strict)
     print(f"fast clip against strict clip: {p:.1f} dB")
     assert p > FAST_MIN_PSNR_DB
+
+
+@pytest.mark.parametrize("w,h", [(4707, 16), (4595, 16), (4499, 16), (4179, 16), (8611, 64), (8613, 64), (7811, 64), (8227, 64),
+                                 (9091, 64), (10819, 64)])
+def test_every_pixel_of_a_pyramid_is_written(dev, w, h):
+    """Widths at which an output of the next level starts within two roundings of a tile's end (the tile's end over
+    the step is its number and 0.5 to 1.5 units in the last place), so that an approximate quotient could leave
+    it to no tile: the pyramid of a black image after one of noise, in the same scratch, is zero everywhere."""
+    s = tw.FlowSettings(quality=5 if w <= 6000 else 4, fast_mode=True)
+    noise = np.random.RandomState(w).randint(0, 256, w * h * 4).astype(np.uint8)
+    dev.build_pyramid(noise, w, h, 0, s)
+    for level in dev.build_pyramid(np.zeros(w * h * 4, np.uint8), w, h, 0, s):
+        assert not np.any(level)

@@ -90,9 +90,10 @@ __device__ __forceinline__ void pyramid_step(const PyramidStep& P, float* sm, in
     // the outputs xa .. (nx of them), ya .. (ny) whose first tap can lie in the tile: its ends over the step
     int xa = 0, nx = 0, ya = 0, ny = 0;
     if (P.dst) {
+        // (rounded correctly in the fast mode too: a quotient below an output's number would leave it to no tile)
         auto range = [](int at, int len, float step, int n, int& lo, int& count) {
-            lo = (int)((float)at / step);
-            count = min((at + T < len - 1 ? min((int)((float)(at + T) / step), n - 1) : n - 1) - lo + 1, G::CELLS);
+            lo = (int)__fdiv_rn((float)at, step);
+            count = min((at + T < len - 1 ? min((int)__fdiv_rn((float)(at + T), step), n - 1) : n - 1) - lo + 1, G::CELLS);
         };
         range(X0, w, P.sx, P.dw, xa, nx);
         range(Y0, h, P.sy, P.dh, ya, ny);
