@@ -70,6 +70,14 @@ def _objects_stale(src, obj):
     return os.path.getmtime(src) > t or any(os.path.getmtime(h) > t for h in heads)
 
 
+def fast_flags(flags):
+    """The fast mode's build of the solver's translation units: FMA contraction, approximate division
+    and square root, denormals flushed; its kernels in namespace tw::fast (TW_FAST_VARIANT)."""
+    swap = {"-fmad=false": "-fmad=true", "-prec-div=true": "-prec-div=false", "-prec-sqrt=true": "-prec-sqrt=false",
+            "-ftz=false": "-ftz=true"}
+    return [swap.get(f, f) for f in flags] + ["-DTW_FAST_VARIANT"]
+
+
 def build(force=False, verbose=False):
     """Compiles every translation unit to an object in _build/ (in parallel), then links the library."""
     if not force and not stale():
@@ -79,18 +87,13 @@ def build(force=False, verbose=False):
     env = dict(os.environ)
     env.pop("CXX", None)  # host compiler: the system g++ (ccbin default)
     compile_flags = [f for f in FLAGS if f not in ("-shared", "-cudart", "shared")]
-    # the fast mode's build of the solver's translation units: FMA contraction, approximate division
-    # and square root, denormals flushed; its kernels in namespace tw::fast (TW_FAST_VARIANT)
-    fast_flags = [{"-fmad=false": "-fmad=true", "-prec-div=true": "-prec-div=false",
-                   "-prec-sqrt=true": "-prec-sqrt=false", "-ftz=false": "-ftz=true"}.get(f, f)
-                  for f in compile_flags] + ["-DTW_FAST_VARIANT"]
 
     def compile_one(unit):
         name, fast = unit
         src = os.path.join(CSRC, name)
         obj = os.path.join(BUILD, name[:-3] + ("_fast.o" if fast else ".o"))
         if force or _objects_stale(src, obj):
-            cmd = [NVCC] + (fast_flags if fast else compile_flags) + ["-c", "-o", obj, src]
+            cmd = [NVCC] + (fast_flags(compile_flags) if fast else compile_flags) + ["-c", "-o", obj, src]
             if verbose:
                 print(" ".join(cmd))
             r = subprocess.run(cmd, env=env, cwd=CSRC, capture_output=True, text=True)

@@ -335,10 +335,10 @@ __device__ __forceinline__ void bm_cell(float t, float top, int last, bool& ok, 
     f = c - (float)i;
 }
 
-// The level block matching reads, along one line: B row major (element (x, y) at [y * w + x]), or with COLS
-// its transpose ([x * h + y]), so that a line's patches are contiguous.
 // The costs (flow.rs:474-523) of two vectors at one position as the two lanes of packed arithmetic: lane .x
-// and lane .y their cells' first elements (at0, at1) and fractions; p: the 3 x 3 patch of A there, row by row.
+// and lane .y their cells' first elements (at0, at1) and fractions; p: the 3 x 3 patch of A there, row by row. B is
+// row major (element (x, y) at [y * w + x]), or with COLS the transpose ([x * h + y]), so that the patches along a
+// line are contiguous.
 // The products carry negated weights, so that their sum adds to the patch value; the squares are the same
 // bits. z: -0.0 (see the packed pairs above).
 template <bool COLS, bool LDG = true>
@@ -378,7 +378,8 @@ __device__ __forceinline__ float2 bm_cost2(const float* __restrict__ B, int pitc
     return s;
 }
 
-// The cost of one vector there.
+// The cost of one vector there, the same bits as a lane of bm_cost2 (in the fast mode too, where the compiler would
+// contract the plain sums its own way: a run's test compares the one with the other).
 template <bool COLS, bool LDG = true>
 __device__ __forceinline__ float bm_cost1(const float* __restrict__ B, int pitch, const float p[9], float fx, float fy, int at) {
     float T[4][4];
@@ -386,6 +387,20 @@ __device__ __forceinline__ float bm_cost1(const float* __restrict__ B, int pitch
     for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) T[COLS ? j : i][COLS ? i : j] = plane_load<LDG>(B + at + i * pitch + j);
+#ifdef TW_FAST_VARIANT
+    const float w11 = __fmul_rn(fy, fx), n10 = __fsub_rn(w11, fx), n01 = __fsub_rn(w11, fy);
+    const float n00 = __fsub_rn(__fadd_rn(__fsub_rn(fx, 1.0f), fy), w11);
+    float s = -0.0f;
+#pragma unroll
+    for (int b = 0; b < 3; b++)
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const float d = __fmaf_rn(-w11, T[b + 1][a + 1], __fmaf_rn(n01, T[b + 1][a], __fmaf_rn(n10, T[b][a + 1],
+                            __fmaf_rn(n00, T[b][a], p[b * 3 + a]))));
+            s = __fmaf_rn(d, d, s);
+        }
+    return s;
+#else
     const float w11 = fy * fx, w10 = fx - w11, w01 = fy - w11, w00 = ((1.0f - fx) - fy) + w11;
     float sq[9];
 #pragma unroll
@@ -400,6 +415,7 @@ __device__ __forceinline__ float bm_cost1(const float* __restrict__ B, int pitch
 #pragma unroll
     for (int k = 2; k < 8; k++) s = s + sq[k];
     return sq[8] + s;
+#endif
 }
 
 // sample.rs:31-41 for a coordinate known to lie in [0, len - 1] (or a NaN): the conversion needs no range
