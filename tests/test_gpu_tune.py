@@ -95,3 +95,39 @@ def test_tuning_entries_are_checked(dev):
     for bad in [(-1, 256, 256, 256), (3, 256, 256, 256), (0, 1024, 256, 256), (0, 100, 256, 256), (0, 256, 2048, 256)]:
         with pytest.raises(tw.BadParam):
             dev.tuning_set(64, 48, *bad)
+
+
+@pytest.mark.parametrize("tile", ["16x16", "32x64", "32x32", "64x32", "64x64"])
+@pytest.mark.parametrize("threads", [256, 512])
+@pytest.mark.parametrize("size", [(15, 17), (31, 63), (32, 64), (33, 65), (161, 131)])
+@pytest.mark.parametrize("points", [None, (-1.0, -1.0)])
+@pytest.mark.parametrize("above_first", [False, True])
+def test_every_shape_of_a_table_at_the_ends_of_its_tiles(dev, tmp_path, tile, threads, size, points, above_first):
+    """Levels a pixel smaller and larger than one or several tiles with each shape a saved table can hold (the
+    defaults choose 32 x 64 only for levels of more than 148 tiles of 32 x 32). The points put vectors of
+    exactly -1.0, the sentinel of the border rule, near the corners."""
+    w, h = size
+    rng = np.random.RandomState(w * 3 + h)
+    x = np.kron(rng.randint(0, 256, ((h + 2) // 3, (w + 2) // 3, 4)), np.ones((3, 3, 1)))[:h, :w].astype(np.uint8)
+    y = np.roll(x, 1, axis=1)
+    y[:, 0] = rng.randint(0, 256, (h, 4))
+    x, y = np.ascontiguousarray(x).reshape(-1), np.ascontiguousarray(y).reshape(-1)
+    pairs = None
+    if points:
+        at = np.array([[1.0, 1.0], [w - 1.0, 1.0], [1.0, h - 1.0], [w / 2, h / 2]], np.float32)
+        pairs = np.concatenate([at, at + np.float32(points)], 1).astype(np.float32)
+    want, xl, yl, _, _, ud, uw = O.solve_pyramids_with(x, y, w, h, 0, None, None, pairs, quality=5, above_first=above_first)
+    s = tw.FlowSettings(quality=5, taps_above_first=above_first)
+    levels = tw.flow_geometry(s, w, h)[2]
+    path = tmp_path / "tune.json"
+    try:
+        for lw, lh in levels:
+            dev.tuning_set(lw, lh, 0, threads, 256, 256)
+        path.write_text(dev.tuning_table().replace('"32x32"', f'"{tile}"'))
+        dev.tuning_clear()
+        assert dev.autotune(s, w, h, path=str(path)) == 0
+        assert [v["iter_tile"] for v in json.loads(dev.tuning_table())["levels"].values()] == [tile] * len(levels)
+        got, _ = dev.solve_pyramids(s, w, h, xl, yl, None, None, ud, uw)
+    finally:
+        dev.tuning_clear()
+    assert got.tobytes() == want.tobytes()
