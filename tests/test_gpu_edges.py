@@ -276,3 +276,19 @@ def test_sharpening_mask_at_the_ends_of_its_tiles(dev, size, fmt, density):
     cs = tw.EngineSettings(taps_above_first=True)
     got = dev.compose_vectors(cs, sel, a, b, w, h, fmt, flows[0], flows[1], (w, h))
     assert same(got, O.compose_vectors3(a, b, w, h, fmt, flows[0], flows[1], w, h, sel, cs))
+
+
+def test_algorithmic_bytes_of_a_level(dev):
+    """The bytes a level's kernels cannot do without, as the profiler counts them (what the layout adds, such as the
+    determinant beside the tensor, is not among them): per pixel 44 for the level's start, 36 for an iteration, 60
+    where it makes the next one's B, and 32 for the B after the finest level's block matching."""
+    w, h = 33, 65  # one level above the coarse ones, in 16 x 16 tiles
+    rng = np.random.RandomState(1)
+    x, y = (rng.randint(0, 256, w * h * 4).astype(np.uint8) for _ in range(2))
+    s = tw.FlowSettings(quality=5)
+    for kernel, launches, per_pixel in [("k_level_init_16x16", 1, 44), ("k_level_iter_16x16", 3, 60 + 36 + 36),
+                                        ("k_calc_b_pitched", 1, 32)]:
+        dev.profile_begin(kernel)
+        dev.solve(x, y, w, h, 0, s)
+        _, n, b = dev.profile_end()
+        assert (n, b) == (launches, per_pixel * w * h)

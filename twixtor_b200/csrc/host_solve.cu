@@ -115,10 +115,10 @@ void conv_planes(tw_ctx* ctx, float* const* planes, int c, int w, int h, const T
 }
 
 // One solver iteration (k_level_iter_*) with the tile shape and block size of the level's choice.
-// Algorithmic bytes per pixel: B (8), the tensor (16) and the flow (8) read, the flow (8) written;
-// with b_out also I1 (4), the I0 gather (4) and the gradient (8) read and B (8) written.
+// Algorithmic bytes per pixel: B (8), the tensor (12; the determinant beside it is the layout's) and the flow (8)
+// read, the flow (8) written; with b_out also I1 (4), the I0 gather (4) and the gradient (8) read and B (8) written.
 void level_iter(tw_ctx* ctx, LevelTune ic, const LevelIterArgs& P, bool fast) {
-    const double b = (P.b_out ? 64.0 : 40.0) * P.w * P.h;
+    const double b = (P.b_out ? 60.0 : 36.0) * P.w * P.h;
     const size_t smem = level_iter_smem(ic.iter_tile);
     auto grid = [&](int tx, int ty) { return dim3((unsigned)((P.w + tx - 1) / tx), (unsigned)((P.h + ty - 1) / ty)); };
     switch (ic.iter_tile) {
@@ -495,13 +495,13 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
         I.start = start;
         I.af = af;
         I.g7 = ctx->g7;
-        // the image read, the gradient and the tensor written (28); the flow and the I0 gather read, B
+        // the image read, the gradient and the tensor written (24); the flow and the I0 gather read, B
         // written (20)
         if (tiles_of(w, h, 16, 16) <= 148)
-            LAUNCHV(ctx, fast, 48.0 * px, k_level_init_16x16, dim3((w + 15) / 16, (h + 15) / 16), 512,
+            LAUNCHV(ctx, fast, 44.0 * px, k_level_init_16x16, dim3((w + 15) / 16, (h + 15) / 16), 512,
                     level_init_smem(LEVEL_TILE_16x16), I);
         else
-            LAUNCHV(ctx, fast, 48.0 * px, k_level_init_32x32, tiles(w, h), tiles_of(w, h, 32, 32) <= 148 ? 512 : 256,
+            LAUNCHV(ctx, fast, 44.0 * px, k_level_init_32x32, tiles(w, h), tiles_of(w, h, 32, 32) <= 148 ? 512 : 256,
                     level_init_smem(LEVEL_TILE_32x32), I);
         LevelIterArgs P;
         std::memset(&P, 0, sizeof P);
@@ -533,7 +533,7 @@ int solve_pyramids_dev(tw_ctx* ctx, const float* x, const float* y, const float*
             if (it == 1 && l == 0) {
                 if (!s.skip_refine) block_match(ctx, A, B, AT, BT, f, ft, w, h, fast, nullptr);
                 user();
-                LAUNCHV(ctx, fast, 40.0 * px, k_calc_b_pitched, grid2(w, h), TB, 0, A, B, grad, f, w, h, mask_y, bb[0], P.bp);
+                LAUNCHV(ctx, fast, 32.0 * px, k_calc_b_pitched, grid2(w, h), TB, 0, A, B, grad, f, w, h, mask_y, bb[0], P.bp);
             }
         }
         if (match_last) block_match(ctx, A, B, AT, BT, f, ft, w, h, fast, udu ? nullptr : any + l);
