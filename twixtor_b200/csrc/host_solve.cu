@@ -146,9 +146,6 @@ LevelTune level_tune(tw_ctx* ctx, int w, int h) {
     return it != ctx->tune_table.end() ? it->second : default_tune(w, h);
 }
 
-// Threads per CTA of the tiled pyramid kernels: a level of few tiles is latency bound
-// (every CTA walks its stages one after the other), so its CTAs get more threads and each thread
-// fewer elements per stage; a level with tiles enough to fill the GPU keeps 256.
 // ---- a step of a pyramid: the blur5 of src (or of the luma of luma_src), its band and transposed band, and the
 // next size's plane, each where asked for. Tiles of 32 x 32, or of 16 x 16 while the larger ones would not fill
 // the chip's 148 SMs (a 240 x 135 level: see pyramid_step's figures).

@@ -5,8 +5,9 @@
 // real-time render thread where a driver allocation can stall or is forbidden. They can still pass
 // their own device buffers for the inputs and the output. This entry point runs the four block
 // matching sweeps (flow.rs:551-622) on such buffers without allocating anything: its only scratch
-// (a copy of the field, the transposes of the two images and of the field for the column sweeps) lives in the file-scope device array below, which every GPU that loads the
-// library holds until the process exits.
+// (a copy of the field, the transposes of the two images and of the field for the column sweeps)
+// lives in the file-scope device array below, which every GPU that loads the library holds until the
+// process exits.
 #include <cuda_runtime.h>
 
 #include "../../include/twixtor_b200.h"

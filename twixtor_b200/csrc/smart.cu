@@ -223,9 +223,7 @@ __global__ void k_cov_holes(const uint8_t* __restrict__ c1, const uint8_t* __res
     if (__syncthreads_or(hole) && threadIdx.x == 0) atomicOr(any_hole, 1);
 }
 
-// ---- the hole fill on plane stacks (holefill.rs) ------------------------------------------------------
-
-// ---- the fill's levels in tiles ----------------------------------------------------------------------
+// ---- the hole fill (holefill.rs): its levels in tiles ---------------------------------------------------
 
 // One element of a pass along a line held in shared memory: element t (global index in [0, len)) of
 // the line at line[(t - origin) * stride]; the interior chain or the 1 channel border rule (conv.rs:101-137,
@@ -597,7 +595,8 @@ __device__ __forceinline__ void fill_push_image(FillShared<6>& S, const FillPush
 // One level down (holefill.rs:352-404): the values over their weights, the coarser solution where there is no
 // weight, and the Gaussian of it; a pair of channels (blockIdx.z). At level 0 (an image) the holes take it and
 // the other pixels stay as they are, but for a NaN that the rule's division by 1 quiets; a tile without a
-// hole has nothing to do. No tile reads what another writes: a hole's own sample is not looked at.
+// hole has nothing to do. A tile's halo may read a sample while its own tile quiets it: the NaN that was there
+// and the quieted one give the same bits after the division by 1; a hole's own sample is not looked at.
 //
 // Bound by issue. The launches of a 1080p level 0 (combine, blur, combine, store) took 10 + 48 + 10 + 15 us.
 __global__ void __launch_bounds__(FILL_THREADS) k_fill_push(const __grid_constant__ FillPush P) {

@@ -310,9 +310,8 @@ __device__ __forceinline__ void bm_push(int* q, int* n, bool want, int val) {
 // q (q = i forward, q = len-1-i reverse) both are the same forward recurrence
 // v'[q] = accept(q, v'[q-1]) ? v'[q-1] : v[q], so every v'[q] is the vector of its run's start, and
 // a run started at j ends at end[j], the first position past j that refuses v[j]. The sweep:
-//   1. c0[i], the cost of the current vector (the reverse sweep recomputes it only where the forward
-//      sweep replaced the vector, those positions listed by the forward sweep), and the test of
-//      v[q-1] at every q: end[q-1] = q where it refuses, the others queued;
+//   1. c0[i], the cost of the current vector, and the test of v[q-1], evaluated as a pair at every q:
+//      end[q-1] = q where it refuses, the others queued;
 //   2. the queued candidates extended one position per stage (BM_STAGES stages, the survivors
 //      compacted after each), then the rest by groups of BM_GROUP lanes testing as many positions at once;
 //   3. the chain of run starts 0, end[0], end[end[0]], ... in 32-position chunks, one warp per
